@@ -66,6 +66,12 @@ def _signatures(lib):
         "mllm_linear_stream_f32_tall_rows": [c_int, c_int],
         "mllm_linear_stream_f32_kernel_of": [c_int, c_int, c_int],
         "mllm_linear_stream_f32_bind_error": [c_void_p],
+        "mllm_linear_split_f32": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int,
+                                  c_void_p],
+        "mllm_linear_split_f32_qkv": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_void_p,
+                                      c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
+        "mllm_linear_split_f32_bind_error": [c_void_p],
+        "mllm_linear_split_f32_error": [c_void_p],
         "mllm_linear_stream_f32_error": [c_void_p],
         "mllm_linear_tcgen05": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int,
                                 c_int, c_void_p],
@@ -213,14 +219,14 @@ def _bind_error_word(lib) -> None:
         return
     word = torch.zeros(1, dtype=torch.int32).pin_memory()
     for name in ("mllm_tcgen05_bind_error", "mllm_attention_tcgen05_bind_error", "mllm_attention_decode_bind_error",
-                 "mllm_linear_stream_f32_bind_error"):
+                 "mllm_linear_stream_f32_bind_error", "mllm_linear_split_f32_bind_error"):
         if getattr(lib, name)(word.data_ptr()) != 0:
             raise KernelError(lib.mllm_last_error().decode(errors="replace"))
     _error_word = word
 
 
 _WHO = {1: "the tcgen05 product", 2: "the tcgen05 attention", 3: "the decode attention",
-        4: "the float32 weight-streaming product"}
+        4: "the float32 weight-streaming product", 5: "the float32 product of many rows"}
 
 
 def raise_if_kernel_gave_up() -> None:
@@ -319,6 +325,11 @@ def check_device_errors() -> None:
         raise KernelError(lib.mllm_last_error().decode(errors="replace"))
     if code.value:
         raise KernelError("the float32 weight-streaming product gave up waiting for its weights")
+    if lib.mllm_linear_split_f32_error(ctypes.byref(code)) != 0:
+        raise KernelError(lib.mllm_last_error().decode(errors="replace"))
+    if code.value:
+        raise KernelError(f"the float32 product of many rows gave up waiting: code {code.value} "
+                          "(1, 5 the cutting warps, 2-3 the MMA issuer, 4 the epilogue, 6 the TMA producer)")
 
 
 _stream_handle = None     # set by stream_scope(); None: ask torch on every call
@@ -650,6 +661,16 @@ def _norm_ok_f32(n: NormedInput) -> bool:
             and n.beta.data_ptr() % 16 == 0)
 
 
+def _split_f32_ok(x, weight, M, K) -> bool:
+    """Float32 products of more rows than the weight-streaming kernel takes go to the tensor cores in exact pieces
+    (csrc/linear_split_f32.cu) wherever rows can be read 16 bytes at a time: at 2,048 rows GPT-2 small's four products
+    take 24 / 42 / 58 / 73 us instead of 84 / 187 / 275 / 251 us on CUDA cores, at 77 rows 17 / 17 / 17 / 53 instead of
+    52 / 52 / 52 / 189 us.  The CUDA-core kernel is left with unaligned operands and with K under 128, where a chain of
+    so few additions is as close to float64 as the pieces are (from 128 on it is further off: 1.5 to 7 times)."""
+    return (x.dtype == torch.float32 and weight.dtype == torch.float32 and M > SMALL_M_F32 and K % 4 == 0 and K >= 128
+            and _rows("x", x) % 4 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
+
+
 def _linear_stream_f32(x, weight, bias, out, act, accumulate, norm: Optional[NormedInput], kv) -> None:
     """The float32 weight-streaming product, with the norm fused on its input and/or the cache write on its output."""
     M = norm.shape[0] if norm is not None else x.shape[0]
@@ -731,6 +752,16 @@ def linear_qkv_cache(x, weight, bias, q_out, k_pages, v_pages, slot_mapping, ws)
               bias.data_ptr() if bias is not None else None, q_out.data_ptr(), _rows("q_out", q_out), M, N, K,
               k_pages.data_ptr(), v_pages.data_ptr(), slot_mapping.data_ptr(), q_size, Hkv, dh, ps, _stream())
         return q_out
+    if (q_out.dtype == torch.float32 and _split_f32_ok(x, weight, M, K) and q_size % 32 == 0 and dh % 32 == 0
+            and _rows("q_out", q_out) % 4 == 0 and q_out.data_ptr() % 16 == 0 and k_pages.is_contiguous()
+            and v_pages.is_contiguous() and k_pages.data_ptr() % 16 == 0 and v_pages.data_ptr() % 16 == 0):
+        # the same in 32-bit
+        if bias is not None:
+            _cuda("bias", bias, torch.float32)
+        _call("mllm_linear_split_f32_qkv", x.data_ptr(), _rows("x", x), weight.data_ptr(),
+              bias.data_ptr() if bias is not None else None, q_out.data_ptr(), _rows("q_out", q_out), M, N, K,
+              k_pages.data_ptr(), v_pages.data_ptr(), slot_mapping.data_ptr(), q_size, Hkv, dh, ps, _stream())
+        return q_out
     qkv = ws.buf("qkv", M, N, q_out.dtype)
     linear(x, weight, bias, out=qkv)
     kv_write(qkv[:, q_size:q_size + Hkv * dh], qkv[:, q_size + Hkv * dh:], k_pages, v_pages, slot_mapping)
@@ -791,8 +822,16 @@ def linear(x, weight, bias, out, act: Optional[str] = None, accumulate: bool = F
         elif x.dtype == torch.float32 and out.dtype == torch.float32 and _stream_f32_ok(weight, M, K) \
                 and lda % 4 == 0 and x.data_ptr() % 16 == 0:
             impl = "stream_f32"
+        elif _split_f32_ok(x, weight, M, K):
+            impl = "split_f32"
     if impl == "stream_f32":
         _linear_stream_f32(x, weight, bias, out, act, accumulate, None, None)
+        return out
+    if impl == "split_f32":
+        if not _split_f32_ok(x, weight, M, K):
+            raise KernelError(f"linear: split_f32 takes float32, more than {SMALL_M_F32} rows of at least 128 and 16-byte aligned rows")
+        _call("mllm_linear_split_f32", x.data_ptr(), lda, weight.data_ptr(), bias.data_ptr() if bias is not None else None,
+              out.data_ptr(), ldo, M, N, K, _ACT[act], int(accumulate), _stream())
         return out
     if impl in ("smallm", "tcgen05"):
         _call("mllm_linear_" + impl, x.data_ptr(), lda, weight.data_ptr(),

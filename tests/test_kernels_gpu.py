@@ -455,6 +455,76 @@ def test_linear_many_rows_float32_in_k_slices(ops, M, N, K):
         assert torch.equal(part, full[lo:hi]), (lo, hi)
 
 
+@pytest.mark.parametrize("M,N,K", [(65, 64, 128), (128, 1, 132), (129, 191, 768), (300, 1003, 260), (2048, 768, 3072),
+                                   (200, 2304, 768), (77, 50257, 192), (552, 1024, 4096)])
+def test_linear_float32_in_pieces_on_tensor_cores(ops, M, N, K):
+    """The 32-bit product of many rows in exact bfloat16 pieces: every epilogue against float64, no further from float64
+    than the chain of fmaf (for values of both signs and for positive ones, where a bias would add up), a row's bits
+    independent of the rows beside it, and infinities and NaN where the chain has them."""
+    x, w, b = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5), rnd(N, seed=3)
+    ref = x.double() @ w.double().t()
+    for act in (None, "gelu_tanh", "gelu_erf"):
+        out = torch.full((M, N + 3), 7.0, device=DEV)[:, :N]          # rows that the copy engine cannot write
+        ops.linear(x, w, b, out=out, act=act, impl="split_f32")
+        want = ref + b.double()
+        want = want if act is None else torch.nn.functional.gelu(want, approximate="tanh" if act == "gelu_tanh" else "none")
+        assert (out.double() - want).abs().max() < 4e-6 * max(1.0, want.abs().max().item())
+    full = torch.empty(M, N, device=DEV)
+    ops.linear(x, w, None, out=full)                                  # what the dispatcher picks
+    forced = torch.empty(M, N, device=DEV)
+    ops.linear(x, w, None, out=forced, impl="split_f32")
+    assert torch.equal(full, forced)
+    wide = torch.zeros(M, K + 8, device=DEV)
+    wide[:, 4:4 + K] = x
+    acc = rnd(M, N, seed=4)
+    acc0 = acc.clone()
+    ops.linear(wide[:, 4:4 + K], w, None, out=acc, accumulate=True)
+    assert torch.equal(acc, acc0 + full)                              # one addition in 32-bit
+    for xs, ws in ((x, w), (x.abs(), w.abs())):
+        exact = xs.double() @ ws.double().t()
+        err = []
+        for impl in ("split_f32", "simt"):
+            out = torch.empty(M, N, device=DEV)
+            ops.linear(xs, ws, None, out=out, impl=impl)
+            err.append(((out.double() - exact).norm() / exact.norm()).item())
+        assert err[0] <= err[1] * 1.02, err
+    for lo, hi in ((0, 65), (M - 65, M), (M // 2 - 32, M // 2 + 33)):
+        part = torch.empty(65, N, device=DEV)
+        ops.linear(x[lo:hi], w, None, out=part, impl="split_f32")
+        assert torch.equal(part, full[lo:hi]), (lo, hi)
+    x[3, 5], x[9, 1], x[20, 0], w[0, 7], w[N // 2, 0] = float("inf"), float("nan"), 3.4e38, -float("inf"), 2.0
+    out, plain = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    ops.linear(x, w, None, out=out, impl="split_f32")
+    ops.linear(x, w, None, out=plain, impl="simt")
+    assert torch.equal(out.isnan(), plain.isnan()) and torch.equal(out.isposinf(), plain.isposinf())
+    assert torch.equal(out.isneginf(), plain.isneginf())
+    ops.check_device_errors()
+
+
+@pytest.mark.parametrize("M,H,Hkv,dh,page,K", [(300, 12, 12, 64, 16, 768), (65, 4, 2, 32, 8, 128), (130, 3, 3, 16, 4, 192)])
+def test_linear_float32_in_pieces_writes_the_cache(ops, M, H, Hkv, dh, page, K):
+    """The Q|K|V projection of many 32-bit rows (its epilogue stores keys and values where a block of 32 columns lies in
+    one head, else the copy kernel does) against the product followed by the copy kernel; slots below zero stay out."""
+    from mini_llm_b200.engine.context import Workspace
+    ws = Workspace(torch.device(DEV), 512)
+    q_size, kv = H * dh, Hkv * dh
+    N, P = q_size + 2 * kv, 40 + M // page
+    x, w, b = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5), rnd(N, seed=3)
+    slots = torch.randperm(P * page, generator=torch.Generator().manual_seed(4))[:M].to(torch.int32)
+    if dh % 32 == 0:
+        slots[7] = -1
+    slots = slots.to(DEV)
+    qkv = torch.empty(M, N, device=DEV)
+    ops.linear(x, w, b, out=qkv)
+    wk, gk = (torch.full((P, Hkv, page, dh), 9.0, device=DEV) for _ in range(2))
+    wv, gv = wk.clone(), gk.clone()
+    keep = slots >= 0
+    ops.kv_write(qkv[keep][:, q_size:q_size + kv], qkv[keep][:, q_size + kv:], wk, wv, slots[keep])
+    q = ops.linear_qkv_cache(x, w, b, torch.empty(M, q_size, device=DEV), gk, gv, slots, ws)
+    assert torch.equal(q, qkv[:, :q_size]) and torch.equal(gk, wk) and torch.equal(gv, wv)
+    ops.check_device_errors()
+
+
 def _paged_case(dtype, seqs, H, Hkv, dh, page, num_pages, seed, sharp_key=None):
     """seqs: list of (context_len, q_len).  Returns everything the kernel needs plus dense K/V per sequence."""
     g = torch.Generator().manual_seed(seed)
