@@ -96,7 +96,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     uint32_t* tmem_slot = (uint32_t*)(o_free + 1);
     volatile int* failed = (volatile int*)(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int h = blockIdx.x, tile = blockIdx.y;
 
     if (threadIdx.x == 0) {
@@ -168,51 +168,50 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = make_idesc(BQ, BKV);
-            constexpr uint32_t idesc_o = make_idesc_bmn(BQ, DH);
-            const uint32_t t_o = tmem_base + TMEM_O;
-            const uint64_t q_desc = make_smem_desc(smem_u32(sQ));
-            auto issue_s = [&](int i) {                       // S(i) = Q K(i)^T into the S buffer i & 1
-                const uint64_t k_desc = make_smem_desc(smem_u32(sKV + (size_t)(i % STAGES) * 2 * KV_BYTES));
+        // (the warp as a whole runs the loop, one elected lane issues: tcgen05.cuh says why)
+        constexpr uint32_t idesc_s = make_idesc(BQ, BKV);
+        constexpr uint32_t idesc_o = make_idesc_bmn(BQ, DH);
+        const uint32_t t_o = tmem_base + TMEM_O;
+        const uint64_t q_desc = make_smem_desc(smem_u32(sQ)), kv_desc = make_smem_desc(smem_u32(sKV)),
+                       p_desc = make_smem_desc(smem_u32(sP));
+        auto all_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); };
+        auto issue_s = [&](int i) {                       // S(i) = Q K(i)^T into the S buffer i & 1
+            const uint64_t k_desc = kv_desc + (uint64_t)((i % STAGES) * (2 * KV_BYTES >> 4));
 #pragma unroll
-                for (int k = 0; k < DH / 16; ++k)
-                    umma_f16(tmem_base + (uint32_t)(i & 1) * 128, q_desc + 2 * k, k_desc + 2 * k, idesc_s, k != 0);
-                umma_commit(&s_full[i & 1]);
-                umma_commit(&k_empty[i % STAGES]);             // the keys of this block have been read
-            };
-            bool ok = mbar_wait(q_full, 0) && mbar_wait(&k_full[0], 0);
-            if (!ok) *failed = 2;
-            if (ok) {
+            for (int k = 0; k < DH / 16; ++k)
+                umma_f16_warp(tmem_base + (uint32_t)(i & 1) * 128, q_desc + 2 * k, k_desc + 2 * k, idesc_s, k != 0);
+            umma_commit_warp(&s_full[i & 1]);
+            umma_commit_warp(&k_empty[i % STAGES]);       // the keys of this block have been read
+        };
+        bool ok = all_wait(q_full, 0) && all_wait(&k_full[0], 0);
+        if (!ok) *failed = 2;
+        if (ok) {
+            tc_fence_after();
+            issue_s(0);
+        }
+        for (int i = 0; i < nblk && ok; ++i) {
+            if (i + 1 < nblk) {
+                // S of the next block goes ahead of this block's P V: its buffer was read two blocks ago
+                if (!all_wait(&k_full[(i + 1) % STAGES], ((i + 1) / STAGES) & 1)) { *failed = 3; break; }
                 tc_fence_after();
-                issue_s(0);
+                issue_s(i + 1);
             }
-            for (int i = 0; i < nblk && ok && !*failed; ++i) {
-                if (i + 1 < nblk) {
-                    // S of the next block goes ahead of this block's P V: its buffer was read two blocks ago
-                    if (!mbar_wait(&k_full[(i + 1) % STAGES], ((i + 1) / STAGES) & 1)) { *failed = 3; break; }
-                    tc_fence_after();
-                    issue_s(i + 1);
-                }
-                // O_blk = P(i) V(i) (hi term, then lo term) once the weights are written and O_blk of block i-1 was read
-                if (!mbar_wait(p_full, i & 1)) { *failed = 4; break; }
-                if (i > 0 && !mbar_wait(o_free, (i - 1) & 1)) { *failed = 5; break; }
-                if (!mbar_wait(&v_full[i % STAGES], (i / STAGES) & 1)) { *failed = 6; break; }
-                tc_fence_after();
-                const uint32_t v_addr = smem_u32(sKV + (size_t)(i % STAGES) * 2 * KV_BYTES + KV_BYTES);
-                const uint32_t p_addr = smem_u32(sP + (size_t)(i & 1) * 2 * P_BYTES);
+            // O_blk = P(i) V(i) (hi term, then lo term) once the weights are written and O_blk of block i-1 was read
+            if (!all_wait(p_full, i & 1)) { *failed = 4; break; }
+            if (i > 0 && !all_wait(o_free, (i - 1) & 1)) { *failed = 5; break; }
+            if (!all_wait(&v_full[i % STAGES], (i / STAGES) & 1)) { *failed = 6; break; }
+            tc_fence_after();
+            const uint64_t v_desc = kv_desc + (uint64_t)(((i % STAGES) * 2 * KV_BYTES + KV_BYTES) >> 4);
+            const uint64_t pi_desc = p_desc + (uint64_t)((i & 1) * (2 * P_BYTES >> 4));
 #pragma unroll
-                for (int term = 0; term < 2; ++term) {
+            for (int term = 0; term < 2; ++term) {
 #pragma unroll
-                    for (int kk = 0; kk < BKV / 16; ++kk) {
-                        const uint64_t a_desc = make_smem_desc(p_addr + term * P_BYTES + (kk / 4) * (P_BYTES / 2)) + 2 * (kk % 4);
-                        const uint64_t b_desc = make_smem_desc(v_addr + kk * 2048);
-                        umma_f16(t_o, a_desc, b_desc, idesc_o, (term | kk) != 0);
-                    }
-                }
-                umma_commit(o_full);
-                umma_commit(&v_empty[i % STAGES]);            // this block's values have been read
+                for (int kk = 0; kk < BKV / 16; ++kk)
+                    umma_f16_warp(t_o, pi_desc + (uint64_t)(((term * P_BYTES + (kk / 4) * (P_BYTES / 2)) >> 4) + 2 * (kk % 4)),
+                                  v_desc + (uint64_t)(kk * (2048 >> 4)), idesc_o, (term | kk) != 0);
             }
+            umma_commit_warp(o_full);
+            umma_commit_warp(&v_empty[i % STAGES]);       // this block's values have been read
         }
     } else {
         // ---------------------------------------------------------------- softmax: one query row per thread

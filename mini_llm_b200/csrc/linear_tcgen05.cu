@@ -82,7 +82,7 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
     volatile int* failed = (volatile int*)(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int nk = (K + C::KB * BK - 1) / (C::KB * BK);       // stages per tile; k-blocks beyond K are zeros
 
     if (threadIdx.x == 0) {
@@ -99,71 +99,76 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     // The weights are written by no kernel of the step: the W tiles of the first stages are asked for before the
     // wait on the previous kernel; their A tiles follow after it and complete the same barriers.
     int pre = 0;                                                 // stages whose W tiles are already on their way
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
         const int my_tiles = (int)blockIdx.x < num_tiles ? (num_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
         pre = min(C::STAGES, my_tiles * nk);
+        int n0 = (blockIdx.x % tiles_n) * BN, tile = blockIdx.x, kt = 0;
         for (int g = 0; g < pre; ++g) {
-            const int tile = blockIdx.x + (g / nk) * gridDim.x, kt = g % nk;
-            const int n0 = (tile % tiles_n) * BN;
             uint8_t* a_dst = tiles + (size_t)g * C::STAGE_BYTES;
-            mbar_expect_tx(&full[g], C::STAGE_BYTES);
+            mbar_expect_tx_warp(&full[g], C::STAGE_BYTES);
 #pragma unroll
             for (int b = 0; b < C::KB; ++b)
-                tma_load_2d(a_dst + b * C::BLOCK_BYTES + C::A_BYTES, &map_w, (kt * C::KB + b) * BK, n0, &full[g]);
+                tma_load_2d_warp(a_dst + b * C::BLOCK_BYTES + C::A_BYTES, &map_w, (kt * C::KB + b) * BK, n0, &full[g]);
+            if (++kt == nk) { kt = 0; tile += gridDim.x; n0 = (tile % tiles_n) * BN; }
         }
     }
     pdl_wait();                 // now what earlier kernels of the step wrote may be read
     pdl_launch();
 
+    // Producer and MMA issuer run their loops as whole warps and one elected lane issues (tcgen05.cuh says why).
     if (warp == 0) {
-        if (lane == 0) {
-            int g = 0;                                           // k-steps issued so far, over all tiles
-            for (int tile = blockIdx.x; tile < num_tiles && !*failed; tile += gridDim.x) {
-                const int m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN;
-                for (int kt = 0; kt < nk; ++kt, ++g) {
-                    const int s = g % C::STAGES;
-                    if (g >= C::STAGES && !mbar_wait(&empty[s], ((g / C::STAGES) - 1) & 1)) { *failed = 1; break; }
-                    if (*failed) break;
-                    uint8_t* a_dst = tiles + (size_t)s * C::STAGE_BYTES;
-                    const bool w_sent = g < pre;
-                    if (!w_sent) mbar_expect_tx(&full[s], C::STAGE_BYTES);
+        int g = 0, s = 0;                                    // k-steps issued so far, over all tiles; their stage
+        uint32_t parity = 0;                                 // of the use of the stage that has to be over
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+            const int m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN;
+            for (int kt = 0; kt < nk; ++kt, ++g) {
+                if (g >= C::STAGES && !mbar_wait(&empty[s], parity)) *failed = 1;
+                ok = __all_sync(0xffffffffu, !*failed);
+                if (!ok) break;
+                uint8_t* a_dst = tiles + (size_t)s * C::STAGE_BYTES;
+                const bool w_sent = g < pre;
+                if (!w_sent) mbar_expect_tx_warp(&full[s], C::STAGE_BYTES);
 #pragma unroll
-                    for (int b = 0; b < C::KB; ++b) {
-                        tma_load_2d(a_dst + b * C::BLOCK_BYTES, &map_a, (kt * C::KB + b) * BK, m0, &full[s]);
-                        if (!w_sent)
-                            tma_load_2d(a_dst + b * C::BLOCK_BYTES + C::A_BYTES, &map_w, (kt * C::KB + b) * BK, n0, &full[s]);
-                    }
+                for (int b = 0; b < C::KB; ++b) {
+                    tma_load_2d_warp(a_dst + b * C::BLOCK_BYTES, &map_a, (kt * C::KB + b) * BK, m0, &full[s]);
+                    if (!w_sent)
+                        tma_load_2d_warp(a_dst + b * C::BLOCK_BYTES + C::A_BYTES, &map_w, (kt * C::KB + b) * BK, n0, &full[s]);
+                }
+                if (++s == C::STAGES) {
+                    s = 0;
+                    if (g >= C::STAGES) parity ^= 1;         // the first round waits for nothing
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc(BM, BN);
-            int g = 0, ti = 0;
-            for (int tile = blockIdx.x; tile < num_tiles && !*failed; tile += gridDim.x, ++ti) {
-                const int buf = ti & 1;
-                if (ti >= 2 && !mbar_wait(&acc_empty[buf], ((ti >> 1) - 1) & 1)) { *failed = 4; break; }
+        constexpr uint32_t idesc = make_idesc(BM, BN);
+        const uint64_t desc0 = make_smem_desc(smem_u32(tiles));
+        int s = 0, ti = 0;
+        uint32_t parity = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++ti) {
+            const int buf = ti & 1;
+            if (ti >= 2 && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], ((ti >> 1) - 1) & 1))) { *failed = 4; break; }
+            tc_fence_after();
+            const uint32_t d_tmem = tmem_base + (uint32_t)(buf * C::ACC_COLS);
+            for (int kt = 0; kt < nk; ++kt) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&full[s], parity));
+                if (!ok) { *failed = 2; break; }
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + (uint32_t)(buf * C::ACC_COLS);
-                bool ok = true;
-                for (int kt = 0; kt < nk; ++kt, ++g) {
-                    const int s = g % C::STAGES;
-                    if (!mbar_wait(&full[s], (g / C::STAGES) & 1)) { *failed = 2; ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t a_addr = smem_u32(tiles + (size_t)s * C::STAGE_BYTES);
+                const uint64_t a_desc = desc0 + (uint64_t)(s * (C::STAGE_BYTES >> 4));
 #pragma unroll
-                    for (int b = 0; b < C::KB; ++b) {
-                        const uint64_t a_desc = make_smem_desc(a_addr + b * C::BLOCK_BYTES);
-                        const uint64_t b_desc = make_smem_desc(a_addr + b * C::BLOCK_BYTES + C::A_BYTES);
+                for (int b = 0; b < C::KB; ++b) {
 #pragma unroll
-                        for (int k = 0; k < BK / 16; ++k)      // 32 bytes along K inside the swizzle atom = +2 in the address field
-                            umma_f16(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, (kt | b | k) != 0);
-                    }
-                    umma_commit(&empty[s]);                 // the stage is free once these MMAs have read it
+                    for (int k = 0; k < BK / 16; ++k)      // 32 bytes along K inside the swizzle atom = +2 in the address field
+                        umma_f16_warp(d_tmem, a_desc + (uint64_t)(b * (C::BLOCK_BYTES >> 4) + 2 * k),
+                                      a_desc + (uint64_t)((b * C::BLOCK_BYTES + C::A_BYTES) / 16 + 2 * k), idesc, (kt | b | k) != 0);
                 }
-                if (!ok) break;
-                umma_commit(&acc_full[buf]);                // the accumulator is complete once all of them are done
+                umma_commit_warp(&empty[s]);                // the stage is free once these MMAs have read it
+                if (++s == C::STAGES) { s = 0; parity ^= 1; }
             }
+            if (!ok) break;
+            umma_commit_warp(&acc_full[buf]);               // the accumulator is complete once all of them are done
         }
     } else {
         const int q = warp & 3;                             // the quarter of the 128 TMEM lanes this warp may read
