@@ -29,27 +29,41 @@ __global__ void layernorm_kernel(const float* x, const int* __restrict__ rows,
         o[d] = from_f32<TOut>((xr[d] - mean) * inv * gamma[d] + beta[d]);
 }
 
-// One warp per row, the row held in registers (up to 2048 columns): one read of the row, the
+// One warp per row, the row held in registers (up to 2048 columns, KEEP runs of 128): one read of the row, the
 // centred second pass runs on registers, 16-byte loads and stores.  Same arithmetic order for
-// a row whatever the number of rows.
-template <typename TOut>
-__global__ void __launch_bounds__(256)
+// a row whatever the number of rows.  What bounds it is the chain of memory round trips, not bytes, so gamma and beta
+// (weights) are in registers before the wait on the previous kernel: inside a step a launch took 4.6 us at
+// 64 to 77 rows of 768 and 9.2 us at 24 rows of 1600 with them read after the statistics, 1.8 and 2.7 us now.  Four
+// rows per CTA (eight before) spread few rows over the SMs.
+constexpr int ROWS = 4;
+
+template <typename TOut, int KEEP>
+__global__ void __launch_bounds__(ROWS * 32)
 layernorm_warp_kernel(const float* x, const int* __restrict__ rows, const float* __restrict__ gamma,
                       const float* __restrict__ beta, TOut* __restrict__ out, int R, int D, float eps) {
-    constexpr int KEEP = 16;
+    const int r = blockIdx.x * ROWS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= R) return;
+    float4 g[KEEP], b[KEEP];
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i) {
+        const int k = lane * 4 + i * 128;
+        if (k < D) {
+            g[i] = __ldg(reinterpret_cast<const float4*>(gamma + k));
+            b[i] = __ldg(reinterpret_cast<const float4*>(beta + k));
+        }
+    }
+    const float* xr = x + (size_t)(rows ? rows[r] : r) * D;
     pdl_wait();
     pdl_launch();
-    const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (r >= R) return;
-    const float* xr = x + (size_t)(rows ? rows[r] : r) * D;
     float4 v[KEEP];
     float s = 0.f;
 #pragma unroll
     for (int i = 0; i < KEEP; ++i) {
         const int k = lane * 4 + i * 128;
         v[i] = k < D ? *reinterpret_cast<const float4*>(xr + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-        s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
     }
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i) s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
     const float mean = warp_sum(s) / (float)D;
     float q = 0.f;
 #pragma unroll
@@ -65,10 +79,8 @@ layernorm_warp_kernel(const float* x, const int* __restrict__ rows, const float*
     for (int i = 0; i < KEEP; ++i) {
         const int k = lane * 4 + i * 128;
         if (k >= D) break;
-        const float4 g = __ldg(reinterpret_cast<const float4*>(gamma + k));
-        const float4 b = __ldg(reinterpret_cast<const float4*>(beta + k));
-        const float y0 = (v[i].x - mean) * inv * g.x + b.x, y1 = (v[i].y - mean) * inv * g.y + b.y;
-        const float y2 = (v[i].z - mean) * inv * g.z + b.z, y3 = (v[i].w - mean) * inv * g.w + b.w;
+        const float y0 = (v[i].x - mean) * inv * g[i].x + b[i].x, y1 = (v[i].y - mean) * inv * g[i].y + b[i].y;
+        const float y2 = (v[i].z - mean) * inv * g[i].z + b[i].z, y3 = (v[i].w - mean) * inv * g[i].w + b[i].w;
         if constexpr (sizeof(TOut) == 4) {
             *reinterpret_cast<float4*>(o + k) = make_float4(y0, y1, y2, y3);
         } else {
@@ -81,6 +93,16 @@ layernorm_warp_kernel(const float* x, const int* __restrict__ rows, const float*
     }
 }
 
+template <typename TOut>
+int launch_warp(const float* x, const int* rows, const float* gamma, const float* beta, void* out, int R, int D, float eps,
+                cudaStream_t stream) {
+    auto kern = D <= 768 ? layernorm_warp_kernel<TOut, 6> : D <= 1024 ? layernorm_warp_kernel<TOut, 8> :
+                D <= 1664 ? layernorm_warp_kernel<TOut, 13> : layernorm_warp_kernel<TOut, 16>;
+    MLLM_CUDA(mllm_launch(kern, dim3((R + ROWS - 1) / ROWS), dim3(ROWS * 32), 0, stream, true, x, rows, gamma, beta,
+                          (TOut*)out, R, D, eps));
+    return 0;
+}
+
 MLLM_EXPORT int mllm_layernorm(const float* x, const int* rows, const float* gamma, const float* beta,
                                void* out, int R, int D, float eps, int out_dtype, cudaStream_t stream) {
     if (R <= 0) return 0;
@@ -88,14 +110,8 @@ MLLM_EXPORT int mllm_layernorm(const float* x, const int* rows, const float* gam
     const bool fast = D % 4 == 0 && D <= 2048 && (uintptr_t)x % 16 == 0 && (uintptr_t)gamma % 16 == 0 &&
                       (uintptr_t)beta % 16 == 0 && (uintptr_t)out % 16 == 0;
     if (fast && (out_dtype == MLLM_F32 || out_dtype == MLLM_BF16)) {
-        const int grid = (R + 7) / 8;
-        if (out_dtype == MLLM_F32)
-            MLLM_CUDA(mllm_launch(layernorm_warp_kernel<float>, dim3(grid), dim3(256), 0, stream, true, x, rows, gamma,
-                                  beta, (float*)out, R, D, eps));
-        else
-            MLLM_CUDA(mllm_launch(layernorm_warp_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, stream, true, x, rows,
-                                  gamma, beta, (__nv_bfloat16*)out, R, D, eps));
-        return 0;
+        return out_dtype == MLLM_F32 ? launch_warp<float>(x, rows, gamma, beta, out, R, D, eps, stream)
+                                     : launch_warp<__nv_bfloat16>(x, rows, gamma, beta, out, R, D, eps, stream);
     }
     int threads = D >= 1024 ? 256 : (D >= 256 ? 128 : ((D + 31) / 32) * 32);
     if (out_dtype == MLLM_F32)
