@@ -39,19 +39,23 @@ class StepLayout:
     max_pages: Tuple[int, ...]
     n_tiles: int = 0
     n_tiles_wide: int = 0
+    n_single: int = 0
     offsets: Dict[str, int] = field(default_factory=dict)
     total: int = 0
 
     @classmethod
     def make(cls, T: int, S: int, R: int, max_pages: Sequence[int], n_tiles: int = 0,
-             n_tiles_wide: int = 0) -> "StepLayout":
-        lay = cls(T, S, R, tuple(max_pages), n_tiles, n_tiles_wide)
+             n_tiles_wide: int = 0, n_single: int = 0) -> "StepLayout":
+        lay = cls(T, S, R, tuple(max_pages), n_tiles, n_tiles_wide, n_single)
         off = 0
         for name, n in (("token_ids", T), ("positions", T), ("token_seq", T), ("logit_rows", R),
                         ("state_slots", S), ("cu_q", S + 1), ("q_start", S), ("ctx_len", S),
                         ("attn_tiles", 3 * n_tiles), ("attn_tiles_wide", 3 * n_tiles_wide)):
             lay.offsets[name] = off
             off += _pad4(n)
+        if n_single:
+            lay.offsets["single_rows"] = off
+            off += _pad4(n_single)
         for g, mp in enumerate(max_pages):
             lay.offsets[f"slot_mapping.{g}"] = off
             off += _pad4(T)
@@ -61,7 +65,7 @@ class StepLayout:
         return lay
 
     def key(self):
-        return (self.T, self.S, self.R, self.max_pages, self.n_tiles, self.n_tiles_wide)
+        return (self.T, self.S, self.R, self.max_pages, self.n_tiles, self.n_tiles_wide, self.n_single)
 
 
 class Workspace:
@@ -138,6 +142,10 @@ class StepContext:
         # the same tokens cut into tiles of ATTN_TILE_WIDE rows, for the tcgen05 attention
         self.attn_tiles_wide = sec("attn_tiles_wide", 3 * layout.n_tiles_wide)
         self.n_tiles_wide = layout.n_tiles_wide
+        # flat rows of the requests that bring one token to a step in which others bring more; where there are any, their
+        # tiles stand at the end of both lists
+        self.n_single = layout.n_single
+        self.single_rows = sec("single_rows", self.n_single) if self.n_single else None
         self.groups: List[GroupView] = []
         for g, mp in enumerate(layout.max_pages):
             bt = dev[o[f"block_table.{g}"]:o[f"block_table.{g}"] + self.S * mp].view(self.S, mp)
@@ -150,6 +158,7 @@ class StepContext:
         self.q_starts = list(q_starts)
         self.max_q_len = max(self.q_lens) if self.q_lens else 0
         self.max_ctx_len = max((a + b for a, b in zip(self.q_starts, self.q_lens)), default=0)
+        self.max_single_ctx_len = max((a + 1 for a, b in zip(self.q_starts, self.q_lens) if b == 1), default=0)
         self.decode_only = self.max_q_len == 1
         # what a layer's arrangement leaves for the next one within the step (a residual write that the next layer's
         # read takes along); nothing is carried from one step to the next
@@ -161,11 +170,12 @@ ATTN_TILE_WIDE = 128     # query rows per tile of csrc/attention_tcgen05.cu
 
 
 def attention_tiles(q_lens: Sequence[int], q_starts: Optional[Sequence[int]] = None,
-                    tile_rows: int = ATTN_TILE) -> List[int]:
+                    tile_rows: int = ATTN_TILE, singles_last: bool = False) -> List[int]:
     """Cut every request's new tokens into tiles of at most ``tile_rows`` rows: triples of
     (request index in the batch, flat index of the tile's first token, rows).  With the
     positions at which the portions start, the tiles that see the most keys come first,
-    so that the longest walks of the attention kernel start earliest."""
+    so that the longest walks of the attention kernel start earliest.  ``singles_last``: requests with
+    one new token come after all others, so that a launch over the others takes the head of the list."""
     tiles = []
     base = 0
     for s, n in enumerate(q_lens):
@@ -176,6 +186,8 @@ def attention_tiles(q_lens: Sequence[int], q_starts: Optional[Sequence[int]] = N
         base += n
     if q_starts is not None:
         tiles.sort(key=lambda t: -t[0])          # stable: equal lengths keep the batch order
+    if singles_last:
+        tiles.sort(key=lambda t: q_lens[t[1]] == 1)
     out: List[int] = []
     for _, s, t0, rows in tiles:
         out += [s, t0, rows]
@@ -183,7 +195,7 @@ def attention_tiles(q_lens: Sequence[int], q_starts: Optional[Sequence[int]] = N
 
 
 def pack_step(layout: StepLayout, host: np.ndarray, *, token_ids, positions, token_seq, logit_rows, state_slots,
-              cu_q, q_start, ctx_len, slot_mappings, block_tables, attn_tiles=(), attn_tiles_wide=()) -> None:
+              cu_q, q_start, ctx_len, slot_mappings, block_tables, attn_tiles=(), attn_tiles_wide=(), single_rows=()) -> None:
     """Write every section into the int32 array ``host`` (length >= layout.total)."""
     o = layout.offsets
 
@@ -203,6 +215,8 @@ def pack_step(layout: StepLayout, host: np.ndarray, *, token_ids, positions, tok
         put("attn_tiles", attn_tiles)
     if layout.n_tiles_wide:
         put("attn_tiles_wide", attn_tiles_wide)
+    if layout.n_single:
+        put("single_rows", single_rows)
     for g, mp in enumerate(layout.max_pages):
         put(f"slot_mapping.{g}", slot_mappings[g])
         bt = np.zeros((layout.S, mp), dtype=np.int32)

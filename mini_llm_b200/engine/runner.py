@@ -97,6 +97,9 @@ class ModelRunner:
         # a part that reads device data on the host while it runs sets graph_safe = False
         self._graph_ok = all(getattr(self.model.part(label), "graph_safe", True)
                              for label, _ in self.spec.all_part_specs())
+        # a mixer whose attention takes the single tokens of a mixed step by themselves
+        self._singles_apart = any(getattr(self.model.part(label), "singles_apart", False)
+                                  for label, _ in self.spec.all_part_specs())
         self._capture_at_once = self.engine.graph_capture == "at_once"
         if self._capture_at_once and self.cache.state_layers:
             raise StepError("graph_capture='at_once' runs a new step shape twice; a mixer with a state of its own "
@@ -240,14 +243,17 @@ class ModelRunner:
         for g in range(ng):
             mp = max(len(t) for t in tables[g])
             max_pages.append(max(16, 1 << (mp - 1).bit_length()))   # powers of two: few distinct shapes for captured graphs
-        tiles = [] if T == S else attention_tiles(q_lens, q_start)
-        wide = [] if T == S else attention_tiles(q_lens, q_start, ATTN_TILE_WIDE)
-        layout = StepLayout.make(T, S, len(logit_rows), max_pages, len(tiles) // 3, len(wide) // 3)
+        apart = self._singles_apart and T != S
+        tiles = [] if T == S else attention_tiles(q_lens, q_start, singles_last=apart)
+        wide = [] if T == S else attention_tiles(q_lens, q_start, ATTN_TILE_WIDE, singles_last=apart)
+        singles = [int(cu_q[s]) for s, n in enumerate(q_lens) if n == 1] if apart else []
+        layout = StepLayout.make(T, S, len(logit_rows), max_pages, len(tiles) // 3, len(wide) // 3, len(singles))
         i, host = self._staging(layout.total)
         self._last_layout_total = layout.total
         pack_step(layout, host.numpy(), token_ids=token_ids, positions=positions, token_seq=token_seq,
                   logit_rows=logit_rows, state_slots=slots, cu_q=cu_q, q_start=q_start, ctx_len=ctx_len,
-                  slot_mappings=slot_maps, block_tables=tables, attn_tiles=tiles, attn_tiles_wide=wide)
+                  slot_mappings=slot_maps, block_tables=tables, attn_tiles=tiles, attn_tiles_wide=wide,
+                  single_rows=singles)
         self._dev[:layout.total].copy_(host[:layout.total], non_blocking=True)
         self._host_events[i].record()
         self._pending_ids = pending
@@ -300,7 +306,8 @@ class ModelRunner:
             self._graph_seen.clear()
             self._graph_families.clear()
             self._graph_version = self._buffer_version()
-        key = (ctx.layout.key(), ops.decode_splits(ctx.max_ctx_len) if ctx.decode_only else 0,
+        key = (ctx.layout.key(), ops.decode_splits(ctx.max_ctx_len) if ctx.decode_only else
+               ops.decode_splits(ctx.max_single_ctx_len) if ctx.n_single else 0,
                ops.latent_splits(ctx.max_ctx_len))      # every host-side number a launch's grid depends on
         g = self._graphs.get(key)
         if g is not None:

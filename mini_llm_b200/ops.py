@@ -85,6 +85,9 @@ def _signatures(lib):
         "mllm_attention_decode": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                   c_ll, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
                                   c_int, c_int, c_int, c_int, c_void_p],
+        "mllm_attention_decode_rows": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
+                                       c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
+                                       c_int, c_int, c_int, c_int, c_void_p],
         "mllm_attention_decode_last_staging": [],
         "mllm_attention_flash": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p,
                                  c_void_p, c_ll, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
@@ -2004,19 +2007,18 @@ attention_launches = {}     # attention kernel name -> launches so far (tests ch
 use_tcgen05_attention = True    # False: prompt portions stay on the mma.sync kernel (for comparisons and profiles)
 
 
-def _flash_tc_ok(q, k_pages, out, ctx, head_dim, ps, ldq, ldo) -> bool:
+def _flash_tc_ok(q, k_pages, out, n_wide, head_dim, ps, ldq, ldo) -> bool:
     return (q.dtype == torch.bfloat16 and head_dim == 64 and 8 <= ps <= 128 and ps & (ps - 1) == 0
-            and getattr(ctx, "n_tiles_wide", 0) > 0 and ldq % 8 == 0 and q.data_ptr() % 16 == 0 and ldo % 8 == 0
+            and n_wide > 0 and ldq % 8 == 0 and q.data_ptr() % 16 == 0 and ldo % 8 == 0
             and out.data_ptr() % 16 == 0 and k_pages.is_contiguous() and k_pages.data_ptr() % 16 == 0)
 
 
 _TILED_WIDE_HEAD_DIMS = (16, 32, 48, 64)
 
 
-def _tiled_wide_ok(q, head_dim, ctx, ldq) -> bool:
+def _tiled_wide_ok(q, head_dim, n_wide, tokens, ldq) -> bool:
     """Long prompt portions (128-row tiles mostly full) with heads up to 64, where no tensor-core kernel applies."""
-    nw = getattr(ctx, "n_tiles_wide", 0)
-    return (head_dim in _TILED_WIDE_HEAD_DIMS and nw > 0 and ctx.T >= 256 and ctx.T >= 80 * nw
+    return (head_dim in _TILED_WIDE_HEAD_DIMS and n_wide > 0 and tokens >= 256 and tokens >= 80 * n_wide
             and ldq % (16 // q.element_size()) == 0 and q.data_ptr() % 16 == 0)
 
 
@@ -2041,44 +2043,64 @@ def paged_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, nu
     if head_dim % 16 != 0 or not (16 <= head_dim <= 256):
         raise KernelError(f"paged_attention: head size {head_dim} is not a multiple of 16 in 16..256")
     bt_stride = _rows("block_table", block_table)
+    n_tiles, n_wide, tokens, singles = getattr(ctx, "n_tiles", 0), getattr(ctx, "n_tiles_wide", 0), T, 0
+    decode_ok = head_dim in _DECODE_HEAD_DIMS[q.dtype] and ldq % 8 == 0 and q.data_ptr() % 16 == 0
     if impl is None:
         impl = "simt"
-        if getattr(ctx, "decode_only", False) and head_dim in _DECODE_HEAD_DIMS[q.dtype] and ldq % 8 == 0 \
-                and q.data_ptr() % 16 == 0:
+        if decode_ok and (k_pages.data_ptr() | v_pages.data_ptr()) % 16 == 0 and getattr(ctx, "n_single", 0):
+            # single tokens beside prompt portions: the decode kernel takes them after the portions' launch below, whose
+            # tiles are the head of the lists
+            singles = ctx.n_single
+            n_tiles, n_wide, tokens = n_tiles - singles, n_wide - singles, T - singles
+        if getattr(ctx, "decode_only", False) and decode_ok:
             impl = "decode"
-        elif use_tcgen05_attention and _flash_tc_ok(q, k_pages, out, ctx, head_dim, ps, ldq, ldo) and ctx.T >= 256 \
-                and ctx.T >= 80 * ctx.n_tiles_wide:
+        elif use_tcgen05_attention and _flash_tc_ok(q, k_pages, out, n_wide, head_dim, ps, ldq, ldo) and tokens >= 256 \
+                and tokens >= 80 * n_wide:
             impl = "flash_tc"       # long prompt portions (tiles of 128 rows mostly full): the tensor-memory kernel
-        elif q.dtype == torch.bfloat16 and head_dim in _FLASH_HEAD_DIMS and getattr(ctx, "n_tiles", 0) > 0 \
+        elif q.dtype == torch.bfloat16 and head_dim in _FLASH_HEAD_DIMS and n_tiles > 0 \
                 and ldq % 8 == 0 and q.data_ptr() % 16 == 0 and ldo % 2 == 0:
             impl = "flash"
-        elif _tiled_wide_ok(q, head_dim, ctx, ldq):
+        elif _tiled_wide_ok(q, head_dim, n_wide, tokens, ldq):
             impl = "tiled_wide"     # float32 (or a head size of 48) and long portions: 128 x 128 tiles on CUDA cores
-        elif getattr(ctx, "n_tiles", 0) > 0:
+        elif n_tiles > 0:
             impl = "tiled"          # float32, or a head size the tensor-core kernel does not take
+    if singles:
+        _attend(impl, q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ldo, num_heads, num_kv_heads, head_dim, ps,
+                scale, window, n_tiles, n_wide, None)
+        _attend("decode", q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ldo, num_heads, num_kv_heads, head_dim,
+                ps, scale, window, 0, 0, ctx.single_rows)
+        return
+    _attend(impl, q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ldo, num_heads, num_kv_heads, head_dim, ps, scale,
+            window, n_tiles, n_wide, None)
+
+
+def _attend(impl, q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ldo, num_heads, num_kv_heads, head_dim, ps, scale,
+            window, n_tiles, n_wide, rows) -> None:
+    """One launch of the named attention kernel; ``rows``: the batch's rows that the decode kernel takes (None: all)."""
+    T = q.shape[0] if rows is None else rows.shape[0]
     attention_launches[impl] = attention_launches.get(impl, 0) + 1
     if impl == "tiled_wide":
-        if head_dim not in _TILED_WIDE_HEAD_DIMS or getattr(ctx, "n_tiles_wide", 0) <= 0 or ldq % (16 // q.element_size()):
+        if head_dim not in _TILED_WIDE_HEAD_DIMS or n_wide <= 0 or ldq % (16 // q.element_size()):
             raise KernelError("paged_attention: the 128 x 128 CUDA-core kernel takes head sizes "
                               f"{_TILED_WIDE_HEAD_DIMS}, 16-byte aligned rows and a list of 128-row tiles")
         _call("mllm_attention_tiled_wide", q.data_ptr(), ldq, k_pages.data_ptr(), v_pages.data_ptr(),
-              block_table.data_ptr(), bt_stride, ctx.attn_tiles_wide.data_ptr(), int(ctx.n_tiles_wide),
+              block_table.data_ptr(), bt_stride, ctx.attn_tiles_wide.data_ptr(), int(n_wide),
               ctx.positions.data_ptr(), out.data_ptr(), ldo, num_heads, num_kv_heads, head_dim, ps, float(scale),
               int(window or 0), _dt(q), _stream())
         return
     if impl == "tiled":
         _call("mllm_attention_tiled", q.data_ptr(), ldq, k_pages.data_ptr(), v_pages.data_ptr(),
-              block_table.data_ptr(), bt_stride, ctx.attn_tiles.data_ptr(), int(ctx.n_tiles),
+              block_table.data_ptr(), bt_stride, ctx.attn_tiles.data_ptr(), int(n_tiles),
               ctx.positions.data_ptr(), out.data_ptr(), ldo, num_heads, num_kv_heads, head_dim, ps, float(scale),
               int(window or 0), _dt(q), _stream())
         return
     if impl == "flash_tc":
-        if not _flash_tc_ok(q, k_pages, out, ctx, head_dim, ps, ldq, ldo):
+        if not _flash_tc_ok(q, k_pages, out, n_wide, head_dim, ps, ldq, ldo):
             raise KernelError("paged_attention: the tcgen05 kernel takes bfloat16, head size 64, pages of 8..128 "
                               "tokens (a power of two), 16-byte aligned rows and a list of 128-row tiles")
         _call("mllm_attention_tcgen05", q.data_ptr(), ldq, T, k_pages.data_ptr(), v_pages.data_ptr(),
               int(k_pages.shape[0]), block_table.data_ptr(), bt_stride, ctx.attn_tiles_wide.data_ptr(),
-              int(ctx.n_tiles_wide), ctx.positions.data_ptr(), out.data_ptr(), ldo, num_heads, num_kv_heads, head_dim,
+              int(n_wide), ctx.positions.data_ptr(), out.data_ptr(), ldo, num_heads, num_kv_heads, head_dim,
               ps, float(scale), int(window or 0), _stream())
         return
     if impl == "flash":
@@ -2086,7 +2108,7 @@ def paged_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, nu
             raise KernelError(f"paged_attention: the tensor-core kernel takes bfloat16 and head sizes "
                               f"{_FLASH_HEAD_DIMS}, not {q.dtype} / {head_dim}")
         _call("mllm_attention_flash", q.data_ptr(), ldq, k_pages.data_ptr(), v_pages.data_ptr(),
-              block_table.data_ptr(), bt_stride, ctx.attn_tiles.data_ptr(), int(ctx.n_tiles),
+              block_table.data_ptr(), bt_stride, ctx.attn_tiles.data_ptr(), int(n_tiles),
               ctx.positions.data_ptr(), out.data_ptr(), ldo, num_heads, num_kv_heads, head_dim, ps, float(scale),
               int(window or 0), _stream())
         return
@@ -2095,7 +2117,7 @@ def paged_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, nu
             raise KernelError(f"paged_attention: the split-key kernel takes head sizes {_DECODE_HEAD_DIMS[q.dtype]} "
                               f"for {q.dtype}, not {head_dim}")
         # splits cover the longest context of the step, rounded up so that captured graphs keep their grid
-        max_splits = decode_splits(ctx.max_ctx_len)
+        max_splits = decode_splits(ctx.max_ctx_len if rows is None else ctx.max_single_ctx_len)
         # Up to DECODE_CLUSTER_SPLITS splits meet in a thread-block cluster and touch no scratch; only beyond that
         # (contexts over 1,024 tokens) or on request do the partial results go through global memory.  Asking for
         # the buffers only then keeps a growing context from ever replacing a buffer under the captured graphs.
@@ -2105,8 +2127,9 @@ def paged_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, nu
             counters = ctx.ws.zeroed("attn_counters", T * num_heads).data_ptr()     # the kernel leaves them zero
         else:
             part_o = part_ml = counters = None
-        _call("mllm_attention_decode", q.data_ptr(), ldq, k_pages.data_ptr(), v_pages.data_ptr(),
-              block_table.data_ptr(), bt_stride, ctx.token_seq.data_ptr(), ctx.positions.data_ptr(), out.data_ptr(),
+        _call("mllm_attention_decode_rows", q.data_ptr(), ldq, k_pages.data_ptr(), v_pages.data_ptr(),
+              block_table.data_ptr(), bt_stride, ctx.token_seq.data_ptr(), ctx.positions.data_ptr(),
+              rows.data_ptr() if rows is not None else None, out.data_ptr(),
               ldo, part_o, part_ml, counters, T, num_heads, num_kv_heads, head_dim, ps, float(scale),
               int(window or 0), max_splits, _dt(q), int(impl == "decode_scratch"), _stream())
         return

@@ -25,6 +25,7 @@ from .projected import ProjectedMixer
 
 class Attention(Mixer):
     accepts_lazy_norm = True
+    singles_apart = True         # in a step with prompt portions the single tokens take the decode kernel
 
     def __init__(self, hidden_size: int, num_heads: int, head_dim: int, scale: float,
                  num_kv_heads: Optional[int] = None, window: Optional[int] = None, bias: bool = True):
