@@ -99,6 +99,11 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int h = blockIdx.x, tile = blockIdx.y;
 
+    if (threadIdx.x == 32) {
+        prefetch_map(&map_q);
+        prefetch_map(&map_k);
+        prefetch_map(&map_v);
+    }
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
         for (int s = 0; s < STAGES; ++s) {

@@ -85,15 +85,6 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint4& a, const u
                  ::"r"(taddr), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w));
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-}
-
 // The plain sum of an element whose tensor-core sum is not finite.
 __device__ __noinline__ float plain_dot(const float* a, const float* w, int K) {
     float s = 0.f;
@@ -131,7 +122,12 @@ linear_split_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     const int nk = (K + BK - 1) / BK;
     const int my_tiles = (num_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;       // the grid has no more CTAs than tiles
     const int steps = my_tiles * nk;
+    if (threadIdx.x == 32) {
+        prefetch_map(&map_a);
+        if (tma_out) prefetch_map(&map_o);
+    }
     if (threadIdx.x == 0) {
+        prefetch_map(&map_w);
         for (int s = 0; s < 2; ++s) {
             mbar_init(&full[s], CUT_WARPS);
             mbar_init(&empty[s], 1);

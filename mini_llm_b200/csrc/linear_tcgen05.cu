@@ -85,7 +85,12 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int nk = (K + C::KB * BK - 1) / (C::KB * BK);       // stages per tile; k-blocks beyond K are zeros
 
+    if (threadIdx.x == 64) {
+        prefetch_map(&map_a);
+        if (tma_out) prefetch_map(&map_o);
+    }
     if (threadIdx.x == 0) {
+        prefetch_map(&map_w);
         for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], EPI_WARPS); }
         *failed = 0;
