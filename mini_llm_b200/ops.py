@@ -66,6 +66,12 @@ def _signatures(lib):
         "mllm_linear_stream_f32_tall_rows": [c_int, c_int],
         "mllm_linear_stream_f32_kernel_of": [c_int, c_int, c_int],
         "mllm_linear_stream_f32_bind_error": [c_void_p],
+        "mllm_linear_cluster": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int,
+                                c_int, c_void_p],
+        "mllm_linear_cluster_qkv": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_void_p,
+                                    c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
+        "mllm_linear_cluster_bind_error": [c_void_p],
+        "mllm_linear_cluster_error": [c_void_p],
         "mllm_linear_split_f32": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int,
                                   c_void_p],
         "mllm_linear_split_f32_qkv": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_void_p,
@@ -222,14 +228,16 @@ def _bind_error_word(lib) -> None:
         return
     word = torch.zeros(1, dtype=torch.int32).pin_memory()
     for name in ("mllm_tcgen05_bind_error", "mllm_attention_tcgen05_bind_error", "mllm_attention_decode_bind_error",
-                 "mllm_linear_stream_f32_bind_error", "mllm_linear_split_f32_bind_error"):
+                 "mllm_linear_stream_f32_bind_error", "mllm_linear_split_f32_bind_error",
+                 "mllm_linear_cluster_bind_error"):
         if getattr(lib, name)(word.data_ptr()) != 0:
             raise KernelError(lib.mllm_last_error().decode(errors="replace"))
     _error_word = word
 
 
 _WHO = {1: "the tcgen05 product", 2: "the tcgen05 attention", 3: "the decode attention",
-        4: "the float32 weight-streaming product", 5: "the float32 product of many rows"}
+        4: "the float32 weight-streaming product", 5: "the float32 product of many rows",
+        6: "the product of a decode batch"}
 
 
 def raise_if_kernel_gave_up() -> None:
@@ -333,6 +341,11 @@ def check_device_errors() -> None:
     if code.value:
         raise KernelError(f"the float32 product of many rows gave up waiting: code {code.value} "
                           "(1, 5 the cutting warps, 2-3 the MMA issuer, 4 the epilogue, 6 the TMA producer)")
+    if lib.mllm_linear_cluster_error(ctypes.byref(code)) != 0:
+        raise KernelError(lib.mllm_last_error().decode(errors="replace"))
+    if code.value:
+        raise KernelError(f"the product of a decode batch gave up waiting: code {code.value} "
+                          "(1 the TMA producer, 2 the MMA issuer, 3 the epilogue)")
 
 
 _stream_handle = None     # set by stream_scope(); None: ask torch on every call
@@ -614,6 +627,18 @@ def _small_m_wins(M: int, N: int, K: int) -> bool:
     return False
 
 
+def _cluster_wins(M: int, N: int, K: int) -> bool:
+    """Whether M rows of bfloat16 go to the kernel that cuts K over the CTAs of a cluster (csrc/linear_cluster.cu).
+    Measured in replayed chains at GPT-2 small's, medium's and XL's four products and 17 to 128 rows.  Long rows of W
+    (K = 4 x width), which the other kernels walk on few SMs, gain at every count (5 to 9 against 11 to 22 us).  With K =
+    width it wins up to 32 rows (3.7 to 9.5 against 4.1 to 14 us; 768 x 768 is a tie at 32); beyond, the exchange of the
+    sums, which grows with the rows, outweighs what the other kernel loses by using fewer SMs, except for narrow results
+    (1024 x 1024 and 1600 x 1600 at 64 rows 4.8 and 6.5 against 5.4 and 8.0 us, 768 x 768 6.0 against 4.6)."""
+    if not 16 < M <= 128 or N >= 16384 or K < 512:
+        return False
+    return M <= 32 or K >= 2048 or (M <= 64 and 1024 <= N <= K)
+
+
 def _fusable(weight, M, K) -> bool:
     return weight.dtype == torch.bfloat16 and M <= SMALL_M and K % 8 == 0 and weight.data_ptr() % 16 == 0
 
@@ -732,6 +757,15 @@ def linear_qkv_cache(x, weight, bias, q_out, k_pages, v_pages, slot_mapping, ws)
             return q_out
     if norm is not None and not _norm_ok(norm):
         x, norm = norm.materialize(), None
+    if (norm is None and q_out.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and _cluster_wins(M, N, K)
+            and x.is_cuda and x.dtype == torch.bfloat16 and K % 8 == 0 and weight.data_ptr() % 16 == 0
+            and _rows("x", x) % 8 == 0 and x.data_ptr() % 16 == 0 and k_pages.is_contiguous() and v_pages.is_contiguous()):
+        if bias is not None:
+            _cuda("bias", bias, torch.float32)
+        _call("mllm_linear_cluster_qkv", x.data_ptr(), _rows("x", x), weight.data_ptr(),
+              bias.data_ptr() if bias is not None else None, q_out.data_ptr(), _rows("q_out", q_out), M, N, K,
+              k_pages.data_ptr(), v_pages.data_ptr(), slot_mapping.data_ptr(), q_size, Hkv, dh, ps, _stream())
+        return q_out
     if q_out.dtype == torch.bfloat16 and _fusable(weight, M, K) and _small_m_wins(M, N, K) and (
             _norm_ok(norm) if norm is not None else
             (x.is_cuda and x.dtype == torch.bfloat16 and _rows("x", x) % 8 == 0 and x.data_ptr() % 16 == 0)):
@@ -821,7 +855,7 @@ def linear(x, weight, bias, out, act: Optional[str] = None, accumulate: bool = F
         impl = "simt"
         if x.dtype == torch.bfloat16 and K % 8 == 0 and lda % 8 == 0 \
                 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0:
-            impl = "smallm" if _small_m_wins(M, N, K) else "tcgen05"
+            impl = "cluster" if _cluster_wins(M, N, K) else "smallm" if _small_m_wins(M, N, K) else "tcgen05"
         elif x.dtype == torch.float32 and out.dtype == torch.float32 and _stream_f32_ok(weight, M, K) \
                 and lda % 4 == 0 and x.data_ptr() % 16 == 0:
             impl = "stream_f32"
@@ -836,7 +870,7 @@ def linear(x, weight, bias, out, act: Optional[str] = None, accumulate: bool = F
         _call("mllm_linear_split_f32", x.data_ptr(), lda, weight.data_ptr(), bias.data_ptr() if bias is not None else None,
               out.data_ptr(), ldo, M, N, K, _ACT[act], int(accumulate), _stream())
         return out
-    if impl in ("smallm", "tcgen05"):
+    if impl in ("smallm", "tcgen05", "cluster"):
         _call("mllm_linear_" + impl, x.data_ptr(), lda, weight.data_ptr(),
               bias.data_ptr() if bias is not None else None, out.data_ptr(), ldo, M, N, K, _ACT[act],
               int(accumulate), _dt(out), _stream())

@@ -455,6 +455,53 @@ def test_linear_many_rows_float32_in_k_slices(ops, M, N, K):
         assert torch.equal(part, full[lo:hi]), (lo, hi)
 
 
+@pytest.mark.parametrize("M,N,K", [(17, 768, 768), (24, 1600, 6400), (32, 4800, 1600), (33, 1, 512), (64, 3072, 768),
+                                   (64, 768, 3072), (65, 2304, 768), (77, 127, 520), (128, 6400, 1600), (1, 129, 4096), (20, 300, 64)])
+def test_linear_of_a_decode_batch_in_cluster_slices(ops, M, N, K):
+    """The bfloat16 product that cuts K over the CTAs of a cluster: both result types, every epilogue and unaligned result
+    rows against float64; a row's bits do not depend on the rows beside it; the fused cache write is the plain product's
+    columns, and a negative slot stores nothing."""
+    dt = torch.bfloat16
+    x, w, b = rnd(M, K, seed=1, dtype=dt), rnd(N, K, seed=2, scale=K ** -0.5, dtype=dt), rnd(N, seed=3)
+    ref = x.double() @ w.double().t()
+    for act in (None, "gelu_tanh", "gelu_erf"):
+        want = ref + b.double()
+        want = want if act is None else torch.nn.functional.gelu(want, approximate="tanh" if act == "gelu_tanh" else "none")
+        for out_dtype, tol in ((torch.float32, 2e-5), (dt, 2 ** -8)):
+            big = torch.full((M, N + 3), 7.0, device=DEV, dtype=out_dtype)
+            ops.linear(x, w, b, out=big[:, :N], act=act, impl="cluster")
+            assert ((big[:, :N].double() - want).abs() / want.abs().clamp(min=1.0)).max() < tol
+            assert torch.all(big[:, N:] == 7.0)
+    full = torch.empty(M, N, device=DEV)
+    ops.linear(x, w, None, out=full, impl="cluster")
+    acc = rnd(M, N, seed=4)
+    acc0 = acc.clone()
+    wide = torch.zeros(M, K + 16, device=DEV, dtype=dt)
+    wide[:, 8:8 + K] = x
+    ops.linear(wide[:, 8:8 + K], w, None, out=acc, accumulate=True, impl="cluster")
+    assert torch.equal(acc, acc0 + full)
+    for lo, hi in ((0, 1), (M // 2, M), (max(0, M - 17), M)):
+        part = torch.empty(hi - lo, N, device=DEV)
+        ops.linear(x[lo:hi], w, None, out=part, impl="cluster")
+        assert torch.equal(part, full[lo:hi]), (lo, hi)
+    if ops._cluster_wins(M, N, K):
+        auto = torch.empty(M, N, device=DEV)
+        ops.linear(x, w, None, out=auto)
+        assert torch.equal(auto, full)
+    if ops._cluster_wins(M, N, K) and N % 96 == 0:
+        from mini_llm_b200.engine.context import Workspace
+        H, dh, page = N // 96, 32, 16
+        slots = torch.randperm(256, generator=torch.Generator().manual_seed(5))[:M].to(torch.int32).to(DEV)
+        qkv = torch.empty(M, N, device=DEV, dtype=dt)
+        ops.linear(x, w, b, out=qkv, impl="cluster")
+        wk, wv, gk, gv = (torch.full((16, H, page, dh), 9.0, device=DEV, dtype=dt) for _ in range(4))
+        ops.kv_write(qkv[1:, H * dh:2 * H * dh], qkv[1:, 2 * H * dh:], wk, wv, slots[1:])
+        slots[0] = -1
+        q = ops.linear_qkv_cache(x, w, b, torch.empty(M, H * dh, device=DEV, dtype=dt), gk, gv, slots, Workspace(torch.device(DEV), 128))
+        assert torch.equal(q, qkv[:, :H * dh]) and torch.equal(gk, wk) and torch.equal(gv, wv)
+    ops.check_device_errors()
+
+
 @pytest.mark.parametrize("M,N,K", [(65, 64, 128), (128, 1, 132), (129, 191, 768), (300, 1003, 260), (2048, 768, 3072),
                                    (200, 2304, 768), (77, 50257, 192), (552, 1024, 4096)])
 def test_linear_float32_in_pieces_on_tensor_cores(ops, M, N, K):
