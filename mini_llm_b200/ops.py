@@ -91,6 +91,10 @@ def _signatures(lib):
         "mllm_attention_decode": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                   c_ll, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
                                   c_int, c_int, c_int, c_int, c_void_p],
+        "mllm_attention_split_f32": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p,
+                                     c_ll, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
+        "mllm_attention_split_f32_bind_error": [c_void_p],
+        "mllm_attention_split_f32_error": [c_void_p],
         "mllm_attention_decode_rows": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                        c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
                                        c_int, c_int, c_int, c_int, c_void_p],
@@ -229,7 +233,7 @@ def _bind_error_word(lib) -> None:
     word = torch.zeros(1, dtype=torch.int32).pin_memory()
     for name in ("mllm_tcgen05_bind_error", "mllm_attention_tcgen05_bind_error", "mllm_attention_decode_bind_error",
                  "mllm_linear_stream_f32_bind_error", "mllm_linear_split_f32_bind_error",
-                 "mllm_linear_cluster_bind_error"):
+                 "mllm_linear_cluster_bind_error", "mllm_attention_split_f32_bind_error"):
         if getattr(lib, name)(word.data_ptr()) != 0:
             raise KernelError(lib.mllm_last_error().decode(errors="replace"))
     _error_word = word
@@ -237,7 +241,7 @@ def _bind_error_word(lib) -> None:
 
 _WHO = {1: "the tcgen05 product", 2: "the tcgen05 attention", 3: "the decode attention",
         4: "the float32 weight-streaming product", 5: "the float32 product of many rows",
-        6: "the product of a decode batch"}
+        6: "the product of a decode batch", 7: "the float32 prefill attention"}
 
 
 def raise_if_kernel_gave_up() -> None:
@@ -346,6 +350,11 @@ def check_device_errors() -> None:
     if code.value:
         raise KernelError(f"the product of a decode batch gave up waiting: code {code.value} "
                           "(1 the TMA producer, 2 the MMA issuer, 3 the epilogue)")
+    if lib.mllm_attention_split_f32_error(ctypes.byref(code)) != 0:
+        raise KernelError(lib.mllm_last_error().decode(errors="replace"))
+    if code.value:
+        raise KernelError(f"the float32 prefill attention gave up waiting: code {code.value} "
+                          "(1 the cutting warps, 2-5 the MMA issuer, 7-8 the softmax warps)")
 
 
 _stream_handle = None     # set by stream_scope(); None: ask torch on every call
@@ -2056,6 +2065,14 @@ def _tiled_wide_ok(q, head_dim, n_wide, tokens, ldq) -> bool:
             and ldq % (16 // q.element_size()) == 0 and q.data_ptr() % 16 == 0)
 
 
+def _attention_split_ok(q, k_pages, v_pages, out, head_dim, n_wide, ldq, ldo) -> bool:
+    """The float32 prefill attention on tensor cores (csrc/attention_split_f32.cu): heads of 64 and rows that can be read 16
+    bytes at a time.  It is ahead of both CUDA-core kernels from 20 tokens on (its header has the figures) and level below."""
+    return (q.dtype == torch.float32 and head_dim == 64 and n_wide > 0 and ldq % 4 == 0 and ldo % 4 == 0
+            and (q.data_ptr() | out.data_ptr() | k_pages.data_ptr() | v_pages.data_ptr()) % 16 == 0
+            and k_pages.is_contiguous() and v_pages.is_contiguous())
+
+
 def paged_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, num_kv_heads, head_dim, scale,
                     window=None, impl: Optional[str] = None) -> None:
     """Causal attention of the step's tokens over the cache.
@@ -2094,6 +2111,8 @@ def paged_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, nu
         elif q.dtype == torch.bfloat16 and head_dim in _FLASH_HEAD_DIMS and n_tiles > 0 \
                 and ldq % 8 == 0 and q.data_ptr() % 16 == 0 and ldo % 2 == 0:
             impl = "flash"
+        elif _attention_split_ok(q, k_pages, v_pages, out, head_dim, n_wide, ldq, ldo):
+            impl = "split_f32"      # float32 with heads of 64: 128 x 128 tiles on tensor cores
         elif _tiled_wide_ok(q, head_dim, n_wide, tokens, ldq):
             impl = "tiled_wide"     # float32 (or a head size of 48) and long portions: 128 x 128 tiles on CUDA cores
         elif n_tiles > 0:
@@ -2121,6 +2140,14 @@ def _attend(impl, q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ld
               block_table.data_ptr(), bt_stride, ctx.attn_tiles_wide.data_ptr(), int(n_wide),
               ctx.positions.data_ptr(), out.data_ptr(), ldo, num_heads, num_kv_heads, head_dim, ps, float(scale),
               int(window or 0), _dt(q), _stream())
+        return
+    if impl == "split_f32":
+        if not _attention_split_ok(q, k_pages, v_pages, out, head_dim, n_wide, ldq, ldo):
+            raise KernelError("paged_attention: split_f32 takes float32, head size 64, 16-byte aligned rows and a list of "
+                              "128-row tiles")
+        _call("mllm_attention_split_f32", q.data_ptr(), ldq, k_pages.data_ptr(), v_pages.data_ptr(),
+              block_table.data_ptr(), bt_stride, ctx.attn_tiles_wide.data_ptr(), int(n_wide), ctx.positions.data_ptr(),
+              out.data_ptr(), ldo, num_heads, num_kv_heads, head_dim, ps, float(scale), int(window or 0), _stream())
         return
     if impl == "tiled":
         _call("mllm_attention_tiled", q.data_ptr(), ldq, k_pages.data_ptr(), v_pages.data_ptr(),

@@ -907,6 +907,62 @@ def test_tiled_attention_mixed_batch(ops, dtype, H, Hkv, dh, page, window):
         assert torch.equal(part, whole[lo:hi]), (lo, hi)
 
 
+@pytest.mark.parametrize("H,Hkv,page,window", [(2, 2, 16, None), (6, 2, 8, None), (4, 1, 24, 37), (2, 2, 64, 200), (3, 3, 1, None)])
+def test_float32_attention_in_pieces_on_tensor_cores(ops, H, Hkv, page, window):
+    """The 32-bit prefill attention in exact bfloat16 pieces (heads of 64): portions of many lengths, any page size, against
+    float64 and no further from it than the CUDA-core kernel; the same queries cut differently give the same bits; with
+    infinities and NaN among keys and values the rows that see them come out as the plain kernel has them."""
+    from mini_llm_b200.engine.context import ATTN_TILE_WIDE, attention_tiles
+    dtype, dh = torch.float32, 64
+
+    def wide(ctx, q_lens, starts):
+        tiles = attention_tiles(q_lens, starts, ATTN_TILE_WIDE)
+        ctx.attn_tiles_wide, ctx.n_tiles_wide = torch.tensor(tiles, dtype=torch.int32, device=DEV), len(tiles) // 3
+        ctx.decode_only = False
+        return ctx
+
+    seqs = [(1, 1), (70, 1), (33, 33), (100, 7), (16, 2), (129, 129), (128, 128), (65, 65), (200, 63), (500, 300),
+            (256, 128), (191, 2), (640, 257)]
+    case = _paged_case(dtype, seqs, H, Hkv, dh, page, num_pages=2800 // page + 40, seed=H + page,
+                       sharp_key={5: [0, 64, 127, 128], 12: [383, 384, 600]})
+    ctx = wide(_ctx_for(case), [n for _, n in seqs], [c - n for c, n in seqs])
+    q, kp, vp, bt = case["q"].to(DEV), case["k_pages"].to(DEV), case["v_pages"].to(DEV), case["bt"].to(DEV)
+    kw = dict(num_heads=H, num_kv_heads=Hkv, head_dim=dh, scale=dh ** -0.5, window=window)
+    out, cores, plain = torch.full_like(q, 7.0), torch.empty_like(q), torch.empty_like(q)
+    ops.paged_attention(q, kp, vp, bt, ctx, out, impl="split_f32", **kw)
+    ops.paged_attention(q, kp, vp, bt, ctx, cores, impl="tiled_wide", **kw)
+    want = _attention_reference(case, H, Hkv, dh, dh ** -0.5, window, dtype).to(DEV)
+    assert ((out.double() - want).abs() / want.abs().clamp(min=1.0)).max() < 2e-5
+    err = [((o.double() - want).norm() / want.norm()).item() for o in (out, cores)]
+    assert err[0] <= err[1] * 1.05, err
+    auto = torch.empty_like(q)
+    before = ops.attention_launches.get("split_f32", 0)
+    ops.paged_attention(q, kp, vp, bt, ctx, auto, **kw)
+    assert torch.equal(auto, out) and ops.attention_launches.get("split_f32", 0) == before + 1
+    # the same bits for other cuts
+    c2 = _paged_case(dtype, [(300, 300)], H, Hkv, dh, page, num_pages=2800 // page + 40, seed=99)
+    q2, args2 = c2["q"].to(DEV), (c2["k_pages"].to(DEV), c2["v_pages"].to(DEV), c2["bt"].to(DEV))
+    whole = torch.empty_like(q2)
+    ops.paged_attention(q2, *args2, wide(_ctx_for(c2), [300], [0]), whole, impl="split_f32", **kw)
+    for lo, hi in ((0, 5), (5, 70), (70, 300), (100, 101), (127, 260)):
+        cb = wide(_Ctx(), [hi - lo], [lo])
+        cb.token_seq = torch.zeros(hi - lo, dtype=torch.int32, device=DEV)
+        cb.positions = torch.arange(lo, hi, dtype=torch.int32, device=DEV)
+        part = torch.empty_like(q2[lo:hi])
+        ops.paged_attention(q2[lo:hi], *args2, cb, part, impl="split_f32", **kw)
+        assert torch.equal(part, whole[lo:hi]), (lo, hi)
+    # values that have no pieces
+    kp[int(bt[9, 250 // page]), 0, 250 % page, 3] = float("inf")
+    vp[int(bt[12, 400 // page]), 0, 400 % page, 5] = -float("inf")
+    vp[int(bt[8, 150 // page]), 0, 150 % page, 60] = float("nan")
+    q[40, 1] = float("nan")
+    ops.paged_attention(q, kp, vp, bt, ctx, out, impl="split_f32", **kw)
+    ops.paged_attention(q, kp, vp, bt, ctx, plain, impl="simt", **kw)
+    assert torch.equal(out.isnan(), plain.isnan()) and torch.equal(out.isinf(), plain.isinf())
+    assert torch.allclose(out, plain, rtol=1e-4, atol=1e-5, equal_nan=True)
+    ops.check_device_errors()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H,Hkv,dh,page,window", [(2, 2, 64, 16, None), (12, 12, 64, 16, None), (6, 2, 32, 8, None), (3, 1, 48, 32, None),
                                                   (4, 4, 16, 4, None), (4, 1, 64, 16, 37), (2, 2, 64, 64, 200)])
