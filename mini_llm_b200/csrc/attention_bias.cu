@@ -22,7 +22,7 @@
 // Four kernels (the fourth, `mma`, is described where it stands).  `simt`: one warp per (token, head), 32 keys at a time: any step, and the plain twin of the
 // others.  `tiled`: 64 queries x 32 keys per CTA and head for prompt portions: queries in shared memory, a key
 // tile staged transposed and a value tile as it is, 2 x 4 scores and 2 x dv/8 outputs per thread.  `split`: single
-// tokens (decode): the keys of a token are cut into splits of 256 starting at multiples of 256 from position 0, a
+// tokens (decode): the keys of a token are cut into splits of 64 starting at multiples of 64 from position 0, a
 // CTA takes one split for up to four query heads that share a key/value head (rows staged once in shared memory),
 // the partial (o, m, l) of the splits are merged in split order by a second kernel.  Key chunks and tiles start at multiples of 32 from position 0 in all three, so a token's
 // sums run in an order that depends on its position only, not on how the step was cut or batched.
@@ -177,7 +177,9 @@ attention_bias_simt_kernel(const T* q, long long q_stride, const T* k_pages, con
 }
 
 // ------------------------------------------------------------------------------------------------ decode
-constexpr int SPLIT = 256;          // keys per split
+// keys per split: with 256 a launch at 4 requests and contexts of 510 took 23.5 us on 32 CTAs that each met the latency of
+// their loads four times; with 64 it takes 11.0 (at 64 requests 75 us either way; the merge 4 us either way)
+constexpr int SPLIT = 64;
 
 // Single tokens.  grid (splits, kv heads x head chunks, tokens).  A CTA takes one split of one token's keys for HG
 // (1, 2 or 4) query heads that share a key/value head, so a key or value row is fetched once for all of them.  The
@@ -202,9 +204,10 @@ attention_bias_split_kernel(const T* q, long long q_stride, const T* k_pages, co
     float* qs = reinterpret_cast<float*>(Vs + (((size_t)tile * dv + VEC - 1) / VEC) * VEC);   // [HG][dk]
     float* so = qs + HG * dk;                                   // [warps][dv] at the end
     float* sml = so + 4 * dv;                                   // [warps][2]
+    const int split = blockIdx.x, nsplit = gridDim.x, t = blockIdx.z;
+    const int seq = __ldcg(token_seq + t), p = __ldcg(positions + t);        // written by the host before the step
     pdl_wait();
     pdl_launch();
-    const int split = blockIdx.x, nsplit = gridDim.x, t = blockIdx.z;
     const int R = H / Hkv, chunks = (R + HG - 1) / HG;
     const int hk = blockIdx.y / chunks, h0 = hk * R + (blockIdx.y % chunks) * HG;
     const int nh = min(HG, hk * R + R - h0);                    // heads this CTA really has
@@ -212,7 +215,6 @@ attention_bias_split_kernel(const T* q, long long q_stride, const T* k_pages, co
     const int wh = warp % HG, wk = warp / HG;                   // this warp's head and key sub-tile
     const int h = h0 + wh;
     const bool live = wh < nh;
-    const int seq = token_seq[t], p = positions[t];
     const int first = first_visible(a, p);
     const int s_lo = split * SPLIT < a.keep ? split * SPLIT : max(first, split * SPLIT), s_hi = min(p, split * SPLIT + SPLIT - 1);
     if (s_lo > s_hi) {                                          // uniform over the CTA
@@ -238,39 +240,32 @@ attention_bias_split_kernel(const T* q, long long q_stride, const T* k_pages, co
     for (int base = (s_lo / tile) * tile; base <= s_hi; base += tile) {
         if (in_gap(a, base, base + tile - 1, first)) continue;  // uniform over the CTA
         __syncthreads();                                        // the tile before is no longer read; qs is complete
+        // the loads of a burst of keys and a burst of values are all in flight before the first is stored
         constexpr int LD = 4;
-        for (int i0 = tid; i0 < tile * kpieces; i0 += nthreads * LD) {
-            uint4 r[LD];
-#pragma unroll
-            for (int u = 0; u < LD; ++u) {
-                const int i = i0 + u * nthreads, key = i / kpieces, piece = i % kpieces, kp = base + key;
-                r[u] = make_uint4(0u, 0u, 0u, 0u);
-                if (i < tile * kpieces && kp >= s_lo && kp <= s_hi && sees(a, kp, first))
-                    r[u] = *reinterpret_cast<const uint4*>(k_pages + (((size_t)bt[kp / page_size] * Hkv + hk) * page_size + kp % page_size) * dk + piece * VEC);
-            }
-#pragma unroll
-            for (int u = 0; u < LD; ++u) {
-                const int i = i0 + u * nthreads;
-                if (i < tile * kpieces) *reinterpret_cast<uint4*>(Ks + (size_t)(i / kpieces) * krow + (i % kpieces) * VEC) = r[u];
-            }
-        }
-        if (vpieces) {
-            for (int i0 = tid; i0 < tile * vpieces; i0 += nthreads * LD) {
-                uint4 r[LD];
-#pragma unroll
-                for (int u = 0; u < LD; ++u) {
-                    const int i = i0 + u * nthreads, key = i / vpieces, piece = i % vpieces, kp = base + key;
-                    r[u] = make_uint4(0u, 0u, 0u, 0u);
-                    if (i < tile * vpieces && kp >= s_lo && kp <= s_hi && sees(a, kp, first))
-                        r[u] = *reinterpret_cast<const uint4*>(v_pages + (((size_t)bt[kp / page_size] * Hkv + hk) * page_size + kp % page_size) * dv + piece * VEC);
-                }
+        const int nkp = tile * kpieces, nvp = tile * vpieces;
+        for (int i0 = tid; i0 < max(nkp, nvp); i0 += nthreads * LD) {
+            uint4 rk[LD], rv[LD];
+            auto fetch = [&](const T* pages, int pieces, int width, int n, uint4 (&r)[LD]) {
 #pragma unroll
                 for (int u = 0; u < LD; ++u) {
                     const int i = i0 + u * nthreads;
-                    if (i < tile * vpieces) *reinterpret_cast<uint4*>(Vs + (size_t)(i / vpieces) * dv + (i % vpieces) * VEC) = r[u];
+                    r[u] = make_uint4(0u, 0u, 0u, 0u);
+                    if (i >= n) continue;
+                    const int key = i / pieces, piece = i % pieces, kp = base + key;
+                    if (kp >= s_lo && kp <= s_hi && sees(a, kp, first))
+                        r[u] = *reinterpret_cast<const uint4*>(pages + (((size_t)bt[kp / page_size] * Hkv + hk) * page_size + kp % page_size) * width + piece * VEC);
                 }
+            };
+            fetch(k_pages, kpieces, dk, nkp, rk);
+            fetch(v_pages, vpieces, dv, nvp, rv);
+#pragma unroll
+            for (int u = 0; u < LD; ++u) {
+                const int i = i0 + u * nthreads;
+                if (i < nkp) *reinterpret_cast<uint4*>(Ks + (size_t)(i / kpieces) * krow + (i % kpieces) * VEC) = rk[u];
+                if (i < nvp) *reinterpret_cast<uint4*>(Vs + (size_t)(i / vpieces) * dv + (i % vpieces) * VEC) = rv[u];
             }
-        } else {
+        }
+        if (!vpieces) {
             for (int i = tid; i < tile * dv; i += nthreads) {
                 const int key = i / dv, d = i % dv, kp = base + key;
                 T val = from_f32<T>(0.f);
@@ -362,32 +357,45 @@ __global__ void __launch_bounds__(WARPS * 32)
 attention_bias_merge_kernel(const float* part_o, const float* part_ml, const int* __restrict__ positions,
                             T* __restrict__ out, long long out_stride, int T_tokens, int H, int dv, int nsplit,
                             BiasArgs a) {
-    pdl_wait();
-    pdl_launch();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long gw = (long long)blockIdx.x * WARPS + warp;
     if (gw >= (long long)T_tokens * H) return;
     const int t = (int)(gw / H), h = (int)(gw % H);
+    const int used = min(nsplit, __ldcg(positions + t) / SPLIT + 1);         // positions: written by the host before the step
     const float* sink = a.sink;
-    const int used = min(nsplit, positions[t] / SPLIT + 1);
+    const float sk = sink ? sink[h] : -INFINITY;
+    pdl_wait();
+    pdl_launch();
     const size_t base = ((size_t)t * H + h) * nsplit;
-    float mm = sink ? sink[h] : -INFINITY;
-    for (int s = 0; s < used; ++s)
-        if (part_ml[(base + s) * 2 + 1] > 0.f) mm = fmaxf(mm, part_ml[(base + s) * 2]);
-    float ll = sink ? expf(sink[h] - mm) : 0.f;              // the sink's term, taken before the splits'
-    constexpr int NACC = MAX_D / 32;
+    // a lane takes a split's maximum and sum, 32 splits at a time; the weighted sum walks the splits in order, its loads
+    // eight splits at a time and ahead of the weights
+    float mm = sk;
+    for (int s = lane; s - lane < used; s += 32)
+        mm = fmaxf(mm, warp_max(s < used && part_ml[(base + s) * 2 + 1] > 0.f ? part_ml[(base + s) * 2] : -INFINITY));
+    float ll = sink ? expf(sk - mm) : 0.f;                   // the sink's term, taken before the splits'
+    constexpr int NACC = MAX_D / 32, U = 8;
     float acc[NACC];
 #pragma unroll
     for (int i = 0; i < NACC; ++i) acc[i] = 0.f;
-    for (int s = 0; s < used; ++s) {
-        const float ls = part_ml[(base + s) * 2 + 1];
-        if (!(ls > 0.f)) continue;
-        const float f = expf(part_ml[(base + s) * 2] - mm);
-        ll += ls * f;
+    for (int s0 = 0; s0 < used; s0 += U) {
+        const int n = min(U, used - s0);
+        float v[U][NACC];
 #pragma unroll
-        for (int i = 0; i < NACC; ++i) {
-            const int d = lane + 32 * i;
-            if (d < dv) acc[i] = fmaf(part_o[(base + s) * dv + d], f, acc[i]);
+        for (int s = 0; s < U; ++s)
+#pragma unroll
+            for (int i = 0; i < NACC; ++i) {
+                const int d = lane + 32 * i;
+                v[s][i] = s < n && d < dv ? part_o[(base + s0 + s) * dv + d] : 0.f;
+            }
+        const float l_mine = lane < n ? part_ml[(base + s0 + lane) * 2 + 1] : 0.f;
+        const float f_mine = l_mine > 0.f ? expf(part_ml[(base + s0 + lane) * 2] - mm) : 0.f;
+#pragma unroll
+        for (int s = 0; s < U; ++s) {
+            const float ls = __shfl_sync(0xffffffffu, l_mine, s), f = __shfl_sync(0xffffffffu, f_mine, s);
+            if (!(ls > 0.f)) continue;                       // a split without visible keys left no sums
+            ll += ls * f;
+#pragma unroll
+            for (int i = 0; i < NACC; ++i) acc[i] = fmaf(v[s][i], f, acc[i]);
         }
     }
     T* orow = out + (size_t)t * out_stride + (size_t)h * dv;
@@ -915,7 +923,7 @@ MLLM_EXPORT int mllm_attention_bias(const void* q, long long q_stride, const voi
             return tile * (dk + vec) * es + ((tile * dv + vec - 1) / vec) * vec * es + sizeof(float) * ((size_t)HG * dk + 4 * (size_t)dv + 8);
         };
         while (KS > 1 && bytes(KS) > 96 * 1024) KS /= 2;
-        // A whole split of 256 keys staged at once (one round of loads instead of up to eight) where it fits and the grid
+        // A whole split staged at once (one round of loads) where it fits and the grid
         // is small: with few CTAs nothing else hides the loads' latency.  In a large grid (measured at batch 64: 0.57
         // against 0.71 ms per step) small tiles win, since more CTAs fit an SM and hide each other's loads.  A warp
         // walks the same chunks in the same order either way, so the result is the same bits.

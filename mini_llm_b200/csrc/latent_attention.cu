@@ -305,24 +305,43 @@ latent_attention_kernel(const float* qa, const T* pages, int row, const int* blo
     }
 }
 
-// One warp per (token, head): out = sum_s o_s e^(m_s - M) / (e^(sink - M) + sum_s l_s e^(m_s - M)) over the token's splits.
-__global__ void __launch_bounds__(256)
-latent_merge_kernel(const float* part_o, const float* part_ml, const int* positions, float* out, int nsplit, int TH, int H,
-                    int R, int span, const float* __restrict__ sink) {
+// One CTA per (token, head): out = sum_s o_s e^(m_s - M) / (e^(sink - M) + sum_s l_s e^(m_s - M)) over the token's splits,
+// in split order.  Every thread takes the maxima and weights for itself (the same addresses in all of them), then a column
+// of the sum at a time.  With a warp per (token, head) the twelve columns of a lane stood one after the other.
+__global__ void __launch_bounds__(128)
+latent_merge_kernel(const float* part_o, const float* part_ml, const int* positions, float* out, int nsplit, int H, int R,
+                    int span, const float* __restrict__ sink) {
+    __shared__ float wgt[128];                               // the weights of 128 splits at a time
     pdl_wait();
-    const int th = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (th >= TH) return;
+    const int th = blockIdx.x, tid = threadIdx.x;
     const int ns = positions[th / H] / span + 1;
     const size_t o = (size_t)th * nsplit;
-    float M = sink ? sink[th % H] : -INFINITY;
+    const float sk = sink ? sink[th % H] : -INFINITY;
+    float M = sk;
+#pragma unroll 8
     for (int s = 0; s < ns; ++s) M = fmaxf(M, part_ml[(o + s) * 2]);
-    float L = sink ? expf(sink[th % H] - M) : 0.f;
-    for (int s = 0; s < ns; ++s) L += part_ml[(o + s) * 2 + 1] * expf(part_ml[(o + s) * 2] - M);
-    for (int d = lane; d < R; d += 32) {
-        float a = 0.f;
-        for (int s = 0; s < ns; ++s) a = fmaf(part_o[(o + s) * R + d], expf(part_ml[(o + s) * 2] - M), a);
-        out[(size_t)th * R + d] = a / L;
+    float L = sink ? expf(sk - M) : 0.f;
+    constexpr int COLS = MAX_R / 128;
+    float a[COLS];
+#pragma unroll
+    for (int i = 0; i < COLS; ++i) a[i] = 0.f;
+    for (int s0 = 0; s0 < ns; s0 += 128) {
+        const int n = min(128, ns - s0);
+        __syncthreads();
+        if (tid < n) wgt[tid] = expf(part_ml[(o + s0 + tid) * 2] - M);
+        __syncthreads();
+#pragma unroll 4
+        for (int s = 0; s < n; ++s) {
+            const float w = wgt[s];
+            L = fmaf(part_ml[(o + s0 + s) * 2 + 1], w, L);
+#pragma unroll
+            for (int i = 0; i < COLS; ++i)
+                if (tid + i * 128 < R) a[i] = fmaf(part_o[(o + s0 + s) * R + tid + i * 128], w, a[i]);
+        }
     }
+#pragma unroll
+    for (int i = 0; i < COLS; ++i)
+        if (tid + i * 128 < R) out[(size_t)th * R + tid + i * 128] = a[i] / L;
 }
 
 template <typename T, int NACC>
@@ -331,7 +350,7 @@ int launch_attention(const float* qa, const void* pages, int row, const int* bt,
                      int ps, float scale, int span, cudaStream_t stream) {
     const int kw = row * (int)sizeof(T) / 4 + 4;
     const int V = 16 / (int)sizeof(T), dkp = (dk + V - 1) / V * V;
-    const size_t smem = (size_t)HB * dkp * 4 + (size_t)2 * 32 * kw * 4;
+    const size_t smem = (size_t)HB * dkp * 4 + (size_t)(span > 32 ? 2 : 1) * 32 * kw * 4;      // a split of one chunk needs one buffer
     static bool raised = false;                     // once per instantiation
     if (smem > 48 * 1024 && !raised) {
         MLLM_CUDA(cudaFuncSetAttribute(latent_attention_kernel<T, NACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
@@ -801,8 +820,8 @@ MLLM_EXPORT int mllm_latent_attention(const float* qa, const void* pages, int ro
     else
         return mllm_fail(1, "latent_attention: unknown dtype code %d", dtype);
     if (rc) return rc;
-    MLLM_CUDA(mllm_launch(latent_merge_kernel, dim3((Tn * H + 7) / 8), dim3(256), 0, stream, true, part_o, part_ml, positions,
-                          out, nsplit, Tn * H, H, R, span, sink));
+    MLLM_CUDA(mllm_launch(latent_merge_kernel, dim3(Tn * H), dim3(128), 0, stream, true, part_o, part_ml, positions, out, nsplit,
+                          H, R, span, sink));
     return 0;
 }
 

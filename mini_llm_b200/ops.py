@@ -1060,9 +1060,8 @@ def biased_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, n
     if impl == "split":
         if _bias_split_keys is None:
             _bias_split_keys = int(library().mllm_attention_bias_split_keys())
-        # splits cover the longest context of the step, rounded up to a power of two so that captured graphs keep their grid
-        need = max(1, -(-int(ctx.max_ctx_len) // _bias_split_keys))
-        nsplit = 1 << (need - 1).bit_length()
+        # splits cover the longest context of the step as ``latent_splits`` rounds it (part of a step's shape for captured graphs)
+        nsplit = max(1, latent_splits(ctx.max_ctx_len) * LATENT_SPAN_DECODE // _bias_split_keys)
         part_o = ctx.ws.buf("battn_part_o", T * num_heads * nsplit, dv, torch.float32).data_ptr()
         part_ml = ctx.ws.buf("battn_part_ml", T * num_heads * nsplit, 2, torch.float32).data_ptr()
     elif impl in ("tiled", "mma"):
@@ -1493,8 +1492,10 @@ def wkv_finish(o, z, weight, out, *, heads: int, eps: float) -> None:
 # --------------------------------------------------------------------------- attention over a cache of latents
 LATENT_MAX_RANK, LATENT_MAX_KEY = 512, 1024      # what csrc/latent_attention.cu takes
 # keys per CTA of the CUDA-core kernel: short splits when a step has single tokens only (a few long contexts must fill
-# the GPU), long ones when it has prompt portions (their tokens fill it, and every split costs a partial result)
-LATENT_SPAN_DECODE, LATENT_SPAN_PROMPT = 128, 1024
+# the GPU), long ones when it has prompt portions (their tokens fill it, and every split costs a partial result).  Splits of
+# 32 instead of 128 keys: 13 against 42 us a launch at 3 requests and contexts of 250 (float32), 15 against 33 at 8 and 500
+# (bfloat16), 41 against 85 at 64 and 200 (float32), with 1 to 3 us more for the merge.
+LATENT_SPAN_DECODE, LATENT_SPAN_PROMPT = 32, 1024
 
 
 def latent_prepare(proj, q_off: int, dkv_off: Optional[int], ctx, slot_mapping, freq, mscale: float, norm_weight, eps: float,
