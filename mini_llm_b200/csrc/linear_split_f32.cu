@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 linear_split_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                         const __grid_constant__ CUtensorMap map_o, const float* A, long long lda,
                         const float* __restrict__ W, const float* __restrict__ bias, float* out, long long ldo, int M,
-                        int N, int K, int act, int accumulate, int tma_out, int tiles_n, int num_tiles, KvOut32 kv) {
+                        int N, int K, int act, int accumulate, int tma_out, int tiles_n, int num_items, int slices, KvOut32 kv) {
     using C = Cfg<BN>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* w_stages = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -91,9 +91,10 @@ linear_split_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     volatile int* failed = (volatile int*)(tmem_slot + 1);
 
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
-    const int nk = (K + BK - 1) / BK;
-    const int my_tiles = (num_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;       // the grid has no more CTAs than tiles
-    const int steps = my_tiles * nk;
+    // An item is a K slice of a tile (slices of whole blocks, all equally long: blocks beyond K are zeros).
+    const int nk = ((K + BK - 1) / BK + slices - 1) / slices;
+    const int my_items = (num_items - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;       // the grid has no more CTAs than items
+    const int steps = my_items * nk;
     if (threadIdx.x == 32) {
         prefetch_map(&map_a);
         if (tma_out) prefetch_map(&map_o);
@@ -190,13 +191,18 @@ linear_split_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         if (warp == TMA_WARP) {
             const int total = 2 * steps, pre = total < C::SLOTS ? total : C::SLOTS;
             // the half block that is brought next, counted up (a division per box would cost as much as its copy)
-            struct Next { int tile, m0, n0, k, slot; } w{(int)blockIdx.x, 0, 0, 0, 0};
-            const int k_end = nk * BK;
-            auto place = [&](Next& x) { x.m0 = (x.tile / tiles_n) * BM; x.n0 = (x.tile % tiles_n) * BN; };
+            struct Next { int item, m0, n0, k, k_end, slot; } w{(int)blockIdx.x, 0, 0, 0, 0, 0};
+            auto place = [&](Next& x) {
+                const int tile = x.item / slices;
+                x.m0 = (tile / tiles_n) * BM;
+                x.n0 = (tile % tiles_n) * BN;
+                x.k = (x.item % slices) * nk * BK;
+                x.k_end = x.k + nk * BK;
+            };
             auto step = [&](Next& x) {
                 if (++x.slot == C::SLOTS) x.slot = 0;
                 x.k += HK;
-                if (x.k == k_end) { x.k = 0; x.tile += gridDim.x; place(x); }
+                if (x.k == x.k_end) { x.item += gridDim.x; place(x); }
             };
             place(w);
             Next a = w;
@@ -257,7 +263,9 @@ linear_split_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         uint8_t* blk = epi + (size_t)(warp - CUT_WARPS) * 4096;
         int it = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+        const int slice_rows = (M + BM - 1) / BM * BM;     // slice z of the partial sums: rows z * slice_rows ... of `out`
+        for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+            const int tile = item / slices, slice = item % slices, k0 = slice * nk * BK;
             float acc[C::HALF];
 #pragma unroll
             for (int j = 0; j < C::HALF; ++j) acc[j] = 0.f;
@@ -295,7 +303,7 @@ linear_split_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 #pragma unroll
                     for (int j = 0; j < 32; ++j)
                         if (!(fabsf(v[j]) <= 3.402823466e38f) && n0 + j < N)
-                            v[j] = plain_dot(A + (size_t)row * lda, W + (size_t)(n0 + j) * K, K);
+                            v[j] = plain_dot(A + (size_t)row * lda + k0, W + (size_t)(n0 + j) * K + k0, min(K - k0, nk * BK));
                 }
                 __syncwarp();
                 if (bias) {
@@ -337,7 +345,7 @@ linear_split_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                     __syncwarp();
                     if (lane == 0) {
                         if (accumulate) tma_reduce_add_2d(&map_o, n0, row0, blk);
-                        else tma_store_2d(&map_o, n0, row0, blk);
+                        else tma_store_2d(&map_o, n0, slice * slice_rows + row0, blk);
                         bulk_commit();
                     }
                 } else {                                        // rows that are not 16-byte aligned: lane = column
@@ -369,6 +377,37 @@ linear_split_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     }
 }
 
+// out = act(ws[0] + ws[1] + ... + bias) (+ out): the K slices of the kernel above, added in slice order, four columns per
+// thread.
+__global__ void __launch_bounds__(256)
+linear_split_f32_finish_kernel(const float* ws, int slices, size_t slice_floats, const float* __restrict__ bias, float* out,
+                               long long ldo, int M, int N, int act, int accumulate, int vec) {
+    const int n4 = N / 4, total = M * n4;
+    pdl_wait();
+    pdl_launch();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const int m = i / n4, n = (i - m * n4) * 4;
+        float* o = out + (size_t)m * ldo + n;
+        float4 old = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (accumulate) old = vec ? *reinterpret_cast<const float4*>(o) : make_float4(o[0], o[1], o[2], o[3]);
+        const float4 b = bias ? make_float4(__ldg(bias + n), __ldg(bias + n + 1), __ldg(bias + n + 2), __ldg(bias + n + 3))
+                              : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float* p = ws + (size_t)m * N + n;
+        float4 v = __ldcg(reinterpret_cast<const float4*>(p));
+#pragma unroll 3
+        for (int z = 1; z < slices; ++z) {
+            const float4 x = __ldcg(reinterpret_cast<const float4*>(p + (size_t)z * slice_floats));
+            v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+        }
+        v.x = apply_act(v.x + b.x, act) + old.x;
+        v.y = apply_act(v.y + b.y, act) + old.y;
+        v.z = apply_act(v.z + b.z, act) + old.z;
+        v.w = apply_act(v.w + b.w, act) + old.w;
+        if (vec) *reinterpret_cast<float4*>(o) = v;
+        else { o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; }
+    }
+}
+
 int sm_count() {
     static int n = 0;
     if (!n) {
@@ -379,47 +418,61 @@ int sm_count() {
     return n;
 }
 
+// K slices, from N and K alone: a narrow result has few tiles (12 to 96 for 768 columns and 77 to 2,048 rows), each of
+// which walked all of K on its SM.  SLICES_NOTE
+int slices_for(int N, int K) { return N <= 1024 && N % 4 == 0 && K >= 512 ? 3 : 1; }
+
 template <int BN>
 int launch(const float* A, long long lda, const float* W, const float* bias, float* out, long long ldo, int M, int N,
-           int K, int act, int accumulate, const KvOut32& kv, cudaStream_t stream) {
+           int K, int act, int accumulate, float* ws, int slices, const KvOut32& kv, cudaStream_t stream) {
     using C = Cfg<BN>;
     CUtensorMap ma, mw, mo = {};
     int rc = get_map(A, lda, M, K, HK, BM, MAP_F32_SW128, &ma);
     if (rc) return rc;
     rc = get_map(W, K, N, K, HK, BN, MAP_F32_SW128, &mw);
     if (rc) return rc;
-    const int tma_out = (uintptr_t)out % 16 == 0 && ldo % 4 == 0;
-    if (tma_out) {
-        rc = get_map(out, ldo, M, kv.k_pages ? kv.q_size : N, 32, 32, MAP_F32_SW128, &mo);
-        if (rc) return rc;
-    }
+    const int tiles_n = (N + BN - 1) / BN, tiles_m = (M + BM - 1) / BM;
+    const int vec = (uintptr_t)out % 16 == 0 && ldo % 4 == 0, tma_out = slices > 1 || vec;
+    if (slices > 1) rc = get_map(ws, N, slices * tiles_m * BM, N, 32, 32, MAP_F32_SW128, &mo);
+    else if (tma_out) rc = get_map(out, ldo, M, kv.k_pages ? kv.q_size : N, 32, 32, MAP_F32_SW128, &mo);
+    if (rc) return rc;
     auto kern = linear_split_f32_kernel<BN>;
     static bool set = false;
     if (!set) {
         MLLM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
         set = true;
     }
-    const int tiles_n = (N + BN - 1) / BN, num_tiles = tiles_n * ((M + BM - 1) / BM);
-    const int grid = num_tiles < sm_count() ? num_tiles : sm_count();
-    MLLM_CUDA(mllm_launch(kern, dim3(grid), dim3(THREADS), C::SMEM, stream, true, ma, mw, mo, A, lda, W, bias, out, ldo, M, N, K,
-                          act, accumulate, tma_out, tiles_n, num_tiles, kv));
+    const int items = tiles_n * tiles_m * slices, grid = items < sm_count() ? items : sm_count();
+    if (slices == 1) {
+        MLLM_CUDA(mllm_launch(kern, dim3(grid), dim3(THREADS), C::SMEM, stream, true, ma, mw, mo, A, lda, W, bias, out, ldo, M, N,
+                              K, act, accumulate, tma_out, tiles_n, items, 1, kv));
+        return 0;
+    }
+    MLLM_CUDA(mllm_launch(kern, dim3(grid), dim3(THREADS), C::SMEM, stream, true, ma, mw, mo, A, lda, W, (const float*)nullptr, ws,
+                          (long long)N, M, N, K, (int)MLLM_ACT_NONE, 0, tma_out, tiles_n, items, slices, kv));
+    const long long quads = (long long)M * N / 4;
+    MLLM_CUDA(mllm_launch(linear_split_f32_finish_kernel, dim3((unsigned)((quads + 255) / 256)), dim3(256), 0, stream, true,
+                          (const float*)ws, slices, (size_t)tiles_m * BM * N, bias, out, ldo, M, N, act, accumulate, vec));
     return 0;
 }
 
 int go(const float* A, long long lda, const float* W, const float* bias, float* out, long long ldo, int M, int N, int K,
-       int act, int accumulate, const KvOut32& kv, cudaStream_t stream) {
+       int act, int accumulate, float* ws, long long ws_floats, const KvOut32& kv, cudaStream_t stream) {
     if (K <= 0 || K % 4 != 0 || lda % 4 != 0)
         return mllm_fail(1, "linear_split_f32: K=%d and the row stride %lld must be multiples of 4", K, lda);
     if ((uintptr_t)A % 16 != 0 || (uintptr_t)W % 16 != 0)
         return mllm_fail(1, "linear_split_f32: operands must be 16-byte aligned");
     const long long tiles_m = (M + BM - 1) / BM;
     if (tiles_m * ((N + 63) / 64) > 0x7fffffffLL) return mllm_fail(1, "linear_split_f32: M=%d, N=%d exceed the grid limit", M, N);
+    int slices = ws && !kv.k_pages ? slices_for(N, K) : 1;
+    if (slices > 1 && (slices * tiles_m * BM * N > ws_floats || (uintptr_t)ws % 16 != 0 || (long long)M * N > 0x3fffffffLL))
+        return mllm_fail(1, "linear_split_f32: %lld floats of scratch for %d slices of %d x %d", ws_floats, slices, M, N);
     // A 64-wide tile takes about three quarters of a 128-wide one's time (1.08 against 1.45 us per block of 64: what
     // W costs halves, the cutting of A stays).
-    const long long r128 = (tiles_m * ((N + 127) / 128) + sm_count() - 1) / sm_count();
-    const long long r64 = (tiles_m * ((N + 63) / 64) + sm_count() - 1) / sm_count();
-    if (r64 * 3 < r128 * 4) return launch<64>(A, lda, W, bias, out, ldo, M, N, K, act, accumulate, kv, stream);
-    return launch<128>(A, lda, W, bias, out, ldo, M, N, K, act, accumulate, kv, stream);
+    const long long r128 = (tiles_m * ((N + 127) / 128) * slices + sm_count() - 1) / sm_count();
+    const long long r64 = (tiles_m * ((N + 63) / 64) * slices + sm_count() - 1) / sm_count();
+    if (r64 * 3 < r128 * 4) return launch<64>(A, lda, W, bias, out, ldo, M, N, K, act, accumulate, ws, slices, kv, stream);
+    return launch<128>(A, lda, W, bias, out, ldo, M, N, K, act, accumulate, ws, slices, kv, stream);
 }
 
 }  // namespace
@@ -435,11 +488,16 @@ MLLM_EXPORT int mllm_linear_split_f32_error(int* code) {
     return 0;
 }
 
-// 32-bit A [M,K] (row stride lda), W [N,K] and out; K and lda multiples of 4, A and W 16-byte aligned.
+// K slices that mllm_linear_split_f32 uses (1: no scratch needed, no second kernel).
+MLLM_EXPORT int mllm_linear_split_f32_slices(int N, int K) { return slices_for(N, K); }
+
+// 32-bit A [M,K] (row stride lda), W [N,K] and out; K and lda multiples of 4, A and W 16-byte aligned.  ws: room for the
+// partial sums, slices * (M rounded up to 128) * N floats, 16-byte aligned (null: no slices).
 MLLM_EXPORT int mllm_linear_split_f32(const float* A, long long lda, const float* W, const float* bias, float* out,
-                                      long long ldo, int M, int N, int K, int act, int accumulate, cudaStream_t stream) {
+                                      long long ldo, int M, int N, int K, int act, int accumulate, float* ws,
+                                      long long ws_floats, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
-    return go(A, lda, W, bias, out, ldo, M, N, K, act, accumulate, KvOut32{}, stream);
+    return go(A, lda, W, bias, out, ldo, M, N, K, act, accumulate, ws, ws_floats, KvOut32{}, stream);
 }
 
 // The Q|K|V projection with the cache write fused in: out [M, q_size] receives the query columns, keys and values go
@@ -455,5 +513,5 @@ MLLM_EXPORT int mllm_linear_split_f32_qkv(const float* A, long long lda, const f
                             "in blocks of 32", N, q_size, kv_heads, head_dim);
     if ((uintptr_t)k_pages % 16 || (uintptr_t)v_pages % 16) return mllm_fail(1, "linear_split_f32: the pages must be 16-byte aligned");
     KvOut32 kv{k_pages, v_pages, slots, q_size, kv_heads, head_dim, page_size};
-    return go(A, lda, W, bias, out, ldo, M, N, K, MLLM_ACT_NONE, 0, kv, stream);
+    return go(A, lda, W, bias, out, ldo, M, N, K, MLLM_ACT_NONE, 0, nullptr, 0, kv, stream);
 }

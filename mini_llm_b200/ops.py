@@ -73,7 +73,8 @@ def _signatures(lib):
         "mllm_linear_cluster_bind_error": [c_void_p],
         "mllm_linear_cluster_error": [c_void_p],
         "mllm_linear_split_f32": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int,
-                                  c_void_p],
+                                  c_void_p, c_ll, c_void_p],
+        "mllm_linear_split_f32_slices": [c_int, c_int],
         "mllm_linear_split_f32_qkv": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_void_p,
                                       c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
         "mllm_linear_split_f32_bind_error": [c_void_p],
@@ -821,6 +822,7 @@ def linear(x, weight, bias, out, act: Optional[str] = None, accumulate: bool = F
     contiguous, bias [N] 32-bit or None, out [M,N] rows contiguous.  float32 operands run
     the true 32-bit FMA kernel; bfloat16 operands accumulate in 32-bit.
     """
+    global launches
     if isinstance(x, NormedInput):
         if impl in (None, "smallm") and _fusable(weight, x.shape[0], weight.shape[1]) and _norm_ok(x) \
                 and (impl == "smallm" or _small_m_wins(x.shape[0], weight.shape[0], weight.shape[1])) \
@@ -876,8 +878,15 @@ def linear(x, weight, bias, out, act: Optional[str] = None, accumulate: bool = F
     if impl == "split_f32":
         if not _split_f32_ok(x, weight, M, K):
             raise KernelError(f"linear: split_f32 takes float32, more than {SMALL_M_F32} rows of at least 128 and 16-byte aligned rows")
+        ws_ptr, ws_floats = None, 0
+        slices = library().mllm_linear_split_f32_slices(N, K)
+        if slices > 1:
+            ws = _scratch("split_f32_slices", x.device, slices * (-(-M // 128) * 128) * N)
+            ws_ptr, ws_floats = ws.data_ptr(), ws.numel()
         _call("mllm_linear_split_f32", x.data_ptr(), lda, weight.data_ptr(), bias.data_ptr() if bias is not None else None,
-              out.data_ptr(), ldo, M, N, K, _ACT[act], int(accumulate), _stream())
+              out.data_ptr(), ldo, M, N, K, _ACT[act], int(accumulate), ws_ptr, ws_floats, _stream())
+        if slices > 1:
+            launches += 1           # the kernel that adds the slices
         return out
     if impl in ("smallm", "tcgen05", "cluster"):
         _call("mllm_linear_" + impl, x.data_ptr(), lda, weight.data_ptr(),
@@ -896,7 +905,6 @@ def linear(x, weight, bias, out, act: Optional[str] = None, accumulate: bool = F
     _call("mllm_linear_simt", x.data_ptr(), lda, weight.data_ptr(), bias.data_ptr() if bias is not None else None,
           out.data_ptr(), ldo, M, N, K, _ACT[act], int(accumulate), _dt(x), _dt(out), ws_ptr, ws_floats, _stream())
     if ws_ptr is not None:
-        global launches
         launches += 1           # the finishing kernel that adds the slices
     return out
 

@@ -503,7 +503,7 @@ def test_linear_of_a_decode_batch_in_cluster_slices(ops, M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(65, 64, 128), (128, 1, 132), (129, 191, 768), (300, 1003, 260), (2048, 768, 3072),
-                                   (200, 2304, 768), (77, 50257, 192), (552, 1024, 4096)])
+                                   (200, 2304, 768), (77, 50257, 192), (552, 1024, 4096), (77, 768, 520), (100, 64, 512)])
 def test_linear_float32_in_pieces_on_tensor_cores(ops, M, N, K):
     """The 32-bit product of many rows in exact bfloat16 pieces: every epilogue against float64, no further from float64
     than the chain of fmaf (for values of both signs and for positive ones, where a bias would add up), a row's bits
