@@ -1,5 +1,5 @@
-// out = act(A[M,K] . W[N,K]^T + bias) (+ out) for 17 to 128 rows of bfloat16: the products of decode batches and of
-// short prompts.
+// out = act(A[M,K] . W[N,K]^T + bias) (+ out) for up to 128 rows of bfloat16: the products of decode batches and of
+// short prompts, and the vocabulary for a few rows.
 //
 // What bounds these is how fast a matrix of a few MB comes out of HBM, and the chain of latencies around it; the
 // arithmetic is nothing.  The persistent kernel (linear_tcgen05.cu) gives a narrow matrix to few SMs (12 for 768

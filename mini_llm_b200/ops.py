@@ -643,9 +643,17 @@ def _cluster_wins(M: int, N: int, K: int) -> bool:
     (K = 4 x width), which the other kernels walk on few SMs, gain at every count (5 to 9 against 11 to 22 us).  With K =
     width it wins up to 32 rows (3.7 to 9.5 against 4.1 to 14 us; 768 x 768 is a tie at 32); beyond, the exchange of the
     sums, which grows with the rows, outweighs what the other kernel loses by using fewer SMs, except for narrow results
-    (1024 x 1024 and 1600 x 1600 at 64 rows 4.8 and 6.5 against 5.4 and 8.0 us, 768 x 768 6.0 against 4.6)."""
-    if not 16 < M <= 128 or N >= 16384 or K < 512:
+    (1024 x 1024 and 1600 x 1600 at 64 rows 4.8 and 6.5 against 5.4 and 8.0 us, 768 x 768 6.0 against 4.6).
+    Up to 16 rows the weight-streaming kernel, which takes a norm into its loads, keeps what it wins (2.0 to 3.8 against 3.0
+    to 4.0 us at K = 768 to 1024; 768 x 3072 is 4.8 against 4.5 us inside a step of one row); rows from 6,144 on go to the
+    cluster (1600 x 6400 at 8 rows 7.4 against 11.5 us), and so does a vocabulary, norm apart: 50257 x 768 at 1 / 8 / 16 rows 17 / 18 / 20 us, against 17 / 21 / 31
+    without the norm and 23 to 37 us inside steps with it; the persistent kernel 21 / 21 / 23."""
+    if not 0 < M <= 128 or K < 512:
         return False
+    if N >= 16384:
+        return M <= 16
+    if M <= 16:
+        return K >= 6144
     return M <= 32 or K >= 2048 or (M <= 64 and 1024 <= N <= K)
 
 
@@ -819,13 +827,15 @@ def linear(x, weight, bias, out, act: Optional[str] = None, accumulate: bool = F
     """out = act(x @ weight^T + bias) (+ out when ``accumulate``).
 
     x [M,K] rows contiguous (a column slice is fine) or a NormedInput, weight [N,K]
-    contiguous, bias [N] 32-bit or None, out [M,N] rows contiguous.  float32 operands run
-    the true 32-bit FMA kernel; bfloat16 operands accumulate in 32-bit.
+    contiguous, bias [N] 32-bit or None, out [M,N] rows contiguous.  float32 operands keep
+    all their bits (fmaf chains, or exact pieces on the tensor cores for many rows); bfloat16
+    operands accumulate in 32-bit.
     """
     global launches
     if isinstance(x, NormedInput):
         if impl in (None, "smallm") and _fusable(weight, x.shape[0], weight.shape[1]) and _norm_ok(x) \
-                and (impl == "smallm" or _small_m_wins(x.shape[0], weight.shape[0], weight.shape[1])) \
+                and (impl == "smallm" or (_small_m_wins(x.shape[0], weight.shape[0], weight.shape[1])
+                                          and not _cluster_wins(x.shape[0], weight.shape[0], weight.shape[1]))) \
                 and x.shape[1] == weight.shape[1] and tuple(out.shape) == (x.shape[0], weight.shape[0]):
             _cuda("out", out, contiguous=False)
             if bias is not None:
@@ -1580,7 +1590,7 @@ def latent_attention(qa, pages, block_table, ctx, out, *, heads: int, rank: int,
     holds its key (the first dk columns) and its value (the first ``rank`` columns) for all heads.
     out[t, h] = sum_j softmax_j((qa[t, h] . row_j[:dk]) * scale) row_j[:rank], 32-bit [T, heads * rank].  ``sink`` (float32
     [heads]): exp(sink[h]) is one more term of the softmax's denominator and of nothing else.
-    ``impl``: "split" (CUDA cores, all 32-bit, splits of 256 keys: single tokens, 32-bit caches, any size) or "mma"
+    ``impl``: "split" (CUDA cores, all 32-bit, splits of 32 or 1,024 keys: single tokens, 32-bit caches, any size) or "mma"
     (tensor cores: steps with prompt portions over a bfloat16 cache); None picks by the step's shape."""
     _cuda("qa", qa, torch.float32)
     _cuda("pages", pages)
@@ -2069,7 +2079,7 @@ _TILED_WIDE_HEAD_DIMS = (16, 32, 48, 64)
 
 
 def _tiled_wide_ok(q, head_dim, n_wide, tokens, ldq) -> bool:
-    """Long prompt portions (128-row tiles mostly full) with heads up to 64, where no tensor-core kernel applies."""
+    """Long prompt portions (128-row tiles mostly full) with heads up to 64, where no tensor-core kernel applies (float32: other heads than 64, unaligned rows)."""
     return (head_dim in _TILED_WIDE_HEAD_DIMS and n_wide > 0 and tokens >= 256 and tokens >= 80 * n_wide
             and ldq % (16 // q.element_size()) == 0 and q.data_ptr() % 16 == 0)
 

@@ -456,7 +456,8 @@ def test_linear_many_rows_float32_in_k_slices(ops, M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(17, 768, 768), (24, 1600, 6400), (32, 4800, 1600), (33, 1, 512), (64, 3072, 768),
-                                   (64, 768, 3072), (65, 2304, 768), (77, 127, 520), (128, 6400, 1600), (1, 129, 4096), (20, 300, 64)])
+                                   (64, 768, 3072), (65, 2304, 768), (77, 127, 520), (128, 6400, 1600), (1, 129, 4096), (20, 300, 64),
+                                   (3, 50257, 768), (16, 20000, 1600)])
 def test_linear_of_a_decode_batch_in_cluster_slices(ops, M, N, K):
     """The bfloat16 product that cuts K over the CTAs of a cluster: both result types, every epilogue and unaligned result
     rows against float64; a row's bits do not depend on the rows beside it; the fused cache write is the plain product's
