@@ -22,7 +22,8 @@ with ``bf16_`` in every key.  ``--dtype bfloat16`` swaps the two.  It prints ONE
               median of three such runs, since K steps may be only a millisecond);
   prefill     2,048 prompt tokens (2 x 1024) in one step: tokens/s, ms, and the share of
               the peak for its dtype that its flops reach (bfloat16: the measured cuBLAS
-              rate; float32: the CUDA cores' nominal FFMA rate, SMs x 128 x 2 x clock);
+              rate; float32: the CUDA cores' nominal FFMA rate, SMs x 128 x 2 x clock, which the
+              products in bfloat16 pieces on the tensor cores exceed);
   roofline    bytes the decode step has to read (every weight once + the cache of the
               live requests) / its time, against the HBM copy bandwidth;
   points      decode tokens/s at batch 1 and 64 with their share of the HBM rate, the
@@ -672,8 +673,8 @@ def run_compare_designs(sizes, dtype: str, batch: int, steps: int, designs=None)
 
 
 def fp32_peak_flops() -> float:
-    """CUDA-core peak of the float32 path (no tensor-core mode exists for true 32-bit products):
-    SMs x 128 lanes x 2 flops x the highest SM clock; nominal, nothing measures it on this pool."""
+    """CUDA-core peak, the yardstick of the float32 path (its prefill products run in exact bfloat16 pieces on the tensor
+    cores and can exceed it): SMs x 128 lanes x 2 flops x the highest SM clock; nominal, nothing measures it on this pool."""
     import torch
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     mhz = 1965.0

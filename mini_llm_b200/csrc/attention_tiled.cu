@@ -1,8 +1,8 @@
 // Causal attention of prompt portions over the paged cache on CUDA cores, tiled:
 // 64 queries against 32 keys at a time, everything in 32-bit.
 //
-// This is the prefill attention of the true 32-bit path (float cache: no tensor core, no
-// reduced-precision product) and of head sizes the tensor-core kernel does not take.  A CTA
+// This is the prefill attention of the 32-bit path with other heads than 64 (attention_split_f32.cu
+// takes those) and of head sizes the bfloat16 tensor-core kernels do not take.  A CTA
 // of 256 threads takes one tile of up to 64 consecutive new tokens of one request (the same
 // tiles as the tensor-core kernel) and one head.  Key tile j covers the absolute positions
 // [32j, 32j+32), whatever the cut of the prompt.  Queries sit in shared memory; a key tile is

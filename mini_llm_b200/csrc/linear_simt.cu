@@ -1,9 +1,9 @@
 // out = act(A[M,K] . W[N,K]^T + bias[N]) (+ out): the plain matrix product of the
 // engine, on CUDA cores with 32-bit FMA accumulation.
 //
-// It is the whole product path of the true 32-bit mode (float operands: no tensor
-// core, no reduced-precision matrix mode) and the plain twin that the tensor-core
-// kernels are tested against (bfloat16 operands widened to 32-bit).  Both operands
+// It takes the 32-bit products that neither linear_stream_f32.cu nor linear_split_f32.cu
+// does (unaligned rows, many rows shorter than 128) and is the plain twin that the
+// tensor-core kernels are tested against (bfloat16 operands widened to 32-bit).  Both operands
 // are read along K, the layout every weight is brought to at load, so the tied head
 // uses the embedding table as it is; the reference multiplies row-major [K,N]
 // weights with its own SGEMM tiles (src/kernels/gemm.cu:238-392) and fuses the same
