@@ -119,8 +119,8 @@ __global__ void __launch_bounds__(THREADS, STG ? (TWO ? 6 : Staged<T, LPK>::CTAS
 attn_decode_kernel(const T* q, long long q_stride, const T* k_pages,      // written by kernels of this step: no __restrict__,
                    const T* v_pages,                                        // the compiler must not read them on the non-coherent path
                    const int* __restrict__ block_table, int bt_stride,
-                   const int* __restrict__ token_seq, const int* __restrict__ positions, const int* __restrict__ rows,
-                   T* __restrict__ out, long long out_stride, float* __restrict__ part_o, float* __restrict__ part_ml,
+                   const int* __restrict__ token_seq, const int* __restrict__ positions, T* __restrict__ out,
+                   long long out_stride, float* __restrict__ part_o, float* __restrict__ part_ml,
                    unsigned int* __restrict__ counters, int H, int Hkv, int page_size, float scale, int window,
                    int max_splits, int spc_arg) {
     const int spc = ONE ? 1 : spc_arg;
@@ -144,8 +144,7 @@ attn_decode_kernel(const T* q, long long q_stride, const T* k_pages,      // wri
     __shared__ float sm_res[(PUSH ? MAX_CLUSTER : MODE == MODE_SCRATCH || ONE ? 1 : MAX_SPC) * RES];
     __shared__ int s_last;
     __shared__ __align__(8) uint64_t s_bar;                   // STAGE: a split's bulk copies complete here
-    const int cx = blockIdx.x, h = blockIdx.y;
-    const int t = rows ? __ldcg(rows + blockIdx.z) : blockIdx.z;      // the token's row in the batch
+    const int cx = blockIdx.x, h = blockIdx.y, t = blockIdx.z;
     // Positions, the request index and the block table are written by the host before the step, and the rows of
     // all keys before the token's own position were written by earlier steps: all of that is read before the
     // wait on the previous kernel, which only brings the queries and the token's own key and value.
@@ -191,7 +190,7 @@ attn_decode_kernel(const T* q, long long q_stride, const T* k_pages,      // wri
     uint4 qw = make_uint4(0, 0, 0, 0);
     float qv[VEC];                                            // loaded after the wait, in the first split's turn
     bool waited = false;
-    const size_t pair = (size_t)blockIdx.z * H + h;
+    const size_t pair = (size_t)t * H + h;
     uint32_t phase = 0;
     if constexpr (STAGE) {
         if (threadIdx.x == 0) {
@@ -495,7 +494,7 @@ int decode_sm_count() {
 
 template <typename T, int LPK>
 int launch(const void* q, long long q_stride, const void* k_pages, const void* v_pages, const int* block_table,
-           int bt_stride, const int* token_seq, const int* positions, const int* rows, void* out, long long out_stride,
+           int bt_stride, const int* token_seq, const int* positions, void* out, long long out_stride,
            float* part_o, float* part_ml, unsigned int* counters, int T_tokens, int H, int Hkv, int page_size,
            float scale, int window, int max_splits, bool scratch_path, cudaStream_t stream) {
     // CTAs per (token, head): few requests get one CTA per split, so that the chain position -> block table ->
@@ -512,8 +511,8 @@ int launch(const void* q, long long q_stride, const void* k_pages, const void* v
     ctas = (max_splits + spc - 1) / spc;
     dim3 grid(ctas, H, T_tokens);
 #define ARGS (const T*)q, q_stride, (const T*)k_pages, (const T*)v_pages, block_table, bt_stride, token_seq, positions, \
-             rows, (T*)out, out_stride, part_o, part_ml, counters, H, Hkv, page_size, scale, window, max_splits, spc
-    using K = void (*)(const T*, long long, const T*, const T*, const int*, int, const int*, const int*, const int*, T*, long long,
+             (T*)out, out_stride, part_o, part_ml, counters, H, Hkv, page_size, scale, window, max_splits, spc
+    using K = void (*)(const T*, long long, const T*, const T*, const int*, int, const int*, const int*, T*, long long,
                        float*, float*, unsigned int*, int, int, int, float, int, int, int);
     constexpr bool CAN_STAGE = Staged<T, LPK>::value;
     // staged whenever the rows fit (measured: never slower, from two requests on faster); bulk copies want
@@ -612,7 +611,7 @@ static int attention_decode_check(const void* q, long long q_stride, const void*
 
 static int attention_decode_impl(const void* q, long long q_stride, const void* k_pages, const void* v_pages,
                                  const int* block_table, int bt_stride, const int* token_seq, const int* positions,
-                                 const int* rows, void* out, long long out_stride, float* part_o, float* part_ml,
+                                 void* out, long long out_stride, float* part_o, float* part_ml,
                                  unsigned int* counters, int T, int H, int Hkv, int dh, int page_size, float scale,
                                  int window, int max_splits, int dtype, bool scratch_path, cudaStream_t stream) {
     if (T <= 0) return 0;
@@ -622,7 +621,7 @@ static int attention_decode_impl(const void* q, long long q_stride, const void* 
     if ((scratch_path || max_splits > 8) && (!part_o || !part_ml || !counters))
         return mllm_fail(1, "attention_decode: %d splits need the scratch buffers", max_splits);
 #define GO(TT, LPK)                                                                                            \
-    return launch<TT, LPK>(q, q_stride, k_pages, v_pages, block_table, bt_stride, token_seq, positions, rows, out, \
+    return launch<TT, LPK>(q, q_stride, k_pages, v_pages, block_table, bt_stride, token_seq, positions, out,    \
                            out_stride, part_o, part_ml, counters, T, H, Hkv, page_size, scale, window,          \
                            max_splits, scratch_path, stream)
     if (dtype == MLLM_BF16) {
@@ -664,23 +663,7 @@ MLLM_EXPORT int mllm_attention_decode(const void* q, long long q_stride, const v
                                       float* part_ml, unsigned int* counters, int T, int H, int Hkv, int dh,
                                       int page_size, float scale, int window, int max_splits, int dtype,
                                       int scratch_only, cudaStream_t stream) {
-    return attention_decode_impl(q, q_stride, k_pages, v_pages, block_table, bt_stride, token_seq, positions, nullptr, out,
-                                 out_stride, part_o, part_ml, counters, T, H, Hkv, dh, page_size, scale, window,
-                                 max_splits, dtype, scratch_only != 0, stream);
-}
-
-// The same for T of the batch's tokens: rows[i] (each below the rows of q, out, token_seq and positions) is the i-th
-// token's row.  The single tokens of a step that carries prompt portions come here: as 64-row tiles with one live row
-// of the prefill kernels they cost as much as full tiles.  GPT-2 medium, 512 prompt tokens beside 40 single ones at
-// contexts of 225 to 900, per block: bfloat16 62 us in one launch, 25 us (tcgen05 kernel, whose rule on full tiles the
-// portion now meets) + 27 us in two; float32 835 us in one, 206 + 48 us in two.
-MLLM_EXPORT int mllm_attention_decode_rows(const void* q, long long q_stride, const void* k_pages, const void* v_pages,
-                                           const int* block_table, int bt_stride, const int* token_seq,
-                                           const int* positions, const int* rows, void* out, long long out_stride,
-                                           float* part_o, float* part_ml, unsigned int* counters, int T, int H, int Hkv,
-                                           int dh, int page_size, float scale, int window, int max_splits, int dtype,
-                                           int scratch_only, cudaStream_t stream) {
-    return attention_decode_impl(q, q_stride, k_pages, v_pages, block_table, bt_stride, token_seq, positions, rows, out,
+    return attention_decode_impl(q, q_stride, k_pages, v_pages, block_table, bt_stride, token_seq, positions, out,
                                  out_stride, part_o, part_ml, counters, T, H, Hkv, dh, page_size, scale, window,
                                  max_splits, dtype, scratch_only != 0, stream);
 }
@@ -752,7 +735,7 @@ MLLM_EXPORT int mllm_attention_decode_noalloc(const void* q, long long q_stride,
     // The array keeps what the last call left.  The partial results are fully rewritten before
     // they are read; the counters must start at zero, so they are cleared on this stream.
     MLLM_CUDA(cudaMemsetAsync(counters, 0, (size_t)T * H * sizeof(unsigned int), stream));
-    return attention_decode_impl(q, q_stride, k_pages, v_pages, block_table, bt_stride, token_seq, positions, nullptr, out,
+    return attention_decode_impl(q, q_stride, k_pages, v_pages, block_table, bt_stride, token_seq, positions, out,
                                  out_stride, part_o, part_ml, counters, T, H, Hkv, dh, page_size, scale, window,
                                  max_splits, dtype, /*scratch_path=*/true, stream);
 }

@@ -39,23 +39,20 @@ class StepLayout:
     max_pages: Tuple[int, ...]
     n_tiles: int = 0
     n_tiles_wide: int = 0
-    n_single: int = 0
+    single_runs: Tuple[Tuple[int, int], ...] = ()
     offsets: Dict[str, int] = field(default_factory=dict)
     total: int = 0
 
     @classmethod
     def make(cls, T: int, S: int, R: int, max_pages: Sequence[int], n_tiles: int = 0,
-             n_tiles_wide: int = 0, n_single: int = 0) -> "StepLayout":
-        lay = cls(T, S, R, tuple(max_pages), n_tiles, n_tiles_wide, n_single)
+             n_tiles_wide: int = 0, single_runs: Sequence[Tuple[int, int]] = ()) -> "StepLayout":
+        lay = cls(T, S, R, tuple(max_pages), n_tiles, n_tiles_wide, tuple(single_runs))
         off = 0
         for name, n in (("token_ids", T), ("positions", T), ("token_seq", T), ("logit_rows", R),
                         ("state_slots", S), ("cu_q", S + 1), ("q_start", S), ("ctx_len", S),
                         ("attn_tiles", 3 * n_tiles), ("attn_tiles_wide", 3 * n_tiles_wide)):
             lay.offsets[name] = off
             off += _pad4(n)
-        if n_single:
-            lay.offsets["single_rows"] = off
-            off += _pad4(n_single)
         for g, mp in enumerate(max_pages):
             lay.offsets[f"slot_mapping.{g}"] = off
             off += _pad4(T)
@@ -65,7 +62,7 @@ class StepLayout:
         return lay
 
     def key(self):
-        return (self.T, self.S, self.R, self.max_pages, self.n_tiles, self.n_tiles_wide, self.n_single)
+        return (self.T, self.S, self.R, self.max_pages, self.n_tiles, self.n_tiles_wide, self.single_runs)
 
 
 class Workspace:
@@ -142,10 +139,9 @@ class StepContext:
         # the same tokens cut into tiles of ATTN_TILE_WIDE rows, for the tcgen05 attention
         self.attn_tiles_wide = sec("attn_tiles_wide", 3 * layout.n_tiles_wide)
         self.n_tiles_wide = layout.n_tiles_wide
-        # flat rows of the requests that bring one token to a step in which others bring more; where there are any, their
-        # tiles stand at the end of both lists
-        self.n_single = layout.n_single
-        self.single_rows = sec("single_rows", self.n_single) if self.n_single else None
+        # runs (first flat row, rows) of requests that bring one token to a step in which others bring more; where there are
+        # any, their tiles stand at the end of both lists
+        self.single_runs = layout.single_runs
         self.groups: List[GroupView] = []
         for g, mp in enumerate(layout.max_pages):
             bt = dev[o[f"block_table.{g}"]:o[f"block_table.{g}"] + self.S * mp].view(self.S, mp)
@@ -167,6 +163,24 @@ class StepContext:
 
 ATTN_TILE = 64      # query rows per tile of csrc/attention_flash.cu and attention_tiled.cu
 ATTN_TILE_WIDE = 128     # query rows per tile of csrc/attention_tcgen05.cu
+
+
+MAX_SINGLE_RUNS = 4      # runs of single tokens that a mixed step hands to the decode attention, a launch each
+
+
+def single_runs(q_lens: Sequence[int]) -> List[Tuple[int, int]]:
+    """Runs (first flat row, rows) of neighbouring requests with one new token each; none where there are more than
+    MAX_SINGLE_RUNS of them."""
+    runs: List[Tuple[int, int]] = []
+    base = 0
+    for n in q_lens:
+        if n == 1:
+            if runs and sum(runs[-1]) == base:
+                runs[-1] = (runs[-1][0], runs[-1][1] + 1)
+            else:
+                runs.append((base, 1))
+        base += n
+    return runs if len(runs) <= MAX_SINGLE_RUNS else []
 
 
 def attention_tiles(q_lens: Sequence[int], q_starts: Optional[Sequence[int]] = None,
@@ -195,7 +209,7 @@ def attention_tiles(q_lens: Sequence[int], q_starts: Optional[Sequence[int]] = N
 
 
 def pack_step(layout: StepLayout, host: np.ndarray, *, token_ids, positions, token_seq, logit_rows, state_slots,
-              cu_q, q_start, ctx_len, slot_mappings, block_tables, attn_tiles=(), attn_tiles_wide=(), single_rows=()) -> None:
+              cu_q, q_start, ctx_len, slot_mappings, block_tables, attn_tiles=(), attn_tiles_wide=()) -> None:
     """Write every section into the int32 array ``host`` (length >= layout.total)."""
     o = layout.offsets
 
@@ -215,8 +229,6 @@ def pack_step(layout: StepLayout, host: np.ndarray, *, token_ids, positions, tok
         put("attn_tiles", attn_tiles)
     if layout.n_tiles_wide:
         put("attn_tiles_wide", attn_tiles_wide)
-    if layout.n_single:
-        put("single_rows", single_rows)
     for g, mp in enumerate(layout.max_pages):
         put(f"slot_mapping.{g}", slot_mappings[g])
         bt = np.zeros((layout.S, mp), dtype=np.int32)

@@ -21,7 +21,7 @@ from ..cache.manager import CacheManager
 from ..config.base import ConfigError, EngineConfig, ModelConfig, get_architecture, load_config
 from ..parts.model import Model
 from ..weights.loader import load_weights
-from .context import ATTN_TILE_WIDE, StepContext, StepLayout, Workspace, attention_tiles, pack_step
+from .context import ATTN_TILE_WIDE, StepContext, StepLayout, Workspace, attention_tiles, pack_step, single_runs
 
 
 class StepError(RuntimeError):
@@ -243,17 +243,15 @@ class ModelRunner:
         for g in range(ng):
             mp = max(len(t) for t in tables[g])
             max_pages.append(max(16, 1 << (mp - 1).bit_length()))   # powers of two: few distinct shapes for captured graphs
-        apart = self._singles_apart and T != S
-        tiles = [] if T == S else attention_tiles(q_lens, q_start, singles_last=apart)
-        wide = [] if T == S else attention_tiles(q_lens, q_start, ATTN_TILE_WIDE, singles_last=apart)
-        singles = [int(cu_q[s]) for s, n in enumerate(q_lens) if n == 1] if apart else []
-        layout = StepLayout.make(T, S, len(logit_rows), max_pages, len(tiles) // 3, len(wide) // 3, len(singles))
+        runs = single_runs(q_lens) if self._singles_apart and T != S else []
+        tiles = [] if T == S else attention_tiles(q_lens, q_start, singles_last=bool(runs))
+        wide = [] if T == S else attention_tiles(q_lens, q_start, ATTN_TILE_WIDE, singles_last=bool(runs))
+        layout = StepLayout.make(T, S, len(logit_rows), max_pages, len(tiles) // 3, len(wide) // 3, runs)
         i, host = self._staging(layout.total)
         self._last_layout_total = layout.total
         pack_step(layout, host.numpy(), token_ids=token_ids, positions=positions, token_seq=token_seq,
                   logit_rows=logit_rows, state_slots=slots, cu_q=cu_q, q_start=q_start, ctx_len=ctx_len,
-                  slot_mappings=slot_maps, block_tables=tables, attn_tiles=tiles, attn_tiles_wide=wide,
-                  single_rows=singles)
+                  slot_mappings=slot_maps, block_tables=tables, attn_tiles=tiles, attn_tiles_wide=wide)
         self._dev[:layout.total].copy_(host[:layout.total], non_blocking=True)
         self._host_events[i].record()
         self._pending_ids = pending
@@ -307,7 +305,7 @@ class ModelRunner:
             self._graph_families.clear()
             self._graph_version = self._buffer_version()
         key = (ctx.layout.key(), ops.decode_splits(ctx.max_ctx_len) if ctx.decode_only else
-               ops.decode_splits(ctx.max_single_ctx_len) if ctx.n_single else 0,
+               ops.decode_splits(ctx.max_single_ctx_len) if ctx.single_runs else 0,
                ops.latent_splits(ctx.max_ctx_len))      # every host-side number a launch's grid depends on
         g = self._graphs.get(key)
         if g is not None:

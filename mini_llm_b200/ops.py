@@ -96,9 +96,6 @@ def _signatures(lib):
                                      c_ll, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
         "mllm_attention_split_f32_bind_error": [c_void_p],
         "mllm_attention_split_f32_error": [c_void_p],
-        "mllm_attention_decode_rows": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
-                                       c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
-                                       c_int, c_int, c_int, c_int, c_void_p],
         "mllm_attention_decode_last_staging": [],
         "mllm_attention_flash": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p,
                                  c_void_p, c_ll, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
@@ -2117,10 +2114,13 @@ def paged_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, nu
     decode_ok = head_dim in _DECODE_HEAD_DIMS[q.dtype] and ldq % 8 == 0 and q.data_ptr() % 16 == 0
     if impl is None:
         impl = "simt"
-        if decode_ok and (k_pages.data_ptr() | v_pages.data_ptr()) % 16 == 0 and getattr(ctx, "n_single", 0):
-            # single tokens beside prompt portions: the decode kernel takes them after the portions' launch below, whose
-            # tiles are the head of the lists
-            singles = ctx.n_single
+        if decode_ok and (k_pages.data_ptr() | v_pages.data_ptr()) % 16 == 0 and getattr(ctx, "single_runs", ()):
+            # Single tokens beside prompt portions: the decode kernel takes them, run by run, after the portions' launch,
+            # whose tiles are the head of the lists.  As 64-row tiles with one live row of the prefill kernels they cost as
+            # much as full tiles.  GPT-2 medium, 512 prompt tokens beside 40 single ones at contexts of 225 to 900, per
+            # block: bfloat16 62 us in one launch, 25 us (tcgen05 kernel, whose rule on full tiles the portion now meets)
+            # + 27 us in two; float32 835 us in one, 51 + 48 us in two.
+            singles = sum(n for _, n in ctx.single_runs)
             n_tiles, n_wide, tokens = n_tiles - singles, n_wide - singles, T - singles
         if getattr(ctx, "decode_only", False) and decode_ok:
             impl = "decode"
@@ -2139,17 +2139,18 @@ def paged_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, nu
     if singles:
         _attend(impl, q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ldo, num_heads, num_kv_heads, head_dim, ps,
                 scale, window, n_tiles, n_wide, None)
-        _attend("decode", q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ldo, num_heads, num_kv_heads, head_dim,
-                ps, scale, window, 0, 0, ctx.single_rows)
+        for run in ctx.single_runs:
+            _attend("decode", q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ldo, num_heads, num_kv_heads,
+                    head_dim, ps, scale, window, 0, 0, run)
         return
     _attend(impl, q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ldo, num_heads, num_kv_heads, head_dim, ps, scale,
             window, n_tiles, n_wide, None)
 
 
 def _attend(impl, q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ldo, num_heads, num_kv_heads, head_dim, ps, scale,
-            window, n_tiles, n_wide, rows) -> None:
-    """One launch of the named attention kernel; ``rows``: the batch's rows that the decode kernel takes (None: all)."""
-    T = q.shape[0] if rows is None else rows.shape[0]
+            window, n_tiles, n_wide, run) -> None:
+    """One launch of the named attention kernel; ``run`` (first row, rows): what the decode kernel takes (None: all)."""
+    T = q.shape[0] if run is None else run[1]
     attention_launches[impl] = attention_launches.get(impl, 0) + 1
     if impl == "tiled_wide":
         if head_dim not in _TILED_WIDE_HEAD_DIMS or n_wide <= 0 or ldq % (16 // q.element_size()):
@@ -2197,7 +2198,7 @@ def _attend(impl, q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ld
             raise KernelError(f"paged_attention: the split-key kernel takes head sizes {_DECODE_HEAD_DIMS[q.dtype]} "
                               f"for {q.dtype}, not {head_dim}")
         # splits cover the longest context of the step, rounded up so that captured graphs keep their grid
-        max_splits = decode_splits(ctx.max_ctx_len if rows is None else ctx.max_single_ctx_len)
+        max_splits = decode_splits(ctx.max_ctx_len if run is None else ctx.max_single_ctx_len)
         # Up to DECODE_CLUSTER_SPLITS splits meet in a thread-block cluster and touch no scratch; only beyond that
         # (contexts over 1,024 tokens) or on request do the partial results go through global memory.  Asking for
         # the buffers only then keeps a growing context from ever replacing a buffer under the captured graphs.
@@ -2207,9 +2208,10 @@ def _attend(impl, q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ld
             counters = ctx.ws.zeroed("attn_counters", T * num_heads).data_ptr()     # the kernel leaves them zero
         else:
             part_o = part_ml = counters = None
-        _call("mllm_attention_decode_rows", q.data_ptr(), ldq, k_pages.data_ptr(), v_pages.data_ptr(),
-              block_table.data_ptr(), bt_stride, ctx.token_seq.data_ptr(), ctx.positions.data_ptr(),
-              rows.data_ptr() if rows is not None else None, out.data_ptr(),
+        t0, es = (0 if run is None else run[0]), q.element_size()
+        _call("mllm_attention_decode", q.data_ptr() + t0 * ldq * es, ldq, k_pages.data_ptr(), v_pages.data_ptr(),
+              block_table.data_ptr(), bt_stride, ctx.token_seq.data_ptr() + 4 * t0, ctx.positions.data_ptr() + 4 * t0,
+              out.data_ptr() + t0 * ldo * es,
               ldo, part_o, part_ml, counters, T, num_heads, num_kv_heads, head_dim, ps, float(scale),
               int(window or 0), max_splits, _dt(q), int(impl == "decode_scratch"), _stream())
         return

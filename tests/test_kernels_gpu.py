@@ -825,11 +825,11 @@ def test_tcgen05_attention_mixed_batch(ops, H, Hkv, page, window):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H,Hkv,dh,page,window", [(12, 12, 64, 16, None), (4, 1, 32, 8, 37), (2, 2, 128, 4, None), (3, 3, 48, 16, None)])
-@pytest.mark.parametrize("seqs", [[(70, 1), (300, 257), (1, 1), (16, 2), (1024, 1)], [(2, 2), (129, 1)], [(1, 1), (640, 600), (700, 1)]])
+@pytest.mark.parametrize("seqs", [[(70, 1), (300, 257), (1, 1), (9, 1), (16, 2), (1024, 1)], [(2, 2), (129, 1)], [(1, 1), (640, 600), (700, 1)]])
 def test_single_tokens_beside_portions_take_the_decode_kernel(ops, dtype, H, Hkv, dh, page, window, seqs):
     """A step's prompt portions and single tokens in two launches: every row written once, against float64, and the single
     tokens with the bits of a step that has only them.  Head sizes without a decode kernel stay in one launch."""
-    from mini_llm_b200.engine.context import ATTN_TILE_WIDE, attention_tiles
+    from mini_llm_b200.engine.context import ATTN_TILE_WIDE, attention_tiles, single_runs
     case = _paged_case(dtype, seqs, H, Hkv, dh, page, num_pages=2500 // page + 40, seed=dh)
     ctx = _ctx_for(case)
     q_lens, starts = [n for _, n in seqs], [c - n for c, n in seqs]
@@ -840,7 +840,8 @@ def test_single_tokens_beside_portions_take_the_decode_kernel(ops, dtype, H, Hkv
         setattr(ctx, "attn_tiles" + name, torch.tensor(tiles, dtype=torch.int32, device=DEV))
         setattr(ctx, "n_tiles" + name, len(tiles) // 3)
     rows = [sum(q_lens[:i]) for i, n in enumerate(q_lens) if n == 1]
-    ctx.n_single, ctx.single_rows = len(rows), torch.tensor(rows, dtype=torch.int32, device=DEV)
+    ctx.single_runs = single_runs(q_lens)
+    assert [t for t0, n in ctx.single_runs for t in range(t0, t0 + n)] == rows
     ctx.max_single_ctx_len = max(c for c, n in seqs if n == 1)
     q = case["q"].to(dtype).to(DEV)
     kp, vp, bt = case["k_pages"].to(dtype).to(DEV), case["v_pages"].to(dtype).to(DEV), case["bt"].to(DEV)
@@ -848,11 +849,11 @@ def test_single_tokens_beside_portions_take_the_decode_kernel(ops, dtype, H, Hkv
     out = torch.full_like(q, 7.0)
     before = ops.attention_launches.get("decode", 0)
     ops.paged_attention(q, kp, vp, bt, ctx, out, **kw)
-    assert ops.attention_launches.get("decode", 0) == before + (dh != 48)
+    assert ops.attention_launches.get("decode", 0) == before + (len(ctx.single_runs) if dh != 48 else 0)
     want = _attention_reference(case, H, Hkv, dh, dh ** -0.5, window, dtype)
     assert ((out.double().cpu() - want).abs() / want.abs().clamp(min=1.0)).max() < (2e-5 if dtype == torch.float32 else 2 ** -8)
     if dh != 48:
-        alone, sel = _Ctx(), ctx.single_rows.long()
+        alone, sel = _Ctx(), torch.tensor(rows, device=DEV)
         alone.token_seq, alone.positions = ctx.token_seq[sel], ctx.positions[sel]
         alone.ws, alone.max_ctx_len, alone.decode_only = ctx.ws, ctx.max_single_ctx_len, True
         got = torch.empty_like(q[sel])
