@@ -758,6 +758,13 @@ def linear_qkv_cache(x, weight, bias, q_out, k_pages, v_pages, slot_mapping, ws)
     _cuda("slot_mapping", slot_mapping, torch.int32)
     if slot_mapping.numel() != M or q_out.shape[0] != M or v_pages.shape != k_pages.shape:
         raise KernelError(f"linear_qkv_cache: {M} rows, {slot_mapping.numel()} slots, q_out {tuple(q_out.shape)}")
+    _cuda("weight", weight)
+    if x.shape[1] != K:
+        raise KernelError(f"linear_qkv_cache: x {tuple(x.shape)}, weight {tuple(weight.shape)}")
+    if bias is not None:
+        _cuda("bias", bias, torch.float32)
+        if bias.numel() != N:
+            raise KernelError(f"linear_qkv_cache: a bias of {bias.numel()} for {N} columns")
     norm = x if isinstance(x, NormedInput) else None
     if q_out.dtype == torch.float32 and _stream_f32_ok(weight, M, K) and q_out.stride(1) == 1 \
             and k_pages.is_contiguous() and v_pages.is_contiguous():
@@ -765,8 +772,6 @@ def linear_qkv_cache(x, weight, bias, q_out, k_pages, v_pages, slot_mapping, ws)
         if norm is not None and not _norm_ok_f32(norm):
             x, norm = norm.materialize(), None
         if norm is not None or (x.is_cuda and x.dtype == torch.float32 and _rows("x", x) % 4 == 0 and x.data_ptr() % 16 == 0):
-            if bias is not None:
-                _cuda("bias", bias, torch.float32)
             _linear_stream_f32(None if norm is not None else x, weight, bias, q_out, None, False, norm,
                                (k_pages, v_pages, slot_mapping, q_size))
             return q_out
@@ -775,8 +780,6 @@ def linear_qkv_cache(x, weight, bias, q_out, k_pages, v_pages, slot_mapping, ws)
     if (norm is None and q_out.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and _cluster_wins(M, N, K)
             and x.is_cuda and x.dtype == torch.bfloat16 and K % 8 == 0 and weight.data_ptr() % 16 == 0
             and _rows("x", x) % 8 == 0 and x.data_ptr() % 16 == 0 and k_pages.is_contiguous() and v_pages.is_contiguous()):
-        if bias is not None:
-            _cuda("bias", bias, torch.float32)
         _call("mllm_linear_cluster_qkv", x.data_ptr(), _rows("x", x), weight.data_ptr(),
               bias.data_ptr() if bias is not None else None, q_out.data_ptr(), _rows("q_out", q_out), M, N, K,
               k_pages.data_ptr(), v_pages.data_ptr(), slot_mapping.data_ptr(), q_size, Hkv, dh, ps, _stream())
@@ -784,8 +787,6 @@ def linear_qkv_cache(x, weight, bias, q_out, k_pages, v_pages, slot_mapping, ws)
     if q_out.dtype == torch.bfloat16 and _fusable(weight, M, K) and _small_m_wins(M, N, K) and (
             _norm_ok(norm) if norm is not None else
             (x.is_cuda and x.dtype == torch.bfloat16 and _rows("x", x) % 8 == 0 and x.data_ptr() % 16 == 0)):
-        if bias is not None:
-            _cuda("bias", bias, torch.float32)
         _linear_fused(None if norm is not None else x, weight, bias, q_out, None, False, norm,
                       (k_pages, v_pages, slot_mapping, q_size))
         return q_out
@@ -798,8 +799,6 @@ def linear_qkv_cache(x, weight, bias, q_out, k_pages, v_pages, slot_mapping, ws)
             and _rows("q_out", q_out) % 8 == 0 and q_out.data_ptr() % 16 == 0 and k_pages.is_contiguous()
             and v_pages.is_contiguous()):
         # many rows: the tensor-memory product, whose epilogue stores keys and values into their pages
-        if bias is not None:
-            _cuda("bias", bias, torch.float32)
         _call("mllm_linear_tcgen05_qkv", x.data_ptr(), _rows("x", x), weight.data_ptr(),
               bias.data_ptr() if bias is not None else None, q_out.data_ptr(), _rows("q_out", q_out), M, N, K,
               k_pages.data_ptr(), v_pages.data_ptr(), slot_mapping.data_ptr(), q_size, Hkv, dh, ps, _stream())
@@ -808,8 +807,6 @@ def linear_qkv_cache(x, weight, bias, q_out, k_pages, v_pages, slot_mapping, ws)
             and _rows("q_out", q_out) % 4 == 0 and q_out.data_ptr() % 16 == 0 and k_pages.is_contiguous()
             and v_pages.is_contiguous() and k_pages.data_ptr() % 16 == 0 and v_pages.data_ptr() % 16 == 0):
         # the same in 32-bit
-        if bias is not None:
-            _cuda("bias", bias, torch.float32)
         _call("mllm_linear_split_f32_qkv", x.data_ptr(), _rows("x", x), weight.data_ptr(),
               bias.data_ptr() if bias is not None else None, q_out.data_ptr(), _rows("q_out", q_out), M, N, K,
               k_pages.data_ptr(), v_pages.data_ptr(), slot_mapping.data_ptr(), q_size, Hkv, dh, ps, _stream())

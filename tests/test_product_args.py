@@ -1,0 +1,51 @@
+"""What the products' entry points check and choose on the host, without a GPU: the functions of ops run on CPU tensors with
+the launch itself replaced by a recorder, so nothing is computed and no address is used."""
+import pytest
+import torch
+
+
+@pytest.fixture
+def ops(monkeypatch):
+    from mini_llm_b200 import ops
+
+    def named(name, t, dtype=None, contiguous=True):
+        if dtype is not None and t.dtype != dtype:
+            raise ops.KernelError(f"{name} must be {dtype}, got {t.dtype}")
+        if contiguous and not t.is_contiguous():
+            raise ops.KernelError(f"{name} must be contiguous")
+        return t
+
+    ops.calls = []
+    monkeypatch.setattr(ops, "_cuda", named)
+    monkeypatch.setattr(ops, "_call", lambda name, *args: ops.calls.append((name, args)))
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    yield ops
+    del ops.calls
+
+
+def _projection(M, H, dh, K, dtype):
+    N = 3 * H * dh
+    pages = torch.zeros(-(-M // 16), H, 16, dh, dtype=dtype)
+    return dict(x=torch.zeros(M, K, dtype=dtype), weight=torch.zeros(N, K, dtype=dtype), bias=torch.zeros(N),
+                q_out=torch.zeros(M, H * dh, dtype=dtype), k_pages=pages, v_pages=pages.clone(),
+                slot_mapping=torch.arange(M, dtype=torch.int32), ws=None)
+
+
+# rows of every kernel behind the entry: weight-streaming, tensor cores in pieces, cluster slices, the product and the copy
+@pytest.mark.parametrize("M,dh,dtype", [(8, 32, torch.float32), (100, 32, torch.float32), (100, 24, torch.float32),
+                                        (300, 32, torch.bfloat16), (100, 24, torch.bfloat16),
+                                        (24, 24, torch.bfloat16)])
+@pytest.mark.parametrize("what", ["short bias", "long rows of x", "weight in columns"])
+def test_cache_writing_projection_refuses_what_does_not_fit(ops, M, dh, dtype, what):
+    a = _projection(M, 4, dh, 768, dtype)
+    if what == "short bias":
+        a["bias"] = a["bias"][:-1]
+    elif what == "long rows of x":
+        a["x"] = torch.zeros(M, 776, dtype=dtype)
+    else:
+        a["weight"] = torch.zeros(768, a["weight"].shape[0], dtype=dtype).t()
+    from mini_llm_b200.engine.context import Workspace
+    a["ws"] = Workspace(torch.device("cpu"), 512)
+    with pytest.raises(ops.KernelError):
+        ops.linear_qkv_cache(**a)
+    assert not ops.calls
