@@ -89,6 +89,17 @@ class Workspace:
             self.version += 1
         return t[:rows]
 
+    def flat(self, name: str, n: int) -> torch.Tensor:
+        """At least ``n`` 32-bit floats, in a buffer that grows by powers of two (sizes that vary from call to call
+        replace it rarely)."""
+        key = (name, 0, torch.float32)
+        t = self._bufs.get(key)
+        if t is None or t.numel() < n:
+            t = torch.empty(max(1 << (int(n) - 1).bit_length(), 1 << 20), dtype=torch.float32, device=self.device)
+            self._bufs[key] = t
+            self.version += 1
+        return t
+
     def zeroed(self, name: str, n: int) -> torch.Tensor:
         """``n`` int32 words that are zero when first handed out; kernels that use them as
         counters leave them zero."""

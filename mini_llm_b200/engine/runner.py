@@ -284,10 +284,6 @@ class ModelRunner:
         return logits
 
     # ------------------------------------------------------------------ CUDA graphs
-    def _buffer_version(self):
-        """Changes whenever a scratch buffer that a captured graph may point into is replaced."""
-        return (self.ws.version, ops.scratch_version)
-
     def _forward(self, ctx: StepContext) -> Optional[torch.Tensor]:
         """A step is about a hundred launches; issued one by one from Python they cost
         more host time than a decode step or a 2,048-token prefill takes on the GPU.  So a
@@ -297,13 +293,13 @@ class ModelRunner:
         first time runs eagerly.  All graphs are dropped when a scratch buffer is replaced
         by a larger one, since a graph fixes buffer addresses."""
         if not (self.engine.use_cuda_graphs and self._graph_ok):
-            with ops.stream_scope():
+            with ops.stream_scope(self.ws):
                 return self.model.forward(ctx)
-        if self._graph_version != self._buffer_version():
+        if self._graph_version != self.ws.version:
             self._graphs.clear()
             self._graph_seen.clear()
             self._graph_families.clear()
-            self._graph_version = self._buffer_version()
+            self._graph_version = self.ws.version
         key = (ctx.layout.key(), ops.decode_splits(ctx.max_ctx_len) if ctx.decode_only else
                ops.decode_splits(ctx.max_single_ctx_len) if ctx.single_runs else 0,
                ops.latent_splits(ctx.max_ctx_len))      # every host-side number a launch's grid depends on
@@ -321,24 +317,24 @@ class ModelRunner:
         # key splits (a context that grew) needs no new buffers: capture it at first sight.
         family = key[0][:3] + key[0][4:]
         if seen == 0 and family not in self._graph_families:
-            with ops.stream_scope():
+            with ops.stream_scope(self.ws):
                 logits = self.model.forward(ctx)       # first time: eager, buffers get allocated
             if not self._capture_at_once:
                 return logits
             # "at_once": the same step again, captured and replayed, so that even a shape that never comes back
             # is computed by a replayed graph (what the replay tests grade); a step only writes its own tokens'
             # cache slots and scratch, so running it twice changes nothing
-        version = self._buffer_version()
+        version = self.ws.version
         torch.cuda.current_stream().synchronize()
         graph = torch.cuda.CUDAGraph()
         n0 = ops.launches
         with torch.cuda.graph(graph):
-            with ops.stream_scope():
+            with ops.stream_scope(self.ws):
                 logits = self.model.forward(ctx)
         kernels = ops.launches - n0
-        if self._buffer_version() != version:           # a buffer was allocated during capture: do not keep it
+        if self.ws.version != version:           # a buffer was allocated during capture: do not keep it
             self._graph_version = None
-            with ops.stream_scope():
+            with ops.stream_scope(self.ws):
                 return self.model.forward(ctx)
         if len(self._graphs) >= 64:
             old = next(iter(self._graphs))

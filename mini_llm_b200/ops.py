@@ -9,6 +9,7 @@ tensor is not on a CUDA device, the call fails with an error.
 from __future__ import annotations
 
 import ctypes
+import threading
 from typing import Optional
 
 import torch
@@ -355,26 +356,36 @@ def check_device_errors() -> None:
                           "(1 the cutting warps, 2-5 the MMA issuer, 7-8 the softmax warps)")
 
 
-_stream_handle = None     # set by stream_scope(); None: ask torch on every call
+class _Scope(threading.local):
+    handle = None       # set by stream_scope(); None: ask torch on every call
+    stream = None
+    workspace = None
+
+
+_scope = _Scope()
 
 
 class stream_scope:
-    """Within the scope every launch goes to the stream that is current on entry, without
-    asking torch again on each call (a lookup costs more than the launch itself)."""
+    """Within the scope every launch of this thread goes to the stream that is current on entry, without
+    asking torch again on each call (a lookup costs more than the launch itself), and the functions
+    here that need scratch of their own take it from ``workspace``."""
+
+    def __init__(self, workspace=None):
+        self._workspace = workspace
 
     def __enter__(self):
-        global _stream_handle
-        self._old = _stream_handle
-        _stream_handle = torch.cuda.current_stream().cuda_stream
+        self._old = _scope.handle, _scope.stream, _scope.workspace
+        _scope.stream = torch.cuda.current_stream()
+        _scope.handle, _scope.workspace = _scope.stream.cuda_stream, self._workspace
         return self
 
     def __exit__(self, *a):
-        global _stream_handle
-        _stream_handle = self._old
+        _scope.handle, _scope.stream, _scope.workspace = self._old
 
 
 def _stream() -> int:
-    return _stream_handle if _stream_handle is not None else torch.cuda.current_stream().cuda_stream
+    handle = _scope.handle
+    return handle if handle is not None else torch.cuda.current_stream().cuda_stream
 
 
 def _dt(t: torch.Tensor) -> int:
@@ -913,24 +924,14 @@ def linear(x, weight, bias, out, act: Optional[str] = None, accumulate: bool = F
     return out
 
 
-_scratch_bufs = {}
-
-
 def _scratch(name: str, device, floats: int) -> torch.Tensor:
-    """A float32 scratch buffer of this module that only grows (a step shape runs eagerly before it is captured as a
-    graph, so a captured graph never sees the buffer replaced under it unless a larger shape comes later: sizes are
-    rounded up to the next power of two to make that rare, and the runner drops its graphs when it happens)."""
-    global scratch_version
-    key = (name, str(device))
-    buf = _scratch_bufs.get(key)
-    if buf is None or buf.numel() < floats:
-        buf = torch.empty(max(1 << (int(floats) - 1).bit_length(), 1 << 20), dtype=torch.float32, device=device)
-        _scratch_bufs[key] = buf
-        scratch_version += 1
-    return buf
-
-
-scratch_version = 0     # bumped whenever a scratch buffer of this module is replaced
+    """float32 scratch of one call: the scope's workspace's own buffer of that name (the steps of a runner follow one
+    another; other runners, on whatever stream or thread, have other buffers), or an allocation that torch gives back to
+    the call's stream afterwards."""
+    if _scope.workspace is not None:
+        return _scope.workspace.flat(name, floats)
+    with torch.cuda.stream(_scope.stream):          # (None: the current stream)
+        return torch.empty(int(floats), dtype=torch.float32, device=device)
 
 
 # --------------------------------------------------------------------------- cache

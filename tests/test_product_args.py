@@ -49,3 +49,31 @@ def test_cache_writing_projection_refuses_what_does_not_fit(ops, M, dh, dtype, w
     with pytest.raises(ops.KernelError):
         ops.linear_qkv_cache(**a)
     assert not ops.calls
+
+
+def test_slices_of_a_product_are_summed_in_the_callers_own_scratch(ops, monkeypatch):
+    """The float32 product in K slices: every workspace brings its own buffer (two runners on two streams may be between
+    the product and the sum of its slices at the same time), the same one for every call; without a workspace a call
+    allocates for itself."""
+    from types import SimpleNamespace
+    from mini_llm_b200.engine.context import Workspace
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: SimpleNamespace(cuda_stream=0))
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: __import__("contextlib").nullcontext())
+    x, w = torch.zeros(100, 768), torch.zeros(768, 768)
+    assert ops.library().mllm_linear_split_f32_slices(768, 768) > 1
+
+    def scratch(ws, rows=100):
+        with ops.stream_scope(ws):
+            ops.linear(x[:rows], w, None, out=torch.zeros(rows, 768))
+        name, args = ops.calls[-1]
+        assert name == "mllm_linear_split_f32"
+        pointer, floats = args[-3:-1]
+        assert floats >= 3 * 128 * 768
+        return pointer
+
+    a, b = Workspace(torch.device("cpu"), 128), Workspace(torch.device("cpu"), 128)
+    assert scratch(a) == scratch(a, 70) != scratch(b) == scratch(b)
+    assert scratch(None) not in (scratch(a), scratch(b))
+    version = a.version
+    x = torch.zeros(1000, 768)
+    assert scratch(a, 1000) and a.version > version          # a larger buffer is seen by whoever keeps its address
