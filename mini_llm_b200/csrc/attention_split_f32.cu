@@ -19,8 +19,8 @@
 // 53 / 190 / 489; 512 tokens after 450 and 16 heads 50 / 187 / 299; 200 tokens and 12 heads 19 / 51 / 71 (19 us is what an
 // isolated launch costs the host; 16 tokens: 19 / 27 / 18).
 //
-// A tile whose queries, keys or values are not all finite (the pieces of an infinity are not) is computed again by
-// plain_rows() with fmaf, one key after the other, so that infinities and NaN come out as they should.
+// A tile whose queries, keys or values do not all have pieces (infinities, NaN, values above the largest bfloat16) is
+// computed again by plain_rows() with fmaf, one key after the other, so that infinities and NaN come out as they should.
 //
 // Every wait is bounded: after the limit the kernel records an error code, frees its tensor memory and returns.
 #include "tcgen05.cuh"
@@ -44,9 +44,9 @@ __device__ int g_attn_split_error = 0;
 
 __host__ __device__ constexpr uint32_t make_idesc_bmn(int m, int n) { return make_idesc(m, n) | (1u << 16); }
 
-__device__ __forceinline__ bool finite4(const float4& v) {
-    return fabsf(v.x) <= 3.402823466e38f && fabsf(v.y) <= 3.402823466e38f && fabsf(v.z) <= 3.402823466e38f &&
-           fabsf(v.w) <= 3.402823466e38f;
+// Whether the values have pieces (infinities, NaN and the largest finite values have not).
+__device__ __forceinline__ bool has_pieces(const float4& v) {
+    return fabsf(v.x) <= SPLIT_MAX && fabsf(v.y) <= SPLIT_MAX && fabsf(v.z) <= SPLIT_MAX && fabsf(v.w) <= SPLIT_MAX;
 }
 
 // 8 consecutive values of row `row` (piece g of 8) into the three swizzled planes at `plane0`
@@ -104,7 +104,7 @@ attention_split_f32_kernel(const float* q, long long q_stride, const float* k_pa
     uint64_t* o_full = p_full + 1;
     uint32_t* tmem_slot = (uint32_t*)(o_full + 1);
     volatile int* failed = (volatile int*)(tmem_slot + 1);
-    volatile int* odd = failed + 1;                               // some operand is not finite
+    volatile int* odd = failed + 1;                               // some operand has no pieces
 
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int h = blockIdx.x, tile = blockIdx.y;
@@ -225,7 +225,7 @@ attention_split_f32_kernel(const float* q, long long q_stride, const float* k_pa
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                fine &= finite4(x[u][0]) && finite4(x[u][1]);
+                fine &= has_pieces(x[u][0]) && has_pieces(x[u][1]);
                 put_row8(dst, (half & 1) * 64 + u * 16 + r0, g, x[u][0], x[u][1]);
             }
             if (half & 1) {
@@ -252,7 +252,7 @@ attention_split_f32_kernel(const float* q, long long q_stride, const float* k_pa
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 x[e] = row < rows ? *reinterpret_cast<const float4*>(p + 4 * e) : make_float4(0.f, 0.f, 0.f, 0.f);
-                fine &= finite4(x[e]);
+                fine &= has_pieces(x[e]);
             }
             put_row8(sQ, row, g, x[0], x[1]);
             put_row8(sQ, row, g + 1, x[2], x[3]);

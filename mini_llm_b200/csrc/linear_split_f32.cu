@@ -1,10 +1,9 @@
 // out = act(A[M,K] . W[N,K]^T + bias) (+ out) with 32-bit operands and more than 64 rows, on the fifth-generation
 // tensor cores: the product of prefill and mixed steps on the 32-bit path.
 //
-// A 32-bit value x is cut exactly into three bfloat16 pieces, x = h + m + l: h is x without its lower 16 bits, m the
-// rest without its lower 16 bits, l what then remains (24 significant bits = 3 x 8; nothing is lost above the
-// smallest bfloat16, 2^-133).  Of the nine products of pieces the six largest are formed: hh, hm, mh, mm, hl, lh; the
-// rest is below 2^-23 of |a w| at most and 2^-26 on average.  A product of two bfloat16 is exact in the tensor core.
+// A 32-bit value x is cut exactly into three bfloat16 pieces, x = h + m + l, by rounding to nearest twice (split_f32.cuh).
+// Of the nine products of pieces the six largest are formed: hh, hm, mh, mm, hl, lh; the rest is at most 2^-24 of |a w|
+// and has either sign.  A product of two bfloat16 is exact in the tensor core.
 // The tensor memory holds the sum over 64 of K only: every 64 wide block is read out and added to a sum in registers
 // by plain 32-bit additions, and within a block the small terms come first, so that the accumulator's own rounding
 // (which drops bits instead of rounding to nearest) meets only 4 additions of full-size terms.  Against float64 the
@@ -20,8 +19,8 @@
 //  * warps 8-15 drain the accumulators and run the epilogue.
 // The sum over K of an element runs in an order that depends on K alone.
 //
-// An element whose sum is not finite (an operand is infinite or NaN, or the sum overflows: inf - inf appears in the
-// pieces) is computed again as a chain of fmaf over the 32-bit operands, so infinities come out as they should.
+// An element whose sum is not finite (an operand is infinite, NaN or above the largest bfloat16, or the sum overflows:
+// inf - inf appears in the pieces) is computed again as a chain of fmaf over the 32-bit operands, so infinities come out as they should.
 //
 // Every wait is bounded: after the limit the kernel records an error code, frees its tensor memory and returns.
 #include "tcgen05.cuh"

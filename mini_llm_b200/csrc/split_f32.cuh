@@ -8,16 +8,26 @@ namespace tc {
 template <int R> __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
 template <int R> __device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
 
-// Two consecutive values -> their three pieces, packed (the first value in the lower half).  Truncation keeps every
-// subtraction exact, and the third piece needs no more than the 8 bits a bfloat16 has.
+// Two consecutive values -> their three pieces, packed (the first value in the lower half).  h is x rounded to the nearest
+// bfloat16, m the rest rounded likewise, l what then remains.  Every subtraction is exact: with |x| in [2^e, 2^(e+1)) the
+// rest after h is a multiple of 2^(e-23) of at most 2^(e-8), the rest after m one of at most 2^(e-17), which needs 7 of the
+// 8 bits a bfloat16 has.  Rounding instead of cutting bits off keeps the dropped products of pieces (m l, l m, l l) below
+// 2^-24 of the product (6e-8; cut off they reach 2^-21 and all have the product's sign, so that sums shrink by 4e-8), and
+// they have either sign (tests/test_product_args.py has both cuts in numpy).  Values beyond the largest bfloat16 round to
+// infinity: SPLIT_MAX is the limit that the kernels look for.  Below 2^-110 the last piece runs into the smallest bfloat16,
+// 2^-133, and what lies under that is lost.
+constexpr float SPLIT_MAX = 3.38953139e38f;
+
+__device__ __forceinline__ uint32_t bf16x2_rn(float x0, float x1) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(x1), "f"(x0));
+    return r;
+}
 __device__ __forceinline__ void cut2(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l) {
-    const uint32_t u0 = __float_as_uint(x0), u1 = __float_as_uint(x1);
-    h = __byte_perm(u0, u1, 0x7632);
-    const float r0 = x0 - __uint_as_float(u0 & 0xffff0000u), r1 = x1 - __uint_as_float(u1 & 0xffff0000u);
-    const uint32_t v0 = __float_as_uint(r0), v1 = __float_as_uint(r1);
-    m = __byte_perm(v0, v1, 0x7632);
-    const float s0 = r0 - __uint_as_float(v0 & 0xffff0000u), s1 = r1 - __uint_as_float(v1 & 0xffff0000u);
-    l = __byte_perm(__float_as_uint(s0), __float_as_uint(s1), 0x7632);
+    h = bf16x2_rn(x0, x1);
+    const float r0 = x0 - __uint_as_float(h << 16), r1 = x1 - __uint_as_float(h & 0xffff0000u);
+    m = bf16x2_rn(r0, r1);
+    l = bf16x2_rn(r0 - __uint_as_float(m << 16), r1 - __uint_as_float(m & 0xffff0000u));
 }
 
 // 8 values -> the 16 bytes of each piece

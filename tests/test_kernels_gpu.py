@@ -1214,3 +1214,72 @@ def test_a_kernel_that_gives_up_is_noticed_by_the_host(ops):
     with pytest.raises(ops.KernelError, match="decode attention"):
         ops.check_device_errors()            # the thorough check synchronises by itself
     ops.check_device_errors()
+
+
+def _just_under(shape, seed, signed):
+    """Values just under 1 + 2^-7, the worst place of a cut into bfloat16 pieces that drops bits instead of rounding: every
+    dropped product then has the sign of the whole one, 2^-22 of it on average."""
+    g = torch.Generator().manual_seed(seed)
+    v = (1 + 2.0 ** -7 - 2.0 ** -14 * torch.rand(*shape, generator=g, dtype=torch.float64)).float()
+    return (v * (torch.randint(0, 2, shape, generator=g) * 2 - 1) if signed else v).to(DEV)
+
+
+@pytest.mark.parametrize("signed", [False, True])
+@pytest.mark.parametrize("K", [128, 768, 3072])
+def test_float32_pieces_at_their_worst_values(ops, K, signed):
+    """The product in pieces is no further from float64 than the chain of fmaf where the cut matters most.  What bias is
+    left comes from the accumulator, which drops bits: at most the last bit, 2^-23 of the sum, in one of the four full-size
+    additions of a block of 64, half of that on average."""
+    x, w = _just_under((200, K), K, signed), _just_under((1100, K), K + 1, signed)
+    exact = x.double() @ w.double().t()
+    err = []
+    for impl in ("split_f32", "simt"):
+        out = torch.empty(200, 1100, device=DEV)
+        ops.linear(x, w, None, out=out, impl=impl)
+        err.append(((out.double() - exact).norm() / exact.norm()).item())
+        if impl == "split_f32" and not signed:
+            assert ((out.double() - exact) / exact).mean().abs() < 2 ** -23
+    assert err[0] <= err[1], err
+    # the largest finite values round to infinity as pieces: such sums are formed again by K fmaf, each off by 2^-24 at most
+    x[7, 3], w[:, 3], w[12, 3] = 3.4028234e38, 2.0 ** -100, 0.0
+    out = torch.empty(200, 1100, device=DEV)
+    ops.linear(x, w, None, out=out, impl="split_f32")
+    exact = x[7].double() @ w.double().t()
+    assert torch.all((out[7].double() - exact).abs() <= K * 2.0 ** -24 * exact.abs().max()) and torch.isfinite(out[7]).all()
+    ops.check_device_errors()
+
+
+@pytest.mark.parametrize("signed", [False, True])
+def test_float32_attention_pieces_at_their_worst_values(ops, signed):
+    """The same for scores (products of 64) and weighted values, beside the plain kernel's fmaf; keys among the largest
+    finite values."""
+    from mini_llm_b200.engine.context import ATTN_TILE_WIDE, attention_tiles
+    H, dh, page, seqs = 4, 64, 16, [(300, 300), (500, 200)]
+    case = _paged_case(torch.float32, seqs, H, H, dh, page, num_pages=100, seed=3)
+    for i, (K, V) in enumerate(case["dense"]):
+        case["dense"][i] = (_just_under(K.shape, i, signed).cpu(), _just_under(V.shape, 9 + i, signed).cpu())
+        for p in range(len(K)):
+            at = case["bt"][i, p // page], slice(None), p % page
+            case["k_pages"][at], case["v_pages"][at] = case["dense"][i][0][p], case["dense"][i][1][p]
+    case["q"] = _just_under(case["q"].shape, 5, signed).cpu()
+    ctx = _ctx_for(case)
+    tiles = attention_tiles([n for _, n in seqs], [c - n for c, n in seqs], ATTN_TILE_WIDE)
+    ctx.attn_tiles_wide, ctx.n_tiles_wide = torch.tensor(tiles, dtype=torch.int32, device=DEV), len(tiles) // 3
+    ctx.decode_only = False
+    q, kp, vp, bt = case["q"].to(DEV), case["k_pages"].to(DEV), case["v_pages"].to(DEV), case["bt"].to(DEV)
+    kw = dict(num_heads=H, num_kv_heads=H, head_dim=dh, scale=dh ** -0.5)
+    want = _attention_reference(case, H, H, dh, dh ** -0.5, None, torch.float32).to(DEV)
+    err, out = [], {}
+    for impl in ("split_f32", "simt"):
+        out[impl] = torch.empty_like(q)
+        ops.paged_attention(q, kp, vp, bt, ctx, out[impl], impl=impl, **kw)
+        err.append(((out[impl].double() - want).norm() / want.norm()).item())
+    assert err[0] <= err[1], err
+    q[5] *= 2.0 ** -120                                  # scores that stay finite beside a key of 3.4e38
+    kp[int(bt[0, 0]), 1, 2, 7] = 3.4028234e38
+    for impl in out:
+        ops.paged_attention(q, kp, vp, bt, ctx, out[impl], impl=impl, **kw)
+    assert torch.equal(out["split_f32"].isnan(), out["simt"].isnan())
+    # scores of up to 32 are off by 32 x 2^-24 in either kernel, so weights that sum to 1, times values of 1, by 2 x 2e-6
+    assert torch.allclose(out["split_f32"][5], out["simt"][5], rtol=1e-5, atol=4e-6)
+    ops.check_device_errors()

@@ -77,3 +77,36 @@ def test_slices_of_a_product_are_summed_in_the_callers_own_scratch(ops, monkeypa
     version = a.version
     x = torch.zeros(1000, 768)
     assert scratch(a, 1000) and a.version > version          # a larger buffer is seen by whoever keeps its address
+
+
+def _pieces(x, rounded):
+    """The cut of csrc/split_f32.cuh: to nearest, or (what it must not do) by dropping the lower bits."""
+    import numpy as np
+
+    def bf16(v):
+        u = v.view(np.uint32)
+        if rounded:
+            u = (u.astype(np.uint64) + 0x7fff + ((u >> 16) & 1)).astype(np.uint32)
+        return (u & np.uint32(0xffff0000)).view(np.float32)
+
+    h = bf16(x)
+    m = bf16(x - h)
+    low = x - h - m
+    assert np.array_equal(bf16(low), low)
+    return [p.astype(np.float64) for p in (h, m, low)]
+
+
+def test_dropped_products_of_pieces():
+    """Of the nine products of pieces six are formed.  Cut to nearest, all pieces are exact, the three dropped products are
+    below 2^-24 of the whole and have either sign; with bits dropped they reach 2^-21 and never change sign."""
+    import numpy as np
+    rng = np.random.default_rng(1)
+    for lo, hi in ((0x3f800000, 0x40000000), (0x3f80f000, 0x3f810000)):
+        x, y = (rng.integers(lo, hi, 1 << 20).astype(np.uint32).view(np.float32) for _ in range(2))
+        lost = {}
+        for rounded in (True, False):
+            a, b = _pieces(x, rounded), _pieces(y, rounded)
+            assert np.array_equal(a[0] + a[1] + a[2], x.astype(np.float64))
+            lost[rounded] = (a[1] * b[2] + a[2] * b[1] + a[2] * b[2]) / (x.astype(np.float64) * y)
+        assert np.abs(lost[True]).max() < 2 ** -24 and abs(lost[True].mean()) < 2 ** -34
+        assert lost[False].min() >= 0 and lost[False].mean() > 2 ** -25
