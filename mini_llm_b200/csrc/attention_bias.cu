@@ -22,7 +22,7 @@
 // Four kernels (the fourth, `mma`, is described where it stands).  `simt`: one warp per (token, head), 32 keys at a time: any step, and the plain twin of the
 // others.  `tiled`: 64 queries x 32 keys per CTA and head for prompt portions: queries in shared memory, a key
 // tile staged transposed and a value tile as it is, 2 x 4 scores and 2 x dv/8 outputs per thread.  `split`: single
-// tokens (decode): the keys of a token are cut into splits of 64 starting at multiples of 64 from position 0, a
+// tokens (decode): the keys of a token are cut into splits whose places follow from the position (KeyCuts), a
 // CTA takes one split for up to four query heads that share a key/value head (rows staged once in shared memory),
 // the partial (o, m, l) of the splits are merged in split order by a second kernel.  Key chunks and tiles start at multiples of 32 from position 0 in all three, so a token's
 // sums run in an order that depends on its position only, not on how the step was cut or batched.
@@ -177,15 +177,11 @@ attention_bias_simt_kernel(const T* q, long long q_stride, const T* k_pages, con
 }
 
 // ------------------------------------------------------------------------------------------------ decode
-// keys per split: with 256 a launch at 4 requests and contexts of 510 took 23.5 us on 32 CTAs that each met the latency of
-// their loads four times; with 64 it takes 11.0 (at 64 requests 75 us either way; the merge 4 us either way)
-constexpr int SPLIT = 64;
-
 // Single tokens.  grid (splits, kv heads x head chunks, tokens).  A CTA takes one split of one token's keys for HG
 // (1, 2 or 4) query heads that share a key/value head, so a key or value row is fetched once for all of them.  The
-// split is walked in tiles of 32 * KS * NT keys (KS = 4 / HG warps per head; NT chunks per warp: the whole split at once
-// where shared memory allows) that are staged in shared memory with 16-byte loads (all loads of a burst before any
-// store); warp w takes head w % HG and the chunks w / HG, w / HG + KS, ...: its lanes are the 32 keys for the scores (a
+// split is walked in tiles of 32 * KS * NT keys (KS = 4 / HG warps per head, fewer where the shortest split has fewer
+// chunks; NT chunks per warp, in a small grid the whole split where shared memory allows) that are staged in shared memory
+// with 16-byte loads (all loads of a burst before any store); warp w takes head w % HG and the chunks w / HG, w / HG + KS, ...: its lanes are the 32 keys for the scores (a
 // row of K per lane, the query broadcast) and 32 value columns at a time for the weighted sum.  Chunks cover 32
 // consecutive positions starting at multiples of 32 from position 0.
 // Partial results: part_o [T][H][splits][dv], part_ml [T][H][splits][2]; a split without visible keys writes l = 0.
@@ -194,17 +190,20 @@ __global__ void __launch_bounds__(128)
 attention_bias_split_kernel(const T* q, long long q_stride, const T* k_pages, const T* v_pages,
                             const int* __restrict__ block_table, int bt_stride, const int* __restrict__ token_seq,
                             const int* __restrict__ positions, float* __restrict__ part_o, float* __restrict__ part_ml,
-                            int H, int Hkv, int dkq, int dk, int dv, int page_size, int HG, int KS, int NT, BiasArgs a) {
+                            int H, int Hkv, int dkq, int dk, int dv, int page_size, int HG, int KS, int max_nt, KeyCuts cuts,
+                            BiasArgs a) {
     extern __shared__ __align__(16) unsigned char smraw[];
     constexpr int VEC = 16 / sizeof(T);
     const int krow = dk + VEC;                                  // elements per staged key row: 16 bytes of padding
+    const int nsplit = gridDim.x, split = nsplit - 1 - blockIdx.x, t = blockIdx.z;       // the long splits first
+    const int k0 = cuts.first(split), keys = cuts.keys(split);
+    const int NT = min(max_nt, keys / (32 * KS));
     const int tile = 32 * KS * NT;                              // keys staged at a time: NT chunks of 32 per warp
     T* Ks = reinterpret_cast<T*>(smraw);                        // [tile][dk + VEC]
     T* Vs = Ks + (size_t)tile * krow;                           // [tile][dv]
     float* qs = reinterpret_cast<float*>(Vs + (((size_t)tile * dv + VEC - 1) / VEC) * VEC);   // [HG][dk]
     float* so = qs + HG * dk;                                   // [warps][dv] at the end
     float* sml = so + 4 * dv;                                   // [warps][2]
-    const int split = blockIdx.x, nsplit = gridDim.x, t = blockIdx.z;
     const int seq = __ldcg(token_seq + t), p = __ldcg(positions + t);        // written by the host before the step
     pdl_wait();
     pdl_launch();
@@ -216,7 +215,7 @@ attention_bias_split_kernel(const T* q, long long q_stride, const T* k_pages, co
     const int h = h0 + wh;
     const bool live = wh < nh;
     const int first = first_visible(a, p);
-    const int s_lo = split * SPLIT < a.keep ? split * SPLIT : max(first, split * SPLIT), s_hi = min(p, split * SPLIT + SPLIT - 1);
+    const int s_lo = k0 < a.keep ? k0 : max(first, k0), s_hi = min(p, k0 + keys - 1);
     if (s_lo > s_hi) {                                          // uniform over the CTA
         if (tid < nh) { const size_t pi = ((size_t)t * H + h0 + tid) * nsplit + split; part_ml[pi * 2] = -INFINITY; part_ml[pi * 2 + 1] = 0.f; }
         return;
@@ -240,8 +239,8 @@ attention_bias_split_kernel(const T* q, long long q_stride, const T* k_pages, co
     for (int base = (s_lo / tile) * tile; base <= s_hi; base += tile) {
         if (in_gap(a, base, base + tile - 1, first)) continue;  // uniform over the CTA
         __syncthreads();                                        // the tile before is no longer read; qs is complete
-        // the loads of a burst of keys and a burst of values are all in flight before the first is stored
         constexpr int LD = 4;
+        // the loads of a burst of keys and a burst of values are all in flight before the first is stored
         const int nkp = tile * kpieces, nvp = tile * vpieces;
         for (int i0 = tid; i0 < max(nkp, nvp); i0 += nthreads * LD) {
             uint4 rk[LD], rv[LD];
@@ -356,12 +355,12 @@ template <typename T>
 __global__ void __launch_bounds__(WARPS * 32)
 attention_bias_merge_kernel(const float* part_o, const float* part_ml, const int* __restrict__ positions,
                             T* __restrict__ out, long long out_stride, int T_tokens, int H, int dv, int nsplit,
-                            BiasArgs a) {
+                            KeyCuts cuts, BiasArgs a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long gw = (long long)blockIdx.x * WARPS + warp;
     if (gw >= (long long)T_tokens * H) return;
     const int t = (int)(gw / H), h = (int)(gw % H);
-    const int used = min(nsplit, __ldcg(positions + t) / SPLIT + 1);         // positions: written by the host before the step
+    const int used = min(nsplit, cuts.splits(__ldcg(positions + t)));       // positions: written by the host before the step
     const float* sink = a.sink;
     const float sk = sink ? sink[h] : -INFINITY;
     pdl_wait();
@@ -861,14 +860,12 @@ int check_sizes(int H, int Hkv, int dk, int dv, int page_size, int dtype) {
 
 }  // namespace
 
-MLLM_EXPORT int mllm_attention_bias_split_keys() { return SPLIT; }
-
-// impl: 0 simt, 1 tiled (needs tiles), 2 split (single tokens; needs part_o [T*H*nsplit*dv], part_ml [T*H*nsplit*2]),
-// 3 mma (bfloat16 prompt portions on tensor cores; needs tiles).
+// impl: 0 simt, 1 tiled (needs tiles), 2 split (single tokens; needs part_o [T*H*nsplit*dv], part_ml [T*H*nsplit*2] and the
+// cuts of the keys, at least as many splits as the longest context has), 3 mma (bfloat16 prompt portions on tensor cores; needs tiles).
 MLLM_EXPORT int mllm_attention_bias(const void* q, long long q_stride, const void* k_pages, const void* v_pages,
                                     const int* block_table, int bt_stride, const int* token_seq, const int* positions,
                                     const int* tiles, int n_tiles, void* out, long long out_stride, float* part_o,
-                                    float* part_ml, int nsplit, int T, int H, int Hkv, int dkq, int dk, int dv, int page_size,
+                                    float* part_ml, int nsplit, int near, int edge, int far, int T, int H, int Hkv, int dkq, int dk, int dv, int page_size,
                                     float scale, float out_scale, const float* dist_bias, int n_dist,
                                     const float* q_scale, int window, int chunk, const float* sink, float softcap,
                                     const float* slopes, int keep_first, const void* gate, long long gate_stride, int dtype, int impl,
@@ -915,6 +912,8 @@ MLLM_EXPORT int mllm_attention_bias(const void* q, long long q_stride, const voi
     }
     if (impl == 2) {
         if (!part_o || !part_ml || nsplit <= 0) return mllm_fail(1, "attention_bias: the split kernel needs scratch for its partial results");
+        KeyCuts cuts;
+        if (int rc = key_cuts("attention_bias", near, edge, far, &cuts)) return rc;
         const int R = H / Hkv;
         int HG = R >= 4 ? 4 : (R >= 2 ? 2 : 1), KS = 4 / HG;
         const size_t es = dtype == MLLM_F32 ? 4 : 2, vec = 16 / es;
@@ -922,7 +921,7 @@ MLLM_EXPORT int mllm_attention_bias(const void* q, long long q_stride, const voi
             const size_t tile = 32 * (size_t)ks;
             return tile * (dk + vec) * es + ((tile * dv + vec - 1) / vec) * vec * es + sizeof(float) * ((size_t)HG * dk + 4 * (size_t)dv + 8);
         };
-        while (KS > 1 && bytes(KS) > 96 * 1024) KS /= 2;
+        while (KS > 1 && (32 * KS > cuts.near || bytes(KS) > 96 * 1024)) KS /= 2;
         // A whole split staged at once (one round of loads) where it fits and the grid
         // is small: with few CTAs nothing else hides the loads' latency.  In a large grid (measured at batch 64: 0.57
         // against 0.71 ms per step) small tiles win, since more CTAs fit an SM and hide each other's loads.  A warp
@@ -933,31 +932,27 @@ MLLM_EXPORT int mllm_attention_bias(const void* q, long long q_stride, const voi
             MLLM_CUDA(cudaGetDevice(&dev));
             MLLM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         }
-        int NT = 1;
-        if ((long long)nsplit * Hkv * ((R + HG - 1) / HG) * T <= 4LL * sms)
-            while (32 * KS * NT * 2 <= SPLIT && bytes(KS * NT * 2) <= 96 * 1024) NT *= 2;
-        const size_t smem = bytes(KS * NT);
         const int chunks = (R + HG - 1) / HG;
+        const bool few = (long long)nsplit * Hkv * chunks * T <= 4LL * sms;
+        int NT = 1;
+        if (few)
+            while (32 * KS * NT * 2 <= cuts.keys(nsplit - 1) && bytes(KS * NT * 2) <= 96 * 1024) NT *= 2;
+        const size_t smem = bytes(KS * NT);
         if ((long long)Hkv * chunks > 65535 || T > 65535) return mllm_fail(1, "attention_bias: %d heads x %d tokens exceed the split kernel's grid", H, T);
         const dim3 grid(nsplit, Hkv * chunks, T), block(32 * HG * KS);
-        if (dtype == MLLM_F32) {
-            if (smem > 48 * 1024) MLLM_CUDA(cudaFuncSetAttribute(attention_bias_split_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            MLLM_CUDA(mllm_launch(attention_bias_split_kernel<float>, grid, block, smem, stream, true,
-                                  (const float*)q, q_stride, (const float*)k_pages, (const float*)v_pages, block_table,
-                                  bt_stride, token_seq, positions, part_o, part_ml, H, Hkv, dkq, dk, dv, page_size, HG, KS, NT, a));
-            MLLM_CUDA(mllm_launch(attention_bias_merge_kernel<float>, dim3((unsigned)blocks), dim3(WARPS * 32), 0, stream, true,
-                                  (const float*)part_o, (const float*)part_ml, positions, (float*)out, out_stride, T, H, dv,
-                                  nsplit, a));
-        } else {
-            if (smem > 48 * 1024) MLLM_CUDA(cudaFuncSetAttribute(attention_bias_split_kernel<bf>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            MLLM_CUDA(mllm_launch(attention_bias_split_kernel<bf>, grid, block, smem, stream, true,
-                                  (const bf*)q, q_stride, (const bf*)k_pages, (const bf*)v_pages, block_table, bt_stride,
-                                  token_seq, positions, part_o, part_ml, H, Hkv, dkq, dk, dv, page_size, HG, KS, NT, a));
-            MLLM_CUDA(mllm_launch(attention_bias_merge_kernel<bf>, dim3((unsigned)blocks), dim3(WARPS * 32), 0, stream, true,
-                                  (const float*)part_o, (const float*)part_ml, positions, (bf*)out, out_stride, T, H, dv,
-                                  nsplit, a));
-        }
-        return 0;
+        auto go = [&](auto kern, auto merge, auto* tq, auto* tk, auto* tv, auto* to) -> int {
+            if (smem > 48 * 1024) MLLM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            MLLM_CUDA(mllm_launch(kern, grid, block, smem, stream, true, tq, q_stride, tk, tv, block_table, bt_stride, token_seq,
+                                  positions, part_o, part_ml, H, Hkv, dkq, dk, dv, page_size, HG, KS, NT, cuts, a));
+            MLLM_CUDA(mllm_launch(merge, dim3((unsigned)blocks), dim3(WARPS * 32), 0, stream, true, (const float*)part_o,
+                                  (const float*)part_ml, positions, to, out_stride, T, H, dv, nsplit, cuts, a));
+            return 0;
+        };
+        if (dtype == MLLM_F32)
+            return go(attention_bias_split_kernel<float>,
+                      attention_bias_merge_kernel<float>, (const float*)q, (const float*)k_pages, (const float*)v_pages, (float*)out);
+        return go(attention_bias_split_kernel<bf>,
+                  attention_bias_merge_kernel<bf>, (const bf*)q, (const bf*)k_pages, (const bf*)v_pages, (bf*)out);
     }
     if (impl == 3) {
         if (!tiles || n_tiles <= 0) return mllm_fail(1, "attention_bias: the tensor-core kernel needs the step's tile list");

@@ -142,3 +142,27 @@ __device__ __forceinline__ float apply_act(float v, int act) {
     if (act == MLLM_ACT_GELU_ERF) return gelu_erf_f(v);
     return v;
 }
+
+// How the keys of a single token are cut into splits, one per CTA: `near` keys each below position `edge`, then twice as
+// many (at most `far`) up to twice that position, then `far`.  A split's place follows from the position alone, so a token's
+// sums run in the same order whatever else is in the step.
+struct KeyCuts {
+    int near, mid, far, edge, n_near, n_mid;             // n_near splits below edge, n_mid below 2 * edge
+    __host__ __device__ int first(int split) const {
+        return split < n_near ? split * near : split < n_mid ? edge + (split - n_near) * mid : 2 * edge + (split - n_mid) * far;
+    }
+    __host__ __device__ int keys(int split) const { return split < n_near ? near : split < n_mid ? mid : far; }
+    __host__ __device__ int splits(int position) const {      // up to and with this position
+        return position < edge       ? position / near + 1
+               : position < 2 * edge ? n_near + (position - edge) / mid + 1
+                                     : n_mid + (position - 2 * edge) / far + 1;
+    }
+};
+// 0, or a refusal: spans are powers of two from 32 on, the far one no shorter, and every span starts at a multiple of itself.
+inline int key_cuts(const char* who, int near, int edge, int far, KeyCuts* out) {
+    const int mid = 2 * near < far ? 2 * near : far;
+    if (near < 32 || (near & (near - 1)) || far < near || (far & (far - 1)) || edge < 0 || edge % mid || 2 * edge % far)
+        return mllm_fail(1, "%s: splits of %d keys below position %d and of %d beyond", who, near, edge, far);
+    *out = KeyCuts{near, mid, far, edge, edge / near, edge / near + edge / mid};
+    return 0;
+}

@@ -12,13 +12,13 @@
 //                    the absorbed query (W = W_uk^T per head) and the head outputs (W = W_uv per head, with the gate).
 //                    Three kernels: CUDA-core tiles (32-bit weights, odd sizes), tensor-core tiles (bfloat16 weights,
 //                    more than 16 tokens), and for up to 16 tokens a CTA per (token, head) that streams its weights.
-//   latent_attention one CTA per (split of `span` keys, token, block of 8 heads): key rows are staged once for all the
+//   latent_attention one CTA per (split of keys, token, block of 8 heads): key rows are staged once for all the
 //                    heads of the block in chunks of 32 that start at multiples of 32 from position 0; a warp is a
 //                    head, its lanes are the 32 keys for the scores and 64 latent columns at a time for the weighted
 //                    sum; online softmax in 32-bit with expf.  Partial (o, m, l) per split, merged in split order by
-//                    latent_merge.  Splits and chunks are fixed ranges of positions, so at one span a token's sums run
-//                    in the same order whether it came in a prompt portion, alone, or in a batch (the caller takes
-//                    short splits for steps of single tokens, to fill the GPU, and long ones otherwise).  A sink (a
+//                    latent_merge.  Splits and chunks are fixed ranges of positions, so with the same cuts a token's sums
+//                    run in the same order whether it came in a prompt portion, alone, or in a batch (the caller takes
+//                    shorter splits for steps of single tokens, to fill the GPU, than for prompt portions).  A sink (a
 //                    number per head) adds exp(sink) to the softmax's denominator and to nothing else: the merge starts
 //                    from it, and the tensor-core kernel's running maximum and sum do.
 #include "common.cuh"
@@ -27,6 +27,7 @@ namespace {
 
 constexpr int HB = 8;           // heads (warps) per CTA
 constexpr int MAX_SMEM = 227 * 1024;    // dynamic shared memory a CTA can have on this GPU
+constexpr size_t BUFS_LIMIT = 75 * 1024;    // a CTA takes two chunk buffers up to here: three such CTAs fit an SM
 constexpr int MAX_R = 512;      // largest latent size
 constexpr int MAX_DK = 1024;    // largest R + dr
 
@@ -177,10 +178,10 @@ headwise_rows_kernel(const TI* in, long long ld_in, int in_head, const TW* __res
     }
 }
 
-// grid (splits, tokens, head blocks); dynamic shared memory: HB * dkp floats of queries, then two chunks of 32 key rows
+// grid (splits, tokens, head blocks); dynamic shared memory: HB * dkp floats of queries, then `bufs` chunks of 32 key rows
 // of `kw` 32-bit words each (kw = a row's words + 4: rows stay 16-byte aligned for cp.async and 128-bit reads, and eight
-// lanes reading 16 bytes of eight consecutive rows touch all 32 banks).  A CTA walks the keys [split * span, ...) of its
-// token in chunks of 32, the next chunk's rows in flight (cp.async) while the current one is used.
+// lanes reading 16 bytes of eight consecutive rows touch all 32 banks).  A CTA walks the keys of its split in
+// chunks of 32, with two buffers the next chunk's rows in flight (cp.async) while the current one is used.
 __device__ __forceinline__ void cp16(void* dst, const void* src) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
@@ -190,7 +191,7 @@ template <typename T, int NACC>
 __global__ void __launch_bounds__(HB * 32)
 latent_attention_kernel(const float* qa, const T* pages, int row, const int* block_table, int bt_stride,
                         const int* token_seq, const int* positions, float* part_o, float* part_ml, int nsplit, int H,
-                        int R, int dk, int ps, float scale, int kw, int span) {
+                        int R, int dk, int ps, float scale, int kw, int bufs, KeyCuts cuts) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int EPW = 4 / sizeof(T);                  // elements per 32-bit word
     constexpr int V = 16 / sizeof(T);                   // elements per 16 bytes
@@ -198,11 +199,11 @@ latent_attention_kernel(const float* qa, const T* pages, int row, const int* blo
     float* qs = reinterpret_cast<float*>(smem_raw);
     uint32_t* ks = reinterpret_cast<uint32_t*>(qs + HB * dkp);
     pdl_wait();
-    const int t = blockIdx.y, split = blockIdx.x;
+    const int t = blockIdx.y, split = gridDim.x - 1 - blockIdx.x;       // the long splits first
     const int p = positions[t];
-    const int k_lo = split * span;
+    const int k_lo = cuts.first(split);
     if (k_lo > p) return;
-    const int k_hi = min(k_lo + span - 1, p);           // inclusive
+    const int k_hi = min(k_lo + cuts.keys(split) - 1, p);          // inclusive
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h0 = blockIdx.z * HB, h = h0 + warp;
     const int nh = min(HB, H - h0);
@@ -229,10 +230,14 @@ latent_attention_kernel(const float* qa, const T* pages, int row, const int* blo
     for (int i = 0; i < NACC; ++i) acc[i] = 0.f;
     const float* q = qs + warp * dkp;
     int buf = 0;
-    for (int base = k_lo; base <= k_hi; base += 32, buf ^= 1) {
+    for (int base = k_lo; base <= k_hi; base += 32, buf ^= bufs - 1) {
+        if (bufs == 1 && base > k_lo) {
+            __syncthreads();        // the chunk before has been used
+            stage(base, 0);
+        }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();            // this chunk (and the queries) are in; the other buffer has been used
-        if (base + 32 <= k_hi) stage(base + 32, buf ^ 1);
+        if (bufs == 2 && base + 32 <= k_hi) stage(base + 32, buf ^ 1);
         const int nk = min(32, k_hi - base + 1);
         if (h >= H) continue;
         const uint32_t* kc = ks + buf * 32 * kw;
@@ -310,11 +315,11 @@ latent_attention_kernel(const float* qa, const T* pages, int row, const int* blo
 // of the sum at a time.  With a warp per (token, head) the twelve columns of a lane stood one after the other.
 __global__ void __launch_bounds__(128)
 latent_merge_kernel(const float* part_o, const float* part_ml, const int* positions, float* out, int nsplit, int H, int R,
-                    int span, const float* __restrict__ sink) {
+                    KeyCuts cuts, const float* __restrict__ sink) {
     __shared__ float wgt[128];                               // the weights of 128 splits at a time
     pdl_wait();
     const int th = blockIdx.x, tid = threadIdx.x;
-    const int ns = positions[th / H] / span + 1;
+    const int ns = cuts.splits(positions[th / H]);
     const size_t o = (size_t)th * nsplit;
     const float sk = sink ? sink[th % H] : -INFINITY;
     float M = sk;
@@ -347,34 +352,40 @@ latent_merge_kernel(const float* part_o, const float* part_ml, const int* positi
 template <typename T, int NACC>
 int launch_attention(const float* qa, const void* pages, int row, const int* bt, int bt_stride, const int* token_seq,
                      const int* positions, float* part_o, float* part_ml, int nsplit, int Tn, int H, int R, int dk,
-                     int ps, float scale, int span, cudaStream_t stream) {
+                     int ps, float scale, const KeyCuts& cuts, cudaStream_t stream) {
     const int kw = row * (int)sizeof(T) / 4 + 4;
     const int V = 16 / (int)sizeof(T), dkp = (dk + V - 1) / V * V;
-    const size_t smem = (size_t)HB * dkp * 4 + (size_t)(span > 32 ? 2 : 1) * 32 * kw * 4;      // a split of one chunk needs one buffer
+    auto bytes = [&](int bufs) { return (size_t)HB * dkp * 4 + (size_t)bufs * 32 * kw * 4; };
+    // One buffer where every split is a single chunk of 32 keys, and where two would leave fewer than three CTAs per SM: 64
+    // tokens at contexts of 1,000, splits of 128 keys, one / two buffers: bfloat16, 64 heads of rank 512 677 / 764 us, 16 heads
+    // 194 / 226, 12 heads of 384 (three CTAs with two) 142 / 140; float32, 12 heads of 384 197 / 330.
+    const bool single = nsplit <= cuts.n_near ? cuts.near == 32 : cuts.far == 32;
+    const int bufs = single || bytes(2) > BUFS_LIMIT ? 1 : 2;
+    const size_t smem = bytes(bufs);
     static bool raised = false;                     // once per instantiation
     if (smem > 48 * 1024 && !raised) {
         MLLM_CUDA(cudaFuncSetAttribute(latent_attention_kernel<T, NACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
         raised = true;
     }
-    if (smem > MAX_SMEM) return mllm_fail(1, "latent_attention: rows of %d need %zu bytes of shared memory", dk, smem);
+    if (bytes(2) > MAX_SMEM) return mllm_fail(1, "latent_attention: rows of %d need %zu bytes of shared memory", dk, bytes(2));
     MLLM_CUDA(mllm_launch(latent_attention_kernel<T, NACC>, dim3(nsplit, Tn, (H + HB - 1) / HB), dim3(HB * 32), smem, stream,
                           true, qa, (const T*)pages, row, bt, bt_stride, token_seq, positions, part_o, part_ml, nsplit, H,
-                          R, dk, ps, scale, kw, span));
+                          R, dk, ps, scale, kw, bufs, cuts));
     return 0;
 }
 
 template <typename T>
 int pick_attention(int R, const float* qa, const void* pages, int row, const int* bt, int bt_stride, const int* token_seq,
                    const int* positions, float* part_o, float* part_ml, int nsplit, int Tn, int H, int dk, int ps,
-                   float scale, int span, cudaStream_t stream) {
+                   float scale, const KeyCuts& cuts, cudaStream_t stream) {
     if (R <= 128)
         return launch_attention<T, 4>(qa, pages, row, bt, bt_stride, token_seq, positions, part_o, part_ml, nsplit, Tn, H, R,
-                                      dk, ps, scale, span, stream);
+                                      dk, ps, scale, cuts, stream);
     if (R <= 256)
         return launch_attention<T, 8>(qa, pages, row, bt, bt_stride, token_seq, positions, part_o, part_ml, nsplit, Tn, H, R,
-                                      dk, ps, scale, span, stream);
+                                      dk, ps, scale, cuts, stream);
     return launch_attention<T, 16>(qa, pages, row, bt, bt_stride, token_seq, positions, part_o, part_ml, nsplit, Tn, H, R, dk,
-                                   ps, scale, span, stream);
+                                   ps, scale, cuts, stream);
 }
 
 
@@ -799,29 +810,30 @@ MLLM_EXPORT int mllm_headwise_linear(const void* in, long long ld_in, int in_hea
 }
 
 // qa [T][H][dk] 32-bit, pages [slots][row] in `dtype` (a token's row: R latent columns, then dk - R rotated key columns),
-// out [T][H][R] 32-bit; part_o [T * H * nsplit * R], part_ml [T * H * nsplit * 2] scratch; nsplit >= ceil(longest context / span).
+// out [T][H][R] 32-bit; part_o [T * H * nsplit * R], part_ml [T * H * nsplit * 2] scratch; nsplit at least the splits of the longest context.
 MLLM_EXPORT int mllm_latent_attention(const float* qa, const void* pages, int row, const int* block_table, int bt_stride,
                                       const int* token_seq, const int* positions, float* part_o, float* part_ml, int nsplit,
-                                      float* out, int Tn, int H, int R, int dk, int ps, float scale, int span, const float* sink,
+                                      float* out, int Tn, int H, int R, int dk, int ps, float scale, int near, int edge, int far, const float* sink,
                                       int dtype, cudaStream_t stream) {
     if (Tn <= 0) return 0;
     if (R <= 0 || R > MAX_R || dk < R || dk > MAX_DK) return mllm_fail(1, "latent_attention: latent size %d (at most %d), key size %d (at most %d)", R, MAX_R, dk, MAX_DK);
     const int es = dtype == MLLM_F32 ? 4 : 2;
     if (row < dk || (row * es) % 16 != 0 || (uintptr_t)pages % 16 != 0) return mllm_fail(1, "latent_attention: cache rows of %d elements must hold %d and be multiples of 16 bytes", row, dk);
     if (Tn > 65535) return mllm_fail(1, "latent_attention: more than 65535 tokens in a step");
-    if (span < 32 || span % 32) return mllm_fail(1, "latent_attention: a split of %d keys (a multiple of 32)", span);
-    int rc;
+    KeyCuts cuts;
+    int rc = key_cuts("latent_attention", near, edge, far, &cuts);
+    if (rc) return rc;
     if (dtype == MLLM_F32)
         rc = pick_attention<float>(R, qa, pages, row, block_table, bt_stride, token_seq, positions, part_o, part_ml, nsplit, Tn,
-                                   H, dk, ps, scale, span, stream);
+                                   H, dk, ps, scale, cuts, stream);
     else if (dtype == MLLM_BF16)
         rc = pick_attention<__nv_bfloat16>(R, qa, pages, row, block_table, bt_stride, token_seq, positions, part_o, part_ml,
-                                           nsplit, Tn, H, dk, ps, scale, span, stream);
+                                           nsplit, Tn, H, dk, ps, scale, cuts, stream);
     else
         return mllm_fail(1, "latent_attention: unknown dtype code %d", dtype);
     if (rc) return rc;
     MLLM_CUDA(mllm_launch(latent_merge_kernel, dim3(Tn * H), dim3(128), 0, stream, true, part_o, part_ml, positions, out, nsplit,
-                          H, R, span, sink));
+                          H, R, cuts, sink));
     return 0;
 }
 

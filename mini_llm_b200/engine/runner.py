@@ -302,7 +302,7 @@ class ModelRunner:
             self._graph_version = self.ws.version
         key = (ctx.layout.key(), ops.decode_splits(ctx.max_ctx_len) if ctx.decode_only else
                ops.decode_splits(ctx.max_single_ctx_len) if ctx.single_runs else 0,
-               ops.latent_splits(ctx.max_ctx_len))      # every host-side number a launch's grid depends on
+               ops.split_context(ctx.max_ctx_len))      # every host-side number a launch's grid depends on
         g = self._graphs.get(key)
         if g is not None:
             g[0].replay()

@@ -117,10 +117,9 @@ def _signatures(lib):
         "mllm_paged_write": [c_void_p, c_ll, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "mllm_paged_write_kv": [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                 c_int, c_int, c_void_p],
-        "mllm_attention_bias_split_keys": [],
         "mllm_attention_bias": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int,
-                                c_void_p, c_ll, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                                c_float, c_float, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_float, c_void_p, c_int,
+                                c_void_p, c_ll, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+                                c_int, c_int, c_float, c_float, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_float, c_void_p, c_int,
                                 c_void_p, c_ll, c_int, c_int, c_void_p],
         "mllm_qk_norm_rope": [c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float,
                               c_void_p, c_int, c_int, c_void_p, c_void_p, c_ll, c_void_p, c_void_p, c_int, c_void_p, c_int,
@@ -154,7 +153,8 @@ def _signatures(lib):
         "mllm_headwise_linear": [c_void_p, c_ll, c_int, c_void_p, c_void_p, c_ll, c_int, c_void_p, c_ll, c_int, c_int, c_int,
                                  c_int, c_int, c_int, c_int, c_void_p],
         "mllm_latent_attention": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
-                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_void_p],
+                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p, c_int,
+                                  c_void_p],
         "mllm_latent_attention_mma": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int,
                                       c_int, c_int, c_int, c_float, c_void_p, c_void_p],
         "mllm_latent_mma_ok": [c_int, c_int, c_int],
@@ -997,7 +997,31 @@ def _bias_mma_ok(q, k_pages, v_pages, out, dk, dv, ldq, ldo) -> bool:
 
 
 BIAS_ATTN_MAX_DIM = 256        # largest key and value size of csrc/attention_bias.cu
-_bias_split_keys = None
+
+
+def split_context(max_ctx_len: int) -> int:
+    """The context length that the grids over splits of keys are made for: the step's longest rounded up to a power of two
+    (at least 32), so that captured graphs, whose shape it is part of, keep their grids."""
+    return 1 << (max(32, int(max_ctx_len)) - 1).bit_length()
+
+
+def key_splits(ctx_len: int, cuts) -> int:
+    """Splits of the first ``ctx_len`` keys under ``cuts`` = (keys per split below a position, that position, keys per split
+    from twice that position on; twice the first in between): csrc/common.cuh's KeyCuts."""
+    near, edge, far = cuts
+    return (-(-min(ctx_len, edge) // near) + -(-max(0, min(ctx_len, 2 * edge) - edge) // min(2 * near, far))
+            + -(-max(0, ctx_len - 2 * edge) // far))
+
+
+def bias_cuts(num_heads: int, num_kv_heads: int):
+    """How the biased attention cuts a single token's keys.  Short splits near the start let a few requests fill the GPU; far
+    ones are long, since every split starts a block, leaves a partial result and is merged.  us a launch with these cuts / with
+    256 keys throughout, bfloat16, heads of 64 (the biased attention's launch and its merge, caches not in L2):
+    12 heads over 4   1 request of 510 15 / 40, of 1,000 21 / 40; 16 of 1,000 46 / 80; 64 of 510 70 / 79, of 1,000 125 / 120
+    12 heads over 12  1 request of 510 17 / 35, of 1,000 17 / 35; 16 of 1,000 45 / 43; 64 of 510 78 / 74, of 1,000 137 / 134
+    With 64 keys throughout, 64 requests of 1,000 take 138 us (12 over 4) and 188 us (12 over 12, where a block of 64 keys has
+    two warps): heads that share no keys start at 128."""
+    return (128, 1024, 256) if num_heads == num_kv_heads else (64, 512, 256)
 
 
 def biased_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, num_kv_heads, scale, dist_bias=None,
@@ -1017,7 +1041,6 @@ def biased_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, n
     zeros), v_pages [P, kv_heads, page_size, dv], out [T, heads * dv] (rows contiguous; a column slice of a wider
     buffer is fine).
     """
-    global _bias_split_keys
     _cuda("q", q, contiguous=False)
     _cuda("k_pages", k_pages, q.dtype)
     _cuda("v_pages", v_pages, q.dtype)
@@ -1068,13 +1091,11 @@ def biased_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, n
                 impl = "mma"       # prompt portions in bfloat16: tensor cores
     attention_launches["bias_" + impl] = attention_launches.get("bias_" + impl, 0) + 1
     part_o = part_ml = None
-    nsplit = 0
+    nsplit, cuts = 0, (0, 0, 0)
     tiles, n_tiles = None, 0
     if impl == "split":
-        if _bias_split_keys is None:
-            _bias_split_keys = int(library().mllm_attention_bias_split_keys())
-        # splits cover the longest context of the step as ``latent_splits`` rounds it (part of a step's shape for captured graphs)
-        nsplit = max(1, latent_splits(ctx.max_ctx_len) * LATENT_SPAN_DECODE // _bias_split_keys)
+        cuts = bias_cuts(num_heads, num_kv_heads)
+        nsplit = key_splits(split_context(ctx.max_ctx_len), cuts)
         part_o = ctx.ws.buf("battn_part_o", T * num_heads * nsplit, dv, torch.float32).data_ptr()
         part_ml = ctx.ws.buf("battn_part_ml", T * num_heads * nsplit, 2, torch.float32).data_ptr()
     elif impl in ("tiled", "mma"):
@@ -1086,7 +1107,7 @@ def biased_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, n
         raise KernelError(f"biased_attention: unknown implementation {impl!r}")
     _call("mllm_attention_bias", q.data_ptr(), ldq, k_pages.data_ptr(), v_pages.data_ptr(), block_table.data_ptr(),
           _rows("block_table", block_table), ctx.token_seq.data_ptr(), ctx.positions.data_ptr(), tiles, n_tiles,
-          out.data_ptr(), ldo, part_o, part_ml, nsplit, T, num_heads, num_kv_heads, dkq, dk, dv, ps, float(scale),
+          out.data_ptr(), ldo, part_o, part_ml, nsplit, *cuts, T, num_heads, num_kv_heads, dkq, dk, dv, ps, float(scale),
           float(out_scale), dist_bias.data_ptr() if dist_bias is not None else None, n_dist,
           q_scale.data_ptr() if q_scale is not None else None, int(window or 0), int(chunk or 0),
           sink.data_ptr() if sink is not None else None, float(softcap or 0.0),
@@ -1169,10 +1190,9 @@ def mixed_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, nu
 
 
 def mixed_splits(max_ctx_len: int, window=None) -> int:
-    """Chunks of keys that a single token sees at most: as many as the context has (rounded so that the number follows from
-    ``latent_splits``, which is part of a step's shape for captured graphs), or the window can touch."""
+    """Chunks of keys that a single token sees at most: as many as the context has (of ``split_context``), or the window can touch."""
     chunk = int(library().mllm_attention_mixed_chunk())
-    n = max(1, latent_splits(max_ctx_len) * LATENT_SPAN_DECODE // chunk)
+    n = max(1, split_context(max_ctx_len) // chunk)
     return n if not window else min(n, (int(window) + chunk - 2) // chunk + 1)
 
 
@@ -1504,11 +1524,21 @@ def wkv_finish(o, z, weight, out, *, heads: int, eps: float) -> None:
 
 # --------------------------------------------------------------------------- attention over a cache of latents
 LATENT_MAX_RANK, LATENT_MAX_KEY = 512, 1024      # what csrc/latent_attention.cu takes
-# keys per CTA of the CUDA-core kernel: short splits when a step has single tokens only (a few long contexts must fill
-# the GPU), long ones when it has prompt portions (their tokens fill it, and every split costs a partial result).  Splits of
-# 32 instead of 128 keys: 13 against 42 us a launch at 3 requests and contexts of 250 (float32), 15 against 33 at 8 and 500
-# (bfloat16), 41 against 85 at 64 and 200 (float32), with 1 to 3 us more for the merge.
-LATENT_SPAN_DECODE, LATENT_SPAN_PROMPT = 32, 1024
+# a step with prompt portions: its tokens fill the GPU, and every split costs a partial result
+LATENT_CUTS_PROMPT = (1024, 0, 1024)
+
+
+def latent_cuts(heads: int, rank: int, dtype):
+    """How the latent attention on CUDA cores cuts a single token's keys: short near the start, where a few requests must fill
+    the GPU, longer from position 1,024 on.  us a launch with its merge, with these cuts / with 128 keys throughout, caches not
+    in L2:
+    bfloat16, 12 heads of rank 384    1 request of 250 26 / 39, of 8,000 60 / 57; 4 of 500 27 / 41; 64 of 200 45 / 49, of 1,000 142 / 140
+    bfloat16, 128 heads of rank 512   1 request of 250 30 / 47, of 8,000 214 / 205; 64 of 200 341 / 323, of 1,000 1,454 / 1,324
+    float32, 12 heads of rank 384     1 request of 250 21 / 48, of 8,000 82 / 69; 4 of 500 26 / 51; 64 of 200 52 / 63, of 1,000 199 / 197
+    Splits of 32 keys throughout took 172, 1,759 and 203 us at 64 requests of 1,000 and four times the scratch, which with these
+    cuts is that of 128 keys and a constant; in 32-bit, and where heads x rank keeps their partial results small, they are
+    worth it below position 1,024."""
+    return (32 if dtype == torch.float32 and heads * rank <= 32 * 512 else 64), 1024, 128
 
 
 def latent_prepare(proj, q_off: int, dkv_off: Optional[int], ctx, slot_mapping, freq, mscale: float, norm_weight, eps: float,
@@ -1618,22 +1648,15 @@ def latent_attention(qa, pages, block_table, ctx, out, *, heads: int, rank: int,
         return
     if impl != "split":
         raise KernelError(f"latent_attention: unknown implementation {impl!r}")
-    span = LATENT_SPAN_DECODE if getattr(ctx, "decode_only", False) else LATENT_SPAN_PROMPT
-    need = max(1, -(-int(ctx.max_ctx_len) // span))
-    nsplit = 1 << (need - 1).bit_length()       # a power of two: few distinct grids for captured graphs
+    cuts = latent_cuts(heads, rank, pages.dtype) if getattr(ctx, "decode_only", False) else LATENT_CUTS_PROMPT
+    nsplit = key_splits(split_context(ctx.max_ctx_len), cuts)
     part_o = ctx.ws.buf("latent_part_o", T * heads * nsplit, rank, torch.float32)
     part_ml = ctx.ws.buf("latent_part_ml", T * heads * nsplit, 2, torch.float32)
     _call("mllm_latent_attention", qa.data_ptr(), pages.data_ptr(), row, block_table.data_ptr(), _rows("block_table", block_table),
           ctx.token_seq.data_ptr(), ctx.positions.data_ptr(), part_o.data_ptr(), part_ml.data_ptr(), nsplit, out.data_ptr(),
-          T, heads, rank, dk, ps, float(scale), span, sink_ptr, _dt(pages), _stream())
+          T, heads, rank, dk, ps, float(scale), *cuts, sink_ptr, _dt(pages), _stream())
     global launches
     launches += 1           # the kernel that merges the splits
-
-
-def latent_splits(max_ctx_len: int) -> int:
-    """Splits of the latent attention at a context length (part of a step's shape for captured graphs)."""
-    need = max(1, -(-int(max_ctx_len) // LATENT_SPAN_DECODE))
-    return 1 << (need - 1).bit_length()
 
 
 # --------------------------------------------------------------------------- matrix memory

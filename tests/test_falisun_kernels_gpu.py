@@ -451,3 +451,25 @@ def test_router_and_experts(ops, dtype, T, D, E, top, groups, keep, F, shared):
     y2 = torch.full((T, D), 3.0, device=DEV)
     ff.forward(h, ctx, y2, accumulate=True)
     assert (y2 - 3.0 - y).abs().max() < 1e-4 * max(1.0, y.abs().max().item())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,R,dr", [(3, 40, 8), (40, 500, 12)])
+def test_latent_attention_single_tokens_across_the_cuts(ops, dtype, H, R, dr):
+    """Single tokens at contexts on both sides of a split's edge, of the position where the splits get longer and beyond
+    it; a token has the same bits alone as beside longer contexts, whose step has a larger grid."""
+    near, edge, far = ops.latent_cuts(H, R, dtype)
+    seqs = [(c, 1) for c in (1, 31, near, near + 1, 2 * near + 1, edge - 1, edge, edge + 1, edge + 2 * near, edge + 2 * near + 1,
+                             2 * edge, 2 * edge + 1, 2 * edge + far + 1)]
+    scale = 0.1
+    ctx, qa, pages, bt, dense = _latent_case(dtype, seqs, H, R, dr, 16, seed=H)
+    ctx.decode_only = True
+    out = torch.full((ctx.T, H * R), 7.0, device=DEV)
+    ops.latent_attention(qa, pages, bt, ctx, out, heads=H, rank=R, scale=scale)
+    assert _rel(out, _latent_want(ctx, qa, dense, seqs, H, R, scale)) < 2e-5
+    for t, (c, _) in enumerate(seqs):
+        ctx2, alone = _Ctx([(c, 1)]), torch.empty(1, H * R, device=DEV)
+        ctx2.T, ctx2.ws, ctx2.max_ctx_len, ctx2.decode_only, ctx2.n_tiles = 1, ctx.ws, c, True, 0
+        ctx2.token_seq, ctx2.positions = ctx.token_seq[t:t + 1].contiguous(), ctx.positions[t:t + 1].contiguous()
+        ops.latent_attention(qa[t:t + 1].contiguous(), pages, bt, ctx2, alone, heads=H, rank=R, scale=scale)
+        assert torch.equal(alone[0], out[t]), c

@@ -496,3 +496,25 @@ def test_gated_recurrence_keeps_a_row_written_long_ago(ops):
     assert torch.allclose(state[0, 0, 1], v[-1])
     want = v / v.pow(2).mean(-1, keepdim=True).sqrt()
     assert (out - want).abs().max() < 1e-5
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,G,dk,dv", [(2, 2, 64, 64), (4, 2, 40, 24), (5, 1, 16, 9), (3, 3, 256, 256)])
+def test_distance_bias_attention_single_tokens_across_the_cuts(ops, dtype, H, G, dk, dv):
+    """Single tokens at contexts on both sides of a split's edge, of the position where the splits get longer and beyond
+    it, enough of them for the form that many blocks take; a token has the same bits alone, in the form for few blocks."""
+    near, edge, far = ops.bias_cuts(H, G)
+    seqs = [(c, 1) for c in (1, near, near + 1, edge, edge + 1, edge + 2 * near + 1, 2 * edge, 2 * edge + 1, 2 * edge + far + 1, 700)] * 3
+    case = _case(dtype, seqs, H, G, dk, dv, 16, seed=H + dv)
+    tol = _tol(dtype) * 2
+    for kw in (dict(), dict(window=700)):
+        want, got = _want(case, **kw), _run(ops, case, "split", **kw)
+        assert (got - want).abs().max() < tol * max(1.0, want.abs().max().item()), kw
+    got = _run(ops, case, "split")
+    ctx, whole = case["ctx"], dict(case)
+    for t in range(10):
+        one = type(ctx)()
+        one.ws, one.max_ctx_len, one.decode_only, one.n_tiles = ctx.ws, seqs[t][0], True, 0
+        one.token_seq, one.positions = ctx.token_seq[t:t + 1].contiguous(), ctx.positions[t:t + 1].contiguous()
+        whole.update(ctx=one, q=case["q"][t:t + 1].contiguous())
+        assert torch.equal(_run(ops, whole, "split")[0], got[t]), seqs[t]

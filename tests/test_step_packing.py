@@ -91,3 +91,28 @@ def test_pack_and_views_round_trip():
     assert g.block_table[1].tolist() == [2, 0, 3, 4, 0, 0, 0, 0]          # a released page reads as page 0, never negative
     assert g.block_table[2].tolist() == [7, 1, 0, 6, 8, 0, 0, 0]
     assert ctx.max_q_len == 70 and ctx.max_ctx_len == 70 and not ctx.decode_only
+
+
+def test_grids_over_splits_of_keys_follow_from_the_rounded_context():
+    """A captured graph is kept under the rounded context: every number of splits follows from it and covers the context."""
+    from mini_llm_b200 import ops
+
+    def places(cuts, n):                                 # csrc/common.cuh's KeyCuts, split by split
+        near, edge, far = cuts
+        at = 0
+        while at < n:
+            yield at
+            at += near if at < edge else min(2 * near, far) if at < 2 * edge else far
+
+    cuts = [ops.bias_cuts(12, 12), ops.bias_cuts(12, 4), ops.latent_cuts(12, 384, torch.float32),
+            ops.latent_cuts(128, 512, torch.bfloat16), ops.LATENT_CUTS_PROMPT]
+    for c in cuts:
+        near, edge, far = c
+        assert near >= 32 and near & (near - 1) == 0 and far >= near and far & (far - 1) == 0 and 2 * edge % far == 0
+        for n in (1, 31, 32, 33, 512, 1023, 1024, 1025, 1300, 5000, 32768, 40000):
+            r = ops.split_context(n)
+            assert n <= r < 2 * max(n, 32)
+            assert len(list(places(c, n))) == ops.key_splits(n, c) <= ops.key_splits(r, c)
+    # short splits end at a fixed position, so that scratch for long contexts is that of the long ones and a constant
+    for c in cuts[:4]:
+        assert ops.key_splits(1 << 17, c) <= (1 << 17) // c[2] + 32
