@@ -180,12 +180,15 @@ attention_bias_simt_kernel(const T* q, long long q_stride, const T* k_pages, con
 // Single tokens.  grid (splits, kv heads x head chunks, tokens).  A CTA takes one split of one token's keys for HG
 // (1, 2 or 4) query heads that share a key/value head, so a key or value row is fetched once for all of them.  The
 // split is walked in tiles of 32 * KS * NT keys (KS = 4 / HG warps per head, fewer where the shortest split has fewer
-// chunks; NT chunks per warp, in a small grid the whole split where shared memory allows) that are staged in shared memory
+// chunks; NT chunks per warp, with FEW the whole split where shared memory allows, else 1) that are staged in shared memory
 // with 16-byte loads (all loads of a burst before any store); warp w takes head w % HG and the chunks w / HG, w / HG + KS, ...: its lanes are the 32 keys for the scores (a
 // row of K per lane, the query broadcast) and 32 value columns at a time for the weighted sum.  Chunks cover 32
 // consecutive positions starting at multiples of 32 from position 0.
 // Partial results: part_o [T][H][splits][dv], part_ml [T][H][splits][2]; a split without visible keys writes l = 0.
-template <typename T>
+// FEW: the form for small grids, where a block's chain of loads is what takes the time.  In large ones its second burst of
+// loads in registers (112 against 80) costs more than it hides, since fewer blocks fit an SM: 64 requests at contexts of 510,
+// 12 heads of 64 104 against 74 us.
+template <typename T, bool FEW>
 __global__ void __launch_bounds__(128)
 attention_bias_split_kernel(const T* q, long long q_stride, const T* k_pages, const T* v_pages,
                             const int* __restrict__ block_table, int bt_stride, const int* __restrict__ token_seq,
@@ -197,7 +200,7 @@ attention_bias_split_kernel(const T* q, long long q_stride, const T* k_pages, co
     const int krow = dk + VEC;                                  // elements per staged key row: 16 bytes of padding
     const int nsplit = gridDim.x, split = nsplit - 1 - blockIdx.x, t = blockIdx.z;       // the long splits first
     const int k0 = cuts.first(split), keys = cuts.keys(split);
-    const int NT = min(max_nt, keys / (32 * KS));
+    const int NT = FEW ? min(max_nt, keys / (32 * KS)) : 1;
     const int tile = 32 * KS * NT;                              // keys staged at a time: NT chunks of 32 per warp
     T* Ks = reinterpret_cast<T*>(smraw);                        // [tile][dk + VEC]
     T* Vs = Ks + (size_t)tile * krow;                           // [tile][dv]
@@ -240,29 +243,62 @@ attention_bias_split_kernel(const T* q, long long q_stride, const T* k_pages, co
         if (in_gap(a, base, base + tile - 1, first)) continue;  // uniform over the CTA
         __syncthreads();                                        // the tile before is no longer read; qs is complete
         constexpr int LD = 4;
-        // the loads of a burst of keys and a burst of values are all in flight before the first is stored
-        const int nkp = tile * kpieces, nvp = tile * vpieces;
-        for (int i0 = tid; i0 < max(nkp, nvp); i0 += nthreads * LD) {
-            uint4 rk[LD], rv[LD];
-            auto fetch = [&](const T* pages, int pieces, int width, int n, uint4 (&r)[LD]) {
+        if constexpr (FEW) {                                    // keys and values in flight together
+            const int nkp = tile * kpieces, nvp = tile * vpieces;
+            for (int i0 = tid; i0 < max(nkp, nvp); i0 += nthreads * LD) {
+                uint4 rk[LD], rv[LD];
+                auto fetch = [&](const T* pages, int pieces, int width, int n, uint4 (&r)[LD]) {
+#pragma unroll
+                    for (int u = 0; u < LD; ++u) {
+                        const int i = i0 + u * nthreads;
+                        r[u] = make_uint4(0u, 0u, 0u, 0u);
+                        if (i >= n) continue;
+                        const int key = i / pieces, piece = i % pieces, kp = base + key;
+                        if (kp >= s_lo && kp <= s_hi && sees(a, kp, first))
+                            r[u] = *reinterpret_cast<const uint4*>(pages + (((size_t)bt[kp / page_size] * Hkv + hk) * page_size + kp % page_size) * width + piece * VEC);
+                    }
+                };
+                fetch(k_pages, kpieces, dk, nkp, rk);
+                fetch(v_pages, vpieces, dv, nvp, rv);
 #pragma unroll
                 for (int u = 0; u < LD; ++u) {
                     const int i = i0 + u * nthreads;
-                    r[u] = make_uint4(0u, 0u, 0u, 0u);
-                    if (i >= n) continue;
-                    const int key = i / pieces, piece = i % pieces, kp = base + key;
-                    if (kp >= s_lo && kp <= s_hi && sees(a, kp, first))
-                        r[u] = *reinterpret_cast<const uint4*>(pages + (((size_t)bt[kp / page_size] * Hkv + hk) * page_size + kp % page_size) * width + piece * VEC);
+                    if (i < nkp) *reinterpret_cast<uint4*>(Ks + (size_t)(i / kpieces) * krow + (i % kpieces) * VEC) = rk[u];
+                    if (i < nvp) *reinterpret_cast<uint4*>(Vs + (size_t)(i / vpieces) * dv + (i % vpieces) * VEC) = rv[u];
                 }
-            };
-            fetch(k_pages, kpieces, dk, nkp, rk);
-            fetch(v_pages, vpieces, dv, nvp, rv);
-#pragma unroll
-            for (int u = 0; u < LD; ++u) {
-                const int i = i0 + u * nthreads;
-                if (i < nkp) *reinterpret_cast<uint4*>(Ks + (size_t)(i / kpieces) * krow + (i % kpieces) * VEC) = rk[u];
-                if (i < nvp) *reinterpret_cast<uint4*>(Vs + (size_t)(i / vpieces) * dv + (i % vpieces) * VEC) = rv[u];
             }
+        } else {
+            for (int i0 = tid; i0 < tile * kpieces; i0 += nthreads * LD) {
+                uint4 r[LD];
+#pragma unroll
+                for (int u = 0; u < LD; ++u) {
+                    const int i = i0 + u * nthreads, key = i / kpieces, piece = i % kpieces, kp = base + key;
+                    r[u] = make_uint4(0u, 0u, 0u, 0u);
+                    if (i < tile * kpieces && kp >= s_lo && kp <= s_hi && sees(a, kp, first))
+                        r[u] = *reinterpret_cast<const uint4*>(k_pages + (((size_t)bt[kp / page_size] * Hkv + hk) * page_size + kp % page_size) * dk + piece * VEC);
+                }
+#pragma unroll
+                for (int u = 0; u < LD; ++u) {
+                    const int i = i0 + u * nthreads;
+                    if (i < tile * kpieces) *reinterpret_cast<uint4*>(Ks + (size_t)(i / kpieces) * krow + (i % kpieces) * VEC) = r[u];
+                }
+            }
+            if (vpieces)
+                for (int i0 = tid; i0 < tile * vpieces; i0 += nthreads * LD) {
+                    uint4 r[LD];
+#pragma unroll
+                    for (int u = 0; u < LD; ++u) {
+                        const int i = i0 + u * nthreads, key = i / vpieces, piece = i % vpieces, kp = base + key;
+                        r[u] = make_uint4(0u, 0u, 0u, 0u);
+                        if (i < tile * vpieces && kp >= s_lo && kp <= s_hi && sees(a, kp, first))
+                            r[u] = *reinterpret_cast<const uint4*>(v_pages + (((size_t)bt[kp / page_size] * Hkv + hk) * page_size + kp % page_size) * dv + piece * VEC);
+                    }
+#pragma unroll
+                    for (int u = 0; u < LD; ++u) {
+                        const int i = i0 + u * nthreads;
+                        if (i < tile * vpieces) *reinterpret_cast<uint4*>(Vs + (size_t)(i / vpieces) * dv + (i % vpieces) * VEC) = r[u];
+                    }
+                }
         }
         if (!vpieces) {
             for (int i = tid; i < tile * dv; i += nthreads) {
@@ -949,9 +985,9 @@ MLLM_EXPORT int mllm_attention_bias(const void* q, long long q_stride, const voi
             return 0;
         };
         if (dtype == MLLM_F32)
-            return go(attention_bias_split_kernel<float>,
+            return go(few ? attention_bias_split_kernel<float, true> : attention_bias_split_kernel<float, false>,
                       attention_bias_merge_kernel<float>, (const float*)q, (const float*)k_pages, (const float*)v_pages, (float*)out);
-        return go(attention_bias_split_kernel<bf>,
+        return go(few ? attention_bias_split_kernel<bf, true> : attention_bias_split_kernel<bf, false>,
                   attention_bias_merge_kernel<bf>, (const bf*)q, (const bf*)k_pages, (const bf*)v_pages, (bf*)out);
     }
     if (impl == 3) {
