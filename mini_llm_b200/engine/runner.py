@@ -21,7 +21,7 @@ from ..cache.manager import CacheManager
 from ..config.base import ConfigError, EngineConfig, ModelConfig, get_architecture, load_config
 from ..parts.model import Model
 from ..weights.loader import load_weights
-from .context import ATTN_TILE_WIDE, StepContext, StepLayout, Workspace, attention_tiles, pack_step, single_runs
+from .context import ATTN_TILE_WIDE, StepContext, StepLayout, Workspace, attention_tiles, pack_step, single_runs, singles_pay
 
 
 class StepError(RuntimeError):
@@ -97,9 +97,14 @@ class ModelRunner:
         # a part that reads device data on the host while it runs sets graph_safe = False
         self._graph_ok = all(getattr(self.model.part(label), "graph_safe", True)
                              for label, _ in self.spec.all_part_specs())
-        # a mixer whose attention takes the single tokens of a mixed step by themselves
-        self._singles_apart = any(getattr(self.model.part(label), "singles_apart", False)
-                                  for label, _ in self.spec.all_part_specs())
+        # mixers whose attention can take the single tokens of a mixed step by themselves: heads and window of the rule
+        apart = [p for p in (self.model.part(label) for label, _ in self.spec.all_part_specs())
+                 if getattr(p, "singles_apart", False) and ops.has_decode_attention(p.head_dim, self.rt.dtype)]
+        self._singles_apart = bool(apart)
+        self._singles_rule = dict(heads=max((p.num_heads for p in apart), default=0), float32=self.rt.dtype == torch.float32,
+                                  wide=all(p.head_dim == 64 for p in apart) and self.engine.page_size in (8, 16, 32, 64, 128),
+                                  window=None if any(p.window is None for p in apart) else max((p.window for p in apart), default=0),
+                                  sms=ops.sm_count())
         self._capture_at_once = self.engine.graph_capture == "at_once"
         if self._capture_at_once and self.cache.state_layers:
             raise StepError("graph_capture='at_once' runs a new step shape twice; a mixer with a state of its own "
@@ -244,6 +249,8 @@ class ModelRunner:
             mp = max(len(t) for t in tables[g])
             max_pages.append(max(16, 1 << (mp - 1).bit_length()))   # powers of two: few distinct shapes for captured graphs
         runs = single_runs(q_lens) if self._singles_apart and T != S else []
+        if runs and not singles_pay(q_lens, q_start, **self._singles_rule):
+            runs = []
         tiles = [] if T == S else attention_tiles(q_lens, q_start, singles_last=bool(runs))
         wide = [] if T == S else attention_tiles(q_lens, q_start, ATTN_TILE_WIDE, singles_last=bool(runs))
         layout = StepLayout.make(T, S, len(logit_rows), max_pages, len(tiles) // 3, len(wide) // 3, runs)

@@ -2087,6 +2087,15 @@ attention_launches = {}     # attention kernel name -> launches so far (tests ch
 use_tcgen05_attention = True    # False: prompt portions stay on the mma.sync kernel (for comparisons and profiles)
 
 
+def wide_tiles_full(tokens: int, n_wide: int) -> bool:
+    """Whether tiles of 128 rows are mostly full: the rule for the kernels that take those."""
+    return n_wide > 0 and tokens >= 256 and tokens >= 80 * n_wide
+
+
+def has_decode_attention(head_dim: int, dtype) -> bool:
+    return head_dim in _DECODE_HEAD_DIMS[dtype]
+
+
 def _flash_tc_ok(q, k_pages, out, n_wide, head_dim, ps, ldq, ldo) -> bool:
     return (q.dtype == torch.bfloat16 and head_dim == 64 and 8 <= ps <= 128 and ps & (ps - 1) == 0
             and n_wide > 0 and ldq % 8 == 0 and q.data_ptr() % 16 == 0 and ldo % 8 == 0
@@ -2098,7 +2107,7 @@ _TILED_WIDE_HEAD_DIMS = (16, 32, 48, 64)
 
 def _tiled_wide_ok(q, head_dim, n_wide, tokens, ldq) -> bool:
     """Long prompt portions (128-row tiles mostly full) with heads up to 64, where no tensor-core kernel applies (float32: other heads than 64, unaligned rows)."""
-    return (head_dim in _TILED_WIDE_HEAD_DIMS and n_wide > 0 and tokens >= 256 and tokens >= 80 * n_wide
+    return (head_dim in _TILED_WIDE_HEAD_DIMS and wide_tiles_full(tokens, n_wide)
             and ldq % (16 // q.element_size()) == 0 and q.data_ptr() % 16 == 0)
 
 
@@ -2136,17 +2145,17 @@ def paged_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, nu
     if impl is None:
         impl = "simt"
         if decode_ok and (k_pages.data_ptr() | v_pages.data_ptr()) % 16 == 0 and getattr(ctx, "single_runs", ()):
-            # Single tokens beside prompt portions: the decode kernel takes them, run by run, after the portions' launch,
-            # whose tiles are the head of the lists.  As 64-row tiles with one live row of the prefill kernels they cost as
-            # much as full tiles.  GPT-2 medium, 512 prompt tokens beside 40 single ones at contexts of 225 to 900, per
-            # block: bfloat16 62 us in one launch, 25 us (tcgen05 kernel, whose rule on full tiles the portion now meets)
-            # + 27 us in two; float32 835 us in one, 51 + 48 us in two.
+            # Single tokens beside prompt portions, where the step's layout names them (engine/context.py has the rule): the
+            # decode kernel takes them, run by run, after the portions' launch, whose tiles are the head of the lists.  GPT-2
+            # medium, 512 prompt tokens beside 40 single ones at contexts of 225 to 900, per block: bfloat16 62 us in one
+            # launch, 25 us (tcgen05 kernel, whose rule on full tiles the portion now meets) + 27 us in two; float32 835 us in
+            # one launch of the CUDA-core kernel, 51 + 48 us in two.
             singles = sum(n for _, n in ctx.single_runs)
             n_tiles, n_wide, tokens = n_tiles - singles, n_wide - singles, T - singles
         if getattr(ctx, "decode_only", False) and decode_ok:
             impl = "decode"
-        elif use_tcgen05_attention and _flash_tc_ok(q, k_pages, out, n_wide, head_dim, ps, ldq, ldo) and tokens >= 256 \
-                and tokens >= 80 * n_wide:
+        elif use_tcgen05_attention and _flash_tc_ok(q, k_pages, out, n_wide, head_dim, ps, ldq, ldo) \
+                and wide_tiles_full(tokens, n_wide):
             impl = "flash_tc"       # long prompt portions (tiles of 128 rows mostly full): the tensor-memory kernel
         elif q.dtype == torch.bfloat16 and head_dim in _FLASH_HEAD_DIMS and n_tiles > 0 \
                 and ldq % 8 == 0 and q.data_ptr() % 16 == 0 and ldo % 2 == 0:

@@ -1283,3 +1283,10 @@ def test_float32_attention_pieces_at_their_worst_values(ops, signed):
     # scores of up to 32 are off by 32 x 2^-24 in either kernel, so weights that sum to 1, times values of 1, by 2 x 2e-6
     assert torch.allclose(out["split_f32"][5], out["simt"][5], rtol=1e-5, atol=4e-6)
     ops.check_device_errors()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("seqs", [[(1500, 1), (40, 39), (300, 1)], [(1025, 1), (1100, 2), (1, 1)]])
+def test_single_tokens_beside_portions_at_long_contexts(ops, dtype, seqs):
+    """Beyond 1,024 keys the splits of the decode kernel meet in scratch, which the runs of a step share."""
+    test_single_tokens_beside_portions_take_the_decode_kernel(ops, dtype, 4, 2, 64, 16, None, seqs)

@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from mini_llm_b200.engine.context import (ATTN_TILE, ATTN_TILE_WIDE, StepContext, StepLayout, Workspace,
-                                          attention_tiles, pack_step)
+                                          attention_tiles, pack_step, single_runs, singles_pay)
 
 
 def _triples(flat):
@@ -91,6 +91,25 @@ def test_pack_and_views_round_trip():
     assert g.block_table[1].tolist() == [2, 0, 3, 4, 0, 0, 0, 0]          # a released page reads as page 0, never negative
     assert g.block_table[2].tolist() == [7, 1, 0, 6, 8, 0, 0, 0]
     assert ctx.max_q_len == 70 and ctx.max_ctx_len == 70 and not ctx.decode_only
+
+
+def test_single_tokens_leave_the_portions_where_it_pays():
+    """The rule on examples of both sides (heads of GPT-2 small): a token that the portions' launch hides stays in it, one
+    that would make it longer, or many that would need another wave, get launches of their own, but not one per token."""
+    def pay(q_lens, q_starts, float32=False, heads=12, **kw):
+        return singles_pay(q_lens, q_starts, heads, float32, **kw)
+
+    for f32 in (False, True):
+        assert not pay([1, 512], [199, 0], f32)                        # a short context beside a long portion
+        assert pay([1, 512], [899, 0], f32)                            # its walk is the longest
+        assert not pay([1, 512], [899, 0], f32, window=256)            # ... but for a window
+        assert not pay([1, 512], [899, 900], f32)                      # the portion walks as far
+        assert pay([1] * 32 + [512], [499] * 32 + [0], f32)            # another wave
+        assert not pay([1, 256, 1, 256, 1, 256, 1, 256], [499, 0] * 4, f32)
+        assert pay([1] * 40 + [512], [225 + 17 * i for i in range(40)] + [388], f32, heads=16)
+    # bfloat16 tiles of 128 rows stay the portion's where single tokens would leave them half empty
+    assert pay([1] * 6 + [700], [399] * 6 + [0]) and not pay([1] * 6 + [700], [399] * 6 + [0], wide=False)
+    assert single_runs([1, 5, 1, 5, 1, 5, 1, 5, 1]) == [] and single_runs([5, 1, 1, 5, 1]) == [(5, 2), (12, 1)]
 
 
 def test_grids_over_splits_of_keys_follow_from_the_rounded_context():
