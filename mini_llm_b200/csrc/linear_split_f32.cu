@@ -417,8 +417,20 @@ int sm_count() {
     return n;
 }
 
-// K slices, from N and K alone: a narrow result has few tiles (12 to 96 for 768 columns and 77 to 2,048 rows), each of
-// which walked all of K on its SM.  SLICES_NOTE
+// K slices, from N and K alone (a row's sum must not depend on the rows beside it): a narrow result has few tiles, each of
+// which walks all of K on its SM.  Three slices give most where rows are few and take an extra write and read of the sums
+// where the tiles fill the GPU without them.  us with one / three slices:
+//     rows              77          552         2,048        8,192
+//      768 x  768    19 / 14     21 / 18      27 / 27      64 / 79
+//      768 x 3072    56 / 27     58 / 36      78 / 63     216 / 219
+//     1024 x 1024    23 / 16     25 / 21      34 / 42     104 / 136
+//     1024 x 4096    72 / 33     78 / 46     103 / 111    380 / 391
+//      768 x  512    15 / 13     16 / 16      21 / 24      47 / 65     shorter rows gain less than they lose (384: 13 / 12,
+//      768 x  256    11 / 12     12 / 14      14 / 20      29 / 51     14 / 14, 18 / 20, 38 / 52)
+//     1600 x 1024    23 / 16     26 / 30      57 / 63     152 / 204    wider results lose from 552 rows on, 1,280 as well
+//     1600 x 4096    76 / 38     82 / 81     193 / 180    570 / 619    (4096: 77 / 38, 85 / 79, 194 / 144, 478 / 472)
+// 768 x 3072 with two / three / four slices: 34 / 27 / 23 at 77 rows, 36 / 36 / 30 at 552, 47 / 37 / 48 at 1,024, 83 / 63 /
+// 68 at 2,048.
 int slices_for(int N, int K) { return N <= 1024 && N % 4 == 0 && K >= 512 ? 3 : 1; }
 
 template <int BN>
@@ -501,6 +513,7 @@ MLLM_EXPORT int mllm_linear_split_f32(const float* A, long long lda, const float
 
 // The Q|K|V projection with the cache write fused in: out [M, q_size] receives the query columns, keys and values go
 // to their page slots (slots[m] = page * page_size + offset, negative: not stored); q_size and head_dim multiples of 32.
+// It never cuts K, so where mllm_linear_split_f32 would, the sums of the two run in different orders.
 MLLM_EXPORT int mllm_linear_split_f32_qkv(const float* A, long long lda, const float* W, const float* bias, float* out,
                                           long long ldo, int M, int N, int K, float* k_pages, float* v_pages,
                                           const int* slots, int q_size, int kv_heads, int head_dim, int page_size,

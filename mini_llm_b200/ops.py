@@ -751,11 +751,12 @@ def linear_qkv_cache(x, weight, bias, q_out, k_pages, v_pages, slot_mapping, ws)
     """Q|K|V projection whose keys and values go to their page slots; returns the queries.
 
     weight [q_size + 2*kv_heads*head_dim, K]; q_out [M, q_size] is where the queries may be
-    put.  The cache write rides in the product's epilogue - the weight-streaming kernel's with few
-    rows (which also takes a NormedInput's norm into its loads), the tensor-memory kernel's with
-    many - and q_out is returned; where neither applies (32-bit, head sizes that are no multiple
-    of 32) the product writes a [M, N] buffer, kv_write copies keys and values from it, and the
-    buffer's query columns are returned.
+    put.  The cache write rides in the product's epilogue and q_out is returned: the weight-streaming
+    kernels' with few rows (which also take a NormedInput's norm into their loads), the cluster
+    kernel's in bfloat16, the tensor-memory kernels' with many rows, in either precision (a 32-bit
+    product with it never cuts K into slices).  Where none applies (many rows with head sizes that are
+    no multiple of 32, unaligned rows) the product writes a [M, N] buffer, kv_write copies keys and
+    values from it, and the buffer's query columns are returned.
     """
     M = x.shape[0]
     N, K = weight.shape
