@@ -34,7 +34,8 @@ constexpr int BQ = 128, BKV = 128, DH = 64;
 constexpr int PARTS = 4;                             // threads per query row: each takes 32 keys of a block and 16 of the 64 output values
 constexpr int SOFTMAX_WARPS = 4 * PARTS, CUT_WARPS = 8, K_WARP = SOFTMAX_WARPS, V_WARP = K_WARP + 4, MMA_WARP = V_WARP + 4;
 constexpr int THREADS = (SOFTMAX_WARPS + CUT_WARPS + 4) * 32;
-// Registers: 896 threads x 72 = 64,512 at launch; 512 x 88 + 256 x 64 + 128 x 24 = 64,512 after the split.
+// Registers: 896 threads x 72 = 64,512 at launch; 512 x 88 + 256 x 64 + 128 x 24 = 64,512 after the split.  The compiler keeps
+// all of the code to the 72 (12 bytes spill, and 124 in plain_rows).
 constexpr int PLANE = 128 * DH * 2;                  // 16 KB: a piece of the tile's queries, of a block's keys or values
 constexpr int XCH_BYTES = 2 * PARTS * BQ * 4;        // partial row maxima, double-buffered; reused for the row sums at the end
 constexpr size_t SMEM = 1024 + 9 * PLANE + XCH_BYTES + 256;

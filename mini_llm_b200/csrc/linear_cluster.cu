@@ -6,7 +6,8 @@
 // columns) and walks K on each, the weight-streaming kernel (linear_smallm.cu) reads its rows of A again for every 16
 // rows of W.  Here the roles are swapped: 128 rows of W are the M side of a tcgen05.mma, all rows of A (32, 64 or 128 of
 // them, zeros beyond M) its N side, and K is cut into up to 8 slices, one per CTA of a thread-block cluster, so that
-// nearly every SM streams weights and A passes once per 128 rows of W.  The CTAs of a cluster share the rows of A among
+// more SMs stream weights (36 to 144 of 148: 36 for 768 x 768, 48 for 768 x 3072, 104 for 1600 x 6400, 108 for 2304 x 768)
+// and A passes once per 128 rows of W.  The CTAs of a cluster share the rows of A among
 // them: a CTA writes its sums of a row straight from tensor memory into the shared memory of the row's owner, and after
 // one cluster barrier the owner adds the slices in rank order and runs the epilogue (bias, GELU, residual sum, cache
 // write).

@@ -216,7 +216,7 @@ struct MapKeyHash {
 // Element type and swizzle of a tensor map over a row-major [rows, cols] matrix with row stride ld
 // (elements).  The box is box_rows x box_cols; box_cols x element size must equal the swizzle span.
 enum { MAP_BF16_SW128 = 0,      // bfloat16, 64 columns (128 bytes): MMA operands, key/value pages
-       MAP_F32_SW128 = 1,       // 32-bit, 32 columns (128 bytes): the products' output blocks
+       MAP_F32_SW128 = 1,       // 32-bit, 32 columns (128 bytes): output blocks, operands of the 32-bit products in pieces
        MAP_BF16_SW64 = 2 };     // bfloat16, 32 columns (64 bytes): the products' output blocks
 
 inline int get_map(const void* ptr, long long ld, int rows, int cols, int box_cols, int box_rows, int kind,
