@@ -1290,3 +1290,17 @@ def test_float32_attention_pieces_at_their_worst_values(ops, signed):
 def test_single_tokens_beside_portions_at_long_contexts(ops, dtype, seqs):
     """Beyond 1,024 keys the splits of the decode kernel meet in scratch, which the runs of a step share."""
     test_single_tokens_beside_portions_take_the_decode_kernel(ops, dtype, 4, 2, 64, 16, None, seqs)
+
+
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D", [1028, 1600, 2048])
+def test_layernorm_of_many_wide_rows(ops, out_dtype, D):
+    """From 1,025 wide rows on gamma and beta are read late: the same bits for a row as with fewer."""
+    x, gamma, beta = rnd(1030, D, seed=4, scale=3.0) + 1.5, rnd(D, seed=5) + 1.0, rnd(D, seed=6)
+    many, few = (torch.empty(n, D, device=DEV, dtype=out_dtype) for n in (1030, 1024))
+    ops.layernorm(x, gamma, beta, 1e-5, many)
+    ops.layernorm(x[:1024], gamma, beta, 1e-5, few)
+    assert torch.equal(many[:1024], few)
+    want = torch.nn.functional.layer_norm(x.double(), (D,), gamma.double(), beta.double(), 1e-5)
+    tol = 2e-5 if out_dtype == torch.float32 else 2e-2
+    assert (many.double() - want).abs().max() < tol * want.abs().max().item()
