@@ -1292,6 +1292,28 @@ def test_single_tokens_beside_portions_at_long_contexts(ops, dtype, seqs):
     test_single_tokens_beside_portions_take_the_decode_kernel(ops, dtype, 4, 2, 64, 16, None, seqs)
 
 
+def test_fused_float32_projection_beside_the_sliced_product(ops):
+    """A projection whose size linear() cuts into K slices: the fused one adds in another order.  In either, the accumulator
+    drops at most 2^-23 of the magnitudes in each of the four full-size additions of a block of 64, the blocks are added
+    one by one, and slices, bias and what the pieces leave out add a few more 2^-24."""
+    from mini_llm_b200.engine.context import Workspace
+    M, H, dh, K, page = 130, 4, 64, 768, 16
+    N = 3 * H * dh
+    assert ops.library().mllm_linear_split_f32_slices(N, K) > 1
+    x, w, b = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5), rnd(N, seed=3)
+    slots = torch.randperm(20 * page, generator=torch.Generator().manual_seed(4))[:M].to(torch.int32).to(DEV)
+    k, v = (torch.zeros(20, H, page, dh, device=DEV) for _ in range(2))
+    q = ops.linear_qkv_cache(x, w, b, torch.empty(M, H * dh, device=DEV), k, v, slots, Workspace(torch.device(DEV), 256))
+    plain = torch.empty(M, N, device=DEV)
+    ops.linear(x, w, b, out=plain)
+    at = slots.long()
+    fused = torch.cat([q] + [c[at // page, :, at % page].reshape(M, -1) for c in (k, v)], 1)
+    exact = x.double() @ w.double().t() + b.double()
+    bound = (K / 64 + 12) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t() + b.double().abs())
+    assert torch.all((fused - exact).abs() < bound) and torch.all((plain - exact).abs() < bound)
+    ops.check_device_errors()
+
+
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("D", [1028, 1600, 2048])
 def test_layernorm_of_many_wide_rows(ops, out_dtype, D):
