@@ -646,23 +646,35 @@ def _small_m_wins(M: int, N: int, K: int) -> bool:
 
 
 def _cluster_wins(M: int, N: int, K: int) -> bool:
-    """Whether M rows of bfloat16 go to the kernel that cuts K over the CTAs of a cluster (csrc/linear_cluster.cu).
-    Measured in replayed chains at GPT-2 small's, medium's and XL's four products and 17 to 128 rows.  Long rows of W
-    (K = 4 x width), which the other kernels walk on few SMs, gain at every count (5 to 9 against 11 to 22 us).  With K =
-    width it wins up to 32 rows (3.7 to 9.5 against 4.1 to 14 us; 768 x 768 is a tie at 32); beyond, the exchange of the
-    sums, which grows with the rows, outweighs what the other kernel loses by using fewer SMs, except for narrow results
-    (1024 x 1024 and 1600 x 1600 at 64 rows 4.8 and 6.5 against 5.4 and 8.0 us, 768 x 768 6.0 against 4.6).
-    Up to 16 rows the weight-streaming kernel, which takes a norm into its loads, keeps what it wins (2.0 to 3.8 against 3.0
-    to 4.0 us at K = 768 to 1024; 768 x 3072 is 4.8 against 4.5 us inside a step of one row); rows from 6,144 on go to the
-    cluster (1600 x 6400 at 8 rows 7.4 against 11.5 us), and so does a vocabulary, norm apart: 50257 x 768 at 1 / 8 / 16 rows 17 / 18 / 20 us, against 17 / 21 / 31
-    without the norm and 23 to 37 us inside steps with it; the persistent kernel 21 / 21 / 23."""
+    """Whether M rows of bfloat16 go to the kernel that cuts K over the CTAs of a cluster (csrc/linear_cluster.cu).  It gains
+    where the other kernels leave SMs idle, on results that are narrow for the length of their rows, and it loses by the
+    exchange of the sums, which grows with rows and columns.  Chains of matrices that are not in L2, 21 sizes from 512 x 512 to
+    11,008 x 4,096 at 8 to 128 rows, us here / in the kernel that would take it otherwise:
+      65 to 128 rows  results up to half as wide as the rows are long: 1280 x 5120 11 to 13 / 20, 512 x 2048 8.0 to 9.4 / 10.7,
+                      2048 x 8192 25 to 27 / 31.  Beyond: 4096 x 4096 17 to 19 / 19, 2048 x 2048 15 to 18 / 11 (sixteen clusters of
+                      eight 166 KB CTAs do not all run at once), 6144 x 2048 23 to 29 / 13.
+      33 to 64        up to as wide as long: 1024 x 1024 6.3 to 7.0 / 7.5, 4096 x 4096 15 to 16 / 19, 1280 x 5120 10 to 11 / 20.  Short
+                      rows of few columns do not gain (768 x 768 6.3 to 7.3 / 6.6), nor wider results (5120 x 1280 10 to 12 / 10,
+                      8192 x 2048 16 to 17 / 14, 11008 x 4096 36 to 40 / 29).
+      17 to 32        results too wide for one wave of the weight-streaming kernel, as long as K is cut at all: 3840 x 1280 8.4 to 8.9 / 10,
+                      4096 x 4096 14 / 19, 8192 x 2048 14 to 15 / 14 to 20, but 11008 x 4096 (one slice) 32 to 34 / 28.  In its wave the
+                      weight-streaming kernel is ahead (768 x 768 5.8 to 6.1 / 5.1 to 5.6, 2048 x 2048 9 / 7 to 8), except for long
+                      rows: 512 x 2048 6.1 to 6.5 / 6.5 to 7.2, 1280 x 5120 9.6 / 12 to 13.
+      up to 16        the weight-streaming kernel, which takes a norm into its loads, keeps all (2048 x 2048 8.5 / 6.1) but rows from 6,144
+                      on (1600 x 6400 at 8 rows 7.4 / 11.5, 2048 x 8192 14 / 15 to 18) and the vocabulary, norm apart: 50257 x 768 at
+                      1 / 8 / 16 rows 17 / 18 / 20, against 17 / 21 / 31 without the norm and 23 to 37 inside steps with it; the
+                      persistent kernel 21 / 21 / 23."""
     if not 0 < M <= 128 or K < 512:
         return False
     if N >= 16384:
         return M <= 16
     if M <= 16:
         return K >= 6144
-    return M <= 32 or K >= 2048 or (M <= 64 and 1024 <= N <= K)
+    if M <= 32:
+        return N <= 74 * 128 if -(-N // 16) > sm_count() else K >= max(2048, 2 * N)
+    if M <= 64:
+        return N <= K and (N >= 1024 or K >= 2048)
+    return K >= max(2048, 2 * N)
 
 
 def _fusable(weight, M, K) -> bool:

@@ -79,6 +79,18 @@ def test_slices_of_a_product_are_summed_in_the_callers_own_scratch(ops, monkeypa
     assert scratch(a, 1000) and a.version > version          # a larger buffer is seen by whoever keeps its address
 
 
+def test_sizes_that_go_to_the_cluster_kernel(ops, monkeypatch):
+    """bfloat16 products of few rows: narrow results of long rows are cut over a cluster, at every count of rows, and wide ones
+    are not, whose sums would cost more to exchange than the idle SMs do."""
+    monkeypatch.setattr(ops, "sm_count", lambda: 148)
+    for M, N, K in ((128, 768, 3072), (65, 1600, 6400), (64, 1024, 1024), (33, 1024, 4096), (24, 4800, 1600), (24, 1600, 6400),
+                    (8, 1600, 6400), (3, 50257, 768), (16, 50257, 768)):
+        assert ops._cluster_wins(M, N, K), (M, N, K)
+    for M, N, K in ((65, 6144, 2048), (128, 2048, 2048), (96, 8192, 2048), (128, 11008, 4096), (48, 11008, 4096), (64, 6144, 2048),
+                    (24, 2048, 1024), (24, 11008, 4096), (64, 768, 768), (17, 50257, 768), (129, 768, 3072), (64, 768, 448)):
+        assert not ops._cluster_wins(M, N, K), (M, N, K)
+
+
 def _pieces(x, rounded):
     """The cut of csrc/split_f32.cuh: to nearest, or (what it must not do) by dropping the lower bits."""
     import numpy as np
