@@ -14,13 +14,6 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (run on a B200)")
 
 
-@pytest.fixture(autouse=True)
-def fixed_seed():
-    """What a test draws without a generator of its own is the same in every run."""
-    if "torch" in sys.modules:
-        sys.modules["torch"].manual_seed(0)
-
-
 def pytest_collection_modifyitems(config, items):
     import torch
 
