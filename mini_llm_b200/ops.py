@@ -93,6 +93,9 @@ def _signatures(lib):
         "mllm_attention_decode": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                   c_ll, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
                                   c_int, c_int, c_int, c_int, c_void_p],
+        "mllm_attention_decode_beside": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
+                                  c_ll, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
+                                  c_int, c_int, c_int, c_int, c_void_p],
         "mllm_attention_split_f32": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p,
                                      c_ll, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
         "mllm_attention_split_f32_bind_error": [c_void_p],
@@ -2180,19 +2183,24 @@ def paged_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, nu
         elif n_tiles > 0:
             impl = "tiled"          # float32, or a head size the tensor-core kernel does not take
     if singles:
+        # the portions' kernels let their dependents start once the projection is complete: the runs go beside them
+        beside = (impl in ("flash_tc", "split_f32", "tiled_wide") and n_wide > 0) or (impl in ("flash", "tiled") and n_tiles > 0)
         _attend(impl, q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ldo, num_heads, num_kv_heads, head_dim, ps,
                 scale, window, n_tiles, n_wide, None)
-        for run in ctx.single_runs:
+        for i, run in enumerate(ctx.single_runs):
+            if i > 0 and decode_splits(ctx.max_single_ctx_len) > DECODE_CLUSTER_SPLITS:
+                beside = False          # the runs share the scratch in which splits of long contexts meet: one after the other
             _attend("decode", q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ldo, num_heads, num_kv_heads,
-                    head_dim, ps, scale, window, 0, 0, run)
+                    head_dim, ps, scale, window, 0, 0, run, beside)
         return
     _attend(impl, q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ldo, num_heads, num_kv_heads, head_dim, ps, scale,
             window, n_tiles, n_wide, None)
 
 
 def _attend(impl, q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ldo, num_heads, num_kv_heads, head_dim, ps, scale,
-            window, n_tiles, n_wide, run) -> None:
-    """One launch of the named attention kernel; ``run`` (first row, rows): what the decode kernel takes (None: all)."""
+            window, n_tiles, n_wide, run, beside: bool = False) -> None:
+    """One launch of the named attention kernel; ``run`` (first row, rows): what the decode kernel takes (None: all), and
+    ``beside``: it need not wait for the launch before it."""
     T = q.shape[0] if run is None else run[1]
     attention_launches[impl] = attention_launches.get(impl, 0) + 1
     if impl == "tiled_wide":
@@ -2252,10 +2260,9 @@ def _attend(impl, q, ldq, k_pages, v_pages, block_table, bt_stride, ctx, out, ld
         else:
             part_o = part_ml = counters = None
         t0, es = (0 if run is None else run[0]), q.element_size()
-        _call("mllm_attention_decode", q.data_ptr() + t0 * ldq * es, ldq, k_pages.data_ptr(), v_pages.data_ptr(),
-              block_table.data_ptr(), bt_stride, ctx.token_seq.data_ptr() + 4 * t0, ctx.positions.data_ptr() + 4 * t0,
-              out.data_ptr() + t0 * ldo * es,
-              ldo, part_o, part_ml, counters, T, num_heads, num_kv_heads, head_dim, ps, float(scale),
+        _call("mllm_attention_decode_beside" if beside else "mllm_attention_decode", q.data_ptr() + t0 * ldq * es, ldq,
+              k_pages.data_ptr(), v_pages.data_ptr(), block_table.data_ptr(), bt_stride, ctx.token_seq.data_ptr() + 4 * t0,
+              ctx.positions.data_ptr() + 4 * t0, out.data_ptr() + t0 * ldo * es, ldo, part_o, part_ml, counters, T, num_heads, num_kv_heads, head_dim, ps, float(scale),
               int(window or 0), max_splits, _dt(q), int(impl == "decode_scratch"), _stream())
         return
     if impl != "simt":

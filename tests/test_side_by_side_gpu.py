@@ -1,0 +1,72 @@
+"""Launches that do not wait for the launch before them: replayed many times between the kernels that write what they read and
+the ones that read what they write, they leave the bits of launches that run one after the other."""
+import pytest
+import torch
+
+from test_kernels_gpu import DEV, _ctx_for, _paged_case, ops, rnd  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def _replayed(ops, run, outs, fresh):
+    """``run`` captured and replayed on changing inputs against the same launches without programmatic dependent launch."""
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        run()
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            run()
+        for i in range(12):
+            fresh(i)
+            graph.replay()
+            stream.synchronize()
+            got = [o.clone() for o in outs]
+            ops.set_pdl(False)
+            try:
+                run()
+                stream.synchronize()
+            finally:
+                ops.set_pdl(True)
+            for g, o in zip(got, outs):
+                assert torch.equal(g, o), i
+    ops.check_device_errors()
+
+
+# (context, new tokens): one run of single tokens, several, many behind a portion whose tiles fill the GPU, runs that share scratch
+@pytest.mark.parametrize("seqs", [[(500, 200), (300, 1), (90, 1)], [(700, 1), (260, 130), (33, 1), (150, 1)],
+                                  [(640, 640)] + [(37 * i + 5, 1) for i in range(20)],
+                                  [(1100, 1), (200, 200), (1200, 1), (70, 1)]])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_single_tokens_beside_portions(ops, dtype, seqs):  # noqa: F811
+    from mini_llm_b200.engine.context import ATTN_TILE_WIDE, attention_tiles, single_runs
+    H = Hkv = 12
+    dh, page, D = 64, 16, 768
+    case = _paged_case(dtype, seqs, H, Hkv, dh, page, num_pages=1200, seed=5)
+    ctx = _ctx_for(case)
+    q_lens, starts = [n for _, n in seqs], [c - n for c, n in seqs]
+    T = sum(q_lens)
+    ctx.decode_only = False
+    for name, rows in (("", 64), ("_wide", ATTN_TILE_WIDE)):
+        tiles = attention_tiles(q_lens, starts, rows, singles_last=True)
+        setattr(ctx, "attn_tiles" + name, torch.tensor(tiles, dtype=torch.int32, device=DEV))
+        setattr(ctx, "n_tiles" + name, len(tiles) // 3)
+    ctx.single_runs = single_runs(q_lens)
+    ctx.max_single_ctx_len = max(c for c, n in seqs if n == 1)
+    slots = torch.tensor([int(case["bt"][s, p // page]) * page + p % page
+                          for s, p in zip(case["token_seq"], case["positions"])], dtype=torch.int32, device=DEV)
+    kp, vp, bt = case["k_pages"].to(dtype).to(DEV), case["v_pages"].to(dtype).to(DEV), case["bt"].to(DEV)
+    w_in, w_out = rnd(3 * D, D, seed=1, scale=D ** -0.5, dtype=dtype), rnd(D, D, seed=2, scale=D ** -0.5, dtype=dtype)
+    x, q, att = (torch.empty(T, D, dtype=dtype, device=DEV) for _ in range(3))
+    y = torch.empty(T, D, device=DEV)
+
+    def run():
+        with ops.stream_scope(ctx.ws):
+            queries = ops.linear_qkv_cache(x, w_in, None, q, kp, vp, slots, ctx.ws)
+            ops.paged_attention(queries, kp, vp, bt, ctx, att, num_heads=H, num_kv_heads=Hkv, head_dim=dh, scale=dh ** -0.5)
+            ops.linear(att, w_out, None, out=y)
+
+    x.copy_(rnd(T, D, seed=3, dtype=dtype))
+    before = ops.attention_launches.get("decode", 0)
+    _replayed(ops, run, [att, y], lambda i: x.copy_(rnd(T, D, seed=10 + i, dtype=dtype)))
+    assert ops.attention_launches["decode"] > before
