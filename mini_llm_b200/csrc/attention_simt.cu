@@ -30,6 +30,7 @@ attention_simt_kernel(const T* q, long long q_stride, const T* k_pages,     // w
                       int window) {
     __shared__ float qs[WARPS][MAX_DH];
     pdl_wait();
+    pdl_launch();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long gw = (long long)blockIdx.x * WARPS + warp;
     if (gw >= (long long)T_tokens * H) return;

@@ -52,6 +52,7 @@ linear_simt_kernel(const TA* A, long long lda, const TW* __restrict__ W, const f
     __shared__ float As[BK][BM + PAD];
     __shared__ float Ws[BK][BN + PAD];
     pdl_wait();
+    pdl_launch();
     const int tid = threadIdx.x;
     const int tx = tid % (BN / TN), ty = tid / (BN / TN);
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
@@ -116,6 +117,7 @@ linear_simt_large_kernel(const TA* A, long long lda, const TW* __restrict__ W,
     __shared__ float As[2][LBK][LBM + 4];
     __shared__ float Ws[2][LBK][LBN + 4];
     pdl_wait();
+    pdl_launch();
     const int tid = threadIdx.x;
     const int tx = tid % 16, ty = tid / 16;
     const int m0 = blockIdx.y * LBM, n0 = blockIdx.x * LBN;

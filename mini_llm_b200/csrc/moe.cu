@@ -60,59 +60,60 @@ __device__ __forceinline__ void token_gate(const T* x, const T* __restrict__ Wg,
     if (lane == 0) *gate = 1.0f / (1.0f + expf(-acc));
 }
 
-// One warp routes one token; `s` is the warp's E floats of shared memory.
+// The scores' inputs: s[e0 ..] = Wr x (+ bias) of four experts by one warp, their loads in flight together.
 template <typename T>
-__device__ __forceinline__ void route_token(const T* x, const RouteArgs<T>& ra, float* s, int* idx, float* wout, int t, int lane) {
+__device__ __forceinline__ void router_logits(const T* x, const RouteArgs<T>& ra, float* s, int e0, int lane) {
     const T* __restrict__ Wr = ra.Wr;
     const float* __restrict__ bias = ra.bias;
-    const int mode = ra.mode, D = ra.D, E = ra.E, top = ra.top, n_groups = ra.n_groups, keep = ra.keep, group_sum = ra.group_sum;
-    const float w_scale = ra.w_scale;
-    if (ra.Wg) token_gate(x, ra.Wg, D, ra.gate + t, lane);
+    const int D = ra.D, E = ra.E;
     constexpr int V = 16 / sizeof(T);                           // elements per 16-byte load
-    const bool vec = D % V == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)Wr % 16 == 0;
-    for (int e0 = 0; e0 < E; e0 += 4) {                         // four experts at a time: their loads are in flight together
-        float a[4] = {0.f, 0.f, 0.f, 0.f};
-        const T* w0 = Wr + (size_t)e0 * D;
-        const T* w1 = Wr + (size_t)min(e0 + 1, E - 1) * D;
-        const T* w2 = Wr + (size_t)min(e0 + 2, E - 1) * D;
-        const T* w3 = Wr + (size_t)min(e0 + 3, E - 1) * D;
-        if (vec) {
-#pragma unroll 2
-            for (int d = lane * V; d < D; d += 32 * V) {
-                const uint4 xv = *reinterpret_cast<const uint4*>(x + d);
-                const uint4 v0 = *reinterpret_cast<const uint4*>(w0 + d), v1 = *reinterpret_cast<const uint4*>(w1 + d);
-                const uint4 v2 = *reinterpret_cast<const uint4*>(w2 + d), v3 = *reinterpret_cast<const uint4*>(w3 + d);
-                const T* px = reinterpret_cast<const T*>(&xv);
-                const T* p0 = reinterpret_cast<const T*>(&v0);
-                const T* p1 = reinterpret_cast<const T*>(&v1);
-                const T* p2 = reinterpret_cast<const T*>(&v2);
-                const T* p3 = reinterpret_cast<const T*>(&v3);
-#pragma unroll
-                for (int c = 0; c < V; ++c) {
-                    const float xf = to_f32(px[c]);
-                    a[0] = fmaf(xf, to_f32(p0[c]), a[0]);
-                    a[1] = fmaf(xf, to_f32(p1[c]), a[1]);
-                    a[2] = fmaf(xf, to_f32(p2[c]), a[2]);
-                    a[3] = fmaf(xf, to_f32(p3[c]), a[3]);
-                }
-            }
-        } else {
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
+    const T* w0 = Wr + (size_t)e0 * D;
+    const T* w1 = Wr + (size_t)min(e0 + 1, E - 1) * D;
+    const T* w2 = Wr + (size_t)min(e0 + 2, E - 1) * D;
+    const T* w3 = Wr + (size_t)min(e0 + 3, E - 1) * D;
+    if (D % V == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)Wr % 16 == 0) {
 #pragma unroll 4
-            for (int d = lane; d < D; d += 32) {
-                const float xv = to_f32(x[d]);
-                a[0] = fmaf(xv, to_f32(w0[d]), a[0]);
-                a[1] = fmaf(xv, to_f32(w1[d]), a[1]);
-                a[2] = fmaf(xv, to_f32(w2[d]), a[2]);
-                a[3] = fmaf(xv, to_f32(w3[d]), a[3]);
+        for (int d = lane * V; d < D; d += 32 * V) {
+            const uint4 xv = *reinterpret_cast<const uint4*>(x + d);
+            const uint4 v0 = *reinterpret_cast<const uint4*>(w0 + d), v1 = *reinterpret_cast<const uint4*>(w1 + d);
+            const uint4 v2 = *reinterpret_cast<const uint4*>(w2 + d), v3 = *reinterpret_cast<const uint4*>(w3 + d);
+            const T* px = reinterpret_cast<const T*>(&xv);
+            const T* p0 = reinterpret_cast<const T*>(&v0);
+            const T* p1 = reinterpret_cast<const T*>(&v1);
+            const T* p2 = reinterpret_cast<const T*>(&v2);
+            const T* p3 = reinterpret_cast<const T*>(&v3);
+#pragma unroll
+            for (int c = 0; c < V; ++c) {
+                const float xf = to_f32(px[c]);
+                a[0] = fmaf(xf, to_f32(p0[c]), a[0]);
+                a[1] = fmaf(xf, to_f32(p1[c]), a[1]);
+                a[2] = fmaf(xf, to_f32(p2[c]), a[2]);
+                a[3] = fmaf(xf, to_f32(p3[c]), a[3]);
             }
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const float v = warp_sum(a[u]);
-            if (lane == 0 && e0 + u < E) s[e0 + u] = v + (bias ? bias[e0 + u] : 0.f);
+    } else {
+#pragma unroll 4
+        for (int d = lane; d < D; d += 32) {
+            const float xv = to_f32(x[d]);
+            a[0] = fmaf(xv, to_f32(w0[d]), a[0]);
+            a[1] = fmaf(xv, to_f32(w1[d]), a[1]);
+            a[2] = fmaf(xv, to_f32(w2[d]), a[2]);
+            a[3] = fmaf(xv, to_f32(w3[d]), a[3]);
         }
     }
-    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const float v = warp_sum(a[u]);
+        if (lane == 0 && e0 + u < E) s[e0 + u] = v + (bias ? bias[e0 + u] : 0.f);
+    }
+}
+
+// One warp chooses one token's experts from its E logits in shared memory; idx may be followed by a second place.
+template <typename T>
+__device__ __forceinline__ void choose_experts(const RouteArgs<T>& ra, float* s, int* idx, int* idx2, float* wout, int lane) {
+    const int mode = ra.mode, E = ra.E, top = ra.top, n_groups = ra.n_groups, keep = ra.keep;
+    const float w_scale = ra.w_scale;
     if (mode == 1) {
         // the largest logits, and a softmax over them alone
         if (lane == 0) {
@@ -124,6 +125,7 @@ __device__ __forceinline__ void route_token(const T* x, const RouteArgs<T>& ra, 
                     if (s[e] > bv) { bv = s[e]; best = e; }
                 if (k == 0) mx = bv;
                 idx[k] = best;
+                if (idx2) idx2[k] = best;
                 wout[k] = expf(bv - mx);
                 wsum += wout[k];
                 s[best] = -INFINITY;                             // taken
@@ -150,74 +152,70 @@ __device__ __forceinline__ void route_token(const T* x, const RouteArgs<T>& ra, 
         for (int e = lane; e < E; e += 32) s[e] = s[e] / sum;
     }
     __syncwarp();
-    if (n_groups == 1) {
-        // the warp looks for the largest together: a lane's experts are lane, lane + 32, ..., and among equals the lowest wins
-        float wsum = 0.f;
-        for (int k = 0; k < top; ++k) {
-            int best = E;
-            float bv = -INFINITY;
-            for (int e = lane; e < E; e += 32) {
-                const float v = ra.correction ? s[e] + ra.correction[e] : s[e];
-                if (s[e] >= 0.f && (best == E || v > bv)) { bv = v; best = e; }
+    if (n_groups > 1 && keep < n_groups) {
+        // a lane scores the groups lane and lane + 32 (there are at most 64); the warp keeps the largest, the lowest number
+        // among equals; experts outside the kept groups are marked by a negative score (scores are >= 0)
+        const int per = E / n_groups;
+        float score[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int g = lane + 32 * u;
+            float gm = -1.f, g2 = 0.f;                          // the largest score of the group and the one after it
+            for (int e = g * per; g < n_groups && e < (g + 1) * per; ++e) {
+                if (s[e] > gm) { g2 = fmaxf(gm, 0.f); gm = s[e]; }
+                else if (s[e] > g2) g2 = s[e];
             }
+            if (ra.group_sum == 2 && per > 1 && g < n_groups) gm += g2;
+            score[u] = gm;
+        }
+        unsigned long long kept = 0ull;
+        for (int k = 0; k < keep; ++k) {
+            int best = 64;
+            float bv = -1.f;
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                if (!((kept >> (lane + 32 * u)) & 1ull) && score[u] > bv) { bv = score[u]; best = lane + 32 * u; }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
                 const int ob = __shfl_xor_sync(0xffffffffu, best, o);
-                if (ob < E && (best == E || ov > bv || (ov == bv && ob < best))) { bv = ov; best = ob; }
+                if (ov > bv || (ov == bv && ob < best)) { bv = ov; best = ob; }
             }
-            best = min(best, E - 1);                             // never beyond the experts, whatever the scores are
-            const float sc = s[best];
-            __syncwarp();
-            if (lane == 0) {
-                idx[k] = best;
-                wout[k] = sc;
-                s[best] = -1.f;                                  // taken (scores are >= 0)
-            }
-            wsum += sc;
-            __syncwarp();
+            if (best < 64) kept |= 1ull << best;
         }
-        for (int k = lane; k < top; k += 32) wout[k] = ra.renorm ? wout[k] / (wsum + 1e-20f) * w_scale : wout[k] * w_scale;
+        __syncwarp();                                            // every lane has read its groups
+        for (int e = lane; e < E; e += 32)
+            if (!((kept >> (e / per)) & 1ull)) s[e] = -1.f - s[e];
         __syncwarp();
-        return;
     }
-    if (lane == 0) {
-        // experts outside the kept groups are marked by a negative score (scores are >= 0)
-        if (n_groups > 1 && keep < n_groups) {
-            const int per = E / n_groups;
-            unsigned long long kept = 0ull;                 // at most 64 groups
-            for (int k = 0; k < keep; ++k) {
-                int best = -1;
-                float bv = -1.f;
-                for (int g = 0; g < n_groups; ++g) {
-                    if ((kept >> g) & 1ull) continue;
-                    float gm = -1.f, g2 = 0.f;             // the largest score of the group and the one after it
-                    for (int e = g * per; e < (g + 1) * per; ++e) {
-                        if (s[e] > gm) { g2 = fmaxf(gm, 0.f); gm = s[e]; }
-                        else if (s[e] > g2) g2 = s[e];
-                    }
-                    if (group_sum == 2 && per > 1) gm += g2;
-                    if (gm > bv) { bv = gm; best = g; }
-                }
-                if (best >= 0) kept |= 1ull << best;
-            }
-            for (int g = 0; g < n_groups; ++g)
-                if (!((kept >> g) & 1ull))
-                    for (int e = g * per; e < (g + 1) * per; ++e) s[e] = -1.f - s[e];
+    // the warp looks for the largest together: a lane's experts are lane, lane + 32, ..., and among equals the lowest wins
+    float wsum = 0.f;
+    for (int k = 0; k < top; ++k) {
+        int best = E;
+        float bv = -INFINITY;
+        for (int e = lane; e < E; e += 32) {
+            const float v = ra.correction ? s[e] + ra.correction[e] : s[e];
+            if (s[e] >= 0.f && (best == E || v > bv)) { bv = v; best = e; }
         }
-        float wsum = 0.f;
-        for (int k = 0; k < top; ++k) {
-            int best = 0;
-            float bv = -INFINITY;
-            for (int e = 0; e < E; ++e)
-                if (s[e] > bv) { bv = s[e]; best = e; }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+            const int ob = __shfl_xor_sync(0xffffffffu, best, o);
+            if (ob < E && (best == E || ov > bv || (ov == bv && ob < best))) { bv = ov; best = ob; }
+        }
+        best = min(best, E - 1);                                 // never beyond the experts, whatever the scores are
+        const float sc = s[best];
+        __syncwarp();
+        if (lane == 0) {
             idx[k] = best;
-            wout[k] = bv;
-            wsum += bv;
-            s[best] = -8.f;                                  // taken
+            if (idx2) idx2[k] = best;
+            wout[k] = sc;
+            s[best] = -1.f;                                      // taken (scores are >= 0)
         }
-        for (int k = 0; k < top; ++k) wout[k] = ra.renorm ? wout[k] / (wsum + 1e-20f) * w_scale : wout[k] * w_scale;
+        wsum += sc;
+        __syncwarp();
     }
+    for (int k = lane; k < top; k += 32) wout[k] = ra.renorm ? wout[k] / (wsum + 1e-20f) * w_scale : wout[k] * w_scale;
     __syncwarp();
 }
 
@@ -228,14 +226,19 @@ __device__ __forceinline__ void sort_pairs(const int* idx, int n, int E, int* of
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&cnt[idx[i]], 1);
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {                                  // the counts become offsets, 32 at a time
         int run = 0;
-        for (int e = 0; e < E; ++e) {
-            const int c = cnt[e];
-            cnt[e] = run;
-            run += c;
+        for (int e0 = 0; e0 <= E; e0 += 32) {
+            const int e = e0 + threadIdx.x, c = e < E ? cnt[e] : 0;
+            int upto = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                if ((int)threadIdx.x >= o) upto += v;
+            }
+            if (e <= E) cnt[e] = run + upto - c;
+            run += __shfl_sync(0xffffffffu, upto, 31);
         }
-        cnt[E] = run;
     }
     __syncthreads();
     for (int e = threadIdx.x; e <= E; e += blockDim.x) offsets[e] = cnt[e];
@@ -259,33 +262,55 @@ __global__ void __launch_bounds__(128)
 moe_route_kernel(const T* h, long long ld, int Tn, int* idx, float* wout, RouteArgs<T> ra) {
     extern __shared__ float sc[];
     pdl_wait();
+    pdl_launch();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * 4 + warp;
     if (t >= Tn) return;
-    route_token(h + (size_t)t * ld, ra, sc + warp * ra.E, idx + (size_t)t * ra.top, wout + (size_t)t * ra.top, t, lane);
+    const T* x = h + (size_t)t * ld;
+    float* s = sc + warp * ra.E;
+    if (ra.Wg) token_gate(x, ra.Wg, ra.D, ra.gate + t, lane);
+    for (int e0 = 0; e0 < ra.E; e0 += 4) router_logits(x, ra, s, e0, lane);
+    __syncwarp();
+    choose_experts(ra, s, idx + (size_t)t * ra.top, (int*)nullptr, wout + (size_t)t * ra.top, lane);
 }
 
 __global__ void __launch_bounds__(1024)
 moe_sort_kernel(const int* idx, int n, int E, int* offsets, int* sorted) {
     __shared__ int cnt[MAX_E + 1];
     pdl_wait();
+    pdl_launch();
     sort_pairs(idx, n, E, offsets, sorted, cnt);
 }
 
-// Few tokens (decode steps): one CTA of 8 warps routes them all and orders the pairs, in one launch.
-// dynamic shared memory: 8 * E floats, then E + 1 ints
+// Few tokens (decode steps): one CTA routes them all and orders the pairs, in one launch.  All of it is latency: the
+// router's rows are asked into L2 before the wait, the logits of four experts of one token are a warp's task (one round of
+// loads), a warp then chooses for a token, and the pairs are ordered from shared memory.  8 experts of 768 columns and 3
+// tokens in a decode step: 8.7 us, with a warp per token and one lane choosing 19.9 us.
+// dynamic shared memory: Tn * E floats, then E + 1 ints, then Tn * top ints
+constexpr int ROUTE_WARPS = 16;
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(ROUTE_WARPS * 32)
 moe_route_sort_kernel(const T* h, long long ld, int Tn, int* idx, float* wout, int* offsets, int* sorted, RouteArgs<T> ra) {
     extern __shared__ float sc[];
-    const int E = ra.E, top = ra.top;
-    int* cnt = reinterpret_cast<int*>(sc + 8 * E);
+    const int E = ra.E, top = ra.top, quads = (E + 3) / 4;
+    int* cnt = reinterpret_cast<int*>(sc + Tn * E);
+    int* chosen = cnt + E + 1;
+    const size_t bytes = (size_t)E * ra.D * sizeof(T);
+    for (size_t b = (size_t)threadIdx.x * 128; b < bytes; b += ROUTE_WARPS * 32 * 128)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(ra.Wr) + b));
     pdl_wait();
+    pdl_launch();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int t = warp; t < Tn; t += 8)
-        route_token(h + (size_t)t * ld, ra, sc + warp * E, idx + (size_t)t * top, wout + (size_t)t * top, t, lane);
-    __syncthreads();                                         // the CTA's own writes of idx are visible to all its threads
-    sort_pairs(idx, Tn * top, E, offsets, sorted, cnt);
+    const int tasks = Tn * quads;
+    for (int i = warp; i < tasks + (ra.Wg ? Tn : 0); i += ROUTE_WARPS) {
+        if (i >= tasks) token_gate(h + (size_t)(i - tasks) * ld, ra.Wg, ra.D, ra.gate + (i - tasks), lane);
+        else router_logits(h + (size_t)(i / quads) * ld, ra, sc + i / quads * E, i % quads * 4, lane);
+    }
+    __syncthreads();
+    for (int t = warp; t < Tn; t += ROUTE_WARPS)
+        choose_experts(ra, sc + t * E, idx + (size_t)t * top, chosen + t * top, wout + (size_t)t * top, lane);
+    __syncthreads();
+    sort_pairs(chosen, Tn * top, E, offsets, sorted, cnt);
 }
 
 // an activation of one argument on a product (an expert without a gate); 0: none
@@ -304,6 +329,30 @@ struct SelfRows {
     int E_total, top;
 };
 
+// The expert, first row and row count of tile blockIdx.x, tiles of ROWS pairs counted expert by expert (expert -1: beyond the
+// last; expert E: pairs of identity experts, E up to E_total).  The offsets come in at once: walked one by one they cost a
+// round trip to memory each.
+template <int ROWS>
+__device__ __forceinline__ void find_tile(const int* offsets, int E, int E_total, int* s_off, int* s_e, int* s_r0, int* s_cnt) {
+    for (int e = threadIdx.x; e <= E_total; e += blockDim.x) s_off[e] = offsets[e];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int tile = blockIdx.x, found = -1, r0 = 0, c = 0;
+        for (int e = 0; e < E; ++e) {
+            const int lo = s_off[e], n = s_off[e + 1] - lo;
+            const int tiles = (n + ROWS - 1) / ROWS;
+            if (tile < tiles) { found = e; r0 = lo + tile * ROWS; c = min(ROWS, n - tile * ROWS); break; }
+            tile -= tiles;
+        }
+        if (found < 0 && E_total > E) {
+            const int lo = s_off[E] + tile * ROWS, n = s_off[E_total] - lo;
+            if (n > 0) { found = E; r0 = lo; c = min(ROWS, n); }
+        }
+        *s_e = found; *s_r0 = r0; *s_cnt = c;
+    }
+    __syncthreads();
+}
+
 template <typename TA, typename TW, typename TO>
 __global__ void __launch_bounds__(256)
 moe_grouped_kernel(const TA* A, long long lda, const TW* __restrict__ W, TO* out, long long ldo, const int* offsets,
@@ -313,23 +362,10 @@ moe_grouped_kernel(const TA* A, long long lda, const TW* __restrict__ W, TO* out
     __shared__ float Ws[64][33];
     __shared__ float Us[64][33];
     __shared__ int rows_a[32], rows_o[32];
-    __shared__ int s_e, s_r0, s_cnt;
+    __shared__ int s_e, s_r0, s_cnt, s_off[MAX_E + 1];
     pdl_wait();
-    if (threadIdx.x == 0) {
-        int tile = blockIdx.x, e = 0, found = -1, r0 = 0, c = 0;
-        for (; e < E; ++e) {
-            const int lo = offsets[e], n = offsets[e + 1] - lo;
-            const int tiles = (n + 31) / 32;
-            if (tile < tiles) { found = e; r0 = lo + tile * 32; c = min(32, n - tile * 32); break; }
-            tile -= tiles;
-        }
-        if (found < 0 && self.rows) {
-            const int lo = offsets[E] + tile * 32, n = offsets[self.E_total] - lo;
-            if (n > 0) { found = E; r0 = lo; c = min(32, n); }
-        }
-        s_e = found; s_r0 = r0; s_cnt = c;
-    }
-    __syncthreads();
+    pdl_launch();
+    find_tile<32>(offsets, E, self.rows ? self.E_total : E, s_off, &s_e, &s_r0, &s_cnt);
     const int e = s_e, cnt = s_cnt;
     if (e < 0) return;
     if (threadIdx.x < 32) {
@@ -400,56 +436,58 @@ moe_grouped_kernel(const TA* A, long long lda, const TW* __restrict__ W, TO* out
 }
 
 // ------------------------------------------------------------------------------------------------ few pairs (decode steps)
-// grid (pairs, column blocks of 64), 8 warps.  The pair's input row is staged in shared memory as 32-bit; a warp owns 8
-// columns, its lanes split K with 16-byte loads of the 8 weight rows (all in flight at once), and the sums meet by
-// a butterfly.  Every weight of the pair's expert leaves L2 once per pair: with few pairs that is the whole cost.
+// grid (pairs, column blocks of 16), 8 warps.  The pair's input row is staged in shared memory as 32-bit; a warp owns 2
+// columns, its lanes split K with 16-byte loads of the weight rows, four steps of K in flight at once, and the sums meet by
+// a butterfly.  Every weight of the pair's expert is read once per pair: with few pairs the cost is the chain of round trips
+// to memory, so the pair's expert is found by all threads at once, a warp takes few columns and a launch many warps.  512 x 768
+// gated and 768 x 512 at 6 pairs in a decode step: 7.2 us (8 columns a warp, the expert found one offset after the
+// other: 10.8 us).
+constexpr int ROW_COLS = 2;
 template <typename TA, typename TW, typename TO>
 __global__ void __launch_bounds__(256)
 moe_rows_kernel(const TA* A, long long lda, const TW* __restrict__ W, TO* out, long long ldo, const int* offsets,
                 const int* sorted, int E, int N, int K, int a_div, int out_by_pair, int gated, float limit, float alpha,
                 int uact, SelfRows<TA> self) {
     extern __shared__ float xs[];                                // [K]
-    __shared__ int s_e;
     pdl_wait();
+    pdl_launch();
     const int i = blockIdx.x;
+    int e = 0;                                                   // the pair's expert: how many later ones start at or before it
+    for (int e0 = 1; e0 < E; e0 += 256) e += __syncthreads_count(e0 + (int)threadIdx.x < E && offsets[e0 + threadIdx.x] <= i);
     if (i >= offsets[E]) {                                       // a pair of an identity expert (uniform over the CTA)
-        const int col = blockIdx.y * 64 + threadIdx.x;
-        if (self.rows && threadIdx.x < 64 && col < N) {
+        const int col = blockIdx.y * 8 * ROW_COLS + threadIdx.x;
+        if (self.rows && threadIdx.x < 8 * ROW_COLS && col < N) {
             const int p = sorted[i];
             out[(size_t)(out_by_pair ? p : i) * ldo + col] = from_f32<TO>(to_f32(self.rows[(size_t)(p / self.top) * self.ld + col]));
         }
         return;
-    }
-    if (threadIdx.x == 0) {
-        int e = 0;
-        while (e < E - 1 && offsets[e + 1] <= i) ++e;
-        s_e = e;
     }
     const int pair = sorted[i];
     const TA* a = A + (size_t)(a_div > 0 ? pair / a_div : i) * lda;
     for (int k = threadIdx.x; k < K; k += 256) xs[k] = to_f32(a[k]);
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n0 = blockIdx.y * 64 + warp * 8;
+    const int n0 = (blockIdx.y * 8 + warp) * ROW_COLS;
     if (n0 >= N) return;
     const size_t wrows = gated ? (size_t)2 * N : (size_t)N;
-    const TW* We = W + (size_t)s_e * wrows * K;
+    const TW* We = W + (size_t)e * wrows * K;
     constexpr int V = 16 / sizeof(TW);                           // weights per 16-byte load
-    float acc[8], acu[8];
+    float acc[ROW_COLS], acu[ROW_COLS];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) acc[u] = acu[u] = 0.f;
+    for (int u = 0; u < ROW_COLS; ++u) acc[u] = acu[u] = 0.f;
     const bool vec = K % V == 0 && ((uintptr_t)W % 16 == 0);
     if (vec) {
+#pragma unroll 4
         for (int k = lane * V; k < K; k += 32 * V) {
-            uint4 w[8], wu[8];
+            uint4 w[ROW_COLS], wu[ROW_COLS];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
+            for (int u = 0; u < ROW_COLS; ++u) {
                 const int n = min(n0 + u, N - 1);
                 w[u] = *reinterpret_cast<const uint4*>(We + (size_t)n * K + k);
                 if (gated) wu[u] = *reinterpret_cast<const uint4*>(We + (size_t)(N + n) * K + k);
             }
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
+            for (int u = 0; u < ROW_COLS; ++u) {
                 const TW* p = reinterpret_cast<const TW*>(&w[u]);
                 const TW* q = reinterpret_cast<const TW*>(&wu[u]);
 #pragma unroll
@@ -462,7 +500,7 @@ moe_rows_kernel(const TA* A, long long lda, const TW* __restrict__ W, TO* out, l
     } else {
         for (int k = lane; k < K; k += 32) {
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
+            for (int u = 0; u < ROW_COLS; ++u) {
                 const int n = min(n0 + u, N - 1);
                 acc[u] = fmaf(xs[k], to_f32(We[(size_t)n * K + k]), acc[u]);
                 if (gated) acu[u] = fmaf(xs[k], to_f32(We[(size_t)(N + n) * K + k]), acu[u]);
@@ -471,7 +509,7 @@ moe_rows_kernel(const TA* A, long long lda, const TW* __restrict__ W, TO* out, l
     }
     const size_t orow = (size_t)(out_by_pair ? pair : i) * ldo;
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
+    for (int u = 0; u < ROW_COLS; ++u) {
         float v = warp_sum(acc[u]);
         if (gated) v = gate_mul(v, warp_sum(acu[u]), gated, limit, alpha);
         else v = unary_act(v, uact);
@@ -513,24 +551,11 @@ moe_grouped_mma_kernel(const __nv_bfloat16* A, long long lda, const __nv_bfloat1
     constexpr int STAGE = (GM + GN * (1 + GATED)) * GROW;        // elements per stage
     bf* sm = reinterpret_cast<bf*>(gsm);
     __shared__ int rows_a[GM], rows_o[GM];
-    __shared__ int s_e, s_r0, s_cnt;
+    __shared__ int s_e, s_r0, s_cnt, s_off[MAX_E + 1];
     pdl_wait();
+    pdl_launch();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid == 0) {
-        int tile = blockIdx.x, found = -1, r0 = 0, c = 0;
-        for (int e = 0; e < E; ++e) {
-            const int lo = offsets[e], n = offsets[e + 1] - lo;
-            const int tiles = (n + GM - 1) / GM;
-            if (tile < tiles) { found = e; r0 = lo + tile * GM; c = min(GM, n - tile * GM); break; }
-            tile -= tiles;
-        }
-        if (found < 0 && self.rows) {
-            const int lo = offsets[E] + tile * GM, n = offsets[self.E_total] - lo;
-            if (n > 0) { found = E; r0 = lo; c = min(GM, n); }
-        }
-        s_e = found; s_r0 = r0; s_cnt = c;
-    }
-    __syncthreads();
+    find_tile<GM>(offsets, E, self.rows ? self.E_total : E, s_off, &s_e, &s_r0, &s_cnt);
     const int e = s_e, cnt = s_cnt;
     if (e < 0) return;
     if (tid < GM) {
@@ -614,6 +639,7 @@ moe_grouped_mma_kernel(const __nv_bfloat16* A, long long lda, const __nv_bfloat1
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(const float* pair_out, const float* w, float* y, long long ldy, int Tn, int D, int top, int accumulate) {
     pdl_wait();
+    pdl_launch();
     const long long total = (long long)Tn * D;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const int t = (int)(i / D), d = (int)(i % D);
@@ -648,12 +674,19 @@ MLLM_EXPORT int mllm_moe_route(const void* h, long long ld, const void* Wr, cons
     const RouteArgs<float> rf{(const float*)Wr, bias, correction, (const float*)Wg, gate, mode, D, E, top, n_groups, keep, group_sum, renorm, w_scale};
     const RouteArgs<bf> rb{(const bf*)Wr, bias, correction, (const bf*)Wg, gate, mode, D, E, top, n_groups, keep, group_sum, renorm, w_scale};
     if (Tn <= MOE_FEW_TOKENS) {
-        const size_t smem = (size_t)8 * E * 4 + (size_t)(E + 1) * 4;
+        const size_t smem = ((size_t)Tn * E + E + 1 + (size_t)Tn * top) * 4;
+        static bool raised = false;
+        if (smem > 48 * 1024 && !raised) {
+            MLLM_CUDA(cudaFuncSetAttribute(moe_route_sort_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+            MLLM_CUDA(cudaFuncSetAttribute(moe_route_sort_kernel<bf>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+            raised = true;
+        }
+        const dim3 few(ROUTE_WARPS * 32);
         if (dtype == MLLM_F32)
-            MLLM_CUDA(mllm_launch(moe_route_sort_kernel<float>, dim3(1), dim3(256), smem, stream, true, (const float*)h, ld, Tn, idx, w,
+            MLLM_CUDA(mllm_launch(moe_route_sort_kernel<float>, dim3(1), few, smem, stream, true, (const float*)h, ld, Tn, idx, w,
                                   offsets, sorted, rf));
         else
-            MLLM_CUDA(mllm_launch(moe_route_sort_kernel<bf>, dim3(1), dim3(256), smem, stream, true, (const bf*)h, ld, Tn, idx, w,
+            MLLM_CUDA(mllm_launch(moe_route_sort_kernel<bf>, dim3(1), few, smem, stream, true, (const bf*)h, ld, Tn, idx, w,
                                   offsets, sorted, rb));
         return 0;
     }
@@ -694,7 +727,8 @@ MLLM_EXPORT int mllm_moe_grouped(const void* A, long long lda, const void* W, vo
     const int gated = kind == 0 ? act : 0;
     const int uact = kind == 2 ? act : 0;
     if (n_pairs <= MOE_FEW_PAIRS && (size_t)K * 4 <= 96 * 1024) {
-        const dim3 fg(n_pairs, (N + 63) / 64);
+        const dim3 fg(n_pairs, (N + 8 * ROW_COLS - 1) / (8 * ROW_COLS));
+        if (fg.y > 65535) return mllm_fail(1, "moe_grouped: too many columns");
         const size_t smem = (size_t)K * 4;
 #define MLLM_ROWS(TA, TW, TO, SELF)                                                                                            \
         do {                                                                                                             \
