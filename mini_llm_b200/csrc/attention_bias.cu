@@ -898,6 +898,7 @@ int check_sizes(int H, int Hkv, int dk, int dv, int page_size, int dtype) {
 
 // impl: 0 simt, 1 tiled (needs tiles), 2 split (single tokens; needs part_o [T*H*nsplit*dv], part_ml [T*H*nsplit*2] and the
 // cuts of the keys, at least as many splits as the longest context has), 3 mma (bfloat16 prompt portions on tensor cores; needs tiles).
+// 4 and 5 are the two launches of 2, the splits and their merge, apart: what is launched between them runs beside the splits.
 MLLM_EXPORT int mllm_attention_bias(const void* q, long long q_stride, const void* k_pages, const void* v_pages,
                                     const int* block_table, int bt_stride, const int* token_seq, const int* positions,
                                     const int* tiles, int n_tiles, void* out, long long out_stride, float* part_o,
@@ -946,7 +947,7 @@ MLLM_EXPORT int mllm_attention_bias(const void* q, long long q_stride, const voi
         }
         return 0;
     }
-    if (impl == 2) {
+    if (impl == 2 || impl == 4 || impl == 5) {
         if (!part_o || !part_ml || nsplit <= 0) return mllm_fail(1, "attention_bias: the split kernel needs scratch for its partial results");
         KeyCuts cuts;
         if (int rc = key_cuts("attention_bias", near, edge, far, &cuts)) return rc;
@@ -978,8 +979,10 @@ MLLM_EXPORT int mllm_attention_bias(const void* q, long long q_stride, const voi
         const dim3 grid(nsplit, Hkv * chunks, T), block(32 * HG * KS);
         auto go = [&](auto kern, auto merge, auto* tq, auto* tk, auto* tv, auto* to) -> int {
             if (smem > 48 * 1024) MLLM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            MLLM_CUDA(mllm_launch(kern, grid, block, smem, stream, true, tq, q_stride, tk, tv, block_table, bt_stride, token_seq,
-                                  positions, part_o, part_ml, H, Hkv, dkq, dk, dv, page_size, HG, KS, NT, cuts, a));
+            if (impl != 5)
+                MLLM_CUDA(mllm_launch(kern, grid, block, smem, stream, true, tq, q_stride, tk, tv, block_table, bt_stride, token_seq,
+                                      positions, part_o, part_ml, H, Hkv, dkq, dk, dv, page_size, HG, KS, NT, cuts, a));
+            if (impl == 4) return 0;
             MLLM_CUDA(mllm_launch(merge, dim3((unsigned)blocks), dim3(WARPS * 32), 0, stream, true, (const float*)part_o,
                                   (const float*)part_ml, positions, to, out_stride, T, H, dv, nsplit, cuts, a));
             return 0;

@@ -115,7 +115,7 @@ def _signatures(lib):
                          c_float, c_float, c_int, c_void_p],
         "mllm_gated_recurrence_wide": [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_void_p,
                                        c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int, c_int,
-                                       c_void_p],
+                                       c_int, c_void_p],
         "mllm_gated_act": [c_void_p, c_ll, c_void_p, c_ll, c_int, c_int, c_int, c_float, c_float, c_void_p, c_int, c_void_p],
         "mllm_paged_write": [c_void_p, c_ll, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "mllm_paged_write_kv": [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
@@ -147,7 +147,7 @@ def _signatures(lib):
         "mllm_softcap": [c_void_p, c_ll, c_int, c_int, c_float, c_void_p],
         "mllm_gated_recurrence": [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_void_p,
                                   c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_float, c_float, c_int,
-                                  c_int, c_void_p],
+                                  c_int, c_int, c_void_p],
         "mllm_norm_scale_add": [c_void_p, c_ll, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_ll, c_void_p, c_float,
                                 c_float, c_void_p, c_ll, c_int, c_int, c_float, c_int, c_void_p],
         "mllm_latent_prepare": [c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
@@ -1042,7 +1042,7 @@ def bias_cuts(num_heads: int, num_kv_heads: int):
 
 def biased_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, num_kv_heads, scale, dist_bias=None,
                      q_scale=None, out_scale: float = 1.0, window=None, chunk=None, sink=None, softcap: float = 0.0,
-                     slopes=None, keep_first: int = 0, gate=None, impl: Optional[str] = None) -> None:
+                     slopes=None, keep_first: int = 0, gate=None, impl: Optional[str] = None, company=None) -> None:
     """Causal attention over the cache with keys and values of different sizes, an additive score bias
     ``dist_bias[head, i - j]`` (float32 [heads, n]) and a factor ``q_scale[position]`` (float32 [n]) on the query:
     out[t] = out_scale * softmax_j((q_t . k_j) * scale * q_scale[p_t] + dist_bias[h, p_t - j]) v_j.
@@ -1051,7 +1051,8 @@ def biased_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, n
     term of the softmax's denominator and of nothing else.  ``softcap`` c > 0: the scaled product s becomes
     c * tanh(s / c) before any bias is added; ``slopes`` (float32 [heads]): slopes[h] * (p_t - j) is taken off the score.
     ``keep_first`` f: the first f positions stay visible beyond the window or the chunk.  ``gate`` [T, heads * dv] in q's
-    dtype: the result is multiplied, entry by entry, with sigmoid(gate).
+    dtype: the result is multiplied, entry by entry, with sigmoid(gate).  ``company``: a function that launches what need not
+    wait for this attention; it is called right behind the launch that walks the keys (before the splits are merged).
 
     q [T, heads * dkq], k_pages [P, kv_heads, page_size, dk] with dk >= dkq a multiple of 8 (key rows padded with
     zeros), v_pages [P, kv_heads, page_size, dv], out [T, heads * dv] (rows contiguous; a column slice of a wider
@@ -1121,17 +1122,27 @@ def biased_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, n
                               f"multiples of 16 up to {BIAS_ATTN_MMA_MAX_DIM} and 16-byte aligned rows")
     elif impl != "simt":
         raise KernelError(f"biased_attention: unknown implementation {impl!r}")
-    _call("mllm_attention_bias", q.data_ptr(), ldq, k_pages.data_ptr(), v_pages.data_ptr(), block_table.data_ptr(),
-          _rows("block_table", block_table), ctx.token_seq.data_ptr(), ctx.positions.data_ptr(), tiles, n_tiles,
-          out.data_ptr(), ldo, part_o, part_ml, nsplit, *cuts, T, num_heads, num_kv_heads, dkq, dk, dv, ps, float(scale),
-          float(out_scale), dist_bias.data_ptr() if dist_bias is not None else None, n_dist,
-          q_scale.data_ptr() if q_scale is not None else None, int(window or 0), int(chunk or 0),
-          sink.data_ptr() if sink is not None else None, float(softcap or 0.0),
-          slopes.data_ptr() if slopes is not None else None, int(keep_first), gate.data_ptr() if gate is not None else None,
-          _rows("gate", gate) if gate is not None else 0, _dt(q), {"simt": 0, "tiled": 1, "split": 2, "mma": 3}[impl],
-          _stream())
-    if impl == "split":
+    def launch(code):
+        _call("mllm_attention_bias", q.data_ptr(), ldq, k_pages.data_ptr(), v_pages.data_ptr(), block_table.data_ptr(),
+              _rows("block_table", block_table), ctx.token_seq.data_ptr(), ctx.positions.data_ptr(), tiles, n_tiles,
+              out.data_ptr(), ldo, part_o, part_ml, nsplit, *cuts, T, num_heads, num_kv_heads, dkq, dk, dv, ps, float(scale),
+              float(out_scale), dist_bias.data_ptr() if dist_bias is not None else None, n_dist,
+              q_scale.data_ptr() if q_scale is not None else None, int(window or 0), int(chunk or 0),
+              sink.data_ptr() if sink is not None else None, float(softcap or 0.0),
+              slopes.data_ptr() if slopes is not None else None, int(keep_first), gate.data_ptr() if gate is not None else None,
+              _rows("gate", gate) if gate is not None else 0, _dt(q), code, _stream())
+
+    if impl != "split":
+        launch({"simt": 0, "tiled": 1, "mma": 3}[impl])
+        if company is not None:
+            company()
+    elif company is not None:
+        launch(4)               # the splits
+        company()
+        launch(5)               # their merge
+    else:
         global launches
+        launch(2)
         launches += 1           # the kernel that merges the splits
 
 
@@ -2055,13 +2066,15 @@ recurrence_launches = {}       # "step" / "wide" -> launches so far
 
 
 def gated_recurrence(a, z, v, f_bias, lower, norm_weight, eps: float, state, ctx, out, *, heads: int, out_scale: float = 1.0,
-                     write_state: bool = True, impl: Optional[str] = None) -> None:
+                     write_state: bool = True, impl: Optional[str] = None, beside: bool = False) -> None:
     """The gated linear recurrence of csrc/gated_recurrence.cu over the step's tokens, request by request:
     f = lower + (1 - lower) * sigmoid(z + f_bias); S <- diag(f) S + (1 - f) v^T; o = S^T silu(a);
     out = out_scale * rms_norm(o) * norm_weight per head.  a, z [T, heads * ek], v, out [T, heads * ev] (rows
     contiguous; column slices are fine), state [slots, heads, ek, ev] float32, indexed by ctx.state_slots.
     ``impl``: "step" (one CTA per request and head with the norm fused: single tokens) or "wide" (the recurrence
-    spread over 32-column CTAs, then the norm kernel: prompt portions); None picks by the step's shape."""
+    spread over 32-column CTAs, then the norm kernel: prompt portions); None picks by the step's shape.
+    ``beside``: the launch before this one is a kernel that waits for what this one reads and lets its dependents start only
+    then; this one runs beside it (csrc/gated_recurrence.cu)."""
     _cuda("a", a, contiguous=False)
     _cuda("z", z, a.dtype, contiguous=False)
     _cuda("v", v, a.dtype, contiguous=False)
@@ -2088,7 +2101,7 @@ def gated_recurrence(a, z, v, f_bias, lower, norm_weight, eps: float, state, ctx
         _call("mllm_gated_recurrence_wide", a.data_ptr(), _rows("a", a), z.data_ptr(), _rows("z", z), v.data_ptr(),
               _rows("v", v), f_bias.data_ptr(), lower.data_ptr(), state.data_ptr(), ctx.cu_q.data_ptr(),
               ctx.state_slots.data_ptr(), raw.data_ptr(), _rows("raw", raw), ctx.S, heads, ek, ev, int(write_state),
-              _dt(a), _stream())
+              int(beside), _dt(a), _stream())
         rmsnorm(raw, norm_weight, eps, out, unit_offset=False, heads=heads, scale=out_scale)
         return
     if impl != "step":
@@ -2096,7 +2109,7 @@ def gated_recurrence(a, z, v, f_bias, lower, norm_weight, eps: float, state, ctx
     _call("mllm_gated_recurrence", a.data_ptr(), _rows("a", a), z.data_ptr(), _rows("z", z), v.data_ptr(), _rows("v", v),
           f_bias.data_ptr(), lower.data_ptr(), norm_weight.data_ptr(), state.data_ptr(), ctx.cu_q.data_ptr(),
           ctx.state_slots.data_ptr(), out.data_ptr(), _rows("out", out), ctx.S, heads, ek, ev, float(eps), float(out_scale),
-          int(write_state), _dt(a), _stream())
+          int(write_state), int(beside), _dt(a), _stream())
 
 
 attention_launches = {}     # attention kernel name -> launches so far (tests check which kernel a step took)

@@ -131,10 +131,18 @@ class ParallelMixer(Mixer):
         wide = self.out_weight.shape[1]
         mid = ctx.ws.buf("mix_core", T, -(-wide // 8) * 8, self.rt.act_dtype)[:, :wide]
         r = c = 0
+        args = []
         for b, s in zip(self.branches, self.scales):
-            b.core(proj[:, r:r + b.in_width], ctx, cache, mid[:, c:c + b.core_width], out_scale=s)
+            args.append((b, (proj[:, r:r + b.in_width], ctx, cache, mid[:, c:c + b.core_width], s)))
             r += b.in_width
             c += b.core_width
+        pair = len(args) == 2 and getattr(args[0][0], "takes_company", False) and getattr(args[1][0], "goes_beside", False)
+        if pair:                            # the cores read the projection and nothing of each other
+            (first, a), (second, b) = args
+            first.core(*a, company=lambda: second.core(*b, beside=True))
+        else:
+            for part, a in args:
+                part.core(*a)
         ops.linear(mid, self.out_weight, None, out=out_accum, accumulate=accumulate)
 
 
