@@ -1,76 +1,65 @@
 // Causal attention of prompt portions over the paged cache on the fifth-generation tensor
 // cores: tiles of 128 queries against blocks of 128 keys, head size 64, bfloat16.
 //
-// A CTA takes one tile of up to 128 consecutive new tokens of one request and one head.
-// Warp 0 is the producer: the query tile and, block by block, the key and value pages come
-// in through TMA (cp.async.bulk.tensor, 128-byte swizzle; a page of 8, 16 ... 128 tokens of
-// one head is a box of page_size rows x 64 values; pages that no row of the tile can see
-// are fetched from beyond the pool, which the copy engine fills with zeros).  Warp 1 (one
-// lane) issues the MMAs: S = Q.K^T (tcgen05.mma 128 x 128 x 16, four per block) into tensor
-// memory, and, once the softmax warps have turned S into weights, O_blk = P.V (128 x 64 x 16,
-// eight per term; V is read as it lies in the pages, an MN-major operand) into a second range
-// of tensor memory.  Warps 2-17 are the softmax: four threads share a query row (a warp may
-// only read its own quarter of the tensor memory's lanes, and one warp reads it slowly, about
-// 5 GB/s, so sixteen warps read side by side); each reads 32 of the block's 128 scores with
-// tcgen05.ld, the four exchange their maxima through shared memory, and they keep the online
-// softmax of the row in 32-bit registers
-//   m' = max(m, s), alpha = exp(m - m'), p = exp(s - m'), o = o*alpha + p.v, l = l*alpha + sum p
-// (the reference's recurrence, src/kernels/prefill/flashattention.cu:129-168, with base-2
-// exponentials and the scale folded in), write the weights of the block to shared memory as
-// two bfloat16 terms p = hi + lo (the product then keeps about 16 bits of them), and add
-// O_blk into their row of o.  S and the weights are double-buffered: the MMAs of S for block
-// i+1 are issued before those of P.V for block i, and a softmax thread adds O_blk of block i
-// only after it has turned S of block i+1 into weights, so neither side waits for the other's
-// hand-over (an mbarrier round trip costs about as much as the arithmetic of a block).
+// A CTA takes one tile of up to 128 consecutive new tokens of one request and one head.  Its keys, in blocks of 64, are dealt
+// to four streams that know nothing of each other until the end: block b (positions [64 b, 64 b + 64)) belongs to stream b % 4.
+// A stream has 64 columns of tensor memory for its scores and 64 for its sums, and
+//  * a producer warp that brings its key and value pages with TMA (cp.async.bulk.tensor, 128-byte swizzle; a page of one head is
+//    a box of page_size rows x 64 values; pages that no row of the tile can see are fetched from beyond the pool, i.e. zeros);
+//  * an issuing warp: S = Q.K^T (tcgen05.mma 128 x 64 x 16), and O += P.V with P as the MMA's tensor-memory operand and V as it
+//    lies in the pages, an MN-major operand;
+//  * four softmax warps, a thread per query row: read 64 scores, write the weights p = hi + lo, two bfloat16 terms (the product
+//    then keeps about 16 bits of them), over the scores, and keep the row's maximum and sum in 32-bit
+//      m' = max(m, s), p = exp(s - m'), O = O*exp(m - m') + p.v, l = l*exp(m - m') + sum p
+//    (the reference's recurrence, src/kernels/prefill/flashattention.cu:129-168, with base-2 exponentials and the scale
+//    folded in).  The sums stay in tensor memory; m and O move only where a score exceeds m by more than 2^8 (until then p
+//    grows beyond 1, in 32-bit and in both terms alike), which after the first blocks is rare.
+// At the end a row's four streams meet: out = sum_g O_g 2^(m_g - m) / sum_g l_g 2^(m_g - m), in the order of g.
 //
-// Block j always covers the absolute positions [128 j, 128 j + 128), so the order of the
-// additions for a query does not depend on how the prompt was cut or what else is in the
-// batch.  Every wait on an mbarrier is bounded; after the limit the kernel records an
+// What bounds it: the softmax, about 11 instructions per score on 4 x 32 lanes, 1,400 cycles per 128 x 128 scores; the MMAs
+// take a fifth of that.  A stream's own chain (scores, weights, product and the hand-overs between, some 900 cycles a block
+// beside its arithmetic) is hidden by the other three.  With all sixteen warps on one block of 128 keys, maxima exchanged, P
+// through shared memory and O added in registers, every hand-over stood in the way of all of them: 4,200 cycles per 128 x 128.
+// 2 x 1,024 tokens, 12 heads: 17 us a launch, 22 us so; 512 tokens behind 450, 16 heads: 17 and 25 us.
+//
+// A block's place and stream follow from positions, so the order of the additions for a query does not depend on how the
+// prompt was cut or what else is in the batch.  Every wait on an mbarrier is bounded; after the limit the kernel records an
 // error code that the host reads, lets its copies land, frees its tensor memory and returns.
 //
 // The reference's prefill attention handles one score at a time with block-wide reductions
 // (src/kernels/prefill/flashattention.cu:7-32) and reads the step's own Q|K|V buffer.
-#include "tcgen05.cuh"
+#include "split_f32.cuh"
 
 namespace {
 
 using namespace tc;
 
-constexpr int BQ = 128, BKV = 128, DH = 64;
-constexpr int PARTS = 4;                             // threads per query row: each takes 32 keys of a block and 16 of the 64 output values
-constexpr int SOFTMAX_WARPS = 4 * PARTS;
-constexpr int THREADS = (3 + SOFTMAX_WARPS) * 32;  // key producer, MMA issuer, softmax warps, value producer
+constexpr int BQ = 128, BKV = 64, DH = 64, STREAMS = 4;
+constexpr int SOFTMAX_WARPS = 4 * STREAMS, ISSUE_WARP = SOFTMAX_WARPS, LOAD_WARP = ISSUE_WARP + STREAMS;   // 16, 4 and 4 warps
+constexpr int THREADS = (LOAD_WARP + STREAMS) * 32;
 constexpr int Q_BYTES = BQ * DH * 2;                 // 16 KB
-constexpr int KV_BYTES = BKV * DH * 2;               // 16 KB each for K and V of a block
-constexpr int P_BYTES = BQ * BKV * 2;                // 32 KB per term: two sub-tiles of 128 rows x 64 keys
+constexpr int KV_BYTES = BKV * DH * 2;               // 8 KB each for K and V of a block
 constexpr int STAGES = 2;
-constexpr int XCH_BYTES = 2 * PARTS * BQ * 4;        // partial row maxima, double-buffered; reused for the row sums at the end
-constexpr size_t SMEM = 1024 + Q_BYTES + STAGES * 2 * KV_BYTES + 2 * 2 * P_BYTES + XCH_BYTES + 512;
-constexpr uint32_t TMEM_COLS = 512;                  // S of even blocks in columns 0..127, of odd blocks in 128..255, O_blk in 256..319
-constexpr uint32_t TMEM_O = 256;
+constexpr int ML_BYTES = 2 * STREAMS * BQ * 4;       // every stream's row maxima and sums
+constexpr size_t SMEM = 1024 + Q_BYTES + STREAMS * STAGES * 2 * KV_BYTES + ML_BYTES + 512;
+constexpr uint32_t TMEM_COLS = 512, TMEM_O = STREAMS * BKV;      // scores (then weights: 32 columns hi, 32 lo), then sums
 constexpr float LOG2E = 1.4426950408889634f;
+constexpr float LAZY = 8.f;                          // how far (in powers of two) a score may exceed the maximum in use
 
 __device__ int g_attn_error = 0;                     // first error code seen by this kernel
 
 // Instruction descriptor with the B operand MN-major (bit 16): D=F32, A=B=BF16.
 __host__ __device__ constexpr uint32_t make_idesc_bmn(int m, int n) { return make_idesc(m, n) | (1u << 16); }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-}
 __device__ __forceinline__ float fast_exp2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&v);
-}
+// A stream's barriers: a stage's keys and values have arrived, its MMAs have read both; a block's scores, weights and sums are there.
+struct Stream {
+    uint64_t k_full[STAGES], v_full[STAGES], empty[STAGES], s_full, p_full, o_full;
+};
 
 __global__ void __launch_bounds__(THREADS, 1)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -81,19 +70,12 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* sQ = base;
-    uint8_t* sKV = sQ + Q_BYTES;                                  // [STAGES][K 16 KB | V 16 KB]
-    uint8_t* sP = sKV + STAGES * 2 * KV_BYTES;                    // [2 buffers][hi term | lo term]
-    float* xch = reinterpret_cast<float*>(sP + 2 * 2 * P_BYTES);  // [2][PARTS][BQ]
-    uint64_t* q_full = (uint64_t*)(sP + 2 * 2 * P_BYTES + XCH_BYTES);
-    uint64_t* k_full = q_full + 1;                                // [STAGES]
-    uint64_t* k_empty = k_full + STAGES;                          // [STAGES]: keys are free again once S was computed
-    uint64_t* v_full = k_empty + STAGES;                          // [STAGES]
-    uint64_t* v_empty = v_full + STAGES;                          // [STAGES]: values are free again once P V was computed
-    uint64_t* s_full = v_empty + STAGES;                          // [2]: one per S buffer
-    uint64_t* p_full = s_full + 2;
-    uint64_t* o_full = p_full + 1;
-    uint64_t* o_free = o_full + 1;
-    uint32_t* tmem_slot = (uint32_t*)(o_free + 1);
+    uint8_t* sKV = sQ + Q_BYTES;                                  // [STREAMS][STAGES][K 8 KB | V 8 KB]
+    float* sm_m = reinterpret_cast<float*>(sKV + STREAMS * STAGES * 2 * KV_BYTES);     // [STREAMS][BQ]
+    float* sm_l = sm_m + STREAMS * BQ;
+    Stream* streams = reinterpret_cast<Stream*>(sm_l + STREAMS * BQ);
+    uint64_t* q_full = (uint64_t*)(streams + STREAMS);
+    uint32_t* tmem_slot = (uint32_t*)(q_full + 1);
     volatile int* failed = (volatile int*)(tmem_slot + 1);
 
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
@@ -106,258 +88,221 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     }
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
-        for (int s = 0; s < STAGES; ++s) {
-            mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1);
-            mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1);
+        for (int g = 0; g < STREAMS; ++g) {
+            Stream& st = streams[g];
+            for (int s = 0; s < STAGES; ++s) { mbar_init(&st.k_full[s], 1); mbar_init(&st.v_full[s], 1); mbar_init(&st.empty[s], 1); }
+            mbar_init(&st.s_full, 1);
+            mbar_init(&st.p_full, 4);
+            mbar_init(&st.o_full, 1);
         }
-        mbar_init(&s_full[0], 1);
-        mbar_init(&s_full[1], 1);
-        mbar_init(p_full, SOFTMAX_WARPS);
-        mbar_init(o_full, 1);
-        mbar_init(o_free, SOFTMAX_WARPS);
         *failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
+    if (warp == ISSUE_WARP) tmem_alloc(tmem_slot, TMEM_COLS);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-    pdl_wait();
-    pdl_launch();
-
-    const int seq = tiles[tile * 3], tok0 = tiles[tile * 3 + 1], rows = tiles[tile * 3 + 2];
-    const int pos0 = positions[tok0];
-    const int pos_max = pos0 + rows - 1;
+    const uint32_t tmem = *tmem_slot;
+    // tiles, positions and block tables are written by the host before the step
+    const int seq = __ldcg(tiles + tile * 3), tok0 = __ldcg(tiles + tile * 3 + 1), rows = __ldcg(tiles + tile * 3 + 2);
+    const int pos0 = __ldcg(positions + tok0), pos_max = pos0 + rows - 1;
     const int hk = h / (H / Hkv);
-    int first_key = 0;
-    if (window > 0 && pos0 - window + 1 > 0) first_key = pos0 - window + 1;
-    const int j_lo = first_key / BKV, j_hi = pos_max / BKV;
-    const int nblk = j_hi - j_lo + 1;
+    const int first_key = window > 0 && pos0 - window + 1 > 0 ? pos0 - window + 1 : 0;
+    const int b_lo = first_key / BKV, b_hi = pos_max / BKV;
+    const int g = warp < SOFTMAX_WARPS ? warp >> 2 : (warp - SOFTMAX_WARPS) % STREAMS;       // this warp's stream
+    // blocks of stream x: first_block(x), first_block(x) + 4, ... up to b_hi
+    auto first_block = [&](int x) { return b_lo + ((x - b_lo) & (STREAMS - 1)); };
+    auto blocks_of = [&](int x) { const int b = first_block(x); return b > b_hi ? 0 : (b_hi - b) / STREAMS + 1; };
+    const int steps = blocks_of(g);
+    Stream& st = streams[g];
+    const uint32_t t_s = tmem + (uint32_t)(g * BKV), t_o = tmem + TMEM_O + (uint32_t)(g * DH);
 
-    const int V_WARP = 2 + SOFTMAX_WARPS;
-    if (warp == 0 || warp == V_WARP) {
-        // ---------------------------------------------------------------- producers: warp 0 brings the queries and
-        // the keys, the last warp the values, each as soon as the stage it writes to is free
-        const bool keys = warp == 0;
-        const CUtensorMap* map = keys ? &map_k : &map_v;
-        uint64_t* full = keys ? k_full : v_full;
-        uint64_t* empty = keys ? k_empty : v_empty;
-        const int ppb = BKV / page_size;                          // pages per block
+    if (warp >= LOAD_WARP) {
+        // ---------------------------------------------------------------- the stream's pages; lane p brings page p of a block
+        const int box = page_size < BKV ? page_size : BKV, boxes = BKV / box;
         const int* bt = block_table + (size_t)seq * bt_stride;
-        if (keys && lane == 0) {
+        auto row_of = [&](int b) {                                // the pool row at which this lane's box of block b starts
+            const int k0 = b * BKV + lane * box;
+            if (lane >= boxes || b > b_hi || k0 > pos_max || k0 + box <= first_key) return pool_rows;     // beyond the pool: zeros
+            const int page = __ldcg(bt + k0 / page_size);
+            return page < 0 ? pool_rows : (page * Hkv + hk) * page_size + k0 % page_size;
+        };
+        int b = first_block(g), row = row_of(b);
+        pdl_wait();
+        pdl_launch();
+        if (g == 0 && lane == 0) {
             mbar_expect_tx(q_full, Q_BYTES);
             tma_load_2d(sQ, &map_q, h * DH, tok0, q_full);
         }
-        for (int i = 0; i < nblk; ++i) {
-            const int j = j_lo + i, s = i % STAGES;
-            bool ok = true;
+        for (int i = 0; i < steps; ++i, b += STREAMS) {
+            const int s = i % STAGES;
+            const int next = row_of(b + STREAMS);
+            bool ok = i < STAGES || mbar_wait(&st.empty[s], ((i / STAGES) - 1) & 1);
+            if (!ok) *failed = 1;
+            if (!__all_sync(0xffffffffu, ok && !*failed)) break;
             if (lane == 0) {
-                if (i >= STAGES) ok = mbar_wait(&empty[s], ((i / STAGES) - 1) & 1);
-                if (!ok) *failed = 1;
-                if (ok && !*failed) mbar_expect_tx(&full[s], KV_BYTES);
+                mbar_expect_tx(&st.k_full[s], KV_BYTES);
+                mbar_expect_tx(&st.v_full[s], KV_BYTES);
             }
-            ok = __shfl_sync(0xffffffffu, (int)(ok && !*failed), 0) != 0;
-            if (!ok) break;
-            // lane p brings page p of the block: keys [128 j + p * page_size, + page_size)
-            for (int p = lane; p < ppb; p += 32) {
-                const int k0 = j * BKV + p * page_size;
-                int row = pool_rows;                              // beyond the pool: the box is filled with zeros
-                if (k0 <= pos_max && k0 + page_size > first_key) {
-                    const int page = bt[k0 / page_size];
-                    if (page >= 0) row = (page * Hkv + hk) * page_size;
-                }
-                uint8_t* dst = sKV + (size_t)s * 2 * KV_BYTES + (keys ? 0 : KV_BYTES) + (size_t)p * page_size * (DH * 2);
-                tma_load_2d(dst, map, 0, row, &full[s]);
+            __syncwarp();
+            if (lane < boxes) {
+                uint8_t* dst = sKV + (size_t)(g * STAGES + s) * 2 * KV_BYTES + (size_t)lane * box * (DH * 2);
+                tma_load_2d(dst, &map_k, 0, row, &st.k_full[s]);
+                tma_load_2d(dst + KV_BYTES, &map_v, 0, row, &st.v_full[s]);
             }
+            row = next;
         }
-    } else if (warp == 1) {
-        // ---------------------------------------------------------------- MMA issuer
+    } else if (warp >= ISSUE_WARP) {
+        // ---------------------------------------------------------------- the stream's MMAs
         // (the warp as a whole runs the loop, one elected lane issues: tcgen05.cuh says why)
-        constexpr uint32_t idesc_s = make_idesc(BQ, BKV);
-        constexpr uint32_t idesc_o = make_idesc_bmn(BQ, DH);
-        const uint32_t t_o = tmem_base + TMEM_O;
-        const uint64_t q_desc = make_smem_desc(smem_u32(sQ)), kv_desc = make_smem_desc(smem_u32(sKV)),
-                       p_desc = make_smem_desc(smem_u32(sP));
-        auto all_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); };
-        auto issue_s = [&](int i) {                       // S(i) = Q K(i)^T into the S buffer i & 1
-            const uint64_t k_desc = kv_desc + (uint64_t)((i % STAGES) * (2 * KV_BYTES >> 4));
-#pragma unroll
-            for (int k = 0; k < DH / 16; ++k)
-                umma_f16_warp(tmem_base + (uint32_t)(i & 1) * 128, q_desc + 2 * k, k_desc + 2 * k, idesc_s, k != 0);
-            umma_commit_warp(&s_full[i & 1]);
-            umma_commit_warp(&k_empty[i % STAGES]);       // the keys of this block have been read
-        };
-        bool ok = all_wait(q_full, 0) && all_wait(&k_full[0], 0);
-        if (!ok) *failed = 2;
-        if (ok) {
+        pdl_wait();
+        pdl_launch();
+        constexpr uint32_t idesc_s = make_idesc(BQ, BKV), idesc_o = make_idesc_bmn(BQ, DH);
+        const uint64_t q_desc = make_smem_desc(smem_u32(sQ)),
+                       kv_desc = make_smem_desc(smem_u32(sKV + (size_t)g * STAGES * 2 * KV_BYTES));
+        auto all_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity) && !*failed); };
+        bool ok = steps == 0 || all_wait(q_full, 0);
+        if (!ok && !*failed) *failed = 2;
+        for (int i = 0; i < steps && ok; ++i) {
+            const int s = i % STAGES;
+            const uint64_t k_desc = kv_desc + (uint64_t)(s * (2 * KV_BYTES >> 4)), v_desc = k_desc + (uint64_t)(KV_BYTES >> 4);
+            // the scores' columns are free once the product that read the last block's weights there is complete
+            if (i > 0 && !all_wait(&st.o_full, (i - 1) & 1)) { if (!*failed) *failed = 3; break; }
+            if (!all_wait(&st.k_full[s], (i / STAGES) & 1)) { if (!*failed) *failed = 4; break; }
             tc_fence_after();
-            issue_s(0);
-        }
-        for (int i = 0; i < nblk && ok; ++i) {
-            if (i + 1 < nblk) {
-                // S of the next block goes ahead of this block's P V: its buffer was read two blocks ago
-                if (!all_wait(&k_full[(i + 1) % STAGES], ((i + 1) / STAGES) & 1)) { *failed = 3; break; }
-                tc_fence_after();
-                issue_s(i + 1);
-            }
-            // O_blk = P(i) V(i) (hi term, then lo term) once the weights are written and O_blk of block i-1 was read
-            if (!all_wait(p_full, i & 1)) { *failed = 4; break; }
-            if (i > 0 && !all_wait(o_free, (i - 1) & 1)) { *failed = 5; break; }
-            if (!all_wait(&v_full[i % STAGES], (i / STAGES) & 1)) { *failed = 6; break; }
-            tc_fence_after();
-            const uint64_t v_desc = kv_desc + (uint64_t)(((i % STAGES) * 2 * KV_BYTES + KV_BYTES) >> 4);
-            const uint64_t pi_desc = p_desc + (uint64_t)((i & 1) * (2 * P_BYTES >> 4));
 #pragma unroll
-            for (int term = 0; term < 2; ++term) {
+            for (int k = 0; k < DH / 16; ++k) umma_f16_warp(t_s, q_desc + 2 * k, k_desc + 2 * k, idesc_s, k != 0);
+            umma_commit_warp(&st.s_full);
+            if (!all_wait(&st.v_full[s], (i / STAGES) & 1)) { if (!*failed) *failed = 5; break; }
+            if (!all_wait(&st.p_full, i & 1)) { if (!*failed) *failed = 6; break; }
+            tc_fence_after();
+#pragma unroll
+            for (int term = 0; term < 2; ++term)                  // hi, then lo
 #pragma unroll
                 for (int kk = 0; kk < BKV / 16; ++kk)
-                    umma_f16_warp(t_o, pi_desc + (uint64_t)(((term * P_BYTES + (kk / 4) * (P_BYTES / 2)) >> 4) + 2 * (kk % 4)),
-                                  v_desc + (uint64_t)(kk * (2048 >> 4)), idesc_o, (term | kk) != 0);
-            }
-            umma_commit_warp(o_full);
-            umma_commit_warp(&v_empty[i % STAGES]);       // this block's values have been read
+                    umma_f16_ts_warp(t_o, t_s + (uint32_t)(term * (BKV / 2) + kk * 8), v_desc + (uint64_t)(kk * (2048 >> 4)), idesc_o,
+                                     (i | term | kk) != 0);
+            umma_commit_warp(&st.o_full);
+            umma_commit_warp(&st.empty[s]);
         }
     } else {
+        pdl_wait();
+        pdl_launch();
         // ---------------------------------------------------------------- softmax: one query row per thread
         const int q4 = warp & 3;                              // the quarter of the tensor-memory lanes this warp may read
-        const int part = (warp - 2) >> 2;                     // which 32 keys of a block and which 16 output values
         const int r = q4 * 32 + lane;                         // row of the tile
         const int qp = pos0 + r;                              // its absolute position (rows beyond the tile are not stored)
-        const uint32_t t_lane = tmem_base + ((uint32_t)(q4 * 32) << 16);
-        const uint32_t t_o = t_lane + TMEM_O + part * 16;
+        const uint32_t t_lane = (uint32_t)(q4 * 32) << 16;
         const float sl2 = scale * LOG2E;
-        float o[16];
-#pragma unroll
-        for (int d = 0; d < 16; ++d) o[d] = 0.f;
-        float m_run = -INFINITY, l_part = 0.f, alpha_prev = 1.f;
-        // A warp that gave up on a wait stays in step with the three that share its rows: it skips the work but
-        // still arrives at their barriers, which also carry whether all of them are still running, so nobody waits for a warp that left.
+        float m_run = -INFINITY, l_run = 0.f;
         bool alive = true;
-        uint32_t v[32];
-        auto row_barrier = [&](bool fine) -> bool {          // barrier of the 4 warps of this quarter; true if all are fine
-            uint32_t all;
-            asm volatile(
-                "{\n\t.reg .pred p, q;\n\t"
-                "setp.ne.b32 p, %1, 0;\n\t"
-                "bar.red.and.pred q, %2, %3, p;\n\t"
-                "selp.u32 %0, 1, 0, q;\n\t}"
-                : "=r"(all) : "r"((uint32_t)fine), "r"(1 + q4), "n"(PARTS * 32) : "memory");
-            return all != 0;
-        };
-        // o = o * alpha + O_blk for the block whose P V was issued last
-        auto add_block = [&](int i, float alpha) -> bool {
-            bool fine = mbar_wait(o_full, i & 1);
-            if (!fine) *failed = 8;
-            fine = __all_sync(0xffffffffu, fine && !*failed);
-            if (!fine) return false;
+        for (int i = 0; i < steps; ++i) {
+            const int k0 = (first_block(g) + i * STREAMS) * BKV;
+            bool got = mbar_wait(&st.s_full, i & 1);
+            if (!got) *failed = 7;
+            alive = __all_sync(0xffffffffu, got && !*failed);
+            if (!alive) break;
             tc_fence_after();
-            uint32_t w[16];
-            tmem_ld16(t_o, w);
+            uint32_t v[2][32];
+            tmem_ld32_issue(t_s + t_lane, v[0]);
+            tmem_ld32_issue(t_s + t_lane + 32, v[1]);
             tmem_ld_wait();
+            if (k0 + BKV - 1 > pos0 + q4 * 32 || window > 0) {        // some row of the warp does not see all keys
 #pragma unroll
-            for (int e = 0; e < 16; ++e) o[e] = fmaf(o[e], alpha, __uint_as_float(w[e]));
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(o_free);
-            return true;
-        };
-        for (int i = 0; i < nblk; ++i) {
-            const int j = j_lo + i;
-            if (alive) {
-                bool got = mbar_wait(&s_full[i & 1], (i >> 1) & 1);
-                if (!got) *failed = 7;
-                alive = __all_sync(0xffffffffu, got && !*failed);
+                for (int e = 0; e < 64; ++e)
+                    if (k0 + e > qp || (window > 0 && k0 + e <= qp - window)) v[e >> 5][e & 31] = __float_as_uint(-INFINITY);
             }
-            const int k0 = j * BKV + part * 32;                   // first key of this thread's 32
-            const bool need_mask = (j * BKV + BKV - 1 > pos0) || (window > 0);     // uniform over the CTA
-            float sc[32];
-            float mx = -INFINITY;
-            if (alive) {
-                tc_fence_after();
-                tmem_ld32_issue(t_lane + (uint32_t)(i & 1) * 128 + part * 32, v);
-                tmem_ld_wait();
+            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-                for (int e = 0; e < 32; ++e) {
-                    float sv = __uint_as_float(v[e]);
-                    if (need_mask && (k0 + e > qp || (window > 0 && k0 + e <= qp - window))) sv = -INFINITY;
-                    sc[e] = sv;
-                    mx = fmaxf(mx, sv);
+            for (int e = 0; e < 64; ++e) mx[e & 3] = fmaxf(mx[e & 3], __uint_as_float(v[e >> 5][e & 31]));
+            const float mb = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2;
+            const bool moves = mb > m_run + LAZY;             // (from -inf on: any visible key)
+            if (__any_sync(0xffffffffu, moves)) {
+                // rows that keep their maximum are multiplied by one
+                const float alpha = moves ? fast_exp2(m_run - mb) : 1.f;
+                if (moves) m_run = mb;
+                l_run *= alpha;
+                if (i > 0) {
+#pragma unroll
+                    for (int c = 0; c < DH; c += 16) {
+                        uint32_t w[16];
+                        tmem_ld16_issue(t_o + t_lane + c, w);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) w[e] = __float_as_uint(__uint_as_float(w[e]) * alpha);
+                        tmem_st8(t_o + t_lane + c, make_uint4(w[0], w[1], w[2], w[3]), make_uint4(w[4], w[5], w[6], w[7]));
+                        tmem_st8(t_o + t_lane + c + 8, make_uint4(w[8], w[9], w[10], w[11]), make_uint4(w[12], w[13], w[14], w[15]));
+                    }
                 }
             }
-            // the row's maximum over the block: the four threads of the row meet in shared memory
-            float* xb = xch + (i & 1) * PARTS * BQ;
-            xb[part * BQ + r] = mx;
-            alive = row_barrier(alive);
-            if (!alive) continue;                                 // all four warps of the quarter take this branch together
+            const float muse = m_run == -INFINITY ? 0.f : m_run;
+            float rs[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int p = 0; p < PARTS; ++p) mx = fmaxf(mx, xb[p * BQ + r]);
-            const float m_new = fmaxf(m_run, mx * sl2);
-            const float muse = m_new == -INFINITY ? 0.f : m_new;
-            const float alpha = fast_exp2(m_run - muse);
-            m_run = m_new;
-            // weights -> shared memory as hi + lo, their sum
-            uint8_t* dst_hi = sP + (size_t)(i & 1) * 2 * P_BYTES + (part / 2) * (P_BYTES / 2) + (size_t)r * 128;
-            uint8_t* dst_lo = dst_hi + P_BYTES;
-            float rs = 0.f;
+            for (int c = 0; c < 4; ++c) {                         // 16 keys: 8 columns of each term
+                uint32_t hi[8], lo[8];
 #pragma unroll
-            for (int g8 = 0; g8 < 4; ++g8) {                      // 8 keys = one 16-byte piece
-                uint32_t hi4[4], lo4[4];
-#pragma unroll
-                for (int e2 = 0; e2 < 4; ++e2) {
-                    const int e = g8 * 8 + e2 * 2;
-                    const float p0 = fast_exp2(fmaf(sc[e], sl2, -muse)), p1 = fast_exp2(fmaf(sc[e + 1], sl2, -muse));
-                    rs += p0 + p1;
-                    const uint32_t hh = pack_bf16(p0, p1);
-                    hi4[e2] = hh;
-                    lo4[e2] = pack_bf16(p0 - __uint_as_float(hh << 16), p1 - __uint_as_float(hh & 0xffff0000u));
+                for (int e = 0; e < 8; ++e) {
+                    const int k = c * 16 + 2 * e;
+                    const float p0 = fast_exp2(fmaf(__uint_as_float(v[k >> 5][k & 31]), sl2, -muse)),
+                                p1 = fast_exp2(fmaf(__uint_as_float(v[k >> 5][(k & 31) + 1]), sl2, -muse));
+                    rs[e & 3] += p0 + p1;
+                    hi[e] = bf16x2_rn(p0, p1);
+                    lo[e] = bf16x2_rn(p0 - __uint_as_float(hi[e] << 16), p1 - __uint_as_float(hi[e] & 0xffff0000u));
                 }
-                const int piece = (part & 1) * 4 + g8;            // 16-byte piece of the 128-byte row; swizzled by r & 7 as the MMA expects
-                const int off = ((piece ^ (r & 7)) << 4);
-                *reinterpret_cast<uint4*>(dst_hi + off) = make_uint4(hi4[0], hi4[1], hi4[2], hi4[3]);
-                *reinterpret_cast<uint4*>(dst_lo + off) = make_uint4(lo4[0], lo4[1], lo4[2], lo4[3]);
+                tmem_st8(t_s + t_lane + c * 8, make_uint4(hi[0], hi[1], hi[2], hi[3]), make_uint4(hi[4], hi[5], hi[6], hi[7]));
+                tmem_st8(t_s + t_lane + 32 + c * 8, make_uint4(lo[0], lo[1], lo[2], lo[3]), make_uint4(lo[4], lo[5], lo[6], lo[7]));
             }
-            l_part = l_part * alpha + rs;
-            fence_async_smem();                                   // the weights become visible to the tensor core's reads
+            l_run += (rs[0] + rs[1]) + (rs[2] + rs[3]);
+            tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(p_full);
-            // the block before this one: its P V has had the time of this block's softmax to finish
-            if (i > 0) alive = add_block(i - 1, alpha_prev);
-            alpha_prev = alpha;
+            if (lane == 0) mbar_arrive(&st.p_full);
         }
-        if (alive) alive = add_block(nblk - 1, alpha_prev);
-        // the row's sum: the four partial sums added in a fixed order
-        alive = row_barrier(alive);                               // the last maxima have been read
-        xch[part * BQ + r] = l_part;
-        alive = row_barrier(alive);
-        if (alive && r < rows) {
-            float l = 0.f;
+        if (alive && steps > 0) {
+            bool got = mbar_wait(&st.o_full, (steps - 1) & 1);
+            if (!got) *failed = 8;
+        }
+        // the four streams of a row meet; thread (g, r) writes the columns 16 g ..
+        sm_m[g * BQ + r] = m_run;
+        sm_l[g * BQ + r] = l_run;
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + q4), "n"(STREAMS * 32) : "memory");
+        tc_fence_after();
+        float m = -INFINITY, l = 0.f, o[16];
 #pragma unroll
-            for (int p = 0; p < PARTS; ++p) l += xch[p * BQ + r];
+        for (int x = 0; x < STREAMS; ++x) m = fmaxf(m, sm_m[x * BQ + r]);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) o[e] = 0.f;
+#pragma unroll
+        for (int x = 0; x < STREAMS; ++x) {
+            if (blocks_of(x) == 0) continue;                      // uniform: the stream's columns were never written
+            const float mx = sm_m[x * BQ + r], f = mx == -INFINITY ? 0.f : fast_exp2(mx - m);
+            uint32_t w[16];
+            tmem_ld16_issue(tmem + TMEM_O + t_lane + (uint32_t)(x * DH + g * 16), w);
+            tmem_ld_wait();
+            l = fmaf(f, sm_l[x * BQ + r], l);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) o[e] = fmaf(f, __uint_as_float(w[e]), o[e]);
+        }
+        if (r < rows && !*failed) {
             const float inv = 1.f / l;
-            __nv_bfloat16* orow = out + (size_t)(tok0 + r) * out_stride + (size_t)h * DH + part * 16;
+            __nv_bfloat16* orow = out + (size_t)(tok0 + r) * out_stride + (size_t)h * DH + g * 16;
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                uint4 pk;
-                pk.x = pack_bf16(o[c * 8] * inv, o[c * 8 + 1] * inv);
-                pk.y = pack_bf16(o[c * 8 + 2] * inv, o[c * 8 + 3] * inv);
-                pk.z = pack_bf16(o[c * 8 + 4] * inv, o[c * 8 + 5] * inv);
-                pk.w = pack_bf16(o[c * 8 + 6] * inv, o[c * 8 + 7] * inv);
-                *reinterpret_cast<uint4*>(orow + c * 8) = pk;
-            }
+            for (int c = 0; c < 2; ++c)
+                *reinterpret_cast<uint4*>(orow + c * 8) =
+                    make_uint4(bf16x2_rn(o[c * 8] * inv, o[c * 8 + 1] * inv), bf16x2_rn(o[c * 8 + 2] * inv, o[c * 8 + 3] * inv),
+                               bf16x2_rn(o[c * 8 + 4] * inv, o[c * 8 + 5] * inv), bf16x2_rn(o[c * 8 + 6] * inv, o[c * 8 + 7] * inv));
         }
     }
     tc_fence_before();
     __syncthreads();
     if (*failed) {
         if (threadIdx.x == 0) { atomicCAS(&g_attn_error, 0, *failed); report_to_host(200 + *failed); }
-        for (int i = 0; i < 2000; ++i) __nanosleep(100);          // copies already issued may still be landing
+        for (int i = 0; i < 2000; ++i) __nanosleep(100);          // copies and MMAs already issued may still be running
         __syncthreads();
     }
-    if (warp == 1) {
+    if (warp == ISSUE_WARP) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, TMEM_COLS);
+        tmem_dealloc(tmem, TMEM_COLS);
     }
 }
 
@@ -387,7 +332,7 @@ MLLM_EXPORT int mllm_attention_tcgen05(const void* q, long long q_stride, int T,
     if (n_tiles <= 0) return 0;
     if (dh != DH) return mllm_fail(1, "attention_tcgen05: head size %d is not 64", dh);
     if (Hkv <= 0 || H % Hkv != 0) return mllm_fail(1, "attention_tcgen05: %d heads over %d key/value heads", H, Hkv);
-    if (page_size < 8 || page_size > BKV || (page_size & (page_size - 1)))
+    if (page_size < 8 || page_size > 128 || (page_size & (page_size - 1)))
         return mllm_fail(1, "attention_tcgen05: page size %d is not a power of two in 8..128", page_size);
     if (n_tiles > 65535) return mllm_fail(1, "attention_tcgen05: %d query tiles are more than one launch takes", n_tiles);
     if (!(scale > 0.f)) return mllm_fail(1, "attention_tcgen05: the score scale must be positive, got %g", (double)scale);
@@ -400,9 +345,10 @@ MLLM_EXPORT int mllm_attention_tcgen05(const void* q, long long q_stride, int T,
     CUtensorMap mq, mk, mv;
     int rc = get_map(q, q_stride, T, H * DH, DH, BQ, MAP_BF16_SW128, &mq);
     if (rc) return rc;
-    rc = get_map(k_pages, DH, (int)pool_rows, DH, DH, page_size, MAP_BF16_SW128, &mk);
+    const int box = page_size < BKV ? page_size : BKV;
+    rc = get_map(k_pages, DH, (int)pool_rows, DH, DH, box, MAP_BF16_SW128, &mk);
     if (rc) return rc;
-    rc = get_map(v_pages, DH, (int)pool_rows, DH, DH, page_size, MAP_BF16_SW128, &mv);
+    rc = get_map(v_pages, DH, (int)pool_rows, DH, DH, box, MAP_BF16_SW128, &mv);
     if (rc) return rc;
     auto kern = attention_tcgen05_kernel;
     static bool set = false;
