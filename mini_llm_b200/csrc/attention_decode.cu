@@ -134,14 +134,15 @@ attn_decode_body(const T* q, long long q_stride, const T* k_pages, const T* v_pa
     constexpr bool STAGE = STG;
     static_assert(!STG || Staged<T, LPK>::value, "a split's rows do not fit the staging area");
     static_assert(!TWO || (STG && NG * UNR * 2 == SPLIT), "two rounds of staging need groups that take a split in two rounds");
+    constexpr bool APART = !ONE || TWO;                       // several stages: keys and values arrive and are replaced on their own
     constexpr int STAGE_KEYS = TWO ? SPLIT / 2 : SPLIT;       // keys that the staging area holds
     __shared__ float sm_m[NG], sm_l[NG], sm_w[NG];
     extern __shared__ __align__(16) uint4 s_stage[];          // STAGE: a split's keys, then its values: [key][16-byte piece]
     __shared__ float sm_o_own[STAGE ? 1 : NG * DH];
-    float* sm_o = STAGE ? reinterpret_cast<float*>(s_stage) : sm_o_own;   // staged: the groups' outputs reuse the keys' space
+    float* sm_o = STAGE ? reinterpret_cast<float*>(s_stage + (APART ? STAGE_KEYS * LPK : 0)) : sm_o_own;    // staged: the groups' outputs reuse the values' space
     __shared__ float sm_res[(PUSH ? MAX_CLUSTER : MODE == MODE_SCRATCH || ONE ? 1 : MAX_SPC) * RES];
     __shared__ int s_last;
-    __shared__ __align__(8) uint64_t s_bar;                   // STAGE: a split's bulk copies complete here
+    __shared__ __align__(8) uint64_t s_bar[2];                // STAGE: the bulk copies of keys and of values complete here
     const int cx = blockIdx.x, h = blockIdx.y, t = blockIdx.z;
     // Positions, the request index and the block table are written by the host before the step, and the rows of
     // all keys before the token's own position were written by earlier steps: all of that is read before the
@@ -192,7 +193,8 @@ attn_decode_body(const T* q, long long q_stride, const T* k_pages, const T* v_pa
     uint32_t phase = 0;
     if constexpr (STAGE) {
         if (threadIdx.x == 0) {
-            tc::mbar_init(&s_bar, 1);
+            tc::mbar_init(&s_bar[0], 1);
+            if constexpr (APART) tc::mbar_init(&s_bar[1], 1);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         __syncthreads();
@@ -230,56 +232,66 @@ attn_decode_body(const T* q, long long q_stride, const T* k_pages, const T* v_pa
     // (39.5 against 36.5 us in float32, 22.7 against 22.0 us in bfloat16 at batch 64).
     if constexpr (!ONE && !STAGE) ask_for((my_lo + 1) * SPLIT, (my_lo + 2) * SPLIT);
 
+    // Staging.  A stage is the rows of up to STAGE_KEYS keys; keys and values have a place and a barrier each, so the next
+    // stage's keys are asked for as soon as this one's scores are taken, its values once this one's are summed: the copies fly
+    // while the CTA computes (24 x 25 heads at 1,023 keys: bfloat16 32.5 us a launch, 35.0 with one barrier for both; float32 53.5
+    // and 58.2; 8 x 12 at 768, float32 9.0 and 10.3).  A CTA with one stage (!APART) waits for both at once: apart they cost a decode
+    // step of one request 0.8 us a layer.  `arrange` says how much is coming, `bring` asks for the rows [a, b) of the stage that starts at lo,
+    // thread c for those of the c-th page that the range touches.  Rows of earlier steps go out before the wait on the
+    // previous kernel, the token's own row (position p) after it.  Rows that are not visible are not copied: their places
+    // hold whatever was there, and the arithmetic below skips them.
+    uint4* sk = s_stage;
+    uint4* sv = s_stage + STAGE_KEYS * LPK;
+    constexpr uint32_t ROW = DH * (uint32_t)sizeof(T);
+    auto stage_end = [&](int lo) { return min(lo + STAGE_KEYS, p + 1); };
+    auto arrange = [&](int which, int lo) {
+        if (threadIdx.x == 0) tc::mbar_expect_tx(&s_bar[which], (uint32_t)max(0, stage_end(lo) - max(lo, first)) * (APART ? ROW : 2 * ROW));
+    };
+    auto bring = [&](bool keys, bool values, int lo, int a, int b) {
+        if (b <= a) return;
+        const int pg0 = page_index(a), pg1 = page_index(b - 1);
+        for (int pg = pg0 + (int)threadIdx.x; pg <= pg1; pg += THREADS) {
+            const int r0 = max(a, pg * page_size), r1 = min(b, (pg + 1) * page_size);
+            const size_t off = (((size_t)__ldcg(bt + pg) * Hkv + hk) * page_size + (r0 - pg * page_size)) * DH;
+            const uint32_t bytes = (uint32_t)(r1 - r0) * ROW;
+            if (keys) tc::bulk_load(sk + (r0 - lo) * LPK, k_pages + off, bytes, &s_bar[0]);
+            if (values) tc::bulk_load(sv + (r0 - lo) * LPK, v_pages + off, bytes, &s_bar[APART]);
+        }
+    };
+    auto next_stage = [&](int which, int lo) {                // its place has been read: the copies may overwrite it
+        arrange(which, lo);
+        bring(which == 0, which == 1, lo, max(lo, first), stage_end(lo));
+    };
+    auto arrived = [&](int which) {
+        if (!tc::mbar_wait(&s_bar[which], phase)) {           // gave up: tell the host, let copies in flight land, go on
+            if (threadIdx.x == 0) { atomicCAS(&g_decode_error, 0, 1); tc::report_to_host(301); }
+            for (int i = 0; i < 2000; ++i) __nanosleep(100);
+        }
+    };
+    if constexpr (STAGE) {
+        const int lo = my_lo * SPLIT, hi = stage_end(lo), v_lo = max(lo, first);
+        arrange(0, lo);
+        if constexpr (APART) arrange(1, lo);
+        bring(true, true, lo, v_lo, min(hi, p));
+        wait_and_load_q();
+        if (p >= v_lo && p < hi) bring(true, true, lo, p, p + 1);
+    }
+
 #pragma unroll 1
-    for (int split = my_lo; split <= my_hi; ++split) {
+    for (int split = my_lo; split <= (ONE ? my_lo : my_hi); ++split) {
         const int k_lo = split * SPLIT, k_hi = min(k_lo + SPLIT, p + 1);
         float m = -INFINITY, l = 0.f, o[VEC];
 #pragma unroll
         for (int i = 0; i < VEC; ++i) o[i] = 0.f;
-        uint4* sk = s_stage;
-        uint4* sv = s_stage + STAGE_KEYS * LPK;
-        // Brings the visible rows of [lo, hi) into the staging area (row r to place r - lo), page by page: thread c
-        // brings the rows of the c-th page that the range touches.  Rows of earlier steps go out before the wait on
-        // the previous kernel, the token's own row (position p) after it.  Rows that are not visible are not
-        // copied: their places hold whatever was there, and the arithmetic below skips them.
-        auto stage = [&](int lo, int hi) {
-            constexpr uint32_t ROW = DH * (uint32_t)sizeof(T);
-            const int v_lo = max(lo, first);
-            const int pre_hi = min(hi, p);
-            if (threadIdx.x == 0) tc::mbar_expect_tx(&s_bar, (uint32_t)max(0, hi - v_lo) * ROW * 2);
-            if (pre_hi > v_lo) {
-                const int pg0 = page_index(v_lo), pg1 = page_index(pre_hi - 1);
-                for (int pg = pg0 + (int)threadIdx.x; pg <= pg1; pg += THREADS) {
-                    const int r0 = max(v_lo, pg * page_size), r1 = min(pre_hi, (pg + 1) * page_size);
-                    const size_t off = (((size_t)__ldcg(bt + pg) * Hkv + hk) * page_size + (r0 - pg * page_size)) * DH;
-                    const uint32_t bytes = (uint32_t)(r1 - r0) * ROW;
-                    tc::bulk_load(sk + (r0 - lo) * LPK, k_pages + off, bytes, &s_bar);
-                    tc::bulk_load(sv + (r0 - lo) * LPK, v_pages + off, bytes, &s_bar);
-                }
-            }
-            if (!waited) wait_and_load_q();
-            if (threadIdx.x == 0 && p >= v_lo && p < hi) {
-                const size_t off = (((size_t)__ldcg(bt + page_index(p)) * Hkv + hk) * page_size + page_offset(p)) * DH;
-                tc::bulk_load(sk + (p - lo) * LPK, k_pages + off, ROW, &s_bar);
-                tc::bulk_load(sv + (p - lo) * LPK, v_pages + off, ROW, &s_bar);
-            }
-            if (!tc::mbar_wait(&s_bar, phase)) {              // gave up: tell the host, let copies in flight land, go on
-                if (threadIdx.x == 0) { atomicCAS(&g_decode_error, 0, 1); tc::report_to_host(301); }
-                for (int i = 0; i < 2000; ++i) __nanosleep(100);
-            }
-            phase ^= 1;
-        };
-        if constexpr (STAGE && !TWO) stage(k_lo, k_hi);
         if constexpr (!ONE && !STAGE) ask_for((split + 2) * SPLIT, (split + 3) * SPLIT);
 #pragma unroll 1
         for (int kb = k_lo + gi; kb < k_lo + SPLIT; kb += NG * UNR) {   // same trip count for every lane
             const int s_base = TWO ? kb - gi : k_lo;          // the key whose row lies first in the staging area
-            if constexpr (TWO) {
-                if (s_base > k_lo) {                          // second round: every group has left the first half
-                    tc::fence_async_smem();
-                    __syncthreads();
-                }
-                stage(s_base, min(s_base + STAGE_KEYS, k_hi));
+            // does this round begin a stage, end it, and does another one follow
+            const bool opens = TWO || kb - gi == k_lo, closes = TWO || kb - gi + NG * UNR >= k_lo + SPLIT;
+            const bool half_way = TWO && kb - gi == k_lo, more = half_way || (!ONE && split < my_hi);
+            if constexpr (STAGE) {
+                if (opens) arrived(0);
             }
             bool ok[UNR];
 #pragma unroll
@@ -334,6 +346,14 @@ attn_decode_body(const T* q, long long q_stride, const T* k_pages, const T* v_pa
                 s[u] = ok[u] ? d : -INFINITY;
                 mx = fmaxf(mx, s[u]);
             }
+            if constexpr (STAGE) {
+                if constexpr (APART) if (closes && more) {      // (uniform) every group has its scores
+                    tc::fence_async_smem();
+                    __syncthreads();
+                    next_stage(0, s_base + STAGE_KEYS);
+                }
+                if constexpr (APART) if (opens) arrived(1);
+            }
             if (mx != -INFINITY) {                               // uniform within the group; no shuffles inside
                 const float alpha = Exp<T>::of(m - mx);
                 l *= alpha;
@@ -352,9 +372,17 @@ attn_decode_body(const T* q, long long q_stride, const T* k_pages, const T* v_pa
                 }
                 m = mx;
             }
+            if constexpr (STAGE) {
+                if constexpr (TWO) if (half_way) {            // the values of the split's second half
+                    tc::fence_async_smem();
+                    __syncthreads();
+                    next_stage(1, s_base + STAGE_KEYS);
+                }
+                if (closes) phase ^= 1;
+            }
         }
         // the groups of the CTA are merged in group order
-        if constexpr (STAGE) __syncthreads();                 // every group has read its keys: their space takes the outputs
+        if constexpr (STAGE) __syncthreads();                 // every group has read its values: their space takes the outputs
         if (li == 0) { sm_m[gi] = m; sm_l[gi] = l; }
 #pragma unroll
         for (int i = 0; i < VEC; ++i) sm_o[gi * DH + li * VEC + i] = o[i];
@@ -385,9 +413,10 @@ attn_decode_body(const T* q, long long q_stride, const T* k_pages, const T* v_pa
             if (MODE == MODE_SCRATCH) { part_ml[slot * 2] = M; part_ml[slot * 2 + 1] = L; }
             else { res[DH] = M; res[DH + 1] = L; }
         }
-        if (split < my_hi) {
+        if (!ONE && split < my_hi) {
             if constexpr (STAGE) tc::fence_async_smem();      // the next split's copies overwrite what was written here
             __syncthreads();                                  // the group buffers are free for the next split
+            if constexpr (STAGE && !ONE) next_stage(1, (split + 1) * SPLIT);
         }
     }
     if (single) return;
@@ -518,14 +547,23 @@ int launch(const void* q, long long q_stride, const void* k_pages, const void* v
            float* part_o, float* part_ml, unsigned int* counters, int T_tokens, int H, int Hkv, int page_size,
            float scale, int window, int max_splits, bool scratch_path, bool beside, cudaStream_t stream) {
     // CTAs per (token, head): few requests get one CTA per split, so that the chain position -> block table ->
-    // rows is as short as it can be; many requests let a CTA walk several splits, which keeps the number of
-    // CTAs near four per SM-slot instead of growing with the batch.  Which keys are added together, and in
-    // which order, is the same either way.
+    // rows is as short as it can be; many requests let a CTA walk several splits.  With staging as many as run at once, six per
+    // SM (us a launch so / with one split per CTA up to 24 CTAs per SM, four per SM beyond; heads of 64, contexts not in L2):
+    //   bfloat16  64 x 12 heads at 250 keys 10.8 / 15.1; 16 x 25 at 300 to 1,023 20.4 / 26.2; 8 x 25 at 900 14.3 / 16.1; 32 x 12 at
+    //             700 17.5 / 20.0; 48 x 12 at 160 to 600 19.5 / 22.4; 32 x 16 at 1,000 34.0 / 37.7; as before from 600 pairs on
+    //   float32   64 x 12 at 250 17.9 / 21.8; 16 x 25 32.9 / 38.2; 32 x 12 28.1 / 30.5; 32 x 16 55.9 / 62.0; 4 or 8 x 12 unchanged
+    // Which keys are added together, and in which order, is the same either way.
     const long long pairs = (long long)T_tokens * H;
-    long long want = (4LL * decode_sm_count() + pairs - 1) / pairs;
-    int ctas = (int)(want < 1 ? 1 : (want > max_splits ? max_splits : want));
-    // measured: one split per CTA stays ahead until the grid reaches about 24 CTAs per SM
-    if (max_splits <= MAX_CLUSTER && pairs * max_splits <= 24LL * decode_sm_count()) ctas = max_splits;
+    const bool stg = Staged<T, LPK>::value && ((uintptr_t)k_pages | (uintptr_t)v_pages) % 16 == 0;
+    int ctas;
+    if (stg) {
+        const long long want = 6LL * decode_sm_count() / pairs;
+        ctas = (int)(want < 1 ? 1 : (want > max_splits ? max_splits : want));
+    } else {
+        const long long want = (4LL * decode_sm_count() + pairs - 1) / pairs;
+        ctas = (int)(want < 1 ? 1 : (want > max_splits ? max_splits : want));
+        if (max_splits <= MAX_CLUSTER && pairs * max_splits <= 24LL * decode_sm_count()) ctas = max_splits;
+    }
     int spc = (max_splits + ctas - 1) / ctas;
     if (spc > MAX_SPC) spc = MAX_SPC;
     ctas = (max_splits + spc - 1) / spc;
@@ -535,9 +573,7 @@ int launch(const void* q, long long q_stride, const void* k_pages, const void* v
     using K = void (*)(const T*, long long, const T*, const T*, const int*, int, const int*, const int*, T*, long long,
                        float*, float*, unsigned int*, int, int, int, float, int, int, int, int);
     constexpr bool CAN_STAGE = Staged<T, LPK>::value;
-    // staged whenever the rows fit (measured: never slower, from two requests on faster); bulk copies want
-    // 16-byte aligned pools
-    const bool stg = CAN_STAGE && ((uintptr_t)k_pages | (uintptr_t)v_pages) % 16 == 0;
+    // staged whenever the rows fit (measured: never slower, from two requests on faster); bulk copies want 16-byte aligned pools
     const int mode = scratch_path ? MODE_SCRATCH : ctas == 1 ? MODE_LOCAL : ctas <= MAX_CLUSTER ? MODE_CLUSTER : MODE_SCRATCH;
     const bool one = spc == 1 && mode != MODE_LOCAL;
     K kern;
