@@ -801,6 +801,12 @@ int sm_count();
 // 8 rows, 72 against 92 us at 64); where they do not (1024 x 4096: slices of 1024 are a chunk and a third) it loses
 // up to 16 rows (7.8 against 7.2 us) and wins beyond (27 against 32 us at 64).
 constexpr int REGS_KC = 768;
+// Rows up to which it is taken; beyond, the product on tensor cores is ahead (csrc/linear_batch_f32.cu has the figures: 768 x 3072
+// 13.2 against 13.1 us at 40 rows, 15.0 against 13.1 at 48).
+constexpr int REGS_M = 40;
+// Rows of W from which on products of more than 16 rows go there: with shorter ones it is level or behind (768 x 512: 6.4 against
+// 7.0 us at 32 rows, 8.4 against 8.3 at 64; 256 x 128 3.8 and 5.0 against 7.0 and 9.5).
+constexpr int BATCH_K = 768;
 int regs_slices(int N, int K, int M) {
     if (K <= 2048 || K % 4 != 0) return 0;
     const int tiles = (N + 31) / 32, sms = sm_count();
@@ -890,14 +896,21 @@ MLLM_EXPORT int mllm_linear_stream_f32_many_shape(int N, int K, int* rt, int* sl
 // Rows of x up to which a matrix [N, K] goes to the kernel with the weights in registers (0: never).
 MLLM_EXPORT int mllm_linear_stream_f32_tall_rows(int N, int K) { return tall_rows_for(N, K); }
 
-// Which kernel of this file computes M plain rows (no norm, no cache write) against a matrix [N, K]: 0 threads split K
-// (up to 16 rows), 1 warps own tokens (17 to 64 rows), 2 weights in registers, 3 long rows in cluster slices.  Rows
-// computed by the same kernel have the same bits whatever the batch.
+// Which kernel computes M plain rows (no norm, no cache write) against a matrix [N, K]: 0 threads split K (up to 16 rows),
+// 1 the kernel of many rows (17 to 64: on tensor cores from K = 768 on, else warps own tokens), 2 weights in registers (as tall
+// as a vocabulary from K = 768 on: on tensor cores), 3 long rows in cluster slices (up to 40 rows).  Rows computed by the same
+// kernel have the same bits whatever the batch.
 MLLM_EXPORT int mllm_linear_stream_f32_kernel_of(int M, int N, int K) {
     if (M <= tall_rows_for(N, K)) return 2;
-    if (regs_slices(N, K, M)) return 3;
+    if (M <= REGS_M && regs_slices(N, K, M)) return 3;
     return M <= FEW_M ? 0 : 1;
 }
+
+// csrc/linear_batch_f32.cu: the same products in exact pieces on tensor cores.
+MLLM_EXPORT int mllm_linear_batch_f32(const float* A, long long lda, const float* W, const float* bias, float* out,
+                                      long long ldo, int M, int N, int K, int act, int accumulate, float* k_pages,
+                                      float* v_pages, const int* slots, int q_size, int kv_heads, int head_dim, int page_size,
+                                      cudaStream_t stream);
 
 MLLM_EXPORT int mllm_linear_stream_f32_bind_error(int* word) { return tc::bind_host_error(word); }
 
@@ -934,6 +947,13 @@ MLLM_EXPORT int mllm_linear_stream_f32(const void* x, long long ldx, const void*
     KvArgs kv = {(float*)k_pages, (float*)v_pages, slots, q_size, kv_heads, head_dim, page_size};
     const int tiles = (N + R - 1) / R;
     const int tall_rw = M <= tall_rows_for(N, K) ? tall_shape(N, K) : 0;
+    const int regs_s = !norm && !kvw && M <= REGS_M ? regs_slices(N, K, M) : 0;
+    const bool vocabulary = tall_rw && (N + 31) / 32 >= 8 * sm_count();
+    // A vocabulary's rows have the same bits at every count of them, so without a norm to fuse it takes the tensor cores from one
+    // row on, although up to 8 rows the weights in registers would be ahead (34 against 45 us at 8 rows of 768, 52 against 44 at 16).
+    if (!norm && K >= BATCH_K && (vocabulary ? !kvw : M > FEW_M && !tall_rw && !regs_s))
+        return mllm_linear_batch_f32((const float*)x, ldx, (const float*)W, bias, (float*)out, ldo, M, N, K, act, accumulate, kv.k_pages,
+                                     kv.v_pages, slots, q_size, kv_heads, head_dim, page_size, stream);
     if (tall_rw) {
         // weights from HBM into registers, x in shared memory once per CTA, CTAs that stay and walk the tiles
         const size_t smem = (size_t)((M + 7) / 8 * 8) * ((K + 127) / 128 * 128) * 4;
@@ -957,8 +977,7 @@ MLLM_EXPORT int mllm_linear_stream_f32(const void* x, long long ldx, const void*
                               (const float*)W, bias, (float*)out, ldo, M, N, K, act, accumulate, ln, kv));
         return 0;
     }
-    const int regs_s = regs_slices(N, K, M);
-    if (regs_s && !norm && !kvw) {
+    if (regs_s) {
         // long rows: K slices in a cluster, chunks in registers
         const int S = regs_s;
         const int Ls = ((K + S - 1) / S + 127) / 128 * 128;
@@ -1038,7 +1057,7 @@ MLLM_EXPORT int mllm_linear_stream_f32(const void* x, long long ldx, const void*
                                      S, T, act, accumulate, ln, kv));
         return 0;
     }
-    // 17 to 64 rows: tile height and K slices from (N, K) alone, so that the CTAs fill the SMs once as fully as possible
+    // 17 to 64 rows that are short: tile height and K slices from (N, K) alone, so that the CTAs fill the SMs once as fully as possible
     int RT = 32, S = 1;
     if (mllm_linear_stream_f32_many_shape(N, K, &RT, &S))
         return mllm_fail(1, "linear_stream_f32: K=%d is too long for shared memory", K);

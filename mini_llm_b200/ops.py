@@ -73,6 +73,10 @@ def _signatures(lib):
                                     c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
         "mllm_linear_cluster_bind_error": [c_void_p],
         "mllm_linear_cluster_error": [c_void_p],
+        "mllm_linear_batch_f32": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int, c_void_p,
+                                  c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
+        "mllm_linear_batch_f32_bind_error": [c_void_p],
+        "mllm_linear_batch_f32_error": [c_void_p],
         "mllm_linear_split_f32": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int,
                                   c_void_p, c_ll, c_void_p],
         "mllm_linear_split_f32_slices": [c_int, c_int],
@@ -235,7 +239,7 @@ def _bind_error_word(lib) -> None:
     word = torch.zeros(1, dtype=torch.int32).pin_memory()
     for name in ("mllm_tcgen05_bind_error", "mllm_attention_tcgen05_bind_error", "mllm_attention_decode_bind_error",
                  "mllm_linear_stream_f32_bind_error", "mllm_linear_split_f32_bind_error",
-                 "mllm_linear_cluster_bind_error", "mllm_attention_split_f32_bind_error"):
+                 "mllm_linear_cluster_bind_error", "mllm_attention_split_f32_bind_error", "mllm_linear_batch_f32_bind_error"):
         if getattr(lib, name)(word.data_ptr()) != 0:
             raise KernelError(lib.mllm_last_error().decode(errors="replace"))
     _error_word = word
@@ -243,7 +247,8 @@ def _bind_error_word(lib) -> None:
 
 _WHO = {1: "the tcgen05 product", 2: "the tcgen05 attention", 3: "the decode attention",
         4: "the float32 weight-streaming product", 5: "the float32 product of many rows",
-        6: "the product of a decode batch", 7: "the float32 prefill attention"}
+        6: "the product of a decode batch", 7: "the float32 prefill attention",
+        8: "the float32 product of a decode batch"}
 
 
 def raise_if_kernel_gave_up() -> None:
@@ -357,6 +362,11 @@ def check_device_errors() -> None:
     if code.value:
         raise KernelError(f"the float32 prefill attention gave up waiting: code {code.value} "
                           "(1 the cutting warps, 2-5 the MMA issuer, 7-8 the softmax warps)")
+    if lib.mllm_linear_batch_f32_error(ctypes.byref(code)) != 0:
+        raise KernelError(lib.mllm_last_error().decode(errors="replace"))
+    if code.value:
+        raise KernelError(f"the float32 product of a decode batch gave up waiting: code {code.value} "
+                          "(1, 5-6 the cutting warps, 2-3 the MMA issuer, 4 the draining warps, 7 the TMA producer)")
 
 
 class _Scope(threading.local):
