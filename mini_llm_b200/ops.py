@@ -187,6 +187,10 @@ def _signatures(lib):
                             c_void_p, c_ll, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_float, c_int, c_int, c_void_p],
         "mllm_moe_route": [c_void_p, c_ll, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
                            c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p],
+        "mllm_moe_split_f32": [c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
+                               c_int, c_int, c_float, c_float, c_void_p, c_void_p],
+        "mllm_moe_split_f32_bind_error": [c_void_p],
+        "mllm_moe_split_f32_error": [c_void_p],
         "mllm_moe_grouped": [c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                              c_int, c_int, c_int, c_float, c_float, c_void_p, c_ll, c_int, c_int, c_int, c_void_p],
         "mllm_retention_step_ok": [c_int, c_int],
@@ -239,7 +243,8 @@ def _bind_error_word(lib) -> None:
     word = torch.zeros(1, dtype=torch.int32).pin_memory()
     for name in ("mllm_tcgen05_bind_error", "mllm_attention_tcgen05_bind_error", "mllm_attention_decode_bind_error",
                  "mllm_linear_stream_f32_bind_error", "mllm_linear_split_f32_bind_error",
-                 "mllm_linear_cluster_bind_error", "mllm_attention_split_f32_bind_error", "mllm_linear_batch_f32_bind_error"):
+                 "mllm_linear_cluster_bind_error", "mllm_attention_split_f32_bind_error", "mllm_linear_batch_f32_bind_error",
+                 "mllm_moe_split_f32_bind_error"):
         if getattr(lib, name)(word.data_ptr()) != 0:
             raise KernelError(lib.mllm_last_error().decode(errors="replace"))
     _error_word = word
@@ -248,7 +253,7 @@ def _bind_error_word(lib) -> None:
 _WHO = {1: "the tcgen05 product", 2: "the tcgen05 attention", 3: "the decode attention",
         4: "the float32 weight-streaming product", 5: "the float32 product of many rows",
         6: "the product of a decode batch", 7: "the float32 prefill attention",
-        8: "the float32 product of a decode batch"}
+        8: "the float32 product of a decode batch", 9: "the float32 product of routed experts"}
 
 
 def raise_if_kernel_gave_up() -> None:
@@ -367,6 +372,11 @@ def check_device_errors() -> None:
     if code.value:
         raise KernelError(f"the float32 product of a decode batch gave up waiting: code {code.value} "
                           "(1, 5-6 the cutting warps, 2-3 the MMA issuer, 4 the draining warps, 7 the TMA producer)")
+    if lib.mllm_moe_split_f32_error(ctypes.byref(code)) != 0:
+        raise KernelError(lib.mllm_last_error().decode(errors="replace"))
+    if code.value:
+        raise KernelError(f"the float32 product of routed experts gave up waiting: code {code.value} "
+                          "(1, 5 the cutting warps, 2-3 the MMA issuer, 4 the epilogue, 6 the TMA producer)")
 
 
 class _Scope(threading.local):
@@ -2024,6 +2034,11 @@ def moe_route(h, router, idx, weights, offsets, order, *, top: int, groups: int 
         launches += 1       # the ordering is a launch of its own
 
 
+MOE_SPLIT_PAIRS = 33            # pairs from which 32-bit experts take the tensor cores (up to 32 every pair streams its weights):
+                                # csrc/moe_split_f32.cu has the figures, from 34 pairs on it is 2.4 to 5.5 times faster
+use_moe_split_f32 = True        # False: 32-bit experts stay on CUDA cores (for comparisons)
+
+
 def moe_grouped(a, weight, out, offsets, order, *, top: int, first: bool, act: str = "silu", limit: float = 0.0,
                 alpha: float = 1.0, identity: int = 0, self_rows=None) -> None:
     """The experts' products over the pairs in ``order``.  ``first``: a [T, K] (row = pair // top), weight [E, 2F, K]
@@ -2052,6 +2067,17 @@ def moe_grouped(a, weight, out, offsets, order, *, top: int, first: bool, act: s
         raise KernelError(f"moe_grouped: activation {act!r} (limit {limit})")
     if (first and out.dtype != a.dtype) or (not first and out.dtype != torch.float32):
         raise KernelError("moe_grouped: the first product keeps the dtype, the second gives 32-bit")
+    if (use_moe_split_f32 and a.dtype == torch.float32 and not identity and n_pairs >= MOE_SPLIT_PAIRS and K % 4 == 0 and K >= 128
+            and _rows("a", a) % 4 == 0 and (a.data_ptr() | weight.data_ptr()) % 16 == 0 and (first or a.stride(0) == K)):
+        # many pairs in 32-bit: tensor cores, in exact pieces
+        global launches
+        rows = _scratch("moe_split_rows", a.device, n_pairs * K) if first else None
+        _call("mllm_moe_split_f32", a.data_ptr(), _rows("a", a), weight.data_ptr(), out.data_ptr(), _rows("out", out),
+              offsets.data_ptr(), order.data_ptr(), n_pairs, E, N, K, int(top) if first else 0, 0 if first else 1,
+              (2 if ungated else 0) if first else 1, _UNGATED_ACT[act] if ungated else _GATE_ACT[act], float(limit), float(alpha),
+              rows.data_ptr() if first else None, _stream())
+        launches += int(first)      # the kernel that gathers the tokens' rows
+        return
     _call("mllm_moe_grouped", a.data_ptr(), _rows("a", a), weight.data_ptr(), out.data_ptr(), _rows("out", out),
           offsets.data_ptr(), order.data_ptr(), n_pairs, E, N, K, int(top) if first else 0, 0 if first else 1,
           (2 if ungated else 0) if first else 1, _UNGATED_ACT[act] if ungated else _GATE_ACT[act], float(limit), float(alpha),

@@ -1,0 +1,59 @@
+"""The float32 products of routed experts over many pairs on tensor cores (csrc/moe_split_f32.cu)."""
+import pytest
+import torch
+
+from test_kernels_gpu import DEV, ops, rnd  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+# pairs per expert: full and ragged tiles, an empty expert, one that has them all; columns that end inside a tile, K inside a block
+@pytest.mark.parametrize("counts", [[64], [128, 0, 1, 129, 70], [7] * 40, [0, 300]])
+@pytest.mark.parametrize("F,D,top,act", [(512, 768, 2, "silu"), (33, 132, 1, "swiglu_clamp"), (100, 260, 2, "relu_sq")])
+def test_routed_experts_in_float32(ops, counts, F, D, top, act):  # noqa: F811
+    E, pairs = len(counts), sum(counts)
+    pairs -= pairs % top
+    counts = list(counts)
+    counts[counts.index(max(counts))] -= sum(counts) - pairs
+    order = torch.randperm(pairs, generator=torch.Generator().manual_seed(1)).to(torch.int32).to(DEV)
+    offsets = torch.tensor([sum(counts[:e]) for e in range(E + 1)], dtype=torch.int32, device=DEV)
+    gated = act != "relu_sq"
+    h = rnd(pairs // top, D, seed=2)
+    w1, w2 = rnd(E, F * (2 if gated else 1), D, seed=3, scale=D ** -0.5), rnd(E, D, F, seed=4, scale=F ** -0.5)
+    mid, out = torch.full((pairs, F), 7.0, device=DEV), torch.full((pairs, D), 7.0, device=DEV)
+    limit = 3.0 if act == "swiglu_clamp" else 0.0
+
+    def run(split):
+        ops.use_moe_split_f32 = split
+        try:
+            ops.moe_grouped(h, w1, mid, offsets, order, top=top, first=True, act=act, limit=limit, alpha=1.7)
+            first = mid.clone()
+            ops.moe_grouped(mid, w2, out, offsets, order, top=top, first=False)
+        finally:
+            ops.use_moe_split_f32 = True
+        return first, out.clone()
+
+    expert = torch.repeat_interleave(torch.arange(E), torch.tensor(counts)).to(DEV)
+    x = h.double()[order.long() // top]
+    y = torch.stack([w1[e].double() @ r for e, r in zip(expert.tolist(), x)])
+    if act == "relu_sq":
+        want = torch.relu(y) ** 2
+    else:
+        g, u = y[:, :F], y[:, F:]
+        if act == "silu":
+            want = torch.nn.functional.silu(g) * u
+        else:
+            g, u = g.clamp(max=limit), u.clamp(-limit, limit)
+            want = g * torch.sigmoid(1.7 * g) * (u + 1.0)
+    got, plain = run(True), run(False)
+    assert (got[0] - want).abs().max() < 2e-5 * max(1.0, want.abs().max().item())
+    assert (got[0] - want).norm() <= 1.1 * (plain[0] - want).norm()
+    want2 = torch.empty(pairs, D, dtype=torch.float64, device=DEV)
+    want2[order.long()] = torch.stack([w2[e].double() @ r for e, r in zip(expert.tolist(), got[0].double())])
+    assert (got[1] - want2).abs().max() < 2e-5 * max(1.0, want2.abs().max().item())
+    # infinities and NaN where the chains of fmaf have them
+    h[1, 3], w1[E - 1, 0, 5] = float("inf"), float("nan")
+    got, plain = run(True), run(False)
+    for a, b in zip(got, plain):
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+    ops.check_device_errors()
