@@ -13,7 +13,8 @@
 // the slice for all 8 weight rows and 8 tokens at a time, so every weight leaves shared memory once and
 // every value of x leaves L2 once per CTA; the 64 sums of a thread meet first inside the warp (a butterfly
 // that halves the values a lane holds at every step: 62 shuffles), then across the warps in shared memory
-// in warp order, then across the slices in rank order.  17 to 64 rows (`many`): every warp takes whole
+// in warp order, then across the slices in rank order.  17 to 64 rows that are shorter than 768 (`many`;
+// longer ones go to csrc/linear_batch_f32.cu): every warp takes whole
 // tokens (warp w the tokens w, w + 8, ...), its lanes split K, and the weights are read from shared memory
 // once per warp, which 8 tokens per warp amortise.
 // Rows up to 2048 long (`tall`: the Q|K|V and up-projections, and the vocabulary) have a kernel whose CTAs stay on
