@@ -330,27 +330,32 @@ struct SelfRows {
 };
 
 // The expert, first row and row count of tile blockIdx.x, tiles of ROWS pairs counted expert by expert (expert -1: beyond the
-// last; expert E: pairs of identity experts, E up to E_total).  The offsets come in at once: walked one by one they cost a
-// round trip to memory each.
+// last; expert E: pairs of identity experts, E up to E_total).  The offsets come in at once, MAX_E experts at a time (an entry
+// point that takes more experts than the routing kernels): walked one by one they cost a round trip to memory each.
 template <int ROWS>
 __device__ __forceinline__ void find_tile(const int* offsets, int E, int E_total, int* s_off, int* s_e, int* s_r0, int* s_cnt) {
-    for (int e = threadIdx.x; e <= E_total; e += blockDim.x) s_off[e] = offsets[e];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int tile = blockIdx.x, found = -1, r0 = 0, c = 0;
-        for (int e = 0; e < E; ++e) {
-            const int lo = s_off[e], n = s_off[e + 1] - lo;
-            const int tiles = (n + ROWS - 1) / ROWS;
-            if (tile < tiles) { found = e; r0 = lo + tile * ROWS; c = min(ROWS, n - tile * ROWS); break; }
-            tile -= tiles;
+    int tile = blockIdx.x, e0 = 0;                           // thread 0 counts the tile down
+    do {
+        const int n = min(MAX_E, E - e0);
+        for (int e = threadIdx.x; e <= n; e += blockDim.x) s_off[e] = offsets[e0 + e];
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int found = -1, r0 = 0, c = 0;
+            for (int e = 0; e < n; ++e) {
+                const int lo = s_off[e], pairs = s_off[e + 1] - lo;
+                const int tiles = (pairs + ROWS - 1) / ROWS;
+                if (tile < tiles) { found = e0 + e; r0 = lo + tile * ROWS; c = min(ROWS, pairs - tile * ROWS); break; }
+                tile -= tiles;
+            }
+            if (found < 0 && e0 + n == E && E_total > E) {
+                const int lo = s_off[n] + tile * ROWS, pairs = offsets[E_total] - lo;
+                if (pairs > 0) { found = E; r0 = lo; c = min(ROWS, pairs); }
+            }
+            *s_e = found; *s_r0 = r0; *s_cnt = c;
         }
-        if (found < 0 && E_total > E) {
-            const int lo = s_off[E] + tile * ROWS, n = s_off[E_total] - lo;
-            if (n > 0) { found = E; r0 = lo; c = min(ROWS, n); }
-        }
-        *s_e = found; *s_r0 = r0; *s_cnt = c;
-    }
-    __syncthreads();
+        __syncthreads();
+        e0 += MAX_E;
+    } while (*s_e < 0 && e0 < E);
 }
 
 template <typename TA, typename TW, typename TO>

@@ -2067,8 +2067,8 @@ def moe_grouped(a, weight, out, offsets, order, *, top: int, first: bool, act: s
         raise KernelError(f"moe_grouped: activation {act!r} (limit {limit})")
     if (first and out.dtype != a.dtype) or (not first and out.dtype != torch.float32):
         raise KernelError("moe_grouped: the first product keeps the dtype, the second gives 32-bit")
-    if (use_moe_split_f32 and a.dtype == torch.float32 and not identity and n_pairs >= MOE_SPLIT_PAIRS and K % 4 == 0 and K >= 128
-            and _rows("a", a) % 4 == 0 and (a.data_ptr() | weight.data_ptr()) % 16 == 0 and (first or a.stride(0) == K)):
+    if (use_moe_split_f32 and a.dtype == torch.float32 and not identity and n_pairs >= MOE_SPLIT_PAIRS and E <= MOE_MAX_EXPERTS
+            and K % 4 == 0 and K >= 128 and _rows("a", a) % 4 == 0 and (a.data_ptr() | weight.data_ptr()) % 16 == 0 and (first or a.stride(0) == K)):
         # many pairs in 32-bit: tensor cores, in exact pieces
         global launches
         rows = _scratch("moe_split_rows", a.device, n_pairs * K) if first else None

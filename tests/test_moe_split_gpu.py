@@ -57,3 +57,35 @@ def test_routed_experts_in_float32(ops, counts, F, D, top, act):  # noqa: F811
     for a, b in zip(got, plain):
         assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
     ops.check_device_errors()
+
+
+# more experts than the routing kernels take, with weights or identity ones: the CUDA-core, mma.sync and few-pairs kernels
+@pytest.mark.parametrize("E,identity", [(1100, 0), (512, 0), (300, 300)])
+@pytest.mark.parametrize("pairs", [20, 300])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_experts_beyond_the_routing_kernels_number(ops, dtype, pairs, E, identity):  # noqa: F811
+    F, D = 24, 136
+    g = torch.Generator().manual_seed(pairs + E)
+    expert = torch.randint(0, E + identity, (pairs,), generator=g)
+    expert[0], expert[1] = 0, E + identity - 1
+    order = torch.argsort(expert, stable=True)
+    offsets = torch.searchsorted(expert[order].contiguous(), torch.arange(E + identity + 1)).to(torch.int32).to(DEV)
+    h = rnd(pairs, D, seed=2, dtype=dtype)
+    w1 = rnd(E, 2 * F, D, seed=3, scale=D ** -0.5, dtype=dtype)
+    w2 = rnd(E, D, F, seed=4, scale=F ** -0.5, dtype=dtype)
+    mid, out = torch.zeros(pairs, F, dtype=dtype, device=DEV), torch.full((pairs, D), 7.0, device=DEV)
+    perm = order.to(torch.int32).to(DEV)
+    ops.moe_grouped(h, w1, mid, offsets, perm, top=1, first=True, identity=identity)
+    ops.moe_grouped(mid, w2, out, offsets, perm, top=1, first=False, identity=identity, self_rows=h if identity else None)
+    eps = 2e-5 if dtype == torch.float32 else 1e-2
+    for i, (p, e) in enumerate(zip(order.tolist(), expert[order].tolist())):
+        x = h[p].double()
+        if e >= E:
+            assert torch.equal(out[p], h[p].float())
+            continue
+        y = w1[e].double() @ x
+        y = torch.nn.functional.silu(y[:F]) * y[F:]
+        assert (mid[i].double() - y).abs().max() <= eps * max(1.0, y.abs().max().item())
+        want = w2[e].double() @ mid[i].double()
+        assert (out[p].double() - want).abs().max() <= 2e-5 * max(1.0, want.abs().max().item())
+    ops.check_device_errors()
