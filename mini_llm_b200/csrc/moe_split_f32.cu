@@ -345,10 +345,11 @@ MLLM_EXPORT int mllm_moe_split_f32(const float* A, long long lda, const float* W
     if ((long long)E * N * 2 > 0x7fffffffLL) return mllm_fail(1, "moe_split_f32: %d experts of %d columns", E, N);
     static int sms = 0;
     if (!sms) {
-        int dev = 0;
+        int dev = 0, n = 0;
         MLLM_CUDA(cudaGetDevice(&dev));
-        MLLM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        MLLM_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
         MLLM_CUDA(cudaFuncSetAttribute(moe_split_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM));
+        sms = n;                    // last: another thread that finds it set launches at once
     }
     if (a_div > 0) {
         MLLM_CUDA(mllm_launch(moe_gather_kernel, dim3(n_pairs), dim3(128), 0, stream, true, A, lda, sorted, xs, K / 4, a_div));
