@@ -72,9 +72,12 @@ def test_single_tokens_beside_portions(ops, dtype, seqs):  # noqa: F811
     assert ops.attention_launches["decode"] > before
 
 
+# several layers: every layer's projection lies at the same addresses, and SMs that run nothing between two layers keep what the
+# last one left in their L1
+@pytest.mark.parametrize("layers", [1, 4])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("seqs", [[(300, 1), (513, 1), (7, 1)], [(200, 200), (90, 30), (64, 1)]])
-def test_recurrence_beside_biased_attention(ops, dtype, seqs):  # noqa: F811
+@pytest.mark.parametrize("seqs", [[(300, 1), (513, 1), (7, 1)], [(200, 200), (90, 30), (64, 1)], [(5, 1)]])
+def test_recurrence_beside_biased_attention(ops, dtype, seqs, layers):  # noqa: F811
     from mini_llm_b200.engine.context import attention_tiles
     H, Hkv, dh, R, ek, ev, page, D = 12, 4, 64, 3, 32, 128, 16, 768
     case = _paged_case(dtype, seqs, H, Hkv, dh, page, num_pages=120, seed=6)
@@ -92,22 +95,22 @@ def test_recurrence_beside_biased_attention(ops, dtype, seqs):  # noqa: F811
     w_out = rnd(D, qs + R * ev, seed=2, scale=D ** -0.5, dtype=dtype)
     f_bias, lower, norm = rnd(rs, seed=3), torch.full((rs,), 0.2, device=DEV), rnd(ev, seed=4) + 1.0
     bias = -0.3 * torch.log1p(torch.arange(600, device=DEV).float()).expand(H, -1).contiguous()
-    state0 = rnd(S, R, ek, ev, seed=7)
-    state, x = state0.clone(), torch.empty(T, D, dtype=dtype, device=DEV)
+    state0 = rnd(layers, S, R, ek, ev, seed=7)
+    state, x, x2 = state0.clone(), torch.empty(T, D, dtype=dtype, device=DEV), torch.empty(T, D, dtype=dtype, device=DEV)
     proj = torch.empty(T, w_in.shape[0], dtype=dtype, device=DEV)
     mid = torch.empty(T, w_out.shape[1], dtype=dtype, device=DEV)
-    y = torch.empty(T, D, device=DEV)
 
     def run():
         state.copy_(state0)
         with ops.stream_scope(ctx.ws):
-            ops.linear(x, w_in, None, out=proj)
-            r = proj[:, qs:]
-            ops.biased_attention(
-                proj[:, :qs], kp, vp, bt, ctx, mid[:, :qs], num_heads=H, num_kv_heads=Hkv, scale=0.125, dist_bias=bias,
-                company=lambda: ops.gated_recurrence(r[:, :rs], r[:, rs:2 * rs], r[:, 2 * rs:], f_bias, lower, norm, 1e-5, state,
-                                                     ctx, mid[:, qs:], heads=R, beside=True))
-            ops.linear(mid, w_out, None, out=y)
+            for i in range(layers):
+                ops.linear(x2 if i else x, w_in, None, out=proj)
+                r = proj[:, qs:]
+                ops.biased_attention(
+                    proj[:, :qs], kp, vp, bt, ctx, mid[:, :qs], num_heads=H, num_kv_heads=Hkv, scale=0.125, dist_bias=bias,
+                    company=lambda: ops.gated_recurrence(r[:, :rs], r[:, rs:2 * rs], r[:, 2 * rs:], f_bias, lower, norm, 1e-5,
+                                                         state[i], ctx, mid[:, qs:], heads=R, beside=True))
+                ops.linear(mid, w_out, None, out=x2)
 
     x.copy_(rnd(T, D, seed=3, dtype=dtype))
-    _replayed(ops, run, [mid, y, state], lambda i: x.copy_(rnd(T, D, seed=10 + i, dtype=dtype)))
+    _replayed(ops, run, [mid, x2, state], lambda i: x.copy_(rnd(T, D, seed=10 + i, dtype=dtype)))
