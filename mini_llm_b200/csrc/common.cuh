@@ -36,6 +36,10 @@ int mllm_fail(int code, const char* fmt, ...);
 // completed and its writes are visible; until then only data that no kernel of the step
 // writes (weights) may be touched.  pdl_launch() lets the kernel after this one start its
 // own prologue.  Without the launch attribute both are no-ops.
+// A kernel may run `beside` the one before it, i.e. leave its wait out, if that one calls pdl_launch() only after its own wait
+// and writes nothing that this one reads or writes: what this one reads was then complete before it could start.  It reads
+// past L1, and one block waits at its end, so that "this kernel has completed" still means that all before it have
+// (attention_decode.cu, gated_recurrence.cu; tests/test_source_rules.py reads the order out of every kernel).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -383,6 +383,7 @@ class _Scope(threading.local):
     handle = None       # set by stream_scope(); None: ask torch on every call
     stream = None
     workspace = None
+    beside = False      # a launch that may run beside the one before it is due: see _with_company
 
 
 _scope = _Scope()
@@ -409,6 +410,16 @@ class stream_scope:
 def _stream() -> int:
     handle = _scope.handle
     return handle if handle is not None else torch.cuda.current_stream().cuda_stream
+
+
+def _with_company(company) -> None:
+    """Calls ``company`` right behind a launch that lets its dependents start only after its own wait: the first launch made
+    there may leave out its wait (``beside``), if it reads nothing that the launch before it writes."""
+    _scope.beside = True
+    try:
+        company()
+    finally:
+        _scope.beside = False
 
 
 def _dt(t: torch.Tensor) -> int:
@@ -1155,10 +1166,10 @@ def biased_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, n
     if impl != "split":
         launch({"simt": 0, "tiled": 1, "mma": 3}[impl])
         if company is not None:
-            company()
+            _with_company(company)
     elif company is not None:
         launch(4)               # the splits
-        company()
+        _with_company(company)
         launch(5)               # their merge
     else:
         global launches
@@ -2110,7 +2121,11 @@ def gated_recurrence(a, z, v, f_bias, lower, norm_weight, eps: float, state, ctx
     ``impl``: "step" (one CTA per request and head with the norm fused: single tokens) or "wide" (the recurrence
     spread over 32-column CTAs, then the norm kernel: prompt portions); None picks by the step's shape.
     ``beside``: the launch before this one is a kernel that waits for what this one reads and lets its dependents start only
-    then; this one runs beside it (csrc/gated_recurrence.cu)."""
+    then; this one runs beside it (csrc/gated_recurrence.cu).  Only as the first launch of an attention's ``company``: behind
+    any other launch it could read what is not there yet, and is refused."""
+    if beside and not _scope.beside:
+        raise KernelError("gated_recurrence: it can run beside an attention only as the first launch of its company")
+    _scope.beside = False
     _cuda("a", a, contiguous=False)
     _cuda("z", z, a.dtype, contiguous=False)
     _cuda("v", v, a.dtype, contiguous=False)

@@ -43,3 +43,52 @@ def test_a_first_call_is_marked_done_after_it_is_done(name):
 
 def test_the_guards_are_found():
     assert sum(len(list(once_guards(_text(n)))) for n in SOURCES) >= 12
+
+
+def kernels(text):
+    """(name, body) of every kernel, and of the device functions that hold a kernel's launch order."""
+    for m in re.finditer(r"__global__[^;{]*?(\w+)\s*\((?:[^(){}]|\([^()]*\))*\)\s*\{", text):
+        yield m.group(1), _block(text, m.end() - 1)
+
+
+# embed_kernel is the first of a step and is launched without the attribute; decode attention lets its dependents start at once and is
+# followed by launches that wait, or by itself
+EARLY = {"embed_kernel", "attn_decode_kernel"}
+
+
+@pytest.mark.parametrize("name", SOURCES)
+def test_dependents_start_only_after_the_wait(name):
+    """What a launch beside this one relies on: its inputs are complete once the kernel before it lets it start."""
+    seen = 0
+    for kernel, body in kernels(_text(name)):
+        if kernel in EARLY:
+            continue
+        at = 0
+        for m in re.finditer(r"pdl_launch\(\)", body):
+            waits = re.findall(r"pdl_wait\(\)", body[at:m.start()])
+            assert waits, f"{kernel} lets its dependents start before its own wait"
+            at, seen = m.end(), seen + 1
+    if re.search(r"pdl_launch\(\)", _text(name)) and not EARLY & {k for k, _ in kernels(_text(name))}:
+        assert seen == len(re.findall(r"pdl_launch\(\)", _text(name)))      # every one of them lies in a kernel that was read
+
+
+def test_kernels_that_leave_their_wait_out_wait_at_their_end():
+    found = 0
+    for name in SOURCES:
+        text = _text(name)
+        if "beside" not in text:
+            continue
+        for kernel, body in kernels(text):
+            if "beside" in body:
+                assert re.search(r"if \((?:r\.)?beside && \(blockIdx\.x[^)]*\) == 0\) pdl_wait\(\);\s*\}\s*$", body), kernel
+                found += 1
+    assert found == 3
+
+
+def test_a_recurrence_runs_beside_nothing_but_an_attention():
+    from mini_llm_b200 import ops
+    with pytest.raises(ops.KernelError, match="company"):
+        ops.gated_recurrence(None, None, None, None, None, None, 1e-5, None, None, None, heads=1, beside=True)
+    again = []
+    ops._with_company(lambda: again.append(ops._scope.beside))
+    assert again == [True] and not ops._scope.beside
