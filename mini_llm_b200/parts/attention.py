@@ -167,8 +167,6 @@ class DistanceBiasAttention(ProjectedMixer):
             steps = torch.div(torch.arange(n, dtype=torch.int64) + 1, self.q_temp_every, rounding_mode="floor").double()
             self.q_scale = (1.0 + self.q_temp_coef * torch.log(steps + 1.0)).float().contiguous().to(rt.device)
 
-    takes_company = True        # core(..., company): another branch's launch may run beside this one's
-
     def core(self, proj, ctx, cache, out, out_scale: float = 1.0, company=None) -> None:
         ops = self.rt.ops
         gv = ctx.groups[cache.group]
@@ -179,6 +177,8 @@ class DistanceBiasAttention(ProjectedMixer):
         ops.biased_attention(q, cache.k_pages, cache.v_pages, gv.block_table, ctx, out, num_heads=self.num_heads,
                              num_kv_heads=self.num_kv_heads, scale=self.scale, dist_bias=self.dist_bias,
                              q_scale=self.q_scale, out_scale=out_scale, window=self.window, company=company)
+
+    core.takes_company = True   # another branch's launch may run beside this one's
 
 
 register_part("mixer", "distance_bias_attention", DistanceBiasAttention)

@@ -133,16 +133,17 @@ class ParallelMixer(Mixer):
         r = c = 0
         args = []
         for b, s in zip(self.branches, self.scales):
-            args.append((b, (proj[:, r:r + b.in_width], ctx, cache, mid[:, c:c + b.core_width], s)))
+            args.append((b, (proj[:, r:r + b.in_width], ctx, cache, mid[:, c:c + b.core_width]), dict(out_scale=s)))
             r += b.in_width
             c += b.core_width
-        pair = len(args) == 2 and getattr(args[0][0], "takes_company", False) and getattr(args[1][0], "goes_beside", False)
+        # marks on the core itself: a part that replaces it takes the ordinary way, whatever it inherits
+        pair = len(args) == 2 and getattr(args[0][0].core, "takes_company", False) and getattr(args[1][0].core, "goes_beside", False)
         if pair:                            # the cores read the projection and nothing of each other
-            (first, a), (second, b) = args
-            first.core(*a, company=lambda: second.core(*b, beside=True))
+            (first, a, sa), (second, b, sb) = args
+            first.core(*a, **sa, company=lambda: second.core(*b, **sb, beside=True))
         else:
-            for part, a in args:
-                part.core(*a)
+            for part, a, sa in args:
+                part.core(*a, **sa)
         ops.linear(mid, self.out_weight, None, out=out_accum, accumulate=accumulate)
 
 

@@ -57,13 +57,13 @@ class GatedLinearRecurrence(ProjectedMixer):
     def cache_need(self):
         return StateNeed((self.num_heads, self.head_dim, self.v_head_dim), "float32")
 
-    goes_beside = True          # core(..., beside=True): it may run beside the launch before it
-
     def core(self, proj, ctx, cache, out, out_scale: float = 1.0, beside: bool = False) -> None:
         K = self.k_size
         self.rt.ops.gated_recurrence(proj[:, :K], proj[:, K:2 * K], proj[:, 2 * K:], self.f_bias, self.lower,
                                      self.norm_weight, self.norm_eps, cache.state, ctx, out, heads=self.num_heads,
                                      out_scale=out_scale, write_state=cache.write, beside=beside)
+
+    core.goes_beside = True     # core(..., beside=True): it may run beside the launch before it
 
 
 register_part("mixer", "gated_linear_recurrence", GatedLinearRecurrence)
