@@ -143,11 +143,11 @@ class CacheManager:
                 g.allocate(dtype, device)
             # layers whose states are alike lie in one tensor, so that admitting a request clears its slot in all of them with
             # one launch (Finuvik: four requests' 16 launches, 15 us of host time each, stood before their prompt step)
-            alike: Dict[StateNeed, List[int]] = {}
+            alike: Dict[Tuple, List[int]] = {}
             for layer, need in self.state_layers.items():
-                alike.setdefault(need, []).append(layer)
-            for need, layers in alike.items():
-                block = torch.zeros((len(layers), max_num_seqs) + tuple(need.shape), dtype=getattr(torch, need.dtype), device=device)
+                alike.setdefault((tuple(need.shape), need.dtype), []).append(layer)
+            for (shape, kind), layers in alike.items():
+                block = torch.zeros((len(layers), max_num_seqs) + shape, dtype=getattr(torch, kind), device=device)
                 self._state_blocks.append(block)
                 for i, layer in enumerate(layers):
                     self.states[layer] = block[i]

@@ -131,3 +131,16 @@ def test_state_slots_are_zeroed_on_admit():
     cm.states[0][s] += 5
     cm.release("a")
     assert cm.admit("b") == s and torch.all(cm.states[0][s] == 0)
+
+
+def test_states_of_a_shape_given_as_a_list():
+    """Alike states lie in one tensor, whatever sequence the shape comes in; a request's slot is cleared in all of them."""
+    cm = CacheManager({0: StateNeed([2, 3]), 1: StateNeed((2, 3)), 2: StateNeed([4], "bfloat16")}, page_size=4, num_pages=2,
+                      max_num_seqs=3)
+    assert [tuple(cm.states[i].shape) for i in range(3)] == [(3, 2, 3), (3, 2, 3), (3, 4)]
+    assert cm.states[0].untyped_storage().data_ptr() == cm.states[1].untyped_storage().data_ptr()
+    for t in cm.states.values():
+        t.fill_(1.0)
+    slot = cm.admit("a")
+    for t in cm.states.values():
+        assert (t[slot] == 0).all() and t.float().sum() == t[0].numel() * 2
