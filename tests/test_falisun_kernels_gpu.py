@@ -55,7 +55,9 @@ class _Ctx:
 
 
 # ------------------------------------------------------------------------------------------------ join
-@pytest.mark.parametrize("R,D,eps", [(5, 48, 1e-5), (3, 1001, 1e-3), (2, 4096, 1e-6), (1, 8, 0.5)])
+# in registers up to 2,048 columns that can be read four at a time (from 1,025 on a thread has a second four), else in loops
+@pytest.mark.parametrize("R,D,eps", [(5, 48, 1e-5), (3, 1001, 1e-3), (2, 4096, 1e-6), (1, 8, 0.5), (3, 1024, 1e-5), (3, 1028, 1e-5),
+                                     (2, 1540, 1e-5), (4, 2048, 1e-6), (2, 2052, 1e-6)])
 def test_norm_scale_add(ops, R, D, eps):
     y, x = rnd(R, D, seed=1, scale=3.0), rnd(R, D, seed=2)
     w, ls = rnd(D, seed=3) + 1.0, rnd(D, seed=4, scale=0.5)
@@ -72,7 +74,8 @@ def test_norm_scale_add(ops, R, D, eps):
 
 
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("R,D,top,eps", [(5, 48, 2, 1e-5), (3, 1001, 1, 1e-3), (2, 4096, 3, 1e-6), (33, 20000, 2, 1e-5)])
+@pytest.mark.parametrize("R,D,top,eps", [(5, 48, 2, 1e-5), (3, 1001, 1, 1e-3), (2, 4096, 3, 1e-6), (33, 20000, 2, 1e-5),
+                                         (3, 1028, 2, 1e-5), (2, 1540, 1, 1e-5), (7, 2048, 4, 1e-6)])
 def test_join_takes_the_weighted_pairs_and_norms_for_the_next_branch(ops, out_dtype, R, D, top, eps):
     """One kernel: the weighted sum over a token's experts (with or without a result to add it to), the norm and scale
     of that sum, the residual sum, and the next branch's norm of the new stream (plain weights or weights around zero)."""
@@ -135,7 +138,9 @@ def test_latent_rows_and_rotated_queries(ops, dtype, H, dn, dr, R, dims, scaling
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("T,H,N,K", [(1, 3, 40, 16), (37, 2, 136, 24), (70, 5, 8, 64), (5, 1, 65, 33)])
+# up to 16 tokens the kernel of few rows, whose first 128 of K are fetched ahead and whose loop takes the rest
+@pytest.mark.parametrize("T,H,N,K", [(1, 3, 40, 16), (37, 2, 136, 24), (70, 5, 8, 64), (5, 1, 65, 33), (3, 2, 64, 128), (2, 3, 70, 129),
+                                     (3, 2, 64, 384), (16, 1, 9, 500)])
 def test_headwise_linear(ops, dtype, T, H, N, K):
     x = rnd(T, H * (K + 4) + 2, seed=1, dtype=dtype)
     W = rnd(H, N, K, seed=2, scale=K ** -0.5, dtype=dtype)

@@ -33,16 +33,13 @@ def _replayed(ops, run, outs, fresh):
     ops.check_device_errors()
 
 
-# (context, new tokens): one run of single tokens, several, many behind a portion whose tiles fill the GPU, runs that share scratch
-@pytest.mark.parametrize("seqs", [[(500, 200), (300, 1), (90, 1)], [(700, 1), (260, 130), (33, 1), (150, 1)],
-                                  [(640, 640)] + [(37 * i + 5, 1) for i in range(20)],
-                                  [(1100, 1), (200, 200), (1200, 1), (70, 1)]])
-@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-def test_single_tokens_beside_portions(ops, dtype, seqs):  # noqa: F811
+def _beside_portions(ops, dtype, seqs, dh, window=None, num_pages=1200):
+    """A projection that writes the cache, the portions' attention with the single tokens' beside it and an output product,
+    replayed; returns which attention kernels were launched."""
     from mini_llm_b200.engine.context import ATTN_TILE_WIDE, attention_tiles, single_runs
     H = Hkv = 12
-    dh, page, D = 64, 16, 768
-    case = _paged_case(dtype, seqs, H, Hkv, dh, page, num_pages=1200, seed=5)
+    page, D = 16, 12 * dh
+    case = _paged_case(dtype, seqs, H, Hkv, dh, page, num_pages=num_pages, seed=5)
     ctx = _ctx_for(case)
     q_lens, starts = [n for _, n in seqs], [c - n for c, n in seqs]
     T = sum(q_lens)
@@ -63,13 +60,36 @@ def test_single_tokens_beside_portions(ops, dtype, seqs):  # noqa: F811
     def run():
         with ops.stream_scope(ctx.ws):
             queries = ops.linear_qkv_cache(x, w_in, None, q, kp, vp, slots, ctx.ws)
-            ops.paged_attention(queries, kp, vp, bt, ctx, att, num_heads=H, num_kv_heads=Hkv, head_dim=dh, scale=dh ** -0.5)
+            ops.paged_attention(queries, kp, vp, bt, ctx, att, num_heads=H, num_kv_heads=Hkv, head_dim=dh, scale=dh ** -0.5,
+                                window=window)
             ops.linear(att, w_out, None, out=y)
 
     x.copy_(rnd(T, D, seed=3, dtype=dtype))
-    before = ops.attention_launches.get("decode", 0)
+    before = dict(ops.attention_launches)
     _replayed(ops, run, [att, y], lambda i: x.copy_(rnd(T, D, seed=10 + i, dtype=dtype)))
-    assert ops.attention_launches["decode"] > before
+    return {k for k, n in ops.attention_launches.items() if n > before.get(k, 0)}
+
+
+# (context, new tokens): one run of single tokens, several, many behind a portion whose tiles fill the GPU, runs that share scratch
+@pytest.mark.parametrize("seqs", [[(500, 200), (300, 1), (90, 1)], [(700, 1), (260, 130), (33, 1), (150, 1)],
+                                  [(640, 640)] + [(37 * i + 5, 1) for i in range(20)],
+                                  [(1100, 1), (200, 200), (1200, 1), (70, 1)]])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_single_tokens_beside_portions(ops, dtype, seqs):  # noqa: F811
+    assert "decode" in _beside_portions(ops, dtype, seqs, 64)
+
+
+# every kernel that portions may take, with heads that decode attention stages and heads that it does not, with and without a window
+@pytest.mark.parametrize("dtype,dh,window,seqs,portions", [
+    (torch.float32, 32, None, [(700, 400), (300, 1), (90, 1)], "tiled_wide"),
+    (torch.float32, 16, 100, [(400, 400), (33, 1), (260, 1)], "tiled_wide"),
+    (torch.float32, 128, None, [(300, 60), (90, 1), (500, 1)], "tiled"),
+    (torch.float32, 64, 130, [(640, 300), (400, 1), (131, 1)], "split_f32"),
+    (torch.bfloat16, 128, 50, [(300, 300), (90, 1), (500, 1)], "flash"),
+    (torch.bfloat16, 16, None, [(200, 60), (300, 1), (33, 1)], "flash"),
+    (torch.bfloat16, 64, 200, [(900, 512), (700, 1), (201, 1)], "flash_tc")])
+def test_single_tokens_beside_every_kernel_of_portions(ops, dtype, dh, window, seqs, portions):  # noqa: F811
+    assert _beside_portions(ops, dtype, seqs, dh, window, num_pages=160) == {portions, "decode"}
 
 
 # several layers: every layer's projection lies at the same addresses, and SMs that run nothing between two layers keep what the
