@@ -8,9 +8,11 @@ pytestmark = pytest.mark.gpu
 
 
 # pairs per expert: full and ragged tiles, an empty expert, one that has them all; columns that end inside a tile, K inside a block
+# of both products, rows of the second's result that are not 16-byte aligned; products that stay on CUDA cores (short or odd K)
 @pytest.mark.parametrize("counts", [[64], [128, 0, 1, 129, 70], [7] * 40, [0, 300]])
-@pytest.mark.parametrize("F,D,top,act", [(512, 768, 2, "silu"), (33, 132, 1, "swiglu_clamp"), (100, 260, 2, "relu_sq")])
-def test_routed_experts_in_float32(ops, counts, F, D, top, act):  # noqa: F811
+@pytest.mark.parametrize("F,D,top,act", [(512, 768, 2, "silu"), (33, 132, 1, "swiglu_clamp"), (100, 260, 2, "relu_sq"), (132, 772, 2, "silu"),
+                                         (260, 302, 1, "relu_sq"), (129 * 4, 300, 2, "swiglu_clamp")])
+def test_routed_experts_in_float32(ops, monkeypatch, counts, F, D, top, act):  # noqa: F811
     E, pairs = len(counts), sum(counts)
     pairs -= pairs % top
     counts = list(counts)
@@ -22,6 +24,9 @@ def test_routed_experts_in_float32(ops, counts, F, D, top, act):  # noqa: F811
     w1, w2 = rnd(E, F * (2 if gated else 1), D, seed=3, scale=D ** -0.5), rnd(E, D, F, seed=4, scale=F ** -0.5)
     mid, out = torch.full((pairs, F), 7.0, device=DEV), torch.full((pairs, D), 7.0, device=DEV)
     limit = 3.0 if act == "swiglu_clamp" else 0.0
+
+    names, call = [], ops._call
+    monkeypatch.setattr(ops, "_call", lambda name, *args: (names.append(name), call(name, *args))[1])
 
     def run(split):
         ops.use_moe_split_f32 = split
@@ -45,7 +50,10 @@ def test_routed_experts_in_float32(ops, counts, F, D, top, act):  # noqa: F811
         else:
             g, u = g.clamp(max=limit), u.clamp(-limit, limit)
             want = g * torch.sigmoid(1.7 * g) * (u + 1.0)
-    got, plain = run(True), run(False)
+    got = run(True)
+    assert names == ["mllm_moe_split_f32" if k % 4 == 0 and k >= 128 else "mllm_moe_grouped" for k in (D, F)]
+    plain = run(False)
+    assert names[2:] == ["mllm_moe_grouped"] * 2
     assert (got[0] - want).abs().max() < 2e-5 * max(1.0, want.abs().max().item())
     assert (got[0] - want).norm() <= 1.1 * (plain[0] - want).norm()
     want2 = torch.empty(pairs, D, dtype=torch.float64, device=DEV)
@@ -56,6 +64,7 @@ def test_routed_experts_in_float32(ops, counts, F, D, top, act):  # noqa: F811
     got, plain = run(True), run(False)
     for a, b in zip(got, plain):
         assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+        assert torch.equal(a.sign()[a.isinf()], b.sign()[b.isinf()])
     ops.check_device_errors()
 
 
