@@ -522,8 +522,10 @@ attn_decode_body(const T* q, long long q_stride, const T* k_pages, const T* v_pa
 // instead, so that this kernel is complete only when the one before it is, which is what the next kernel's wait relies on.
 // A step of GPT-2 medium with a 512-token portion beside 40 single tokens at contexts of 225 to 900: bfloat16 2.44 ms one after the
 // other, 2.02 ms so (25 + 26 us a block), float32 6.13 and 5.18 ms (51 + 46 us a block).
+// (bfloat16 heads of 128 in a cluster: 139 registers as compiled without a bound, three CTAs per SM instead of four: 32 x 16 heads at
+// 1,000 keys 117 instead of 91 us, at 750 to 3,000 279 instead of 233)
 template <typename T, int LPK, int MODE, bool ONE, bool STG, bool TWO = false>
-__global__ void __launch_bounds__(THREADS, STG ? (TWO ? 6 : Staged<T, LPK>::CTAS) : 0)
+__global__ void __launch_bounds__(THREADS, STG ? (TWO ? 6 : Staged<T, LPK>::CTAS) : sizeof(T) == 2 && LPK == 16 && MODE == MODE_CLUSTER ? 4 : 0)
 attn_decode_kernel(const T* q, long long q_stride, const T* k_pages,      // written by kernels of this step: no __restrict__,
                    const T* v_pages,                                        // the compiler must not read them on the non-coherent path
                    const int* __restrict__ block_table, int bt_stride,
