@@ -108,6 +108,10 @@ template <typename T, int LPK> struct Staged {
     static constexpr bool value = LPK * Vec16<T>::N <= 64;                              // heads up to 64, either dtype
     static constexpr int BYTES = 2 * SPLIT * LPK * 16;                                  // a split's keys and values
     static constexpr int CTAS = BYTES <= 32 * 1024 ? 6 : 3;                             // resident CTAs per SM to aim for
+    // Keys and values on barriers of their own pay where a split takes time to bring.  The 8 KB of a bfloat16 head of 16 do not, and
+    // the second barrier's code spills in the 80 registers that six CTAs per SM leave (us a launch, together / apart: 16 x 25 heads at 256 to
+    // 1,023 keys 19.6 / 20.3, 32 x 16 at 1,000 28.7 / 30.0, 64 x 12 at 250 to 1,000 28.9 / 29.7, 32 x 16 at 750 to 3,000 67.3 / 69.6).
+    static constexpr bool APART = LPK * 16 > 32;
 };
 
 // ONE: every CTA takes exactly one split.  STG: keys and values go through shared memory.  TWO: the staging area holds
@@ -134,7 +138,8 @@ attn_decode_body(const T* q, long long q_stride, const T* k_pages, const T* v_pa
     constexpr bool STAGE = STG;
     static_assert(!STG || Staged<T, LPK>::value, "a split's rows do not fit the staging area");
     static_assert(!TWO || (STG && NG * UNR * 2 == SPLIT), "two rounds of staging need groups that take a split in two rounds");
-    constexpr bool APART = !ONE || TWO;                       // several stages: keys and values arrive and are replaced on their own
+    // several stages: keys and values arrive and are replaced on their own (bfloat16 heads of 16: together, see Staged)
+    constexpr bool APART = (!ONE || TWO) && Staged<T, LPK>::APART;
     constexpr int STAGE_KEYS = TWO ? SPLIT / 2 : SPLIT;       // keys that the staging area holds
     __shared__ float sm_m[NG], sm_l[NG], sm_w[NG];
     extern __shared__ __align__(16) uint4 s_stage[];          // STAGE: a split's keys, then its values: [key][16-byte piece]
@@ -261,7 +266,7 @@ attn_decode_body(const T* q, long long q_stride, const T* k_pages, const T* v_pa
     };
     auto next_stage = [&](int which, int lo) {                // its place has been read: the copies may overwrite it
         arrange(which, lo);
-        bring(which == 0, which == 1, lo, max(lo, first), stage_end(lo));
+        bring(which == 0, which == 1 || !APART, lo, max(lo, first), stage_end(lo));
     };
     auto arrived = [&](int which) {
         if (!tc::mbar_wait(&s_bar[which], phase)) {           // gave up: tell the host, let copies in flight land, go on
@@ -424,7 +429,7 @@ attn_decode_body(const T* q, long long q_stride, const T* k_pages, const T* v_pa
         if (!ONE && split < my_hi) {
             if constexpr (STAGE) tc::fence_async_smem();      // the next split's copies overwrite what was written here
             __syncthreads();                                  // the group buffers are free for the next split
-            if constexpr (STAGE && !ONE) next_stage(1, (split + 1) * SPLIT);
+            if constexpr (STAGE && !ONE) next_stage(APART ? 1 : 0, (split + 1) * SPLIT);
         }
     }
     if (single) return;
