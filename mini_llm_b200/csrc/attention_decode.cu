@@ -520,6 +520,10 @@ attn_decode_body(const T* q, long long q_stride, const T* k_pages, const T* v_pa
     }
 }
 
+// 32-bit heads of 128 hold their rows in all the registers there are: a switch at run time costs them 1 to 2 % (8 x 12 heads at 768
+// keys 36.3 against 35.7 us, 32 x 12 at 700 90.9 against 89.9), so for them it is a kernel of its own.
+template <typename T, int LPK> struct FixedOrder { static constexpr bool value = sizeof(T) == 4 && LPK == 32; };
+
 // `beside`: the kernel before this one is the portions' attention of the same step, which reads what this one reads and
 // writes other rows.  It lets its dependents start only after its own wait on the projection has returned (every kernel
 // that mllm_attention_decode_beside may follow does), so the queries, keys and values are there when this kernel starts and
@@ -529,7 +533,7 @@ attn_decode_body(const T* q, long long q_stride, const T* k_pages, const T* v_pa
 // other, 2.02 ms so (25 + 26 us a block), float32 6.13 and 5.18 ms (51 + 46 us a block).
 // (bfloat16 heads of 128 in a cluster: 139 registers as compiled without a bound, three CTAs per SM instead of four: 32 x 16 heads at
 // 1,000 keys 117 instead of 91 us, at 750 to 3,000 279 instead of 233)
-template <typename T, int LPK, int MODE, bool ONE, bool STG, bool TWO = false>
+template <typename T, int LPK, int MODE, bool ONE, bool STG, bool TWO = false, bool BESIDE = false>
 __global__ void __launch_bounds__(THREADS, STG ? (TWO ? 6 : Staged<T, LPK>::CTAS) : sizeof(T) == 2 && LPK == 16 && MODE == MODE_CLUSTER ? 4 : 0)
 attn_decode_kernel(const T* q, long long q_stride, const T* k_pages,      // written by kernels of this step: no __restrict__,
                    const T* v_pages,                                        // the compiler must not read them on the non-coherent path
@@ -538,10 +542,11 @@ attn_decode_kernel(const T* q, long long q_stride, const T* k_pages,      // wri
                    long long out_stride, float* __restrict__ part_o, float* __restrict__ part_ml,
                    unsigned int* __restrict__ counters, int H, int Hkv, int page_size, float scale, int window,
                    int max_splits, int spc_arg, int beside) {
+    const bool along = FixedOrder<T, LPK>::value ? BESIDE : beside != 0;
     attn_decode_body<T, LPK, MODE, ONE, STG, TWO>(q, q_stride, k_pages, v_pages, block_table, bt_stride, token_seq, positions, out,
                                                   out_stride, part_o, part_ml, counters, H, Hkv, page_size, scale, window,
-                                                  max_splits, spc_arg, beside != 0);
-    if (beside && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) pdl_wait();
+                                                  max_splits, spc_arg, along);
+    if (along && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) pdl_wait();
 }
 
 int g_last_staging = 0;   // how the most recent launch staged keys and values: 0 not, 1 a split at a time, 2 half a split
@@ -603,7 +608,8 @@ int launch(const void* q, long long q_stride, const void* k_pages, const void* v
     g_last_staging = two ? 2 : stg ? 1 : 0;
 #define PICK(M, O)                                                                     \
     kern = two ? (K)attn_decode_kernel<T, LPK, M, O, CAN_TWO, CAN_TWO>                 \
-         : stg ? (K)attn_decode_kernel<T, LPK, M, O, CAN_STAGE> : (K)attn_decode_kernel<T, LPK, M, O, false>
+         : stg ? (K)attn_decode_kernel<T, LPK, M, O, CAN_STAGE>                        \
+         : beside ? (K)attn_decode_kernel<T, LPK, M, O, false, false, FixedOrder<T, LPK>::value> : (K)attn_decode_kernel<T, LPK, M, O, false>
     if (mode == MODE_LOCAL) PICK(MODE_LOCAL, false);
     else if (mode == MODE_CLUSTER && one) PICK(MODE_CLUSTER, true);
     else if (mode == MODE_CLUSTER) PICK(MODE_CLUSTER, false);

@@ -80,7 +80,7 @@ def test_kernels_that_leave_their_wait_out_wait_at_their_end():
             continue
         for kernel, body in kernels(text):
             if "beside" in body:
-                assert re.search(r"if \((?:r\.)?beside && \(blockIdx\.x[^)]*\) == 0\) pdl_wait\(\);\s*\}\s*$", body), kernel
+                assert re.search(r"if \((?:r\.beside|along) && \(blockIdx\.x[^)]*\) == 0\) pdl_wait\(\);\s*\}\s*$", body), kernel
                 found += 1
     assert found == 3
 
