@@ -441,15 +441,14 @@ moe_grouped_kernel(const TA* A, long long lda, const TW* __restrict__ W, TO* out
 }
 
 // ------------------------------------------------------------------------------------------------ few pairs (decode steps)
-// grid (pairs, column blocks of 16), 8 warps.  The pair's input row is staged in shared memory as 32-bit; a warp owns 2
-// columns, its lanes split K with 16-byte loads of the weight rows, four steps of K in flight at once, and the sums meet by
-// a butterfly.  Every weight of the pair's expert is read once per pair: with few pairs the cost is the chain of round trips
-// to memory, so the pair's expert is found by all threads at once, a warp takes few columns and a launch many warps.  512 x 768
-// gated and 768 x 512 at 6 pairs in a decode step: 7.2 us (8 columns a warp, the expert found one offset after the
-// other: 10.8 us).
-constexpr int ROW_COLS = 2;
-template <typename TA, typename TW, typename TO>
-__global__ void __launch_bounds__(256)
+// grid (pairs, column blocks of 8 COLS), 8 warps.  The pair's input row is staged in shared memory as 32-bit; a warp owns COLS
+// columns, its lanes split K with 16-byte loads of the weight rows (of 2 columns for four steps of K, of 8 for one: eight loads in
+// flight either way, twice that with a gate), and the sums meet by a butterfly.  Every weight of the pair's expert is read once
+// per pair: with few pairs the cost is the chain of round trips to memory, so the pair's expert is found by all threads at once, a
+// warp takes 2 columns and a launch many warps.  512 x 768 gated and 768 x 512 at 6 pairs in a decode step: 7.2 us (8 columns
+// a warp, the expert found one offset after the other: 10.8 us).  row_cols says when a warp takes 8.
+template <typename TA, typename TW, typename TO, int COLS>
+__global__ void __launch_bounds__(256, sizeof(TW) == 2 ? 4 : COLS == 2 ? 5 : 2)
 moe_rows_kernel(const TA* A, long long lda, const TW* __restrict__ W, TO* out, long long ldo, const int* offsets,
                 const int* sorted, int E, int N, int K, int a_div, int out_by_pair, int gated, float limit, float alpha,
                 int uact, SelfRows<TA> self) {
@@ -460,8 +459,8 @@ moe_rows_kernel(const TA* A, long long lda, const TW* __restrict__ W, TO* out, l
     int e = 0;                                                   // the pair's expert: how many later ones start at or before it
     for (int e0 = 1; e0 < E; e0 += 256) e += __syncthreads_count(e0 + (int)threadIdx.x < E && offsets[e0 + threadIdx.x] <= i);
     if (i >= offsets[E]) {                                       // a pair of an identity expert (uniform over the CTA)
-        const int col = blockIdx.y * 8 * ROW_COLS + threadIdx.x;
-        if (self.rows && threadIdx.x < 8 * ROW_COLS && col < N) {
+        const int col = blockIdx.y * 8 * COLS + threadIdx.x;
+        if (self.rows && threadIdx.x < 8 * COLS && col < N) {
             const int p = sorted[i];
             out[(size_t)(out_by_pair ? p : i) * ldo + col] = from_f32<TO>(to_f32(self.rows[(size_t)(p / self.top) * self.ld + col]));
         }
@@ -472,27 +471,27 @@ moe_rows_kernel(const TA* A, long long lda, const TW* __restrict__ W, TO* out, l
     for (int k = threadIdx.x; k < K; k += 256) xs[k] = to_f32(a[k]);
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n0 = (blockIdx.y * 8 + warp) * ROW_COLS;
+    const int n0 = (blockIdx.y * 8 + warp) * COLS;
     if (n0 >= N) return;
     const size_t wrows = gated ? (size_t)2 * N : (size_t)N;
     const TW* We = W + (size_t)e * wrows * K;
     constexpr int V = 16 / sizeof(TW);                           // weights per 16-byte load
-    float acc[ROW_COLS], acu[ROW_COLS];
+    float acc[COLS], acu[COLS];
 #pragma unroll
-    for (int u = 0; u < ROW_COLS; ++u) acc[u] = acu[u] = 0.f;
+    for (int u = 0; u < COLS; ++u) acc[u] = acu[u] = 0.f;
     const bool vec = K % V == 0 && ((uintptr_t)W % 16 == 0);
     if (vec) {
-#pragma unroll 4
+#pragma unroll (8 / COLS)
         for (int k = lane * V; k < K; k += 32 * V) {
-            uint4 w[ROW_COLS], wu[ROW_COLS];
+            uint4 w[COLS], wu[COLS];
 #pragma unroll
-            for (int u = 0; u < ROW_COLS; ++u) {
+            for (int u = 0; u < COLS; ++u) {
                 const int n = min(n0 + u, N - 1);
                 w[u] = *reinterpret_cast<const uint4*>(We + (size_t)n * K + k);
                 if (gated) wu[u] = *reinterpret_cast<const uint4*>(We + (size_t)(N + n) * K + k);
             }
 #pragma unroll
-            for (int u = 0; u < ROW_COLS; ++u) {
+            for (int u = 0; u < COLS; ++u) {
                 const TW* p = reinterpret_cast<const TW*>(&w[u]);
                 const TW* q = reinterpret_cast<const TW*>(&wu[u]);
 #pragma unroll
@@ -505,7 +504,7 @@ moe_rows_kernel(const TA* A, long long lda, const TW* __restrict__ W, TO* out, l
     } else {
         for (int k = lane; k < K; k += 32) {
 #pragma unroll
-            for (int u = 0; u < ROW_COLS; ++u) {
+            for (int u = 0; u < COLS; ++u) {
                 const int n = min(n0 + u, N - 1);
                 acc[u] = fmaf(xs[k], to_f32(We[(size_t)n * K + k]), acc[u]);
                 if (gated) acu[u] = fmaf(xs[k], to_f32(We[(size_t)(N + n) * K + k]), acu[u]);
@@ -514,7 +513,7 @@ moe_rows_kernel(const TA* A, long long lda, const TW* __restrict__ W, TO* out, l
     }
     const size_t orow = (size_t)(out_by_pair ? pair : i) * ldo;
 #pragma unroll
-    for (int u = 0; u < ROW_COLS; ++u) {
+    for (int u = 0; u < COLS; ++u) {
         float v = warp_sum(acc[u]);
         if (gated) v = gate_mul(v, warp_sum(acu[u]), gated, limit, alpha);
         else v = unary_act(v, uact);
@@ -704,6 +703,30 @@ MLLM_EXPORT int mllm_moe_route(const void* h, long long ld, const void* Wr, cons
     return 0;
 }
 
+// Columns that a warp of moe_rows_kernel takes for 32-bit weights [N, K] (bfloat16: always 2).  With 2 five blocks run on an SM at
+// once, with 8 two, of four times the columns, and a wave of them takes about a third longer: so 8 where that saves enough waves,
+// and more of them where the experts are no fewer than the pairs, so that most weights come from HBM.  Both products of a layer
+// at 8 / 16 / 24 / 32 pairs, us with 2 columns, with 8 and by this rule:
+//     8 experts of   512 x  768   16.1  20.9  27.5  31.0     19.5  20.1  21.0  26.1     16.2  18.2  21.1  26.1
+//     8 experts of 1,024 x  768   20.4  32.1  38.9  45.5     23.4  24.7  34.0  41.7     20.5  24.7  33.9  41.7
+//     8 experts of 2,048 x 2,048  64.5  87.4 123.6 144.8     56.7  81.9 109.6 135.2     58.0  83.3 110.3 134.4
+//    16 experts of   256 x 1,024  15.1  18.9  22.3  24.8     18.5  20.0  24.3  25.1     15.0  16.8  21.4  22.5
+//    64 experts of 1,024 x  768   21.4  37.2  46.0  55.4     25.1  33.4  46.1  57.0     21.5  33.6  46.1  55.4
+int row_cols(int n_pairs, int E, int N, int K) {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        sms = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
+    }
+    const long long room = 220 * 1024 / (K * 4 + 1024);          // blocks whose input row fits an SM's shared memory
+    auto waves = [&](int cols, long long fit) {
+        const long long blocks = (long long)n_pairs * ((N + 8 * cols - 1) / (8 * cols)), at_once = sms * (fit < room ? fit : room);
+        return (blocks + at_once - 1) / at_once;
+    };
+    return (n_pairs > E ? 27 : 30) * waves(8, 2) < 20 * waves(2, 5) ? 8 : 2;
+}
+
 MLLM_EXPORT int mllm_moe_few_tokens() { return MOE_FEW_TOKENS; }
 
 // kind 0: A in `dtype`, gated, out in `dtype` (the experts' first product with its activation `act`: MLLM_ACT_SILU, or
@@ -732,22 +755,24 @@ MLLM_EXPORT int mllm_moe_grouped(const void* A, long long lda, const void* W, vo
     const int gated = kind == 0 ? act : 0;
     const int uact = kind == 2 ? act : 0;
     if (n_pairs <= MOE_FEW_PAIRS && (size_t)K * 4 <= 96 * 1024) {
-        const dim3 fg(n_pairs, (N + 8 * ROW_COLS - 1) / (8 * ROW_COLS));
+        const int cols = dtype == MLLM_F32 ? row_cols(n_pairs, E, N, K) : 2;
+        const dim3 fg(n_pairs, (N + 8 * cols - 1) / (8 * cols));
         if (fg.y > 65535) return mllm_fail(1, "moe_grouped: too many columns");
         const size_t smem = (size_t)K * 4;
-#define MLLM_ROWS(TA, TW, TO, SELF)                                                                                            \
+#define MLLM_ROWS(TA, TW, TO, COLS, SELF)                                                                                        \
         do {                                                                                                             \
             static bool raised = false;                                                                                  \
             if (smem > 48 * 1024 && !raised) {                                                                           \
-                MLLM_CUDA(cudaFuncSetAttribute(moe_rows_kernel<TA, TW, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024)); \
+                MLLM_CUDA(cudaFuncSetAttribute(moe_rows_kernel<TA, TW, TO, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024)); \
                 raised = true;                                                                                           \
             }                                                                                                            \
-            MLLM_CUDA(mllm_launch(moe_rows_kernel<TA, TW, TO>, fg, block, smem, stream, true, (const TA*)A, lda, (const TW*)W, \
+            MLLM_CUDA(mllm_launch(moe_rows_kernel<TA, TW, TO, COLS>, fg, block, smem, stream, true, (const TA*)A, lda, (const TW*)W, \
                                   (TO*)out, ldo, offsets, sorted, E, N, K, a_div, out_by_pair, gated, limit, alpha, uact, SELF)); \
         } while (0)
-        if (dtype == MLLM_F32) MLLM_ROWS(float, float, float, sf);
-        else if (dtype == MLLM_BF16 && kind != 1) MLLM_ROWS(__nv_bfloat16, __nv_bfloat16, __nv_bfloat16, sb);
-        else if (dtype == MLLM_BF16) MLLM_ROWS(__nv_bfloat16, __nv_bfloat16, float, sb);
+        if (dtype == MLLM_F32 && cols == 2) MLLM_ROWS(float, float, float, 2, sf);
+        else if (dtype == MLLM_F32) MLLM_ROWS(float, float, float, 8, sf);
+        else if (dtype == MLLM_BF16 && kind != 1) MLLM_ROWS(__nv_bfloat16, __nv_bfloat16, __nv_bfloat16, 2, sb);
+        else if (dtype == MLLM_BF16) MLLM_ROWS(__nv_bfloat16, __nv_bfloat16, float, 2, sb);
         else return mllm_fail(1, "moe_grouped: unknown dtype code %d", dtype);
 #undef MLLM_ROWS
         return 0;
