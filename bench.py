@@ -673,8 +673,8 @@ def run_compare_designs(sizes, dtype: str, batch: int, steps: int, designs=None)
 
 
 def fp32_peak_flops() -> float:
-    """CUDA-core peak, the yardstick of the float32 path (its prefill products run in exact bfloat16 pieces on the tensor
-    cores and can exceed it): SMs x 128 lanes x 2 flops x the highest SM clock; nominal, nothing measures it on this pool."""
+    """CUDA-core peak, the yardstick of the reference's float32 products: SMs x 128 lanes x 2 flops x the highest SM clock;
+    nominal, not measured."""
     import torch
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     mhz = 1965.0
@@ -683,6 +683,12 @@ def fp32_peak_flops() -> float:
     except Exception:
         pass
     return sms * 128 * 2 * mhz * 1e6
+
+
+def prefill_peak_flops(dtype: str, pk) -> float:
+    """The rate that a prompt step is held against: measured bfloat16 products, and a sixth of that in float32, whose
+    products run as six products of exact bfloat16 pieces."""
+    return pk["bf16_tflops"] * 1e12 / (1 if dtype == "bfloat16" else 6)
 
 
 def bench_prompts(vocab: int, batch: int, n: int = PROMPT_LEN):
@@ -852,9 +858,8 @@ def main() -> int:
 
     def prefill_entry(d, dtype):
         pf = run_prefill(d, dtype)
-        peak_fl = pk["bf16_tflops"] * 1e12 if dtype == "bfloat16" else fp32_peak_flops()
         return {"value": round(pf["tok_s"], 1), "tokens": PREFILL_TOKENS, "ms": round(pf["ms"], 3),
-                "frac": round(pf["flops"] / (pf["ms"] / 1e3) / peak_fl, 4)}
+                "frac": round(pf["flops"] / (pf["ms"] / 1e3) / prefill_peak_flops(dtype, pk), 4)}
 
     points, prefill = {}, None
     with tempfile.TemporaryDirectory(prefix="mini_llm_bench_") as d:

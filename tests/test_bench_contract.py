@@ -1,7 +1,7 @@
 """bench.py's answers that need no GPU: more than one GPU is refused with one line and exit
 code 2, the reference arm answers with one line of its own where it cannot run, and the helpers
 that turn a run into bytes and flops count what they say.  (That the reference arm runs where it
-can is the GPU box's business: tests/test_reference_anchor_gpu.py builds and runs the reference.)"""
+can takes a GPU: tests/test_reference_anchor_gpu.py builds and runs the reference.)"""
 import json
 import os
 import subprocess
@@ -62,3 +62,11 @@ def test_prefill_flops_count_products_and_attention():
     d, inner, T = 8, 32, 4
     want = 2 * T * (3 * d * d + d * d + 2 * d * inner) + 2 * 1 * 10 * d + 4 * d * (1 + 2 + 3 + 4)
     assert bench.prefill_flops(cfg, [T], 1) == want
+
+
+def test_prompt_steps_are_held_against_the_rate_of_the_units_that_run_them():
+    sys.path.insert(0, ROOT)
+    import bench
+    pk = {"bf16_tflops": 1500.0}
+    assert bench.prefill_peak_flops("bfloat16", pk) == 1500e12
+    assert bench.prefill_peak_flops("float32", pk) == 250e12        # six products of pieces for one
