@@ -98,3 +98,30 @@ def test_experts_beyond_the_routing_kernels_number(ops, dtype, pairs, E, identit
         want = w2[e].double() @ mid[i].double()
         assert (out[p].double() - want).abs().max() <= 2e-5 * max(1.0, want.abs().max().item())
     ops.check_device_errors()
+
+
+# two or eight columns a warp, by the waves of either: the same bits as every pair alone
+@pytest.mark.parametrize("pairs,E,F,D", [(24, 8, 512, 768), (32, 8, 500, 1028), (9, 40, 1030, 130), (17, 3, 2048, 516)])
+def test_few_pairs_have_the_bits_of_every_pair_alone(ops, pairs, E, F, D):  # noqa: F811
+    expert = torch.randint(0, E, (pairs,), generator=torch.Generator().manual_seed(pairs)).sort().values
+    h, w1, w2 = rnd(pairs, D, seed=2), rnd(E, 2 * F, D, seed=3, scale=D ** -0.5), rnd(E, D, F, seed=4, scale=F ** -0.5)
+
+    def run(rows):
+        n = rows.stop - rows.start
+        order = torch.arange(n, dtype=torch.int32, device=DEV)
+        offsets = torch.searchsorted(expert[rows].contiguous(), torch.arange(E + 1)).to(torch.int32).to(DEV)
+        mid, out = torch.full((n, F), 7.0, device=DEV), torch.full((n, D), 7.0, device=DEV)
+        ops.moe_grouped(h[rows], w1, mid, offsets, order, top=1, first=True)
+        ops.moe_grouped(mid, w2, out, offsets, order, top=1, first=False)
+        return mid, out
+
+    mid, out = run(slice(0, pairs))
+    for i in range(pairs):
+        y = w1[expert[i]].double() @ h[i].double()
+        y = torch.nn.functional.silu(y[:F]) * y[F:]
+        assert (mid[i] - y).abs().max() < 2e-5 * max(1.0, y.abs().max().item())
+        want = w2[expert[i]].double() @ mid[i].double()
+        assert (out[i] - want).abs().max() < 2e-5 * max(1.0, want.abs().max().item())
+        alone = run(slice(i, i + 1))
+        assert torch.equal(alone[0][0], mid[i]) and torch.equal(alone[1][0], out[i])
+    ops.check_device_errors()
