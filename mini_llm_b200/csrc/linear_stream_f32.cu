@@ -831,15 +831,22 @@ int tall_shape(int N, int K) {
     if (K <= 1024) return 5 * ((N + 31) / 32) >= 3 * sms ? 4 : 2;
     return (N + 15) / 16 >= sms ? 2 : 0;
 }
-// Rows of x up to which it is taken: all that fit shared memory for a matrix as tall as a vocabulary; 48 with 4 weight
-// rows per warp (3072 x 768 at 48 rows: 20.9 against 22.1 us of the kernel for 17 to 64 rows, 3072 x 1024: 24.6
-// against 29.4 us; at 64 rows they are even or it loses), 24 with K over 1024 (4800 x 1600 at 24 rows: 38.5 against
-// 42.9 us, at 32 rows 49.2 against 45.4 us), 16 for narrower matrices (2304 x 768 at 24 rows: 13.0 against 12.4 us).
-int tall_rows_for(int N, int K) {
+// Rows of x up to which it is taken: for a matrix as tall as a vocabulary with a norm all that fit shared memory (16 at most, as
+// many as a norm is fused for), without one all that fit where K is short, else one pass of 8, beyond which the product on
+// tensor cores is ahead (csrc/linear_batch_f32.cu; us here / there at 1, 8, 9, 12 and 16 rows: 50257 x 768 27 / 43, 33 / 43,
+// 43 / 43, 45 / 43, 50 / 43; x 1024 34 / 56, 40 / 56, 52 / 56, 55 / 55, 61 / 55; x 1600 57 / 83, 73 / 83, 107 / 83, 108 / 83, 126 / 83);
+// 48 with 4 weight rows per warp, 24 with K over 1024, 16 for narrower matrices (measured against the kernel for 17 to 64 rows
+// that took the others then: 3072 x 768 at 48 rows 20.9 against 22.1 us, 4800 x 1600 at 24 rows 38.5 against 42.9 us, at 32 rows
+// 49.2 against 45.4 us, 2304 x 768 at 24 rows 13.0 against 12.4 us; the product on tensor cores is ahead of it from about 32 rows on
+// at 3072 x 768, 12.0 against 11 us, and from 17 on at 4800 x 1600, 30 against 16 us).
+int tall_rows_for(int N, int K, bool norm) {
     const int rw = tall_shape(N, K);
     if (!rw) return 0;
     const int fit = tall_rows(K);
-    if ((N + 31) / 32 >= 8 * sm_count()) return fit;
+    if ((N + 31) / 32 >= 8 * sm_count()) {
+        const int most = norm ? FEW_M : K >= BATCH_K ? 8 : fit;
+        return fit < most ? fit : most;
+    }
     const int cap = K > 1024 ? 24 : (rw == 4 ? 48 : FEW_M);
     return fit < cap ? fit : cap;
 }
@@ -894,17 +901,23 @@ MLLM_EXPORT int mllm_linear_stream_f32_many_shape(int N, int K, int* rt, int* sl
     return best < 0 ? 1 : 0;        // 1: no shape fits shared memory (K beyond about 48,000): the caller takes another kernel
 }
 
-// Rows of x up to which a matrix [N, K] goes to the kernel with the weights in registers (0: never).
-MLLM_EXPORT int mllm_linear_stream_f32_tall_rows(int N, int K) { return tall_rows_for(N, K); }
+// Rows of x up to which a matrix [N, K] goes to the kernel with the weights in registers (0: never), without a norm.
+MLLM_EXPORT int mllm_linear_stream_f32_tall_rows(int N, int K) { return tall_rows_for(N, K, false); }
 
-// Which kernel computes M plain rows (no norm, no cache write) against a matrix [N, K]: 0 threads split K (up to 16 rows),
-// 1 the kernel of many rows (17 to 64: on tensor cores from K = 768 on, else warps own tokens), 2 weights in registers (as tall
-// as a vocabulary from K = 768 on: on tensor cores), 3 long rows in cluster slices (up to 40 rows).  Rows computed by the same
-// kernel have the same bits whatever the batch.
+// Whether M rows without a norm go to the product on tensor cores (csrc/linear_batch_f32.cu): rows from BATCH_K on that neither the
+// kernel with the weights in registers nor the one for long rows takes, more than 16 of them or a vocabulary's.
+MLLM_EXPORT int mllm_linear_stream_f32_on_tensor_cores(int M, int N, int K) {
+    if (K < BATCH_K || M <= tall_rows_for(N, K, false) || (M <= REGS_M && regs_slices(N, K, M))) return 0;
+    return M > FEW_M || (tall_shape(N, K) && (N + 31) / 32 >= 8 * sm_count());
+}
+
+// Which kernel computes M plain rows (no norm) against a matrix [N, K]: 0 threads split K (up to 16 rows), 1 the kernel of many
+// rows (on tensor cores where the function above says so, else warps own tokens: for one matrix always the same), 2 weights in
+// registers, 3 long rows in cluster slices (up to 40 rows).  Rows computed by the same kernel have the same bits whatever the batch.
 MLLM_EXPORT int mllm_linear_stream_f32_kernel_of(int M, int N, int K) {
-    if (M <= tall_rows_for(N, K)) return 2;
+    if (M <= tall_rows_for(N, K, false)) return 2;
     if (M <= REGS_M && regs_slices(N, K, M)) return 3;
-    return M <= FEW_M ? 0 : 1;
+    return M > FEW_M || mllm_linear_stream_f32_on_tensor_cores(M, N, K) ? 1 : 0;
 }
 
 // csrc/linear_batch_f32.cu: the same products in exact pieces on tensor cores.
@@ -947,12 +960,9 @@ MLLM_EXPORT int mllm_linear_stream_f32(const void* x, long long ldx, const void*
     LnArgs ln = {(const float*)ln_x, ln_rows, ln_gamma, ln_beta, fabsf(ln_eps), ln_eps < 0.f ? 1 : 0};
     KvArgs kv = {(float*)k_pages, (float*)v_pages, slots, q_size, kv_heads, head_dim, page_size};
     const int tiles = (N + R - 1) / R;
-    const int tall_rw = M <= tall_rows_for(N, K) ? tall_shape(N, K) : 0;
+    const int tall_rw = M <= tall_rows_for(N, K, norm) ? tall_shape(N, K) : 0;
     const int regs_s = !norm && !kvw && M <= REGS_M ? regs_slices(N, K, M) : 0;
-    const bool vocabulary = tall_rw && (N + 31) / 32 >= 8 * sm_count();
-    // A vocabulary's rows have the same bits at every count of them, so without a norm to fuse it takes the tensor cores from one
-    // row on, although up to 8 rows the weights in registers would be ahead (34 against 45 us at 8 rows of 768, 52 against 44 at 16).
-    if (!norm && K >= BATCH_K && (vocabulary ? !kvw : M > FEW_M && !tall_rw && !regs_s))
+    if (!norm && (mllm_linear_stream_f32_on_tensor_cores(M, N, K) || (kvw && M > FEW_M && K >= BATCH_K && !tall_rw)))
         return mllm_linear_batch_f32((const float*)x, ldx, (const float*)W, bias, (float*)out, ldo, M, N, K, act, accumulate, kv.k_pages,
                                      kv.v_pages, slots, q_size, kv_heads, head_dim, page_size, stream);
     if (tall_rw) {

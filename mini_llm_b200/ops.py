@@ -66,6 +66,7 @@ def _signatures(lib):
                                    c_int, c_int, c_int, c_int, c_void_p],
         "mllm_linear_stream_f32_tall_rows": [c_int, c_int],
         "mllm_linear_stream_f32_kernel_of": [c_int, c_int, c_int],
+        "mllm_linear_stream_f32_on_tensor_cores": [c_int, c_int, c_int],
         "mllm_linear_stream_f32_bind_error": [c_void_p],
         "mllm_linear_cluster": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int,
                                 c_int, c_void_p],

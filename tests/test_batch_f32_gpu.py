@@ -7,6 +7,10 @@ from test_kernels_gpu import DEV, ops, rnd  # noqa: F401
 pytestmark = pytest.mark.gpu
 
 
+def _on_tensor_cores(ops, M, N, K):  # noqa: F811
+    return bool(ops.library().mllm_linear_stream_f32_on_tensor_cores(M, N, K))
+
+
 # one tile and one slice, ragged tiles, slices of unequal length, rows of K that end inside a block, CTAs that walk several
 # tiles; both widths of the row side at their edges
 @pytest.mark.parametrize("M", [17, 32, 33, 64])
@@ -38,6 +42,20 @@ def test_float32_product_of_a_batch(ops, M, N, K):  # noqa: F811
     ops.linear(x, w, None, out=plain, impl="simt")
     assert torch.equal(full.isnan(), plain.isnan()) and torch.equal(full.isinf(), plain.isinf())
     assert torch.equal(full.sign().nan_to_num(), plain.sign().nan_to_num()) or N > 1
+    ops.check_device_errors()
+
+
+# a vocabulary's few rows stay with the weights in registers while one pass of eight takes them
+@pytest.mark.parametrize("K", [764, 768, 1600])
+def test_float32_vocabulary_of_few_rows(ops, K):  # noqa: F811
+    N = 38000
+    w, x = rnd(N, K, seed=2, scale=K ** -0.5), rnd(16, K, seed=1)
+    ref, mass = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    for M in (1, 8, 9, 16):
+        assert _on_tensor_cores(ops, M, N, K) == (K >= 768 and M > 8)
+        out = torch.empty(M, N, device=DEV)
+        ops.linear(x[:M], w, None, out=out)
+        assert torch.all((out - ref[:M]).abs() <= (K / 64 + 12) * 2.0 ** -24 * mass[:M])
     ops.check_device_errors()
 
 

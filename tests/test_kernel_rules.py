@@ -15,7 +15,7 @@ def lib():
     from mini_llm_b200.csrc import build
 
     lib = ctypes.CDLL(build.ensure_built())
-    for name in ("mllm_linear_stream_f32_kernel_of",):
+    for name in ("mllm_linear_stream_f32_kernel_of", "mllm_linear_stream_f32_on_tensor_cores"):
         getattr(lib, name).argtypes = [ctypes.c_int] * 3
     lib.mllm_linear_stream_f32_tall_rows.argtypes = [ctypes.c_int] * 2
     try:
@@ -37,15 +37,30 @@ def test_decode_projections_of_gpt2_sizes(lib, D, F):
     for M in (1, 8, 16):
         assert kernel(lib, M, 3 * D, D) == TALL          # Q|K|V
         assert kernel(lib, M, F, D) == TALL              # up-projection
-        assert kernel(lib, M, V, D) == TALL              # the head
+        assert kernel(lib, M, V, D) == (TALL if M <= 8 else MANY)      # the head, without a norm
     # the output projection: narrow and, at XL's width, longer than 1024: the tile kernel's K slices win there
     assert kernel(lib, 8, D, D) == (TALL if D <= 1024 else FEW)
     # the down-projection: cluster slices where their chunks fill the slice, else the tile kernel up to 16 rows
     assert kernel(lib, 8, D, F) == (FEW if D == 1024 else LONG)
     assert kernel(lib, 40, D, F) == LONG
-    # the vocabulary takes every row count that fits shared memory
-    assert lib.mllm_linear_stream_f32_tall_rows(V, D) == {768: 64, 1024: 48, 1600: 32}[D]
-    assert kernel(lib, 64, V, D) == (TALL if D == 768 else MANY)
+    # the vocabulary: one pass of eight rows, then tensor cores; shorter rows stay for every row count that fits shared memory
+    assert lib.mllm_linear_stream_f32_tall_rows(V, D) == 8 and lib.mllm_linear_stream_f32_tall_rows(V, 512) == 64
+    assert kernel(lib, 64, V, D) == MANY and kernel(lib, 64, V, 512) == TALL
+
+
+@pytest.mark.parametrize("D,F", [(768, 3072), (1024, 4096), (1600, 6400)])
+def test_what_runs_on_tensor_cores(lib, D, F):
+    V = 50257
+    for M in range(1, 65):
+        assert lib.mllm_linear_stream_f32_on_tensor_cores(M, V, D) == (M > 8)
+        assert lib.mllm_linear_stream_f32_on_tensor_cores(M, D, F) == (M > 40)
+        assert lib.mllm_linear_stream_f32_on_tensor_cores(M, D, D) == (M > 16)
+        assert lib.mllm_linear_stream_f32_on_tensor_cores(M, F, D) == (M > (24 if D == 1600 else 48))
+        assert lib.mllm_linear_stream_f32_on_tensor_cores(M, 3 * D, D) == (M > {768: 16, 1024: 48, 1600: 24}[D])
+        assert not lib.mllm_linear_stream_f32_on_tensor_cores(M, V, 764) and not lib.mllm_linear_stream_f32_on_tensor_cores(M, D, 764)
+        for N, K in ((V, D), (D, F), (D, D), (F, D)):    # the library's number for it is that of the kernel of many rows
+            if lib.mllm_linear_stream_f32_on_tensor_cores(M, N, K):
+                assert kernel(lib, M, N, K) == MANY
 
 
 def test_row_counts_beyond_the_registers_kernel(lib):
