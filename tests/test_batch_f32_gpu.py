@@ -11,11 +11,14 @@ def _on_tensor_cores(ops, M, N, K):  # noqa: F811
     return bool(ops.library().mllm_linear_stream_f32_on_tensor_cores(M, N, K))
 
 
-# one tile and one slice, ragged tiles, slices of unequal length, rows of K that end inside a block, CTAs that walk several
-# tiles; both widths of the row side at their edges
+# one column, one ragged tile, a column over, slices of unequal length, rows of K that end inside a block, CTAs that walk several
+# tiles; both widths of the row side at their edges.  The last five stay off the tensor cores at all or some row counts: rows
+# under 768, and long rows of few columns up to 40 rows
 @pytest.mark.parametrize("M", [17, 32, 33, 64])
-@pytest.mark.parametrize("N,K", [(1, 128), (127, 132), (129, 520), (300, 1604), (2304, 768), (19001, 260), (50257, 768), (640, 3076)])
+@pytest.mark.parametrize("N,K", [(1, 768), (127, 772), (129, 1604), (300, 1604), (2304, 768), (19001, 2052), (50257, 768), (2500, 3076),
+                                 (1, 128), (127, 132), (129, 520), (19001, 260), (640, 3076)])
 def test_float32_product_of_a_batch(ops, M, N, K):  # noqa: F811
+    assert _on_tensor_cores(ops, M, N, K) == (K >= 768 and (N != 640 or M > 40))
     x, w, b = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5), rnd(N, seed=3)
     ref = x.double() @ w.double().t()
     # four full-size additions of a block drop at most 2^-23 each, blocks, slices and bias add 2^-24 apiece
@@ -24,7 +27,8 @@ def test_float32_product_of_a_batch(ops, M, N, K):  # noqa: F811
     ops.linear(x, w, None, out=full)
     ops.linear(x, w, None, out=plain, impl="simt")
     assert torch.all((full - ref).abs() <= bound)
-    assert (full - ref).norm() <= 1.02 * (plain - ref).norm()
+    # no further off than the chain of fmaf, but for what a single column's few results leave to chance
+    assert (full - ref).norm() <= (1.02 if N > 1 else 2.0) * (plain - ref).norm() + 2.0 ** -24 * ref.norm() * (N == 1)
     big = torch.full((M + 1, N + 3), 7.0, device=DEV)
     big[:M, :N] = 1.5
     ops.linear(x, w, b, out=big[:M, :N], act="gelu_tanh", accumulate=True)
@@ -41,7 +45,7 @@ def test_float32_product_of_a_batch(ops, M, N, K):  # noqa: F811
     ops.linear(x, w, None, out=full)
     ops.linear(x, w, None, out=plain, impl="simt")
     assert torch.equal(full.isnan(), plain.isnan()) and torch.equal(full.isinf(), plain.isinf())
-    assert torch.equal(full.sign().nan_to_num(), plain.sign().nan_to_num()) or N > 1
+    assert plain.isinf().any() and torch.equal(full.sign()[full.isinf()], plain.sign()[plain.isinf()])
     ops.check_device_errors()
 
 
@@ -56,6 +60,19 @@ def test_float32_vocabulary_of_few_rows(ops, K):  # noqa: F811
         out = torch.empty(M, N, device=DEV)
         ops.linear(x[:M], w, None, out=out)
         assert torch.all((out - ref[:M]).abs() <= (K / 64 + 12) * 2.0 ** -24 * mass[:M])
+    ops.check_device_errors()
+
+
+# rows that overlap, and one row for all
+@pytest.mark.parametrize("stride", [0, 4, 760])
+@pytest.mark.parametrize("M", [17, 64])
+def test_float32_product_of_overlapping_rows(ops, M, stride):  # noqa: F811
+    N, K = 300, 772
+    x = rnd(stride * M + K, seed=1).as_strided((M, K), (stride, 1))
+    w, out, want = rnd(N, K, seed=2, scale=K ** -0.5), torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    ops.linear(x, w, None, out=out)
+    ops.linear(x.contiguous(), w, None, out=want)
+    assert torch.equal(out, want)
     ops.check_device_errors()
 
 
