@@ -873,24 +873,23 @@ MLLM_EXPORT int mllm_linear_stream_f32_slices(int N, int K) {
     return S;
 }
 
-constexpr size_t MANY_SMEM_LIMIT = 200 * 1024;
 size_t many_smem_bytes(int RT, int Ks, int S, int MT) {
     return ((size_t)RT * (Ks + MANY_WS_PAD) + (size_t)WARPS * MT * (RT + MANY_RED_PAD) + (S > 1 ? (size_t)(S - 1) * MT * RT : 0)) * 4;
 }
 
-// Tile height (16, 24 or 32 weight rows) and K slices (1, 2, 4 or 8 CTAs of a cluster) of the kernel for 17 to 64 rows,
-// from the matrix alone (never from M): the pair with the least estimated time, waves of CTAs (one CTA per SM) times a
-// CTA's work, its tile's RT x Ks products plus a fixed cost of meeting, reducing and finishing worth about 32 x 256 of
-// them; among equals the taller tile (it reads x less often), then fewer slices.  A slice keeps at least 192 of K.
-MLLM_EXPORT int mllm_linear_stream_f32_many_shape(int N, int K, int* rt, int* slices) {
+// Tile height (16, 24 or 32 weight rows) and K slices (1 or 2 CTAs of a cluster) of the kernel for 17 to 64 rows that are shorter
+// than BATCH_K (so every shape fits shared memory: 166 KB at most), from the matrix alone (never from M): the pair with the
+// least estimated time, waves of CTAs (one CTA per SM) times a CTA's work, its tile's RT x Ks products plus a fixed cost of
+// meeting, reducing and finishing worth about 32 x 256 of them; among equals the taller tile (it reads x less often), then
+// fewer slices.  A slice keeps at least 192 of K.
+void many_shape(int N, int K, int* rt, int* slices) {
     const int sms = sm_count();
     int best_rt = 32, best_s = 1;
     long long best = -1;
     for (int RT = 32; RT >= 16; RT -= 8)
-        for (int S = 1; S <= 8; S *= 2) {
+        for (int S = 1; S <= 2; S *= 2) {
             if (S > 1 && K / S < 192) break;
             const long long ks = ((K + S - 1) / S + 3) / 4 * 4;
-            if (many_smem_bytes(RT, (int)ks, S, MAX_M) > MANY_SMEM_LIMIT) continue;     // (for 64 rows: the choice must not depend on M)
             const long long ctas = (long long)((N + RT - 1) / RT) * S;
             const long long waves = (ctas + sms - 1) / sms;
             const long long cost = waves * ((long long)RT * ks + 8192);
@@ -898,8 +897,8 @@ MLLM_EXPORT int mllm_linear_stream_f32_many_shape(int N, int K, int* rt, int* sl
         }
     *rt = best_rt;
     *slices = best_s;
-    return best < 0 ? 1 : 0;        // 1: no shape fits shared memory (K beyond about 48,000): the caller takes another kernel
 }
+static_assert(BATCH_K <= 768, "tiles of 32 rows and 64 rows of x have to fit shared memory");
 
 // Rows of x up to which a matrix [N, K] goes to the kernel with the weights in registers (0: never), without a norm.
 MLLM_EXPORT int mllm_linear_stream_f32_tall_rows(int N, int K) { return tall_rows_for(N, K, false); }
@@ -997,7 +996,7 @@ MLLM_EXPORT int mllm_linear_stream_f32(const void* x, long long ldx, const void*
         static bool wide_regs = false;
         if (smem > 48 * 1024 && !wide_regs) {
             MLLM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (MAX_M * REGS_KC + MAX_M / 8 * WARPS * 32) * 4));
+                                           (REGS_M * REGS_KC + REGS_M / 8 * WARPS * 32) * 4));
             wide_regs = true;
         }
         cudaLaunchConfig_t cfg = {};
@@ -1070,8 +1069,7 @@ MLLM_EXPORT int mllm_linear_stream_f32(const void* x, long long ldx, const void*
     }
     // 17 to 64 rows that are short: tile height and K slices from (N, K) alone, so that the CTAs fill the SMs once as fully as possible
     int RT = 32, S = 1;
-    if (mllm_linear_stream_f32_many_shape(N, K, &RT, &S))
-        return mllm_fail(1, "linear_stream_f32: K=%d is too long for shared memory", K);
+    many_shape(N, K, &RT, &S);
     const int Ks = ((K + S - 1) / S + 3) / 4 * 4;
     const int MT = M <= 32 ? 32 : 64;
     const size_t smem = many_smem_bytes(RT, Ks, S, MT);
