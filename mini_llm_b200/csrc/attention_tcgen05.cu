@@ -1,5 +1,5 @@
 // Causal attention of prompt portions over the paged cache on the fifth-generation tensor
-// cores: tiles of 128 queries against blocks of 128 keys, head size 64, bfloat16.
+// cores: tiles of 128 queries against blocks of 64 keys in four streams, head size 64, bfloat16.
 //
 // A CTA takes one tile of up to 128 consecutive new tokens of one request and one head.  Its keys, in blocks of 64, are dealt
 // to four streams that know nothing of each other until the end: block b (positions [64 b, 64 b + 64)) belongs to stream b % 4.
@@ -13,7 +13,10 @@
 //      m' = max(m, s), p = exp(s - m'), O = O*exp(m - m') + p.v, l = l*exp(m - m') + sum p
 //    (the reference's recurrence, src/kernels/prefill/flashattention.cu:129-168, with base-2 exponentials and the scale
 //    folded in).  The sums stay in tensor memory; m and O move only where a score exceeds m by more than 2^8 (until then p
-//    grows beyond 1, in 32-bit and in both terms alike), which after the first blocks is rare.
+//    grows beyond 1, in 32-bit and in both terms alike), which after the first blocks is rare.  What that costs in precision lies far
+//    below the rounding of the results (relative error against 64 bits 1.60 to 1.66e-3 with it and with the rounding alone, to 6 digits;
+//    results that are not the correctly rounded ones, 1,024 tokens behind 1,000: 2.4e-3 of them with flat scores, 1.4e-3 with sharp
+//    ones; with m always exact 2.2e-3 and 0.8e-3, and 22.9 instead of 20.1 us a launch for 2 x 1,024 tokens back to back).
 // At the end a row's four streams meet: out = sum_g O_g 2^(m_g - m) / sum_g l_g 2^(m_g - m), in the order of g.
 //
 // What bounds it: the softmax, about 11 instructions per score on 4 x 32 lanes, 1,400 cycles per 128 x 128 scores; the MMAs

@@ -1,5 +1,5 @@
-// out = act(LN?(x)[M,K] . W[N,K]^T + bias) (+ out) for up to 64 rows in true 32-bit (fmaf on CUDA cores,
-// no tensor core, no reduced-precision mode): the products of decode steps on the float32 path, where
+// out = act(LN?(x)[M,K] . W[N,K]^T + bias) (+ out) for up to 64 rows in true 32-bit (in this file fmaf on CUDA cores,
+// no tensor core, no reduced-precision mode; which calls its entry point hands to csrc/linear_batch_f32.cu is said there): the products of decode steps on the float32 path, where
 // the time goes into streaming the 32-bit weights from HBM once and into the dependent round trips
 // between the kernels of a step.
 //
@@ -19,8 +19,9 @@
 // once per warp, which 8 tokens per warp amortise.
 // Rows up to 2048 long (`tall`: the Q|K|V and up-projections, and the vocabulary) have a kernel whose CTAs stay on
 // their SMs: x (normalised) in shared memory once per CTA, a warp's 4 or 2 weight rows in registers straight from
-// HBM, no barrier in its loop.  It takes up to 16 rows of x, and for a matrix as tall as a vocabulary all that fit
-// shared memory (64 at K = 768); where it was measured faster than the tile kernels is written beside its rule.
+// HBM, no barrier in its loop.  It takes up to 16 rows of x, for wide matrices up to 48, of a vocabulary without a norm 8 (64
+// where K is under 768); where it was measured faster than the other kernels is written beside its rules.
+// Rows longer than 2048 (`regs`: the down-projections) are cut into K slices, chunks of them in registers, up to 40 rows.
 // A token's sum runs over k in an order that depends on N, K and on the slices only, never on M, so a
 // token's result does not change with the batch (`few`, `many` and `tall` differ in rounding, as kernels do).
 //
@@ -796,14 +797,14 @@ int tall_rows(int K) {
 int sm_count();
 // K slices with which the kernel for long rows takes M rows of x against a matrix [N, K] (0: another kernel does).
 // From the matrix alone, except for the side of 16 rows.  Measured at the down-projections of GPT-2 small, medium
-// and XL against the tile kernels: with the largest of 4 or 2 slices whose CTAs fit the SMs at once it wins at every
-// row count where the chunks of 768 fill the slice to 4/5 at least (768 x 3072 in 4 slices: 5.0 / 5.1 / 7.0 us at
-// 1 / 8 / 16 rows against 5.6 / 5.9 / 9.4 us, 17.9 against 19.0 us at 64; 1600 x 6400 in 2 slices: 16 against 20 us at
-// 8 rows, 72 against 92 us at 64); where they do not (1024 x 4096: slices of 1024 are a chunk and a third) it loses
-// up to 16 rows (7.8 against 7.2 us) and wins beyond (27 against 32 us at 64).
+// and XL against the kernel in which threads split K: with the largest of 4 or 2 slices whose CTAs fit the SMs at once it wins up
+// to 16 rows where the chunks of 768 fill the slice to 4/5 at least (768 x 3072 in 4 slices: 5.0 / 5.1 / 7.0 us at
+// 1 / 8 / 16 rows against 5.6 / 5.9 / 9.4 us; 1600 x 6400 in 2 slices: 16 against 20 us at 8 rows); where they do not (1024 x 4096:
+// slices of 1024 are a chunk and a third) it loses there (7.8 against 7.2 us) and is taken beyond 16 rows only.
 constexpr int REGS_KC = 768;
-// Rows up to which it is taken; beyond, the product on tensor cores is ahead (csrc/linear_batch_f32.cu has the figures: 768 x 3072
-// 13.2 against 13.1 us at 40 rows, 15.0 against 13.1 at 48).
+// Rows up to which it is taken; beyond, the product on tensor cores is (csrc/linear_batch_f32.cu).  The line is where the two meet at
+// 768 x 3072; longer rows would meet earlier (us here / on tensor cores at 24, 40 and 48 rows: 768 x 3072 9.8 / 11.4, 13.2 / 13.1,
+// 15.3 / 13.2; 1024 x 4096 14.1 / 13.7, 19.5 / 15.6, 22.4 / 15.9; 1600 x 6400 33 / 19, 49 / 22, 57 / 22).
 constexpr int REGS_M = 40;
 // Rows of W from which on products of more than 16 rows go there: with shorter ones it is level or behind (768 x 512: 6.4 against
 // 7.0 us at 32 rows, 8.4 against 8.3 at 64; 256 x 128 3.8 and 5.0 against 7.0 and 9.5).
@@ -820,11 +821,11 @@ int regs_slices(int N, int K, int M) {
 }
 
 // Whether the kernel above takes a matrix, and with how many weight rows per warp (0: not this kernel), from the
-// matrix alone.  Measured against the tile kernels at the layer shapes of GPT-2 small, medium and XL and 1, 8 and 16
+// matrix alone.  Measured against the kernel in which threads split K at the layer shapes of GPT-2 small, medium and XL and 1, 8 and 16
 // rows of x: up to K = 1024 it wins everywhere (3.4-6 us against 3.9-8.5 us), with 4 rows per warp once those
 // tiles of 32 rows fill more than half of the SMs, else with 2; from K = 1025 to 2048 it wins when its tiles of 16
 // rows fill the SMs at least once (N >= 2368 on 148 SMs: 14 against 25 us at 4800 x 1600), and loses for narrower
-// matrices (6.8 against 5.3 us at 1600 x 1600), where the tile kernel's K slices keep more SMs busy.
+// matrices (6.8 against 5.3 us at 1600 x 1600), where that kernel's K slices keep more SMs busy.
 int tall_shape(int N, int K) {
     if (K > 2048) return 0;
     const int sms = sm_count();

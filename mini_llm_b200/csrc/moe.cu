@@ -1,6 +1,7 @@
 // A routed feed-forward (mixture of experts) in which the host reads nothing back:
 //
-//   moe_route       a warp per token: router logits in 32-bit, softmax over all experts, the best `keep` of `n_groups`
+//   moe_route       a warp per token (with up to 16 tokens a warp per four experts' logits of a token, then a warp per token):
+//                   router logits in 32-bit, softmax over all experts, the best `keep` of `n_groups`
 //                   equal groups of neighbouring experts (a group's score is its largest), the `top` best experts inside
 //                   those groups (the lowest index wins among equals), weights = scores / (their sum + 1e-20).
 //                   With `bias` a number per expert is added to the logits first.  `mode` 1: no softmax over all
@@ -15,8 +16,9 @@
 //                   device, so the grid depends on the number of pairs only.  `gated`: W_e is [2F, K] (gate rows, then
 //                   up rows) and the result is act(gate) * up (silu, or the clamped form of gate_mul); an expert without a
 //                   gate has W_e [F, K] and an activation of one argument on the product (`uact`: the square of relu).  Three kernels: CUDA cores, 32 pairs x 64 columns per
-//                   CTA (32-bit weights, odd sizes); tensor cores, 64 x 64 (bfloat16); and for up to 32 pairs (decode
-//                   steps) a CTA per pair and 64 columns whose warps stream the weight rows.
+//                   CTA (32-bit weights, odd sizes; 32-bit products of more pairs go to moe_split_f32.cu where they can); tensor
+//                   cores, 64 x 64 (bfloat16); and for up to 32 pairs (decode steps) a CTA per pair and 16 columns, 64 where
+//                   that saves waves of 32-bit, whose warps stream the weight rows.
 //                   Identity experts (numbers E .. E_total - 1, no weights): their pairs stand last in the order; the first
 //                   product leaves them out and the second copies the token's input row to the pair's result.
 //   moe_combine     y[t] (+)= sum_k weight[t][k] * pair_out[t * top + k], in the order of k.
@@ -703,7 +705,8 @@ MLLM_EXPORT int mllm_moe_route(const void* h, long long ld, const void* Wr, cons
     return 0;
 }
 
-// Columns that a warp of moe_rows_kernel takes for 32-bit weights [N, K] (bfloat16: always 2).  With 2 five blocks run on an SM at
+// Columns that a warp of moe_rows_kernel takes for 32-bit weights [N, K] (bfloat16: always 2, whose eight columns leave room for one
+// block per SM: 8 experts of 512 x 768 at 8 / 16 / 24 / 32 pairs 12.4 / 17.5 / 22.7 / 26.0 us against 16.3 / 21.1 / 28.7 / 32.6).  With 2 five blocks run on an SM at
 // once, with 8 two, of four times the columns, and a wave of them takes about a third longer: so 8 where that saves enough waves,
 // and more of them where the experts are no fewer than the pairs, so that most weights come from HBM.  Both products of a layer
 // at 8 / 16 / 24 / 32 pairs, us with 2 columns, with 8 and by this rule:

@@ -206,11 +206,14 @@ def singles_pay(q_lens: Sequence[int], q_starts: Sequence[int], heads: int, floa
     128 keys, 3 of 64) and one per block it walks; a launch takes its longest tile, or all tiles of all heads over the places
     on the GPU (a tile of 128 rows per SM, two of 64).  A block of 128 keys takes 4 us in 32-bit, 1.3 in bfloat16, like one of 64
     there; a launch of its own costs about 4 us.
-    Measured: GPT-2 small, medium and XL, portions of 64 to 1,024 tokens beside 1 to 32 single ones in 1 to 4 runs at contexts of
-    150 to 900, 292 steps.  Always apart is 2.3 % slower than the better of the two in bfloat16 and 1.2 % in 32-bit, never apart
-    5.7 and 9.3 %, this rule 0.1 % (3.6 % at most).  Examples (us a step, together / apart): small, bfloat16, 512 tokens beside one
-    at 200 653 / 699, at 900 748 / 698, beside 32 at 500 904 / 860; 4 x 256 beside 4 runs at 500 735 / 857; 700 beside 6 at 400 790 /
-    768 (the wide tiles); 32-bit, 512 beside 8 at 500 1,692 / 1,823, beside 16 at 900 2,540 / 2,039."""
+    Fitted while those launches came after the portions' attention: GPT-2 small, medium and XL, portions of 64 to 1,024 tokens
+    beside 1 to 32 single ones in 1 to 4 runs at contexts of 150 to 900, 292 steps, 0.1 % slower than the better of the two (3.6 % at
+    most).  They run beside it now, so a run costs less than the rule charges, and the rule has not been fitted again: of 26 steps
+    measured so, it picks the slower way in two.  Us a call of the runner, together / apart, * where the rule picks the slower:
+      small, bfloat16  512 tokens beside one at 200 707 / 720, at 900 756 / 725, beside 8 at 500 907 / 822 *, beside 32 at 500 1,344 /
+                       1,220; 4 x 256 beside 4 runs at 500 859 / 874; 700 beside 6 at 400 965 / 835; 128 beside 4 at 700 781 / 672
+      small, 32-bit    512 beside 8 at 500 1,857 / 1,900, beside 16 at 900 2,795 / 2,109; 4 x 256 beside 4 runs 2,633 / 2,558 *
+      medium           512 behind 450 beside 40 at 225 to 888, bfloat16 3,190 / 2,777, 32-bit 8,296 / 5,855"""
     ones = [start + 1 for n, start in zip(q_lens, q_starts) if n == 1]
     portions = [(n, start) for n, start in zip(q_lens, q_starts) if n > 1]
     tokens = sum(n for n, _ in portions)

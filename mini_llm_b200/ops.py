@@ -2227,10 +2227,10 @@ def paged_attention(q, k_pages, v_pages, block_table, ctx, out, *, num_heads, nu
         impl = "simt"
         if decode_ok and (k_pages.data_ptr() | v_pages.data_ptr()) % 16 == 0 and getattr(ctx, "single_runs", ()):
             # Single tokens beside prompt portions, where the step's layout names them (engine/context.py has the rule): the
-            # decode kernel takes them, run by run, after the portions' launch, whose tiles are the head of the lists.  GPT-2
-            # medium, 512 prompt tokens beside 40 single ones at contexts of 225 to 900, per block: bfloat16 62 us in one
-            # launch, 25 us (tcgen05 kernel, whose rule on full tiles the portion now meets) + 27 us in two; float32 835 us in
-            # one launch of the CUDA-core kernel, 51 + 48 us in two.
+            # decode kernel takes them, run by run, behind the portions' launch, whose tiles are the head of the lists, and beside
+            # it where it can.  GPT-2 medium, 512 prompt tokens beside 40 single ones at contexts of 225 to 900, a step: bfloat16 3.19 ms
+            # with all in one launch per block (the mma.sync kernel: the tiles are not full enough for the tcgen05 one), 2.78 ms
+            # with them apart, float32 8.30 and 5.86 ms.
             singles = sum(n for _, n in ctx.single_runs)
             n_tiles, n_wide, tokens = n_tiles - singles, n_wide - singles, T - singles
         if getattr(ctx, "decode_only", False) and decode_ok:
