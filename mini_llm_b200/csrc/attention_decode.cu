@@ -572,8 +572,8 @@ int launch(const void* q, long long q_stride, const void* k_pages, const void* v
     //   bfloat16  64 x 12 heads at 250 keys 10.8 / 15.1; 16 x 25 at 300 to 1,023 20.4 / 26.2; 8 x 25 at 900 14.3 / 16.1; 32 x 12 at
     //             700 17.5 / 20.0; 48 x 12 at 160 to 600 19.5 / 22.4; 32 x 16 at 1,000 34.0 / 37.7; as before from 600 pairs on
     //   float32   64 x 12 at 250 17.9 / 21.8; 16 x 25 32.9 / 38.2; 32 x 12 28.1 / 30.5; 32 x 16 55.9 / 62.0; 4 or 8 x 12 unchanged
-    //   heads of 16 and 32, of which more would fit an SM (with the staging of the time / now): bfloat16 64 x 12 at 250 14.8 / 11.9 and
-    //             15.4 / 10.8, 32 x 16 at 1,000 34.5 / 28.7 and 31.1 / 25.0; float32 14.9 / 10.3 and 18.4 / 13.1, 30.2 / 24.1 and 36.6 / 27.8
+    //   heads of 16 and 32, of which more would fit an SM: bfloat16 64 x 12 at 250 11.9 / 14.8 and 10.8 / 15.4, 32 x 16 at 1,000 28.7 / 34.5
+    //             and 25.0 / 31.1; float32 10.3 / 14.9 and 13.1 / 18.4, 24.1 / 30.2 and 27.8 / 36.6
     // Which keys are added together, and in which order, is the same either way.
     const long long pairs = (long long)T_tokens * H;
     const bool stg = Staged<T, LPK>::value && ((uintptr_t)k_pages | (uintptr_t)v_pages) % 16 == 0;

@@ -141,6 +141,13 @@ __device__ __forceinline__ float gate_mul(float g, float u, int act, float limit
     if (act == MLLM_ACT_GELU_ERF) return gelu_erf_f(g) * u;
     return g * u;
 }
+// an activation of one argument on a product (an expert without a gate); 0: none
+__device__ __forceinline__ float unary_act(float v, int uact) {
+    if (uact == MLLM_ACT_RELU_SQ) { const float r = fmaxf(v, 0.f); return r * r; }
+    if (uact == MLLM_ACT_RELU) return fmaxf(v, 0.f);
+    if (uact == MLLM_ACT_GELU_TANH) return gelu_tanh_f(v);
+    return v;
+}
 __device__ __forceinline__ float apply_act(float v, int act) {
     if (act == MLLM_ACT_GELU_TANH) return gelu_tanh_f(v);
     if (act == MLLM_ACT_GELU_ERF) return gelu_erf_f(v);

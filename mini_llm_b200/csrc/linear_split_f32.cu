@@ -56,19 +56,6 @@ struct KvOut32 {
     int q_size, kv_heads, head_dim, page_size;
 };
 
-// The plain sum of an element whose tensor-core sum is not finite.
-__device__ __noinline__ float plain_dot(const float* a, const float* w, int K) {
-    float s = 0.f;
-    for (int k = 0; k < K && s == s; k += 4) {
-        const float4 x = *reinterpret_cast<const float4*>(a + k), y = *reinterpret_cast<const float4*>(w + k);
-        s = fmaf(x.x, y.x, s);
-        s = fmaf(x.y, y.y, s);
-        s = fmaf(x.z, y.z, s);
-        s = fmaf(x.w, y.w, s);
-    }
-    return s;
-}
-
 template <int BN>
 __global__ void __launch_bounds__(THREADS, 1)
 linear_split_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,

@@ -315,14 +315,6 @@ moe_route_sort_kernel(const T* h, long long ld, int Tn, int* idx, float* wout, i
     sort_pairs(chosen, Tn * top, E, offsets, sorted, cnt);
 }
 
-// an activation of one argument on a product (an expert without a gate); 0: none
-__device__ __forceinline__ float unary_act(float v, int uact) {
-    if (uact == MLLM_ACT_RELU_SQ) { const float r = fmaxf(v, 0.f); return r * r; }
-    if (uact == MLLM_ACT_RELU) return fmaxf(v, 0.f);
-    if (uact == MLLM_ACT_GELU_TANH) return gelu_tanh_f(v);
-    return v;
-}
-
 // the input rows that identity experts give back (second product only): rows null means none
 template <typename TA>
 struct SelfRows {

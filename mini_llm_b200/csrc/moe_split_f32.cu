@@ -30,24 +30,6 @@ constexpr size_t SMEM = 1024 /*alignment*/ + 2 * W_STAGE + SLOTS * SLOT + (MAX_E
 
 __device__ int g_moe_error = 0;
 
-__device__ __noinline__ float plain_dot(const float* a, const float* w, int K) {
-    float s = 0.f;
-    for (int k = 0; k < K && s == s; k += 4) {
-        const float4 x = *reinterpret_cast<const float4*>(a + k), y = *reinterpret_cast<const float4*>(w + k);
-        s = fmaf(x.x, y.x, s);
-        s = fmaf(x.y, y.y, s);
-        s = fmaf(x.z, y.z, s);
-        s = fmaf(x.w, y.w, s);
-    }
-    return s;
-}
-__device__ __forceinline__ float unary_act(float v, int uact) {
-    if (uact == MLLM_ACT_RELU_SQ) { const float r = fmaxf(v, 0.f); return r * r; }
-    if (uact == MLLM_ACT_RELU) return fmaxf(v, 0.f);
-    if (uact == MLLM_ACT_GELU_TANH) return gelu_tanh_f(v);
-    return v;
-}
-
 // xs[i] = A[sorted[i] / a_div]: a block per pair, 16 bytes per thread and trip.
 __global__ void __launch_bounds__(128)
 moe_gather_kernel(const float* A, long long lda, const int* sorted, float* xs, int K4, int a_div) {

@@ -1,5 +1,5 @@
 // The exact cut of 32-bit values into three bfloat16 pieces, and what the kernels that multiply in pieces
-// (linear_split_f32.cu, attention_split_f32.cu) share: stores to tensor memory, register shares of warpgroups.
+// (linear_split_f32.cu, linear_batch_f32.cu, moe_split_f32.cu, attention_split_f32.cu) share: stores to tensor memory, register shares of warpgroups.
 #pragma once
 #include "tcgen05.cuh"
 
@@ -44,5 +44,18 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint4& a, const u
                  ::"r"(taddr), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w));
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// The plain sum of an element whose tensor-core sum is not finite; K a multiple of 4, both 16-byte aligned.
+[[maybe_unused]] static __device__ __noinline__ float plain_dot(const float* a, const float* w, int K) {
+    float s = 0.f;
+    for (int k = 0; k < K && s == s; k += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(a + k), y = *reinterpret_cast<const float4*>(w + k);
+        s = fmaf(x.x, y.x, s);
+        s = fmaf(x.y, y.y, s);
+        s = fmaf(x.z, y.z, s);
+        s = fmaf(x.w, y.w, s);
+    }
+    return s;
+}
 
 }  // namespace tc
