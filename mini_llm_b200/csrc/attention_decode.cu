@@ -243,8 +243,9 @@ attn_decode_body(const T* q, long long q_stride, const T* k_pages, const T* v_pa
     // and 58.2; 8 x 12 at 768, float32 9.0 and 10.3).  A CTA with one stage (!APART) waits for both at once: apart they cost a decode
     // step of one request 0.8 us a layer.  `arrange` says how much is coming, `bring` asks for the rows [a, b) of the stage that starts at lo,
     // thread c for those of the c-th page that the range touches.  Rows of earlier steps go out before the wait on the
-    // previous kernel, the token's own row (position p) after it, its page looked up before (1 x 12 heads of 64 at 900 keys, float32:
-    // 5.7 us a launch, 5.95 with the look-up behind the wait and the arrival asked for in every round; 4 x 12 at 500 8.0 and 8.4).  Rows that are not visible are not copied: their places
+    // previous kernel, the token's own row (position p) after it; a CTA with one stage looks its page up before (1 x 12 heads of 64 at
+    // 900 keys, float32: 5.7 us a launch, 5.95 with the look-up behind the wait and the arrival asked for in every round; 4 x 12 at 500
+    // 7.9 and 8.45), one with several stages does not (64 x 32 at 125 to 500, bfloat16: 35.5 us, 36.1 with the look-up before).  Rows that are not visible are not copied: their places
     // hold whatever was there, and the arithmetic below skips them.
     uint4* sk = s_stage;
     uint4* sv = s_stage + STAGE_KEYS * LPK;
@@ -276,16 +277,19 @@ attn_decode_body(const T* q, long long q_stride, const T* k_pages, const T* v_pa
     };
     if constexpr (STAGE) {
         const int lo = my_lo * SPLIT, hi = stage_end(lo), v_lo = max(lo, first);
-        const bool own = threadIdx.x == 0 && p >= v_lo && p < hi;
-        const int own_page = own ? __ldcg(bt + page_index(p)) : 0;
+        const bool own = p >= v_lo && p < hi;
+        int own_page = 0;
+        if constexpr (!APART) own_page = own && threadIdx.x == 0 ? __ldcg(bt + page_index(p)) : 0;
         arrange(0, lo);
         if constexpr (APART) arrange(1, lo);
         bring(true, true, lo, v_lo, min(hi, p));
         wait_and_load_q();
-        if (own) {
+        if constexpr (APART) {
+            if (own) bring(true, true, lo, p, p + 1);
+        } else if (own && threadIdx.x == 0) {
             const size_t off = (((size_t)own_page * Hkv + hk) * page_size + page_offset(p)) * DH;
             tc::bulk_load(sk + (p - lo) * LPK, k_pages + off, ROW, &s_bar[0]);
-            tc::bulk_load(sv + (p - lo) * LPK, v_pages + off, ROW, &s_bar[APART]);
+            tc::bulk_load(sv + (p - lo) * LPK, v_pages + off, ROW, &s_bar[0]);
         }
     }
 
