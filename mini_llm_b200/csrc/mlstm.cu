@@ -39,6 +39,8 @@ __device__ __forceinline__ float log_forget_gate(float z, float cap) {      // l
     const float x = cap * tanhf(z / cap);
     return fminf(x, 0.f) - log1pf(expf(-fabsf(x)));
 }
+// A cp.async of 4 bytes goes through L1, whatever the compiler's flag says: a kernel that uses it lets its lines go (an acquiring
+// fence) after the wait, since an earlier kernel may have left some at the addresses that the last one has written anew.
 __device__ __forceinline__ void cp4(float* dst, const float* src) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
@@ -64,6 +66,7 @@ mlstm_scan_kernel(float* __restrict__ raw, float* __restrict__ aux, int vec, Mls
     float* ns = reinterpret_cast<float*>(gs + 2 * CH);               // [NW][CH]: n . q of the chunk, per warp of rows
     pdl_wait();
     pdl_launch();
+    if (!vec) __threadfence();
     const int seq = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * COLS;
     const int tid = threadIdx.x, nthreads = blockDim.x;
     const int t0 = a.cu_q[seq], n = a.cu_q[seq + 1] - t0;

@@ -36,6 +36,8 @@ struct RotArgs {
     float k_scale;
 };
 
+// A cp.async of 4 bytes goes through L1, whatever the compiler's flag says: a kernel that uses it lets its lines go (an acquiring
+// fence) after the wait, since an earlier kernel may have left some at the addresses that the last one has written anew.
 __device__ __forceinline__ void cp4(float* dst, const float* src) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
@@ -99,6 +101,7 @@ retention_scan_kernel(float* __restrict__ raw, int vec, RetArgs a) {
     const float at = a.decay[h];
     pdl_wait();
     pdl_launch();
+    if (!vec) __threadfence();
     const int t0 = a.cu_q[seq], n = a.cu_q[seq + 1] - t0;
     if (n <= 0) return;
     float* Sg = a.state + (size_t)a.slots[seq] * a.stride + (size_t)h * dk * dv;

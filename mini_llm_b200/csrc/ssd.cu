@@ -20,9 +20,16 @@ constexpr int CHUNK = 16;
 
 __device__ __forceinline__ float silu_f(float v) { return v / (1.0f + expf(-v)); }
 __device__ __forceinline__ float softplus_f(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
+// A cp.async of 4 bytes goes through L1, whatever the compiler's flag says: a kernel that uses it lets its lines go (an acquiring
+// fence) after the wait, since an earlier kernel may have left some at the addresses that the last one has written anew.
 __device__ __forceinline__ void cp4(float* dst, const float* src) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+}
+
+__device__ __forceinline__ void cp16(float* dst, const float* src) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 
 // grid (channel blocks of 256, tokens).  u = proj[:, off : off + C]; state [slots][stride], the conv part at conv_off:
@@ -117,7 +124,7 @@ conv_state_update_kernel(const T* proj, long long ld, int off, float* state, lon
 // Thread (column, rg) owns the ROWS consecutive state rows rg * ROWS ..: it reads its part of B_t and C_t with 16-byte
 // loads (a token's B and C are staged with 4 floats of padding after every ROWS rows, so the eight row groups fall on
 // different banks; rows beyond N are staged as zeros and stay zero in the state).
-template <typename T, int ROWS>
+template <typename T, int ROWS, bool VEC>
 __global__ void __launch_bounds__(256)
 ssd_scan_kernel(const float* xbc, int Cw, int b_off, int c_off, const T* proj, long long ld, int dt_off,
                 const float* __restrict__ dt_bias, const float* __restrict__ A_log, const float* __restrict__ Dh,
@@ -138,6 +145,7 @@ ssd_scan_kernel(const float* xbc, int Cw, int b_off, int c_off, const T* proj, l
     const float a = -expf(A_log[h]), dskip = Dh[h], dtb = dt_bias[h];
     pdl_wait();
     pdl_launch();
+    if (!VEC) __threadfence();
     const bool live = col < P;
     float st[ROWS];
 #pragma unroll
@@ -146,30 +154,35 @@ ssd_scan_kernel(const float* xbc, int Cw, int b_off, int c_off, const T* proj, l
         st[i] = (live && r < N) ? S[(size_t)r * P + col] : 0.f;
     }
     constexpr int BUF = 2 * CHUNK * NP + CHUNK * 32 + 2 * CHUNK;     // floats of one chunk's buffer
-    // a chunk's B, C and x come in by 4-byte cp.async while the chunk before it is walked; its step sizes are read into
-    // a register at the same time and turned into dt and the decay after the walk
+    // a chunk's B, C and x come in by cp.async, 16 bytes at a time where the sizes allow (VEC; 24 heads of 64, us a launch so / 4 bytes
+    // at a time: 3 x 250 tokens, 128 state rows 80 / 83, 256 rows 118 / 134; 1 x 1,000, 64 rows 210 / 219; steps of single tokens
+    // level), while the chunk before it is walked; its step sizes are read into a register at the same time and turned into dt and
+    // the decay after the walk
     float raw_dt = 0.f;
     auto stage = [&](int c0, int buf) {
         const int nc = min(CHUNK, n - c0);
         float* B2 = sm + buf * BUF;
         float* C2 = B2 + CHUNK * NP;
         float* x2 = C2 + CHUNK * NP;
-        for (int i = threadIdx.x; i < nc * 8 * ROWS; i += 256) {
-            const int tt = i / (8 * ROWS), r = i - tt * 8 * ROWS;
+        constexpr int E = VEC ? 4 : 1;                        // floats per copy
+        auto copy = [](float* dst, const float* src) { if constexpr (VEC) cp16(dst, src); else cp4(dst, src); };
+        auto clear = [](float* dst) { if constexpr (VEC) *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f); else *dst = 0.f; };
+        for (int i = threadIdx.x; i < nc * 8 * ROWS / E; i += 256) {
+            const int tt = i / (8 * ROWS / E), r = (i - tt * (8 * ROWS / E)) * E;
             const float* rowp = xbc + (size_t)(t0 + c0 + tt) * Cw;
             const int at = tt * NP + r + (r / ROWS) * PAD;
             if (r < N) {
-                cp4(B2 + at, rowp + b_off + g * N + r);
-                cp4(C2 + at, rowp + c_off + g * N + r);
+                copy(B2 + at, rowp + b_off + g * N + r);
+                copy(C2 + at, rowp + c_off + g * N + r);
             } else {
-                B2[at] = 0.f;
-                C2[at] = 0.f;
+                clear(B2 + at);
+                clear(C2 + at);
             }
         }
-        for (int i = threadIdx.x; i < nc * 32; i += 256) {
-            const int tt = i >> 5, c = i & 31;
-            if (j0 + c < P) cp4(x2 + i, xbc + (size_t)(t0 + c0 + tt) * Cw + (size_t)h * P + j0 + c);
-            else x2[i] = 0.f;
+        for (int i = threadIdx.x; i < nc * (32 / E); i += 256) {
+            const int tt = i / (32 / E), c = i % (32 / E) * E;
+            if (j0 + c < P) copy(x2 + tt * 32 + c, xbc + (size_t)(t0 + c0 + tt) * Cw + (size_t)h * P + j0 + c);
+            else clear(x2 + tt * 32 + c);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
         if (threadIdx.x < nc) raw_dt = to_f32(proj[(size_t)(t0 + c0 + threadIdx.x) * ld + dt_off + h]);
@@ -316,21 +329,27 @@ int scan_launch(int rows, dim3 grid, size_t smem, cudaStream_t stream, const flo
                 const void* proj, long long ld, int dt_off, const float* dt_bias, const float* A_log, const float* Dh,
                 float* state, long long state_stride, const int* cu_q, const int* slots, float* y, int Hm, int N, int P, int G,
                 int write_state) {
-#define MLLM_SCAN(R)                                                                                                     \
+    // rows that can be read 16 bytes at a time
+    const bool vec = ((N | P | Cw | b_off | c_off) & 3) == 0 && (uintptr_t)xbc % 16 == 0;
+#define MLLM_SCAN(R, V)                                                                                                  \
     do {                                                                                                                 \
         static bool raised = false;                                                                                      \
         if (smem > 48 * 1024 && !raised) {                                                                               \
-            MLLM_CUDA(cudaFuncSetAttribute(ssd_scan_kernel<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024)); \
+            MLLM_CUDA(cudaFuncSetAttribute(ssd_scan_kernel<T, R, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024)); \
             raised = true;                                                                                               \
         }                                                                                                                \
-        MLLM_CUDA(mllm_launch(ssd_scan_kernel<T, R>, grid, dim3(256), smem, stream, true, xbc, Cw, b_off, c_off,         \
+        MLLM_CUDA(mllm_launch(ssd_scan_kernel<T, R, V>, grid, dim3(256), smem, stream, true, xbc, Cw, b_off, c_off,      \
                               (const T*)proj, ld, dt_off, dt_bias, A_log, Dh, state, state_stride, cu_q, slots, y, Hm, N, P, \
                               G, write_state));                                                                          \
     } while (0)
-    if (rows <= 4) MLLM_SCAN(4);
-    else if (rows <= 8) MLLM_SCAN(8);
-    else if (rows <= 16) MLLM_SCAN(16);
-    else MLLM_SCAN(32);
+    if (rows <= 4 && vec) MLLM_SCAN(4, true);
+    else if (rows <= 4) MLLM_SCAN(4, false);
+    else if (rows <= 8 && vec) MLLM_SCAN(8, true);
+    else if (rows <= 8) MLLM_SCAN(8, false);
+    else if (rows <= 16 && vec) MLLM_SCAN(16, true);
+    else if (rows <= 16) MLLM_SCAN(16, false);
+    else if (vec) MLLM_SCAN(32, true);
+    else MLLM_SCAN(32, false);
 #undef MLLM_SCAN
     return 0;
 }

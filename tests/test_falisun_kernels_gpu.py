@@ -361,7 +361,9 @@ def _ssd_run(ops, dtype, Hm, Pd, N, G, taps, cuts_per_request, slots, seed):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("Hm,Pd,N,G,taps", [(4, 12, 20, 2, 4), (6, 16, 64, 3, 3), (1, 40, 8, 1, 2), (2, 33, 130, 1, 1), (8, 4, 1, 8, 5)])
+# copies of 16 bytes and of 4, with every number of state rows per thread
+@pytest.mark.parametrize("Hm,Pd,N,G,taps", [(4, 12, 20, 2, 4), (6, 16, 64, 3, 3), (1, 40, 8, 1, 2), (2, 33, 130, 1, 1), (8, 4, 1, 8, 5),
+                                            (3, 64, 128, 1, 4), (2, 36, 256, 1, 2), (2, 20, 66, 1, 4), (3, 33, 36, 3, 3)])
 def test_convolution_and_scan_across_cuts_batches_and_slots(ops, dtype, Hm, Pd, N, G, taps):
     """Three requests of unequal length cut into unequal portions (down to one token, shorter than the convolution's reach),
     batched together, with slots given out of order; against each request run whole by the plain statement."""

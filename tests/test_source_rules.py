@@ -92,3 +92,22 @@ def test_a_recurrence_runs_beside_nothing_but_an_attention():
     again = []
     ops._with_company(lambda: again.append(ops._scope.beside))
     assert again == [True] and not ops._scope.beside
+
+
+@pytest.mark.parametrize("name", SOURCES)
+def test_what_kernels_of_a_step_write_is_not_read_through_l1(name):
+    """The flag that sends plain loads to L2 does not reach cp.async, whose 4- and 8-byte form goes through L1."""
+    assert "cp.async.ca" not in _text(name)
+
+
+@pytest.mark.parametrize("name", SOURCES)
+def test_what_kernels_of_a_step_write_is_not_read_through_l1(name):
+    """The flag that sends plain loads to L2 does not reach cp.async, whose 4-byte form goes through L1: kernels that use it fence
+    behind their wait, before the first copy."""
+    text = _text(name)
+    users = [(k, b) for k, b in kernels(text) if re.search(r"\bcp4\(", b)]
+    assert bool(users) == ("cp.async.ca" in text)
+    assert len(re.findall(r"cp\.async\.ca", text)) <= 1              # the one in cp4
+    for kernel, body in users:
+        m = re.search(r"pdl_wait\(\);\s*pdl_launch\(\);\s*if \(!(?:vec|VEC)\) __threadfence\(\);", body)
+        assert m and m.end() < re.search(r"\bcp4\(", body).start(), kernel
