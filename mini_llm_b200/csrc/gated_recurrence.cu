@@ -64,22 +64,22 @@ gated_recurrence_kernel(const T* a, const T* z, const T* v, T* __restrict__ y, R
     pdl_launch();
     float s[RK];
 #pragma unroll
-    for (int i = 0; i < RK; ++i) s[i] = (col && i0 + i < ek) ? __ldcg(sp + (size_t)(i0 + i) * ev) : 0.f;
+    for (int i = 0; i < RK; ++i) s[i] = (col && i0 + i < ek) ? sp[(size_t)(i0 + i) * ev] : 0.f;
 
     for (int c0 = t0; c0 < t1; c0 += CH) {
         const int n = min(CH, t1 - c0);
         __syncthreads();                    // the chunk before is no longer read
         for (int idx = tid; idx < n * ek; idx += nthreads) {
             const int c = idx / ek, i = idx % ek;
-            const float av = to_f32(__ldcg(a + (size_t)(c0 + c) * r.a_stride + (size_t)h * ek + i));
-            const float zv = to_f32(__ldcg(z + (size_t)(c0 + c) * r.z_stride + (size_t)h * ek + i)) + r.f_bias[h * ek + i];
+            const float av = to_f32(a[(size_t)(c0 + c) * r.a_stride + (size_t)h * ek + i]);
+            const float zv = to_f32(z[(size_t)(c0 + c) * r.z_stride + (size_t)h * ek + i]) + r.f_bias[h * ek + i];
             const float lo = r.lower[h * ek + i];
             qs[c * ek + i] = av / (1.0f + expf(-av));
             fs[c * ek + i] = lo + (1.0f - lo) * (1.0f / (1.0f + expf(-zv)));
         }
         for (int idx = tid; idx < n * ev; idx += nthreads) {
             const int c = idx / ev, d = idx % ev;
-            vs[c * ev + d] = to_f32(__ldcg(v + (size_t)(c0 + c) * r.v_stride + (size_t)h * ev + d));
+            vs[c * ev + d] = to_f32(v[(size_t)(c0 + c) * r.v_stride + (size_t)h * ev + d]);
         }
         __syncthreads();
         if (col) {
@@ -149,14 +149,14 @@ gated_recurrence_wide_kernel(const T* a, const T* z, const T* v, float* __restri
     pdl_launch();
     const int seq = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * WC;
     const int lane = threadIdx.x, g = threadIdx.y, tid = g * 32 + lane, nthreads = G * 32;
-    const int t0 = __ldcg(r.cu_q + seq), t1 = __ldcg(r.cu_q + seq + 1);
-    const int slot = __ldcg(r.slots + seq);
+    const int t0 = r.cu_q[seq], t1 = r.cu_q[seq + 1];
+    const int slot = r.slots[seq];
     const int j = j0 + lane;
     const bool col = j < ev;
     float* sp = r.state + (((size_t)slot * r.Hr + h) * ek) * ev + j;
     float s[WR];
 #pragma unroll
-    for (int i = 0; i < WR; ++i) s[i] = (col && g * WR + i < ek) ? __ldcg(sp + (size_t)(g * WR + i) * ev) : 0.f;
+    for (int i = 0; i < WR; ++i) s[i] = (col && g * WR + i < ek) ? sp[(size_t)(g * WR + i) * ev] : 0.f;
 
     // Every thread owns WLD elements of a chunk's a and z (32 * ekp = 4 * threads of them) and VPT = 32 / G of its v:
     // they are fetched into registers a chunk ahead, while the chunk before is being walked.
@@ -188,13 +188,13 @@ gated_recurrence_wide_kernel(const T* a, const T* z, const T* v, float* __restri
         for (int u = 0; u < WLD; ++u) {
             av[u] = zv[u] = 0.f;
             if (a_tok[u] < n) {
-                av[u] = to_f32(__ldcg(ab + a_off[u]));
-                zv[u] = to_f32(__ldcg(zb + z_off[u]));
+                av[u] = to_f32(ab[a_off[u]]);
+                zv[u] = to_f32(zb[z_off[u]]);
             }
         }
         if (ahead) {
 #pragma unroll
-            for (int u = 0; u < WVMAX; ++u) vv_next[u] = v_tok[u] < n ? to_f32(__ldcg(vb + v_off[u])) : 0.f;
+            for (int u = 0; u < WVMAX; ++u) vv_next[u] = v_tok[u] < n ? to_f32(vb[v_off[u]]) : 0.f;
         }
     };
     // the gate's bias and lower bound of this thread's elements: the same rows in every chunk
@@ -234,7 +234,7 @@ gated_recurrence_wide_kernel(const T* a, const T* z, const T* v, float* __restri
 #pragma unroll
                 for (int u = 0; u < WLD; ++u) {
                     const int idx = base + u * nthreads, c = idx / WC, d = idx % WC;
-                    vv[u] = (idx < n * WC && j0 + d < ev) ? to_f32(__ldcg(v + (size_t)(c0 + c) * r.v_stride + (size_t)h * ev + j0 + d)) : 0.f;
+                    vv[u] = (idx < n * WC && j0 + d < ev) ? to_f32(v[(size_t)(c0 + c) * r.v_stride + (size_t)h * ev + j0 + d]) : 0.f;
                 }
 #pragma unroll
                 for (int u = 0; u < WLD; ++u) {
@@ -343,8 +343,10 @@ MLLM_EXPORT int mllm_gated_recurrence_wide(const void* a, long long a_stride, co
 // beside != 0 (here and above): the launch before this one on the stream is a kernel of the same step that lets its dependents
 // start only after its own wait, and all that this one reads (a, z, v) was written by kernels before that one: this kernel does
 // not wait for it and runs beside it.  One CTA waits at its end, so that this kernel is complete only when the one before is,
-// which is what the next kernel's wait relies on.  What it reads goes past L1 (__ldcg): no wait of its own stands between a
-// line that an earlier layer left in an SM's L1 at the same address and this layer's values.  Behind the biased attention of the other branch of a block (4 requests, 12
+// which is what the next kernel's wait relies on.  What it reads must come from L2, since no wait of its own stands between a line
+// that an earlier layer left in an SM's L1 at the same address and this layer's values: plain loads do, as this library is compiled
+// (csrc/build.py).  Written as __ldcg, which the compiler does not move, they cost bfloat16 prompts 7 % (4 x 500 tokens, 3 heads of
+// 32 x 128: 105 against 98 us a launch).  Behind the biased attention of the other branch of a block (4 requests, 12
 // heads, a context of 510) it lengthens a decode step by 0.6 us a block, after it by 8.8 us.
 MLLM_EXPORT int mllm_gated_recurrence(const void* a, long long a_stride, const void* z, long long z_stride, const void* v,
                                       long long v_stride, const float* f_bias, const float* lower, const float* norm_w,

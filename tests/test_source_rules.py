@@ -111,3 +111,9 @@ def test_what_kernels_of_a_step_write_is_not_read_through_l1(name):
     for kernel, body in users:
         m = re.search(r"pdl_wait\(\);\s*pdl_launch\(\);\s*if \(!(?:vec|VEC)\) __threadfence\(\);", body)
         assert m and m.end() < re.search(r"\bcp4\(", body).start(), kernel
+
+
+def test_plain_loads_go_past_l1():
+    """Kernels that start before the last one has written what they read, or that do not wait for it at all, rely on it."""
+    from mini_llm_b200.csrc import build
+    assert build.NVCC_FLAGS[build.NVCC_FLAGS.index("-dlcm=cg") - 1] == "-Xptxas"
