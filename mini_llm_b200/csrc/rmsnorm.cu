@@ -163,16 +163,17 @@ join_kernel(const float* y, long long y_stride, const float* pairs, const float*
     for (int d = threadIdx.x; d < D; d += blockDim.x) hr[d] = from_f32<TOut>(rowbuf[d] / r2 * (nw[d] + noff));
 }
 
-// The same for rows that can be read 16 bytes at a time, up to 2,048 wide: a thread keeps its 4 or 8 columns in registers, so
-// everything it reads is in flight at once (the weights before the wait), where the loops above meet memory once per trip.
+// The same for rows that can be read 16 bytes at a time, up to 2,048 wide: a thread keeps its columns in registers, 4 (KEEP 1, up to
+// 1,024 wide) or 8, so everything it reads is in flight at once (the weights before the wait), where the loops above meet memory once
+// per trip.  us a launch with the loops / with 8 places for every width / so: 3 rows of 768 5.9 / 3.3 / 2.5, 2,048 rows 12.2 / 14.3 / 9.0,
+// 512 rows of 1,024 5.3 / 6.2 / 3.4, 2,048 rows of 2,048 29.8 / 18.4 / 18.4.
 // A row's cost is then the chain wait - loads - sum - sum.  3 rows of 768 in a decode step, with two pairs each
 // in every second launch: 3.3 us, with the loops 8.0 us.
-template <typename TOut>
+template <typename TOut, int KEEP>
 __global__ void __launch_bounds__(256)
 join_wide_kernel(const float* y, long long y_stride, const float* pairs, const float* pw, int top, const float* __restrict__ w,
                  const float* __restrict__ ls, float* x, long long x_stride, const float* __restrict__ nw, float noff, float neps,
                  TOut* h, long long h_stride, int D, float eps) {
-    constexpr int KEEP = 2;
     __shared__ float scratch[33];
     const size_t r = blockIdx.x;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
@@ -317,12 +318,13 @@ MLLM_EXPORT int mllm_norm_scale_add(const float* y, long long y_stride, const fl
                          (bf_out ? (uintptr_t)h * 2 : (uintptr_t)h);
     if (D % 4 == 0 && D <= 2048 && at % 16 == 0 && (!y || y_stride % 4 == 0) && x_stride % 4 == 0 && (!h || h_stride % 4 == 0)) {
         const dim3 wide(D <= 1024 ? (D / 4 + 31) / 32 * 32 : 256);
-        if (bf_out)
-            MLLM_CUDA(mllm_launch(join_wide_kernel<__nv_bfloat16>, dim3(R), wide, 0, stream, true, y, y_stride, pairs, pw, top, w, ls, x,
-                                  x_stride, nw, noff, neps, (__nv_bfloat16*)h, h_stride, D, eps));
-        else
-            MLLM_CUDA(mllm_launch(join_wide_kernel<float>, dim3(R), wide, 0, stream, true, y, y_stride, pairs, pw, top, w, ls, x,
-                                  x_stride, nw, noff, neps, (float*)h, h_stride, D, eps));
+        auto go = [&](auto kern, auto* to) {
+            return mllm_launch(kern, dim3(R), wide, 0, stream, true, y, y_stride, pairs, pw, top, w, ls, x, x_stride, nw, noff, neps, to,
+                               h_stride, D, eps);
+        };
+        using bf = __nv_bfloat16;
+        if (bf_out) MLLM_CUDA(D <= 1024 ? go(join_wide_kernel<bf, 1>, (bf*)h) : go(join_wide_kernel<bf, 2>, (bf*)h));
+        else MLLM_CUDA(D <= 1024 ? go(join_wide_kernel<float, 1>, (float*)h) : go(join_wide_kernel<float, 2>, (float*)h));
         return 0;
     }
     if (h && h_dtype == MLLM_BF16)
